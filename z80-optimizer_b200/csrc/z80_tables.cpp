@@ -394,6 +394,135 @@ uint32_t seq_relevant(const uint32_t* s, int n, uint32_t out) {
   return out;
 }
 
+namespace {
+// output field g of a state (the layout of op_deps)
+uint32_t flow_field(const Z80S& s, int g) {
+  switch (g) {
+    case 0: return s.a;
+    case 2: return s.b;
+    case 3: return s.c;
+    case 4: return s.d;
+    case 5: return s.e;
+    case 6: return s.h;
+    case 7: return s.l;
+    case 8: return s.sp;
+    case 9: return s.m;
+    default: return (s.f >> (g - kDepF0)) & 1u;
+  }
+}
+void make_flow(int op, OpFlow& f) {
+  static_assert(kFlowFields == kDepFields && kFlowCarry == 1u << kDepF0, "one field layout");
+  z80b_dep::ZB z;
+  // planes named by (field << 4 | plane)
+  auto name8 = [](z80b_dep::ZW (&r)[8], int g) {
+    for (int i = 0; i < 8; i++) {
+      r[i].m = 1u << g;
+      r[i].id = g << 4 | i;
+    }
+  };
+  name8(z.a, 0);
+  name8(z.b, 2);
+  name8(z.c, 3);
+  name8(z.d, 4);
+  name8(z.e, 5);
+  name8(z.h, 6);
+  name8(z.l, 7);
+  name8(z.m, 9);
+  for (int i = 0; i < 16; i++) {
+    z.sp[i].m = kRegSP;
+    z.sp[i].id = 8 << 4 | i;
+  }
+  for (int i = 0; i < 8; i++) {
+    z.f[i].m = 1u << (kDepF0 + i);
+    z.f[i].id = (kDepF0 + i) << 4;
+  }
+  z80b_dep::zb_step(z, uint32_t(op), 0u);
+  f.changed = 0;
+  for (int g = 0; g < kFlowFields; g++) {
+    f.dep[g] = 0;
+    f.src[g] = 0xFF;
+    f.cst[g] = kFlowNoConst;
+  }
+  auto field = [&](int g, const z80b_dep::ZW* r, int n) {
+    bool copy = true;
+    for (int i = 0; i < n; i++) {
+      f.dep[g] |= r[i].m;
+      copy = copy && r[i].id >= 0 && r[i].id == ((r[0].id & ~15) | i);
+    }
+    // a flag bit copies flag bits only, SP itself only
+    if (copy) {
+      const int s = r[0].id >> 4;
+      const bool fits = n == 16 ? s == 8 : (n == 1 ? s >= kDepF0 : s < kDepF0 && s != 8);
+      if (fits) f.src[g] = uint8_t(s);
+    }
+  };
+  field(0, z.a, 8);
+  field(2, z.b, 8);
+  field(3, z.c, 8);
+  field(4, z.d, 8);
+  field(5, z.e, 8);
+  field(6, z.h, 8);
+  field(7, z.l, 8);
+  field(8, z.sp, 16);
+  field(9, z.m, 8);
+  for (int k = 0; k < 8; k++) field(kDepF0 + k, &z.f[k], 1);
+  const int kinds = op_table()[op].imm;
+  static const int kFields[] = {0, 2, 3, 4, 5, 6, 7, 8, 9, 16, 17, 18, 19, 20, 21, 22, 23};
+  // A and the carry, where nothing else matters and no immediate does: all
+  // 512 inputs
+  if (kinds == 0) {
+    uint32_t va[kFlowFields] = {}, vc[kFlowFields] = {};  // seen to depend on A / on the carry
+    std::vector<Z80S> o(512);
+    for (uint32_t x = 0; x < 512; x++) {
+      Z80S s{x & 255u, x >> 8, 0x12, 0x34, 0x56, 0x78, 0x9A, 0xBC, 0xDEF0, 0x5B};
+      z_step(s, uint32_t(op), 0u);
+      o[x] = s;
+    }
+    for (uint32_t x = 0; x < 512; x++)
+      for (int g : kFields) {
+        if (flow_field(o[x], g) != flow_field(o[x & 256u], g)) va[g] = 1;
+        if (flow_field(o[x], g) != flow_field(o[x ^ 256u], g)) vc[g] = 1;
+      }
+    for (int g : kFields) {
+      if (f.src[g] != 0xFF || (f.dep[g] & ~uint32_t(kRegA | kFlowCarry))) continue;
+      if (!va[g]) f.dep[g] &= ~uint32_t(kRegA);
+      if (!vc[g]) f.dep[g] &= ~kFlowCarry;
+    }
+  }
+  // constants: no input matters, so one state shows the value; every
+  // immediate is tried
+  for (int g : kFields) {
+    if (f.src[g] == g) continue;
+    f.changed |= 1u << g;
+    if (f.src[g] != 0xFF || f.dep[g]) continue;
+    const uint32_t n_imm = kinds == 0 ? 1u : (kinds == 1 ? 256u : 65536u);
+    bool same = true, lo = true, hi = true;
+    uint32_t v0 = 0;
+    for (uint32_t imm = 0; imm < n_imm; imm++) {
+      Z80S s{0x12, 0x34, 0x56, 0x78, 0x9A, 0xBC, 0xDE, 0xF0, 0x1234, 0x5B};
+      z_step(s, uint32_t(op), imm);
+      const uint32_t v = flow_field(s, g);
+      if (imm == 0) v0 = v;
+      same = same && v == v0;
+      lo = lo && v == (imm & 255u);
+      hi = hi && v == imm >> 8;
+    }
+    if (same && v0 < 256) f.cst[g] = uint16_t(v0);
+    else if (kinds && lo) f.cst[g] = kFlowImmLo;
+    else if (kinds == 2 && hi) f.cst[g] = kFlowImmHi;
+  }
+}
+}  // namespace
+
+const OpFlow* op_flow() {
+  static OpFlow T[kNumOps];
+  static std::once_flag once;
+  std::call_once(once, [] {
+    for (int op = 0; op < kNumOps; op++) make_flow(op, T[op]);
+  });
+  return T;
+}
+
 uint32_t seq_aflow(const uint32_t* s, int n) {
   const uint8_t* c = op_aclass();
   bool a_is_x = true;

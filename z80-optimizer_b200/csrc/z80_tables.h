@@ -11,6 +11,7 @@
 #include <vector>
 
 #include "z80_isa.h"
+#include "z80_plan.cuh"
 
 namespace z80b {
 
@@ -62,6 +63,11 @@ uint32_t seq_keeps(const uint32_t* s, int n);
 // exactly and that no other compared output depends on: their compared
 // outputs are equal whatever their value, so one value decides.
 uint32_t pair_kept_out(const uint32_t* t, int tn, const uint32_t* c, int cn, uint32_t cmp, uint32_t swept);
+// The flow of every instruction (z80_plan.cuh) for the pair planning: the
+// dependency sets above, sharpened by exhaustive runs where an output
+// depends on A and the carry at most (XOR A and SBC A,A do not depend on A),
+// the outputs that are exact copies of an input field, and the constant ones.
+const OpFlow* op_flow();                  // kNumOps entries
 const char* op_mnemonic(uint16_t op);     // "ADD A, n" style with placeholders
 // The instruction that does op's work with the 8-bit registers renamed:
 // register r (0..5 = B, C, D, E, H, L) plays the part of map[r] (map is a

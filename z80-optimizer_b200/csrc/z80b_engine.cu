@@ -806,8 +806,8 @@ int rounds_on_device(z80b_ctx* ctx, RoundGraph& g, const DevTargets& T, const De
     g.key = key;
     trace("round loop captured (%s pass)", ps ? "length-2" : "length-1");
   }
-  // build, scan (3), [rescan], sweeps, resolve
-  const int per_iter = (ps ? 5 : 4) + 1 + 2 + (R.compact ? 1 : 0) + (R.wide ? 2 : 0);
+  // build, plan, scan (3), [rescan], sweeps, resolve
+  const int per_iter = (ps ? 6 : 5) + 1 + 2 + (R.compact ? 1 : 0) + (R.wide ? 2 : 0);
   CK(cudaMemsetAsync(ctl, 0, sizeof(RoundCtl), s));
   int ke = kbegin(ctx, 1);
   CK(cudaGraphLaunch(g.exec, s));

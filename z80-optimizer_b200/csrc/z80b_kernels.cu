@@ -62,11 +62,8 @@ __device__ uint8_t g_cid[64];
 __device__ uint8_t g_opregs[kNumOps];
 // wide compact sweep: the same per register set of at most four registers
 // (wide_tables)
-// input fields each output field of an opcode depends on (op_deps), and
-// whether it leaves A exactly as it was (op_keeps_a)
-__device__ uint32_t g_dep[kNumOps][kDepFields];
-__device__ uint8_t g_keepa[kNumOps];
-__device__ uint16_t g_keeps[kNumOps];  // fields (read-mask bits) an opcode leaves exactly as they were
+// what each opcode's outputs are computed from (z80_plan.cuh)
+__device__ OpFlow g_flow[kNumOps];
 __device__ int16_t g_wren[kWideSets][kNumOps];
 __device__ int8_t g_worig[kWideSets][4];
 __device__ uint8_t g_wid[64];
@@ -121,39 +118,6 @@ __device__ __forceinline__ uint32_t reg_diff(uint32_t d0, uint32_t d1) {
          ((d1 >> 8) & 0xFFu ? 8u : 0u) | ((d1 >> 16) & 0xFFu ? 16u : 0u) | ((d1 >> 24) ? 32u : 0u);
 }
 
-// Number of A-blocks of the ExhaustiveCheck sweep for a read mask
-// (verifier.go:159-171,428-476); reduced: the reference's sweep of the pair
-// is a reduced one although these reads alone would not make it so (swept
-// registers left out, see put_pair).
-__device__ __forceinline__ unsigned long long sweep_blocks(uint32_t reads, bool reduced = false) {
-  uint32_t ext = reads & (kRegB | kRegC | kRegD | kRegE | kRegH | kRegL | kRegM);
-  int n = __popc(ext);
-  bool sp = (reads & kRegSP) != 0;
-  if (n == 0 && !sp && !reduced) return 2ull;
-  if (n <= 2 && !sp && !reduced) return 2ull << (8 * n);
-  return (2ull << (5 * n)) * (sp ? 16ull : 1ull);
-}
-// Input fields (op_deps layout) that the outputs in `out` of a program can
-// depend on: the dependency sets of its instructions, walked backwards.
-__device__ __forceinline__ uint32_t dev_seq_relevant(const uint32_t* w, uint32_t n, uint32_t out) {
-  for (int i = int(n) - 1; i >= 0; i--) {
-    const uint32_t* d = g_dep[w[i] & 0xFFFFu];
-    uint32_t in = 0;
-    for (uint32_t o = out; o; o &= o - 1) in |= d[__ffs(o) - 1];
-    out = in;
-  }
-  return out;
-}
-__device__ __forceinline__ uint32_t dev_seq_keeps(const uint32_t* w, uint32_t n) {
-  uint32_t k = 0xFFFFu;
-  for (uint32_t i = 0; i < n; i++) k &= g_keeps[w[i] & 0xFFFFu];
-  return k;
-}
-__device__ __forceinline__ bool dev_seq_keeps_a(const uint32_t* w, uint32_t n) {
-  for (uint32_t i = 0; i < n; i++)
-    if (!g_keepa[w[i] & 0xFFFFu]) return false;
-  return true;
-}
 // A-independent sweeps.  When no output of either sequence depends on the
 // input A except A itself passing through (AClass folds of both sequences),
 // every output but A is the same for all 256 values of A, and A_out is
@@ -544,83 +508,77 @@ __device__ __forceinline__ uint32_t alloc_pairs(uint32_t* counter, uint32_t w) {
   return base + incl - w;
 }
 
-// Writes one pair of a round.
-__device__ __forceinline__ void put_pair(const RoundBuf& R, uint32_t p, const DevTargets& T, const DevPool& P,
-                                         const QCOut& q, uint32_t t, uint32_t kind, uint32_t c, uint32_t src,
-                                         uint8_t wlen, uint32_t wend) {
-  PairRec pr;
-  const uint32_t reads = q.meta[t].reads | P.reads[c];
-  pr.target = t;
-  pr.cand = c;
-  pr.keepF = kind ? uint8_t(~target_dead(T, t)) : uint8_t(0xFFu);
-  pr.keepR = kind ? uint8_t((~target_dead_regs(T, t) & 0x3Fu) | 0x80u) : uint8_t(0x3Fu);
-  if (pair_xindep(T, t, P, c)) pr.keepR |= uint8_t(kXIndep);
-  // A swept register that no compared output of either program depends on
-  // (dead registers and flags make this common in masked passes: SET 6, B
-  // with B dead) cannot change the verdict, so one value of it stands for
-  // all the reference sweeps: it is left out of the sweep, whose other
-  // registers keep the reference's values (a reduced sweep stays reduced).
-  // The same holds for the carry, the most significant field of the block
-  // index: when no compared output depends on it, the first half of the
-  // blocks (carry 0) decides.
-  uint32_t swept = reads;
-  pr.sweepf = 0;
-  const uint32_t ext = reads & (kRegB | kRegC | kRegD | kRegE | kRegH | kRegL | kRegM);
-  const uint32_t cmp = kRegA | kRegSP | kRegM | ((uint32_t(pr.keepR) & 0x3Fu) << 2) |
-                       (uint32_t(pr.keepF) << kDepF0);
-  const uint32_t* tw = T.insn + (size_t)t * T.stride;
-  const uint32_t* cw = P.insn + (size_t)c * P.stride;
-  const uint32_t tl = target_len(T, t), cl = pool_len(P, c);
-  // what the compared outputs other than A, and A itself, depend on
-  const uint32_t rest = dev_seq_relevant(tw, tl, cmp & ~uint32_t(kRegA)) | dev_seq_relevant(cw, cl, cmp & ~uint32_t(kRegA));
-  const uint32_t at = dev_seq_relevant(tw, tl, kRegA), ac = dev_seq_relevant(cw, cl, kRegA);
-  const uint32_t rel = rest | at | ac;
-  uint32_t drop = ext & ~rel;
-  // a swept register both programs keep exactly, on which no other compared
-  // output depends, compares equal whatever its value: one value decides
-  const uint32_t both = dev_seq_keeps(tw, tl) & dev_seq_keeps(cw, cl) & ext & ~drop;
-  for (uint32_t b = both; b; b &= b - 1) {
-    const uint32_t r = b & (0u - b);
-    if (!((dev_seq_relevant(tw, tl, cmp & ~r) | dev_seq_relevant(cw, cl, cmp & ~r)) & r)) drop |= r;
+// Puts the window of w survivors at sbase of lane (t, kind) into the pair
+// slots from p0: who the pairs are.  What their sweeps take is worked out by
+// k_pair_plan, a thread per pair (a window is up to 64 pairs and a plan some
+// microseconds: planned here, one thread would plan a window's pairs one
+// after the other).
+__device__ __forceinline__ void put_window(const RoundBuf& R, uint32_t p0, uint32_t w, uint32_t t, uint32_t kind,
+                                           const uint32_t* __restrict__ surv, uint32_t sbase) {
+  for (uint32_t j = 0; j < w; j++) {
+    const uint32_t p = p0 + j;
+    PairRec pr{};
+    pr.target = t;
+    pr.cand = surv[sbase + j];
+    pr.keepR = kind ? 0x80u : 0u;
+    R.pairs[p] = pr;
+    R.pair_src[p] = sbase + j;
+    R.rejected[p] = 0;
+    R.wlen[p] = j == 0 ? uint8_t(w) : uint8_t(0);
+    if (R.wend) {
+      R.wend[p] = p0 + w;
+      R.cdone[p] = 0;
+    }
   }
-  const bool carry_out = (rel & (1u << kDepF0)) == 0;
-  if (drop) {
-    const bool red = (reads & kRegSP) != 0 || __popc(ext) > 2;
-    swept = reads & ~drop;
-    pr.sweepf = uint8_t((red ? 0x80u : 0u) | uint32_t(__popc(drop)) * (red ? 5u : 8u));
+}
+
+// Plans the round's pairs (z80_plan.cuh), one thread each: compared outputs,
+// swept fields, class and chunks.  A pair that its programs prove equivalent
+// gets no chunk and keeps its zero flag; the pairs after it in its window
+// cannot win and are cancelled.  Bound by latency (table loads and local
+// arrays; a few microseconds a pair, thousands of pairs side by side): with
+// the plans made in the round build, windows in one thread, 100,003 masked
+// targets spent 3.4 ms in their 11 rounds, here 0.9 ms.
+__global__ void __launch_bounds__(128) k_pair_plan(DevTargets T, DevPool P, QCOut q, RoundBuf R) {
+  const uint32_t np = min(*R.npairs, R.cap);
+  unsigned long long proven_states = 0;
+  for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < np; p += gridDim.x * blockDim.x) {
+    PairRec pr = R.pairs[p];
+    const uint32_t t = pr.target, c = pr.cand;
+    const bool masked = (pr.keepR & 0x80u) != 0;
+    const uint32_t reads = q.meta[t].reads | P.reads[c];
+    pr.keepF = masked ? uint8_t(~target_dead(T, t)) : uint8_t(0xFFu);
+    pr.keepR = masked ? uint8_t((~target_dead_regs(T, t) & 0x3Fu) | 0x80u) : uint8_t(0x3Fu);
+    const PairPlan pl = plan_pair(g_flow, T.insn + (size_t)t * T.stride, target_len(T, t),
+                                  P.insn + (size_t)c * P.stride, pool_len(P, c), reads, pr.keepF, pr.keepR);
+    pr.reads = pl.reads;
+    pr.sweepf = pl.sweepf;
+    pr.nblocks = pl.nblocks;
+    pr.cmap = 0;
+    if (pl.proven) {
+      pr.nblocks = 0;  // no chunk in any class
+      proven_states += 256ull * plan_blocks(reads, false);
+      if (R.wend)
+        for (uint32_t i = p + 1; i < R.wend[p]; i++) R.rejected[i] = 2;
+    } else {
+      if (pl.a_free || pair_xindep(T, t, P, c)) pr.keepR |= uint8_t(kXIndep);
+      // compact classes: A-dependent pairs, and A-independent ones when those
+      // are swept bit-sliced (units of kXBitsBlocks); the narrow state first
+      if (!(pr.keepR & kXIndep) || R.xunit == kXBitsBlocks) {
+        if (R.compact) pr.cmap = pair_cmap(T, t, P, c);
+        // the wide state: A-dependent pairs only
+        if (!pr.cmap && R.wide && !(pr.keepR & kXIndep)) pr.cmap = pair_wmap(T, t, P, c);
+        // the register state: the rest that name neither SP nor the memory byte
+        if (!pr.cmap && R.wide && pair_regstate(T, t, P, c)) pr.cmap = kRegClass;
+      }
+    }
+    R.pairs[p] = pr;
+    set_chunks(R, p, pr);
   }
-  pr.reads = uint16_t(swept);
-  pr.nblocks = sweep_blocks(swept, (pr.sweepf & 0x80u) != 0);
-  if (carry_out) {
-    pr.nblocks >>= 1;
-    pr.sweepf += 1;
-  }
-  // Two values of A decide the pair when no compared output but A depends
-  // on the input A (a comparison whose flags are dead or overwritten, A
-  // copied into a dead register) and each program keeps A or computes its A
-  // from other inputs: the argument of the A-independent sweeps under the
-  // pair's masks.
-  if (!(rest & kRegA) && (!(at & kRegA) || dev_seq_keeps_a(tw, tl)) && (!(ac & kRegA) || dev_seq_keeps_a(cw, cl)))
-    pr.keepR |= uint8_t(kXIndep);
-  // compact classes: A-dependent pairs, and A-independent ones when those
-  // are swept bit-sliced (units of kXBitsBlocks); the narrow state first
-  pr.cmap = 0;
-  if (!(pr.keepR & kXIndep) || R.xunit == kXBitsBlocks) {
-    if (R.compact) pr.cmap = pair_cmap(T, t, P, c);
-    // the wide state: A-dependent pairs only
-    if (!pr.cmap && R.wide && !(pr.keepR & kXIndep)) pr.cmap = pair_wmap(T, t, P, c);
-    // the register state: the rest that name neither SP nor the memory byte
-    if (!pr.cmap && R.wide && pair_regstate(T, t, P, c)) pr.cmap = kRegClass;
-  }
-  R.pairs[p] = pr;
-  R.pair_src[p] = src;
-  set_chunks(R, p, pr);
-  R.rejected[p] = 0;
-  R.wlen[p] = wlen;
-  if (R.wend) {
-    R.wend[p] = wend;
-    R.cdone[p] = 0;
-  }
+  __syncwarp();
+#pragma unroll
+  for (int o = 16; o; o >>= 1) proven_states += __shfl_xor_sync(kFull, proven_states, o);
+  if (lane_id() == 0 && proven_states) atomicAdd(R.states, proven_states);
 }
 
 // Lane 0, after a warp's chunk of pair p ran to its end without a mismatch:
@@ -648,9 +606,9 @@ __device__ __forceinline__ void chunk_passed(uint32_t* rejected, const uint32_t*
 // One round of the length-1 pass: each unresolved (target, kind) lane puts
 // its window of next survivors into the round (pairs past the buffer's
 // capacity wait for the next round).
-__global__ void k_round_build(DevTargets T, DevPool P, QCOut q, Lanes L, RoundBuf R) {
+__global__ void k_round_build(DevTargets T, QCOut q, Lanes L, RoundBuf R) {
   const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-#pragma unroll
+#pragma unroll 1
   for (uint32_t kind = 0; kind < 2; kind++) {
     uint32_t w = 0, nx = 0, sbase = 0;
     if (t < T.n) {
@@ -670,9 +628,7 @@ __global__ void k_round_build(DevTargets T, DevPool P, QCOut q, Lanes L, RoundBu
     if (!__any_sync(kFull, w != 0)) continue;
     const uint32_t p0 = alloc_pairs(R.npairs, w);
     const uint32_t fit = p0 >= R.cap ? 0u : min(w, R.cap - p0);
-    for (uint32_t j = 0; j < fit; j++)
-      put_pair(R, p0 + j, T, P, q, t, kind, q.surv[sbase + j], sbase + j, j == 0 ? uint8_t(fit) : uint8_t(0),
-               p0 + fit);
+    put_window(R, p0, fit, t, kind, q.surv, sbase);
   }
 }
 
@@ -690,7 +646,7 @@ __global__ void k_pairs_from_survivors(DevTargets T, DevPool P, QCOut q, const u
     pr.target = t;
     pr.cand = c;
     pr.reads = uint16_t(reads);
-    pr.nblocks = sweep_blocks(reads);
+    pr.nblocks = plan_blocks(reads, false);
     pr.keepF = uint8_t(~target_dead(T, t));
     pr.keepR = uint8_t(~target_dead_regs(T, t) & 0x3Fu);
     if (pair_xindep(T, t, P, c)) pr.keepR |= uint8_t(kXIndep);
@@ -988,6 +944,7 @@ __device__ __forceinline__ bool xbits_unit(unsigned long long u, unsigned long l
     // the last field's 32 representatives, state j = representative j
 #pragma unroll
     for (int i = 0; i < 8; i++) vp[i] = __ballot_sync(kFull, (g_rep[lane] >> i) & 1u);
+    fp0 = 0xAAAAAAAAu;  // every swept field left out: the carry is bit 0
   } else {
     // full sweep: the last field's low 5 bits count the states, the rest is
     // the group's value; with no extra register the carry is bit 0
@@ -2200,7 +2157,7 @@ __global__ void __launch_bounds__(kBlock) k_pair_scan(DevTargets T, DevPool P, Q
 // left either end without a winner (bucket exhausted) or wait for a rescan.
 // One round of the length-2 pass: windows over the lane's slots; a lane
 // with its slots used up and its bucket not exhausted asks for a rescan.
-__global__ void k_pair_round_build(DevTargets T, DevPool P, QCOut q1, Lanes L2, PairScan ps, RoundBuf R) {
+__global__ void k_pair_round_build(DevTargets T, Lanes L2, PairScan ps, RoundBuf R) {
   const uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x;
   uint32_t w = 0, sbase = 0;
   if (idx < 2 * T.n) {
@@ -2219,9 +2176,7 @@ __global__ void k_pair_round_build(DevTargets T, DevPool P, QCOut q1, Lanes L2, 
   if (!__any_sync(kFull, w != 0)) return;
   const uint32_t p0 = alloc_pairs(R.npairs, w);
   const uint32_t fit = p0 >= R.cap ? 0u : min(w, R.cap - p0);
-  for (uint32_t j = 0; j < fit; j++)
-    put_pair(R, p0 + j, T, P, q1, idx >> 1, idx & 1u, ps.surv[sbase + j], sbase + j,
-             j == 0 ? uint8_t(fit) : uint8_t(0), p0 + fit);
+  put_window(R, p0, fit, idx >> 1, idx & 1u, ps.surv, sbase);
 }
 
 
@@ -2291,9 +2246,7 @@ void dev_upload_tables(cudaStream_t s) {
   cudaMemcpyToSymbolAsync(g_repsp, rep_sp(), 32, 0, cudaMemcpyHostToDevice, s);
   cudaMemcpyToSymbolAsync(g_aclass, op_aclass(), kNumOps, 0, cudaMemcpyHostToDevice, s);
   {
-    cudaMemcpyToSymbolAsync(g_dep, op_deps(), sizeof(uint32_t) * kNumOps * kDepFields, 0, cudaMemcpyHostToDevice, s);
-    cudaMemcpyToSymbolAsync(g_keepa, op_keeps_a(), kNumOps, 0, cudaMemcpyHostToDevice, s);
-    cudaMemcpyToSymbolAsync(g_keeps, op_keeps(), sizeof(uint16_t) * kNumOps, 0, cudaMemcpyHostToDevice, s);
+    cudaMemcpyToSymbolAsync(g_flow, op_flow(), sizeof(OpFlow) * kNumOps, 0, cudaMemcpyHostToDevice, s);
     const CompactTables& C = compact_tables();
     cudaMemcpyToSymbolAsync(g_cren, C.ren, sizeof C.ren, 0, cudaMemcpyHostToDevice, s);
     cudaMemcpyToSymbolAsync(g_corig, C.orig, sizeof C.orig, 0, cudaMemcpyHostToDevice, s);
@@ -2382,10 +2335,17 @@ void launch_qc_bucket(const DevTargets& T, const DevPool& P, const QCConfig& cfg
   else if (keep) k_qc_bucket<false, true><<<grid, kBlock, 0, s>>>(T, P, cfg, ix, o);
   else k_qc_bucket<false, false><<<grid, kBlock, 0, s>>>(T, P, cfg, ix, o);
 }
+// The pair count is on the device: a grid-stride launch of up to 16 blocks
+// per SM (the pair slots bound it for small jobs).
+static void launch_pair_plan(const DevTargets& T, const DevPool& P, const QCOut& q, const RoundBuf& R, cudaStream_t s) {
+  const unsigned grid = std::min<unsigned>(grid_for(R.cap, 128), unsigned(dev_num_sms() * 16));
+  k_pair_plan<<<grid, 128, 0, s>>>(T, P, q, R);
+}
 void launch_round_build(const DevTargets& T, const DevPool& P, const QCOut& q, const Lanes& L,
                         const RoundBuf& R, cudaStream_t s) {
   if (!T.n) return;
-  k_round_build<<<grid_for(T.n, 256), 256, 0, s>>>(T, P, q, L, R);
+  k_round_build<<<grid_for(T.n, 256), 256, 0, s>>>(T, q, L, R);
+  launch_pair_plan(T, P, q, R, s);
 }
 void launch_pairs_from_survivors(const DevTargets& T, const DevPool& P, const QCOut& q,
                                  const uint8_t* midpass, uint32_t nsurv, const uint32_t* surv_target,
@@ -2736,7 +2696,8 @@ void launch_pair_scan_gated(const DevTargets& T, const DevPool& P, const QCOut& 
 void launch_pair_round_build(const DevTargets& T, const DevPool& P, const QCOut& q1, const Lanes& L2,
                              const PairScan& ps, const RoundBuf& R, cudaStream_t s) {
   if (!T.n) return;
-  k_pair_round_build<<<grid_for(2 * T.n, 256), 256, 0, s>>>(T, P, q1, L2, ps, R);
+  k_pair_round_build<<<grid_for(2 * T.n, 256), 256, 0, s>>>(T, L2, ps, R);
+  launch_pair_plan(T, P, q1, R, s);
 }
 
 
