@@ -24,7 +24,6 @@
 #include <cstring>
 #include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_scan.cuh>
-#include <cub/device/device_select.cuh>
 #include <map>
 #include <memory>
 #include <mutex>
@@ -122,21 +121,20 @@ struct PipeOpts {
 constexpr int kUpChunks = 4;
 constexpr uint32_t kUpChunkMin = 1u << 16;  // targets; smaller jobs upload in one copy
 
-// The 4,531^2 pair pool, its QuickCheck outputs and its bucket indexes (one
-// per dead-register mask, built on first use).  Read-only once built, so all
+// The 4,531^2 pair pool, its QuickCheck outputs and its indexes (one per
+// dead-register mask, built on first use).  Read-only once built, so all
 // contexts of a device share one copy; mu serializes the builds.
 struct PairShared {
   std::mutex mu;
   PoolBufs pool;
   uint32_t valid = 0;                          // unpruned pairs
+  DBuf valid_ids;                              // [valid] their indices, ascending
   std::vector<unsigned long long> eligible;    // [16] unpruned pairs shorter than b bytes
-  DBuf idx[64];
+  DBuf members[64], groups[64], top[64];
   bool ok[64] = {};
-  DBuf ptrs, eligible_dev, keys_tmp, sort_tmp;
-  // the indexes restricted to unpruned pairs of at most 2 / 3 bytes
-  uint32_t n_le[2] = {0, 0};
-  DBuf idx_le[2][64];
-  DBuf ptrs_le[2], sel_tmp, sel_count;
+  DBuf idx, eligible_dev;                      // PairIndex[64]
+  // build scratch: keys and their sorted copy, group numbers
+  DBuf keys, keys_sorted, gid, cub_tmp;
 };
 
 std::mutex g_pairs_mu;
@@ -307,8 +305,9 @@ int fetch(z80b_ctx* ctx, T* host, const T* dev, size_t n = 1) {
 
 // Uploads a candidate list and computes its QuickCheck (and optionally
 // MidCheck) outputs on the device.
+// by_pair: the outputs of a candidate side by side (launch_pool_outputs).
 int build_pool(z80b_ctx* ctx, PoolBufs& P, const uint32_t* insn, uint32_t n, uint32_t len,
-               const uint8_t* lens, bool with_mid) {
+               const uint8_t* lens, bool with_mid, bool by_pair = false) {
   P.loaded = false;
   P.qstate = 0;  // a QuickCheck index of the previous contents is stale
   P.n = n;
@@ -352,14 +351,14 @@ int build_pool(z80b_ctx* ctx, PoolBufs& P, const uint32_t* insn, uint32_t n, uin
   }
   trace("pool: %u candidates uploaded", n);
   launch_pool_outputs(P.insn.as<uint32_t>(), n, len, P.qc.as<uint4>(), with_mid ? P.mid.as<uint4>() : nullptr,
-                      ctx->stream);
+                      by_pair, ctx->stream);
   CKR(check_launch(ctx, "pool_outputs"));
   trace("pool: kernel launched");
   CK(cudaStreamSynchronize(ctx->stream));
   trace("pool: outputs ready");
   P.dev = DevPool{};
   P.dev.insn = P.insn.as<uint32_t>();
-  P.dev.qc = P.qc.as<uint4>();
+  P.dev.qc = by_pair ? nullptr : P.qc.as<uint4>();
   P.dev.mid = with_mid ? P.mid.as<uint4>() : nullptr;
   P.dev.size = P.size.as<uint8_t>();
   P.dev.prune = P.prune.as<uint8_t>();
@@ -402,7 +401,7 @@ int ensure_pairpool(z80b_ctx* ctx) {
       insn[(size_t(a) * n1 + b) * 2 + 1] = p8[b];
     }
   trace("pair pool: %u pairs", n);
-  CKR(build_pool(ctx, S.pool, insn.data(), n, 2, nullptr, false));
+  CKR(build_pool(ctx, S.pool, insn.data(), n, 2, nullptr, false, true));
   // unpruned pairs by encoded size, for the eligible-pair count per target
   std::vector<uint8_t> size(n), prune(n);
   CK(cudaMemcpy(size.data(), S.pool.size.p, n, cudaMemcpyDeviceToHost));
@@ -415,78 +414,68 @@ int ensure_pairpool(z80b_ctx* ctx) {
       by_size[std::min<uint32_t>(size[q], 16)]++;
     }
   S.valid = valid;
-  S.n_le[0] = uint32_t(by_size[0] + by_size[1] + by_size[2]);
-  S.n_le[1] = uint32_t(S.n_le[0] + by_size[3]);
+  for (size_t b = 0; b < by_size.size(); b++)
+    if (by_size[b] && (b < 2 || b >= 2 + kPairSizes))
+      return fail(ctx, Z80B_EINVAL, "a candidate pair takes %u bytes", unsigned(b));
+  std::vector<uint32_t> ids(valid);
+  for (uint32_t q = 0, k = 0; q < n; q++)
+    if (!prune[q]) ids[k++] = q;
+  CK(S.valid_ids.ensure(4ull * valid));
+  CK(cudaMemcpy(S.valid_ids.p, ids.data(), 4ull * valid, cudaMemcpyHostToDevice));
   S.eligible.assign(16, 0);
   for (int b = 1; b < 16; b++) S.eligible[size_t(b)] = S.eligible[size_t(b - 1)] + by_size[size_t(b - 1)];
   CK(S.eligible_dev.ensure(16 * sizeof(unsigned long long)));
   CK(cudaMemcpy(S.eligible_dev.p, S.eligible.data(), 16 * sizeof(unsigned long long), cudaMemcpyHostToDevice));
-  CK(S.ptrs.ensure(64 * sizeof(void*)));
-  CK(cudaMemset(S.ptrs.p, 0, 64 * sizeof(void*)));
-  for (int k = 0; k < 2; k++) {
-    CK(S.ptrs_le[k].ensure(64 * sizeof(void*)));
-    CK(cudaMemset(S.ptrs_le[k].p, 0, 64 * sizeof(void*)));
-  }
-  trace("pair pool ready: %u unpruned (%u of at most 2 bytes, %u of at most 3)", valid, S.n_le[0], S.n_le[1]);
+  CK(S.idx.ensure(64 * sizeof(PairIndex)));
+  CK(cudaMemset(S.idx.p, 0, 64 * sizeof(PairIndex)));
+  trace("pair pool ready: %u unpruned", valid);
   return Z80B_OK;
 }
 
-// Selects index entries of unpruned pairs of at most max_size bytes (pruned
-// pairs' keys are all ones).
-struct ShortPair {
-  const uint8_t* size;
-  uint8_t max_size;
-  __device__ bool operator()(const unsigned long long& key) const {
-    return key != ~0ull && size[uint32_t(key)] <= max_size;
-  }
-};
-
-// Bucket index of the pair pool for one dead-register mask: the pairs'
-// (hash of the masked vector-0 output, pair index) keys, sorted.
+// Index of the pair pool for one dead-register mask (PairIndex): the keys of
+// the unpruned pairs sorted (a stable sort: pair indices ascend within equal
+// keys), cut into groups, and the top table.
 int ensure_pair_index(z80b_ctx* ctx, uint32_t m) {
   PairShared& S = *ctx->pairpool;
   std::lock_guard<std::mutex> lk(S.mu);
   if (S.ok[m]) return Z80B_OK;
-  const DevPool& P = S.pool.dev;
-  const size_t n = P.n;
-  CK(S.keys_tmp.ensure(n * 8));
-  CK(S.idx[m].ensure(n * 8));
-  launch_pair_keys(P, m, S.keys_tmp.as<unsigned long long>(), ctx->stream);
+  const uint32_t n = S.valid;
+  const uint4* out = S.pool.qc.as<uint4>();
+  cudaStream_t s = ctx->stream;
+  CK(S.keys.ensure(8ull * n));
+  CK(S.keys_sorted.ensure(8ull * n));
+  CK(S.gid.ensure(4ull * n));
+  CK(S.members[m].ensure(4ull * n));
+  CK(S.top[m].ensure(4ull * (kPairTop + 1)));
+  launch_pair_keys(S.pool.dev, out, S.valid_ids.as<uint32_t>(), n, m, S.keys.as<unsigned long long>(), s);
   CKR(check_launch(ctx, "pair_keys"));
-  size_t tmp = 0;
-  CK(cub::DeviceRadixSort::SortKeys(nullptr, tmp, S.keys_tmp.as<unsigned long long>(),
-                                    S.idx[m].as<unsigned long long>(), int(n), 0, 64, ctx->stream));
-  CK(S.sort_tmp.ensure(tmp));
-  CK(cub::DeviceRadixSort::SortKeys(S.sort_tmp.p, tmp, S.keys_tmp.as<unsigned long long>(),
-                                    S.idx[m].as<unsigned long long>(), int(n), 0, 64, ctx->stream));
-  ctx->launches += 2;
-  void* ptr = S.idx[m].p;
-  CK(cudaMemcpyAsync(S.ptrs.as<void*>() + m, &ptr, sizeof ptr, cudaMemcpyHostToDevice, ctx->stream));
-  // the short-pair indexes: the entries of pairs of at most 2 / 3 bytes, in
-  // the full index's order (a stable selection)
-  CK(S.sel_count.ensure(sizeof(int)));
-  for (int k = 0; k < 2; k++) {
-    CK(S.idx_le[k][m].ensure(8ull * std::max<uint32_t>(S.n_le[k], 1)));
-    const ShortPair pred{P.size, uint8_t(2 + k)};
-    size_t stmp = 0;
-    CK(cub::DeviceSelect::If(nullptr, stmp, S.idx[m].as<unsigned long long>(), S.idx_le[k][m].as<unsigned long long>(),
-                             S.sel_count.as<int>(), int(n), pred, ctx->stream));
-    CK(S.sel_tmp.ensure(stmp));
-    CK(cub::DeviceSelect::If(S.sel_tmp.p, stmp, S.idx[m].as<unsigned long long>(),
-                             S.idx_le[k][m].as<unsigned long long>(), S.sel_count.as<int>(), int(n), pred,
-                             ctx->stream));
-    ctx->launches += 1;
-    int got = 0;
-    CK(cudaMemcpyAsync(&got, S.sel_count.p, sizeof got, cudaMemcpyDeviceToHost, ctx->stream));
-    CK(cudaStreamSynchronize(ctx->stream));
-    if (uint32_t(got) != S.n_le[k])
-      return fail(ctx, Z80B_ECUDA, "short-pair index holds %d entries, expected %u", got, S.n_le[k]);
-    void* q = S.idx_le[k][m].p;
-    CK(cudaMemcpyAsync(S.ptrs_le[k].as<void*>() + m, &q, sizeof q, cudaMemcpyHostToDevice, ctx->stream));
-  }
-  CK(cudaStreamSynchronize(ctx->stream));
+  size_t tmp = 0, tmp2 = 0;
+  CK(cub::DeviceRadixSort::SortPairs(nullptr, tmp, S.keys.as<unsigned long long>(),
+                                     S.keys_sorted.as<unsigned long long>(), S.valid_ids.as<uint32_t>(),
+                                     S.members[m].as<uint32_t>(), int(n), 0, 64, s));
+  CK(cub::DeviceScan::InclusiveSum(nullptr, tmp2, S.gid.as<uint32_t>(), S.gid.as<uint32_t>(), int(n), s));
+  CK(S.cub_tmp.ensure(std::max(tmp, tmp2)));
+  CK(cub::DeviceRadixSort::SortPairs(S.cub_tmp.p, tmp, S.keys.as<unsigned long long>(),
+                                     S.keys_sorted.as<unsigned long long>(), S.valid_ids.as<uint32_t>(),
+                                     S.members[m].as<uint32_t>(), int(n), 0, 64, s));
+  launch_pair_heads(out, S.keys_sorted.as<unsigned long long>(), S.members[m].as<uint32_t>(), n, m,
+                    S.gid.as<uint32_t>(), s);
+  CKR(check_launch(ctx, "pair_heads"));
+  CK(cub::DeviceScan::InclusiveSum(S.cub_tmp.p, tmp2, S.gid.as<uint32_t>(), S.gid.as<uint32_t>(), int(n), s));
+  uint32_t ng = 0;
+  CKR(fetch(ctx, &ng, S.gid.as<uint32_t>() + (n - 1)));
+  CK(S.groups[m].ensure(16ull * (ng + 1ull)));
+  launch_pair_groups(out, S.keys_sorted.as<unsigned long long>(), S.members[m].as<uint32_t>(), n,
+                     S.gid.as<uint32_t>(), S.groups[m].as<uint4>(), s);
+  CKR(check_launch(ctx, "pair_groups"));
+  launch_pair_top(S.groups[m].as<uint4>(), ng, S.top[m].as<uint32_t>(), s);
+  CKR(check_launch(ctx, "pair_top"));
+  ctx->launches += 3;
+  const PairIndex ix{S.members[m].as<uint32_t>(), S.groups[m].as<uint4>(), S.top[m].as<uint32_t>()};
+  CK(cudaMemcpyAsync(S.idx.as<PairIndex>() + m, &ix, sizeof ix, cudaMemcpyHostToDevice, s));
+  CK(cudaStreamSynchronize(s));
   S.ok[m] = true;
-  trace("pair index for dead-register mask %02X built", m);
+  trace("pair index for dead-register mask %02X built: %u groups", m, ng);
   return Z80B_OK;
 }
 
@@ -772,7 +761,7 @@ int rounds_on_device(z80b_ctx* ctx, RoundGraph& g, const DevTargets& T, const De
       cudaMemsetAsync(ps->refill, 0, 4, s);
       launch_pair_round_build(T, P, q, L, *ps, R, s);
       launch_round_scan(R, ctl, ps->refill, loop, s);
-      launch_pair_scan_gated(T, P, q, L, *ps, ctl, s);
+      launch_pair_scan_gated(T, q, L, *ps, ctl, s);
     } else {
       launch_round_build(T, P, q, L, R, s);
       launch_round_scan(R, ctl, nullptr, loop, s);
@@ -1063,12 +1052,8 @@ int run_pipeline(z80b_ctx* ctx, const DevTargets& T, const PipeOpts& opts, z80b_
       L2 = Lanes{ctx->next2.as<uint32_t>(), ctx->win2.as<uint32_t>(), ctx->windiff2.as<uint16_t>(),
                  ctx->spec2.as<uint8_t>()};
       PairScan ps{};
-      ps.idx = reinterpret_cast<const unsigned long long* const*>(PS.ptrs.p);
-      ps.n_valid = PS.valid;
-      ps.idx_le2 = reinterpret_cast<const unsigned long long* const*>(PS.ptrs_le[0].p);
-      ps.idx_le3 = reinterpret_cast<const unsigned long long* const*>(PS.ptrs_le[1].p);
-      ps.n_le2 = PS.n_le[0];
-      ps.n_le3 = PS.n_le[1];
+      ps.idx = PS.idx.as<PairIndex>();
+      ps.out = PS.pool.qc.as<uint4>();
       ps.cnt = ctx->cnt2.as<uint32_t>();
       ps.resume = ctx->resume2.as<uint32_t>();
       ps.surv = ctx->surv2.as<uint32_t>();
@@ -1081,7 +1066,7 @@ int run_pipeline(z80b_ctx* ctx, const DevTargets& T, const PipeOpts& opts, z80b_
       launch_pair_lanes_init(T, L, q, L2, ps, s);
       CKR(check_launch(ctx, "pair_lanes_init"));
       int kq2 = kbegin(ctx, 0);
-      launch_pair_scan(T, P2, q, L2, ps, s);
+      launch_pair_scan(T, q, L2, ps, s);
       kend(ctx, kq2);
       CKR(check_launch(ctx, "pair_scan"));
       if (dev_rounds)
@@ -1100,7 +1085,7 @@ int run_pipeline(z80b_ctx* ctx, const DevTargets& T, const PipeOpts& opts, z80b_
         if (np == 0) {
           if (nref == 0) break;
           int kr = kbegin(ctx, 0);
-          launch_pair_scan(T, P2, q, L2, ps, s);
+          launch_pair_scan(T, q, L2, ps, s);
           kend(ctx, kr);
           CKR(check_launch(ctx, "pair_scan"));
           continue;

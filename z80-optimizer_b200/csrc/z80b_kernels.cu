@@ -232,7 +232,7 @@ __device__ __forceinline__ unsigned long long chunks_for(unsigned long long nb, 
 // Warp per candidate, lane v runs the candidate on vector v (lanes 0..7
 // QuickCheck, 0..31 MidCheck); the opcode is the same in every lane.
 __global__ void k_pool_outputs(const uint32_t* __restrict__ insn, uint32_t n, uint32_t len,
-                               uint4* __restrict__ qc, uint4* __restrict__ mid) {
+                               uint4* __restrict__ qc, uint4* __restrict__ mid, bool by_pair) {
   const unsigned lane = lane_id();
   const uint32_t gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
@@ -243,7 +243,7 @@ __global__ void k_pool_outputs(const uint32_t* __restrict__ insn, uint32_t n, ui
     uint32_t w[3];
     z_pack(s, w);
     const uint4 q = make_uint4(w[0], w[1], w[2], 0u);
-    if (lane < 8) qc[(size_t)lane * n + c] = q;
+    if (lane < 8) qc[by_pair ? (size_t)c * 8 + lane : (size_t)lane * n + c] = q;
     if (mid) mid[(size_t)lane * n + c] = q;
   }
 }
@@ -1765,14 +1765,14 @@ __global__ void k_verify_small(const uint32_t* __restrict__ tgt, const uint8_t* 
 // The candidates of length 2 are the 4,531^2 odometer pairs of the 8-bit
 // list (pair index = first * 4531 + second, the EnumerateSequences8 order),
 // held as a pool whose QuickCheck outputs are precomputed like the length-1
-// pool.  Instead of comparing every target with all 20.5M pairs, each pair
-// is filed in a sorted index under a hash of its vector-0 output with F left
-// out and the dead registers zeroed (one index per dead-register mask in
-// use).  A target hashes its own vector-0 output the same way, finds its
-// bucket by binary search, and QuickChecks only the bucket's pairs, which
-// the index keeps in enumeration order.  Survivors go to fixed slots per
-// (target, kind) lane; a lane whose slots are used up without a winner
-// rescans its bucket from where it stopped.
+// pool, the eight outputs of a pair in one 128-byte line.  Instead of
+// comparing every target with all 20.5M pairs, an index per dead-register
+// mask in use (PairIndex) sorts the unpruned pairs into groups with the same
+// outputs; a target finds the groups with its own outputs by hash, compares
+// their F bytes under its dead flags, and takes the smallest pair indices of
+// the groups that pass.  Survivors go to fixed slots per (target, kind)
+// lane; a lane whose slots are used up without a winner goes on from the
+// pair after the last one it took.
 
 // Bytes of the packed vector-0 word 0 / word 1 kept in the bucket key.
 __device__ __forceinline__ uint32_t key_keep0(uint32_t dregs) {
@@ -1794,15 +1794,93 @@ __device__ __forceinline__ uint32_t bucket_hash(uint32_t w0, uint32_t w1, uint32
   return uint32_t(h >> 32);
 }
 
-__global__ void k_pair_keys(DevPool P, uint32_t dregs, unsigned long long* __restrict__ keys) {
-  const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= P.n) return;
-  if (P.prune[q]) {
-    keys[q] = ~0ull;  // sorts after every real entry
-    return;
+// Hash of one vector's output (A, live registers, SP, M); the hash of a
+// sequence is the sum over the eight vectors, so that the lanes of a warp can
+// each hash one.
+__device__ __forceinline__ unsigned long long vector_hash(uint32_t w0, uint32_t w1, uint32_t w2, uint32_t v) {
+  unsigned long long h = ((unsigned long long)w0 << 32) | w1;
+  h ^= (unsigned long long)(w2 + (v << 24)) * 0x9E3779B97F4A7C15ull;
+  h ^= h >> 30;
+  h *= 0xBF58476D1CE4E5B9ull;
+  h ^= h >> 27;
+  h *= 0x94D049BB133111EBull;
+  return h ^ (h >> 31);
+}
+__device__ __forceinline__ uint32_t pair_group_key(uint32_t size, unsigned long long h) {
+  return ((size - 2u) << 30) | uint32_t(h >> 34);
+}
+// Thread per unpruned pair (one 128-byte line each).
+__global__ void __launch_bounds__(256) k_pair_keys(DevPool P, const uint4* __restrict__ out,
+                                                   const uint32_t* __restrict__ valid, uint32_t n, uint32_t dregs,
+                                                   unsigned long long* __restrict__ keys) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const uint32_t q = valid[i];
+  const uint32_t k0 = key_keep0(dregs), k1 = key_keep1(dregs);
+  unsigned long long h = 0;
+  uint32_t flo = 0, fhi = 0;
+#pragma unroll
+  for (uint32_t v = 0; v < 8; v++) {
+    const uint4 o = out[(size_t)q * 8 + v];
+    h += vector_hash(o.x & k0, o.y & k1, o.z, v);
+    const uint32_t f = (o.x >> 8) & 0xFFu;
+    if (v < 4) flo |= f << (8 * v);
+    else fhi |= f << (8 * (v - 4));
   }
-  const uint4 o = P.qc[q];
-  keys[q] = ((unsigned long long)bucket_hash(o.x & key_keep0(dregs), o.y & key_keep1(dregs), o.z) << 32) | q;
+  const uint32_t fh = uint32_t(vector_hash(flo, fhi, 0u, 0u) >> 32);
+  keys[i] = ((unsigned long long)pair_group_key(P.size[q], h) << 32) | fh;
+}
+// A position begins a group where its pair's outputs (live registers, A, SP,
+// M, F) differ from the position before it; equal keys are compared in full,
+// so a group never mixes two outputs whose hashes collide.
+__global__ void __launch_bounds__(256) k_pair_heads(const uint4* __restrict__ out,
+                                                    const unsigned long long* __restrict__ keys,
+                                                    const uint32_t* __restrict__ members, uint32_t n, uint32_t dregs,
+                                                    uint32_t* __restrict__ head) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  bool h = i == 0 || keys[i] != keys[i - 1];
+  if (!h) {
+    const uint32_t k0 = key_keep0(dregs) | 0xFF00u, k1 = key_keep1(dregs);
+    const uint4* a = out + (size_t)members[i] * 8;
+    const uint4* b = out + (size_t)members[i - 1] * 8;
+    uint32_t d = 0;
+#pragma unroll
+    for (int v = 0; v < 8; v++) {
+      const uint4 x = a[v], y = b[v];
+      d |= ((x.x ^ y.x) & k0) | ((x.y ^ y.y) & k1) | (x.z ^ y.z);
+    }
+    h = d != 0;
+  }
+  head[i] = h ? 1u : 0u;
+}
+// gid: inclusive sum of the head flags.
+__global__ void __launch_bounds__(256) k_pair_groups(const uint4* __restrict__ out,
+                                                     const unsigned long long* __restrict__ keys,
+                                                     const uint32_t* __restrict__ members, uint32_t n,
+                                                     const uint32_t* __restrict__ gid, uint4* __restrict__ groups) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  if (i == n - 1) groups[gid[i]] = make_uint4(0xFFFFFFFFu, n, 0u, 0u);
+  if (i != 0 && gid[i] == gid[i - 1]) return;
+  const uint4* o = out + (size_t)members[i] * 8;
+  uint32_t f[2] = {0u, 0u};
+#pragma unroll
+  for (int v = 0; v < 8; v++) f[v >> 2] |= ((o[v].x >> 8) & 0xFFu) << (8 * (v & 3));
+  groups[gid[i] - 1] = make_uint4(uint32_t(keys[i] >> 32), i, f[0], f[1]);
+}
+__global__ void k_pair_top(const uint4* __restrict__ groups, uint32_t n_groups, uint32_t* __restrict__ top) {
+  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t > kPairTop) return;
+  uint32_t lo = 0, hi = n_groups;
+  if (t == kPairTop) lo = n_groups;
+  else
+    while (lo < hi) {
+      const uint32_t mid = lo + ((hi - lo) >> 1);
+      if (groups[mid].x < (t << (32 - kPairTopBits))) lo = mid + 1;
+      else hi = mid;
+    }
+  top[t] = lo;
 }
 
 // Lanes of the length-2 pass: a (target, kind) lane takes part when the
@@ -2040,118 +2118,180 @@ __global__ void __launch_bounds__(256) k_qc_compact(QCOut o, uint32_t n) {
   }
 }
 
-// Warp per target: (re)fills the slots of each lane whose slots are used up
-// and whose bucket has pairs left.
-__global__ void __launch_bounds__(kBlock) k_pair_scan(DevTargets T, DevPool P, QCOut q1, Lanes L2, PairScan ps,
+// The first position in [lo, hi) that `below` is false at (true, then false,
+// over the range), hi if none.  Warp-wide, the same in every lane: each step
+// probes the ends of 32 spans.
+template <class Below>
+__device__ __forceinline__ uint32_t warp_first(uint32_t lo, uint32_t hi, Below below) {
+  while (lo < hi) {
+    const uint32_t step = (hi - lo + 31u) / 32u;
+    const uint32_t i = lo + lane_id() * step + (step - 1u);
+    const unsigned m = __ballot_sync(kFull, i < hi && below(i));  // spans that lie below as a whole
+    lo += uint32_t(__popc(m)) * step;
+    if (lo >= hi) return hi;
+    hi = min(hi, lo + (step - 1u));
+  }
+  return lo;
+}
+// Ascending over the lanes: a bitonic merge of a bitonic sequence, and a sort.
+__device__ __forceinline__ uint32_t warp_merge(uint32_t x) {
+#pragma unroll
+  for (int o = 16; o; o >>= 1) {
+    const uint32_t y = __shfl_xor_sync(kFull, x, o);
+    x = (lane_id() & unsigned(o)) ? max(x, y) : min(x, y);
+  }
+  return x;
+}
+__device__ __forceinline__ uint32_t warp_sort(uint32_t x) {
+#pragma unroll
+  for (int k = 2; k <= 32; k <<= 1)
+#pragma unroll
+    for (int o = k >> 1; o; o >>= 1) {
+      const uint32_t y = __shfl_xor_sync(kFull, x, o);
+      const bool up = (lane_id() & unsigned(k)) == 0 || k == 32;
+      x = (((lane_id() & unsigned(o)) == 0) == up) ? min(x, y) : max(x, y);
+    }
+  return x;
+}
+
+// Warp per (target, kind) lane whose slots are used up and whose pairs are
+// not: the kSlots2 smallest survivors from ps.resume on.  The lane's target
+// runs on the eight vectors, one per thread; the groups of its hash are read
+// 128 at a time and their F bytes compared under the dead flags; the members
+// of a group that passes are merged, 32 at a time, into the smallest pair
+// indices so far, which the threads hold in order.  Groups whose first
+// member cannot enter are passed over.
+// Bound by latency: a chain of some ten dependent loads per lane, and for
+// targets that leave little to compare (A kept, registers dead) a walk over
+// the groups of one large bucket.  A walk over the bucket's pairs instead
+// (20.5M pairs, one output compared at a time, one warp per target) took
+// 147 ms for 10,007 uneven targets.
+__global__ void __launch_bounds__(kBlock) k_pair_scan(DevTargets T, QCOut q1, Lanes L2, PairScan ps,
                                                       const RoundCtl* __restrict__ gate) {
   if (gate && gate->np != 0) return;  // device-driven rounds: rescan only after an empty round
   const unsigned lane = lane_id();
   const uint32_t gw = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const uint32_t nw = gridDim.x * (blockDim.x >> 5);
-  for (uint32_t t = gw; t < T.n; t += nw) {
-    bool need[2];
-#pragma unroll
-    for (int kind = 0; kind < 2; kind++) {
-      const uint32_t idx = 2 * t + kind;
-      const uint32_t nx = L2.next[idx];
-      need[kind] = !(nx & kResolved) && nx >= ps.cnt[idx] && ps.resume[idx] != kNone;
-    }
-    if (!need[0] && !need[1]) continue;
+  for (uint32_t idx = gw; idx < 2u * T.n; idx += nw) {
+    const uint32_t resume = ps.resume[idx];
+    const uint32_t nx = L2.next[idx];
+    if ((nx & kResolved) || nx < ps.cnt[idx] || resume == kNone) continue;
+    const uint32_t t = idx >> 1, kind = idx & 1u;
     const uint32_t tl = target_len(T, t);
     const uint32_t pw = lane < tl ? T.insn[(size_t)t * T.stride + lane] : 0u;
     Z80S st = vec_state(int(lane & 7u));
     run_lanes(st, pw, 0, int(tl));
-    uint32_t w[3];
+    uint32_t w[3];  // the target's output on vector lane & 7
     z_pack(st, w);
-    uint32_t tw[8][3];
-#pragma unroll
-    for (int v = 0; v < 8; v++) {
-      tw[v][0] = __shfl_sync(kFull, w[0], v);
-      tw[v][1] = __shfl_sync(kFull, w[1], v);
-      tw[v][2] = __shfl_sync(kFull, w[2], v);
-    }
     const uint32_t tb = q1.meta[t].bytes;
-    const uint32_t dead = target_dead(T, t) & 0xFFu;
-    const uint32_t dregs = target_dead_regs(T, t) & 0x3Fu;
-    for (int kind = 0; kind < 2; kind++) {
-      if (!need[kind]) continue;
-      const uint32_t idx = 2 * t + kind;
-      const uint32_t m = kind ? dregs : 0u;
-      // the index holding only pairs that can be shorter than the target
-      const unsigned long long* ix = tb == 3 ? ps.idx_le2[m] : (tb == 4 ? ps.idx_le3[m] : ps.idx[m]);
-      const uint32_t nv = tb == 3 ? ps.n_le2 : (tb == 4 ? ps.n_le3 : ps.n_valid);
-      const uint32_t h = bucket_hash(tw[0][0] & key_keep0(m), tw[0][1] & key_keep1(m), tw[0][2]);
-      uint32_t lo = 0, hi = 0;
-      if (lane == 0) {
-        lo = lower_bound_u64(ix, nv, (unsigned long long)h << 32);
-        hi = (h == 0xFFFFFFFFu) ? nv : lower_bound_u64(ix, nv, (unsigned long long)(h + 1u) << 32);
-      }
-      lo = __shfl_sync(kFull, lo, 0);
-      hi = __shfl_sync(kFull, hi, 0);
-      // compared bytes: kind 0 everything; kind 1 without the dead flags and registers
-      const uint32_t keep0 = kind ? (0xFFu | ((~dead & 0xFFu) << 8) | ((dregs & 1u) ? 0u : 0xFF0000u) |
-                                     ((dregs & 2u) ? 0u : 0xFF000000u))
-                                  : 0xFFFFFFFFu;
-      const uint32_t keep1 = kind ? key_keep1(dregs) : 0xFFFFFFFFu;
-      uint32_t pos = lo + ps.resume[idx];
-      uint32_t found = 0;
-      bool capped = false;
-      while (pos < hi && !capped) {
-        const uint32_t j = pos + lane;
-        bool pass = false;
-        uint32_t c = 0, diff = 0;
-        if (j < hi) {
-          c = uint32_t(ix[j]);
-          if (P.size[c] < tb) {
-            const uint4 o = P.qc[c];
-            const uint32_t d0 = o.x ^ tw[0][0], d1 = o.y ^ tw[0][1], d2 = o.z ^ tw[0][2];
-            if (((d0 & keep0) | (d1 & keep1) | d2) == 0) {
-              bool full = (d0 | d1 | d2) == 0;
-              uint32_t fd = (d0 >> 8) & 0xFFu, rdf = reg_diff(d0, d1);
-              bool ok = true;
+    const uint32_t dead = kind ? target_dead(T, t) & 0xFFu : 0u;
+    const uint32_t dregs = kind ? target_dead_regs(T, t) & 0x3Fu : 0u;
+    const uint32_t k0 = key_keep0(dregs), k1 = key_keep1(dregs);
+    const uint32_t keepf = (~dead & 0xFFu) * 0x01010101u;
+    const uint32_t keep0 = k0 | ((~dead & 0xFFu) << 8);
+    unsigned long long h = vector_hash(w[0] & k0, w[1] & k1, w[2], lane & 7u);
+    uint32_t flo = 0, fhi = 0;
+    {
+      const uint32_t f = (w[0] >> 8) & 0xFFu, v = lane & 7u;
+      if (v < 4) flo = f << (8 * v);
+      else fhi = f << (8 * (v - 4));
+    }
 #pragma unroll
-              for (int v = 1; v < 8; v++) {
-                const uint4 ov = P.qc[(size_t)v * P.n + c];
-                const uint32_t e0 = ov.x ^ tw[v][0], e1 = ov.y ^ tw[v][1], e2 = ov.z ^ tw[v][2];
-                ok = ok && (((e0 & keep0) | (e1 & keep1) | e2) == 0);
-                full = full && ((e0 | e1 | e2) == 0);
-                fd |= (e0 >> 8) & 0xFFu;
-                rdf |= reg_diff(e0, e1);
+    for (int o = 4; o; o >>= 1) {
+      h += __shfl_xor_sync(kFull, h, o);
+      flo |= __shfl_xor_sync(kFull, flo, o);
+      fhi |= __shfl_xor_sync(kFull, fhi, o);
+    }
+    const PairIndex ix = ps.idx[dregs];
+    uint32_t best = kNone, worst = kNone;  // this thread's survivor; the last thread's
+    for (uint32_t size = 2; size < min(tb, 2u + kPairSizes); size++) {
+      const uint32_t key = pair_group_key(size, h);
+      const uint32_t* top = ix.top + (key >> (32 - kPairTopBits));
+      const uint32_t hi = top[1];
+      const uint32_t g0 = warp_first(top[0], hi, [&](uint32_t i) { return ix.groups[i].x < key; });
+      for (uint32_t base = g0; base < hi; base += 128) {
+        uint4 r[4];
+        bool in[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+          const uint32_t i = base + 32u * u + lane;
+          in[u] = i < hi;
+          r[u] = in[u] ? ix.groups[i] : make_uint4(0u, 0u, 0u, 0u);
+        }
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+          in[u] = in[u] && r[u].x == key;
+          const bool fm = in[u] && (((r[u].z ^ flo) | (r[u].w ^ fhi)) & keepf) == 0;
+          if (!__any_sync(kFull, fm)) continue;
+          const uint32_t first = fm ? ix.members[r[u].y] : kNone;
+          for (unsigned b = __ballot_sync(kFull, first < worst); b; b &= b - 1) {
+            const int j = __ffs(b) - 1;
+            const uint32_t c0 = __shfl_sync(kFull, first, j);
+            if (c0 >= worst) continue;
+            // the group's outputs themselves, on the first member
+            uint32_t d = 0;
+            if (lane < 8) {
+              const uint4 o = ps.out[(size_t)c0 * 8 + lane];
+              d = ((o.x ^ w[0]) & keep0) | ((o.y ^ w[1]) & k1) | (o.z ^ w[2]);
+            }
+            if (__any_sync(kFull, d != 0)) continue;
+            uint32_t pos = __shfl_sync(kFull, r[u].y, j);
+            const uint32_t end = ix.groups[base + 32u * u + j + 1].y;
+            // only members that agree on every flag can agree on everything
+            // (masked lanes leave those to the full lane)
+            const bool maybe_full =
+                kind && __shfl_sync(kFull, r[u].z, j) == flo && __shfl_sync(kFull, r[u].w, j) == fhi;
+            if (c0 < resume)
+              pos = warp_first(pos, end, [&](uint32_t i) { return ix.members[i] < resume; });
+            while (pos < end) {
+              uint32_t c = pos + lane < end ? ix.members[pos + lane] : kNone;
+              if (__shfl_sync(kFull, c, 0) >= worst) break;
+              if (maybe_full) {
+                uint32_t fd = 0;
+                for (int v = 0; v < 8; v++) {
+                  const uint32_t x = __shfl_sync(kFull, w[0], v), y = __shfl_sync(kFull, w[1], v);
+                  const uint32_t z = __shfl_sync(kFull, w[2], v);
+                  if (c != kNone) {
+                    const uint4 o = ps.out[(size_t)c * 8 + v];
+                    fd |= (o.x ^ x) | (o.y ^ y) | (o.z ^ z);
+                  }
+                }
+                if (fd == 0) c = kNone;
+                c = warp_sort(c);
               }
-              pass = ok && (kind ? !full : full);
-              diff = fd | (rdf << 8);
+              best = warp_merge(min(best, __shfl_sync(kFull, c, 31 - int(lane))));
+              worst = __shfl_sync(kFull, best, 31);
+              pos += 32;
             }
           }
         }
-        const unsigned b = __ballot_sync(kFull, pass);
-        const uint32_t room = kSlots2 - found;
-        const uint32_t r = __popc(b & lanemask_lt());
-        if (pass && r < room) {
-          ps.surv[(size_t)idx * kSlots2 + found + r] = c;
-          ps.sdiff[(size_t)idx * kSlots2 + found + r] = uint16_t(diff);
-        }
-        const uint32_t nb = __popc(b);
-        if (nb > room) {
-          // resume after the last survivor that fit
-          uint32_t bb = b;
-          for (uint32_t k = 0; k < room; k++) bb &= bb - 1;
-          pos += uint32_t(__ffs(bb)) - 1u;
-          found = kSlots2;
-          capped = true;
-        } else {
-          found += nb;
-          pos += 32;
-          capped = found == kSlots2;
-        }
+        if (!__all_sync(kFull, in[3])) break;
       }
-      if (lane == 0) {
-        ps.cnt[idx] = found;
-        L2.next[idx] = 0;
-        ps.resume[idx] = pos >= hi ? kNone : pos - lo;
+    }
+    // slots, and the outputs in which each survivor differs
+    uint32_t fd = 0, rdf = 0;
+#pragma unroll
+    for (int v = 0; v < 8; v++) {
+      const uint32_t x = __shfl_sync(kFull, w[0], v), y = __shfl_sync(kFull, w[1], v);
+      if (best != kNone) {
+        const uint4 o = ps.out[(size_t)best * 8 + v];
+        fd |= ((o.x ^ x) >> 8) & 0xFFu;
+        rdf |= reg_diff(o.x ^ x, o.y ^ y);
       }
+    }
+    if (best != kNone) {
+      ps.surv[(size_t)idx * kSlots2 + lane] = best;
+      ps.sdiff[(size_t)idx * kSlots2 + lane] = uint16_t(fd | (rdf << 8));
+    }
+    const uint32_t found = __popc(__ballot_sync(kFull, best != kNone));
+    if (lane == 0) {
+      ps.cnt[idx] = found;
+      L2.next[idx] = 0;
+      ps.resume[idx] = worst == kNone ? kNone : worst + 1u;
     }
   }
 }
+static_assert(kSlots2 == 32, "one slot per thread of the warp");
 
 // One pair per length-2 lane with an untried survivor; lanes with no slot
 // left either end without a winner (bucket exhausted) or wait for a rescan.
@@ -2259,11 +2399,11 @@ void dev_upload_tables(cudaStream_t s) {
   }
 }
 
-void launch_pool_outputs(const uint32_t* insn, uint32_t n, uint32_t len, uint4* qc, uint4* mid,
+void launch_pool_outputs(const uint32_t* insn, uint32_t n, uint32_t len, uint4* qc, uint4* mid, bool by_pair,
                          cudaStream_t s) {
   if (!n) return;
   unsigned grid = std::min<unsigned>(grid_for(n, 4), unsigned(dev_num_sms() * 16));
-  k_pool_outputs<<<grid, 128, 0, s>>>(insn, n, len, qc, mid);
+  k_pool_outputs<<<grid, 128, 0, s>>>(insn, n, len, qc, mid, by_pair);
 }
 void launch_exec(const uint32_t* in, const uint32_t* seqs, const uint8_t* lens, uint32_t len,
                  uint32_t stride, uint32_t n, uint32_t* out, cudaStream_t s) {
@@ -2672,26 +2812,38 @@ void launch_verify_small(const uint32_t* tgt, const uint8_t* tlens, const uint32
   k_verify_small<<<grid, 256, 0, s>>>(tgt, tlens, cand, clens, stride, n, dead, tiers, out, flagdiff);
 }
 
-void launch_pair_keys(const DevPool& P, uint32_t dregs, unsigned long long* keys, cudaStream_t s) {
-  if (!P.n) return;
-  k_pair_keys<<<grid_for(P.n, 256), 256, 0, s>>>(P, dregs, keys);
+void launch_pair_keys(const DevPool& P, const uint4* out, const uint32_t* valid, uint32_t n, uint32_t dregs,
+                      unsigned long long* keys, cudaStream_t s) {
+  if (n) k_pair_keys<<<grid_for(n, 256), 256, 0, s>>>(P, out, valid, n, dregs, keys);
+}
+void launch_pair_heads(const uint4* out, const unsigned long long* keys, const uint32_t* members, uint32_t n,
+                       uint32_t dregs, uint32_t* head, cudaStream_t s) {
+  if (n) k_pair_heads<<<grid_for(n, 256), 256, 0, s>>>(out, keys, members, n, dregs, head);
+}
+void launch_pair_groups(const uint4* out, const unsigned long long* keys, const uint32_t* members, uint32_t n,
+                        const uint32_t* gid, uint4* groups, cudaStream_t s) {
+  if (n) k_pair_groups<<<grid_for(n, 256), 256, 0, s>>>(out, keys, members, n, gid, groups);
+}
+void launch_pair_top(const uint4* groups, uint32_t n_groups, uint32_t* top, cudaStream_t s) {
+  k_pair_top<<<grid_for(kPairTop + 1, 256), 256, 0, s>>>(groups, n_groups, top);
 }
 void launch_pair_lanes_init(const DevTargets& T, const Lanes& L1, const QCOut& q1, const Lanes& L2,
                             const PairScan& ps, cudaStream_t s) {
   if (!T.n) return;
   k_pair_lanes_init<<<grid_for(T.n, 256), 256, 0, s>>>(T, L1, q1, L2, ps);
 }
-void launch_pair_scan(const DevTargets& T, const DevPool& P, const QCOut& q1, const Lanes& L2, const PairScan& ps,
-                      cudaStream_t s) {
+// A warp per lane and no more blocks than that needs; the blocks of a large
+// job retire as their lanes are done, which evens out the few long walks.
+void launch_pair_scan(const DevTargets& T, const QCOut& q1, const Lanes& L2, const PairScan& ps, cudaStream_t s) {
   if (!T.n) return;
-  unsigned grid = std::min<unsigned>(grid_for(T.n, kBlock / 32), unsigned(dev_num_sms() * 8));
-  k_pair_scan<<<grid, kBlock, 0, s>>>(T, P, q1, L2, ps, nullptr);
+  k_pair_scan<<<grid_for(T.n, kBlock / 64), kBlock, 0, s>>>(T, q1, L2, ps, nullptr);
 }
-void launch_pair_scan_gated(const DevTargets& T, const DevPool& P, const QCOut& q1, const Lanes& L2,
-                            const PairScan& ps, const RoundCtl* ctl, cudaStream_t s) {
+// Inside a round graph most launches find nothing to do: a resident grid.
+void launch_pair_scan_gated(const DevTargets& T, const QCOut& q1, const Lanes& L2, const PairScan& ps,
+                            const RoundCtl* ctl, cudaStream_t s) {
   if (!T.n) return;
-  unsigned grid = std::min<unsigned>(grid_for(T.n, kBlock / 32), unsigned(dev_num_sms() * 8));
-  k_pair_scan<<<grid, kBlock, 0, s>>>(T, P, q1, L2, ps, ctl);
+  unsigned grid = std::min<unsigned>(grid_for(T.n, kBlock / 64), unsigned(dev_num_sms() * 8));
+  k_pair_scan<<<grid, kBlock, 0, s>>>(T, q1, L2, ps, ctl);
 }
 void launch_pair_round_build(const DevTargets& T, const DevPool& P, const QCOut& q1, const Lanes& L2,
                              const PairScan& ps, const RoundBuf& R, cudaStream_t s) {

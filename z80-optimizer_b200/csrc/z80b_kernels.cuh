@@ -108,19 +108,28 @@ struct RoundBuf {
                                    // (bit-sliced kernel), else (0 too) the scalar kernel's 128
 };
 
-// Length-2 candidate pass (pair pool): bucket indexes and per-lane slots.
+// Length-2 candidate pass (pair pool): indexes and per-lane slots.
 constexpr uint32_t kSlots2 = 32;  // survivors held per (target, kind) lane
+// Index of the unpruned pairs for one dead-register mask.  The pairs are
+// sorted by (encoded size, hash of A, SP, M and the live registers after all
+// eight QuickCheck vectors, hash of the eight F bytes) and cut into groups
+// of pairs that agree on all of these outputs themselves, not only on the
+// hashes: one comparison with a group's first pair answers the QuickCheck
+// for every member under any dead-flag mask.
+struct PairIndex {
+  const uint32_t* members;  // pair indices, ascending within a group
+  const uint4* groups;      // {pair_group_key, first member's position, F bytes 0-3, F bytes 4-7},
+                            // sorted by key; one more entry ends the last group
+  const uint32_t* top;      // [kPairTop + 1] first group of each range of the key's top bits
+};
+constexpr uint32_t kPairTopBits = 18, kPairTop = 1u << kPairTopBits;
+// Group key: the size class (pairs take 2, 3 or 4 bytes) and 30 hash bits.
+constexpr uint32_t kPairSizes = 3;
 struct PairScan {
-  const unsigned long long* const* idx;  // [64] sorted bucket keys per dead-register mask
-  uint32_t n_valid;                      // entries of each index (the unpruned pairs)
-  // The same indexes over the unpruned pairs of at most 2 and at most 3
-  // bytes ([64] each, in the same order): a target of 3 or 4 bytes can only
-  // take those, and its bucket in the full index is nearly all longer pairs.
-  const unsigned long long* const* idx_le2;
-  const unsigned long long* const* idx_le3;
-  uint32_t n_le2, n_le3;
+  const PairIndex* idx;                  // [64] per dead-register mask (those in use)
+  const uint4* out;                      // [pairs * 8] outputs on the vectors, 128 bytes per pair
   uint32_t* cnt;                         // [2n] survivors in the lane's slots
-  uint32_t* resume;                      // [2n] bucket offset to rescan from; kNone: exhausted
+  uint32_t* resume;                      // [2n] pair index to go on from; kNone: exhausted
   uint32_t* surv;                        // [2n * kSlots2] pair-pool indices
   uint16_t* sdiff;                       // [2n * kSlots2]
   uint32_t* refill;                      // lanes waiting for a rescan (round build)
@@ -143,7 +152,9 @@ void launch_qc_compact(const QCOut& q, uint32_t n, cudaStream_t s);
 void dev_upload_tables(cudaStream_t s);
 int dev_num_sms();
 
-void launch_pool_outputs(const uint32_t* insn, uint32_t n, uint32_t len, uint4* qc, uint4* mid,
+// by_pair: the eight QuickCheck outputs of a candidate side by side (qc[c * 8
+// + v]) instead of vector-major (qc[v * n + c]).
+void launch_pool_outputs(const uint32_t* insn, uint32_t n, uint32_t len, uint4* qc, uint4* mid, bool by_pair,
                          cudaStream_t s);
 void launch_exec(const uint32_t* in_states, const uint32_t* seqs, const uint8_t* lens, uint32_t len,
                  uint32_t stride, uint32_t n, uint32_t* out_states, cudaStream_t s);
@@ -215,8 +226,8 @@ void launch_round_resolve_dev(const RoundBuf& R, const RoundCtl* ctl, const QCOu
                               uint32_t max_spec, cudaStream_t s);
 // k_pair_scan that does its work only when the current round is empty (the
 // rescan step of the length-2 pass).
-void launch_pair_scan_gated(const DevTargets& T, const DevPool& P, const QCOut& q1, const Lanes& L2,
-                            const PairScan& ps, const RoundCtl* ctl, cudaStream_t s);
+void launch_pair_scan_gated(const DevTargets& T, const QCOut& q1, const Lanes& L2, const PairScan& ps,
+                            const RoundCtl* ctl, cudaStream_t s);
 void launch_midcheck(const DevTargets& T, const DevPool& P, const uint32_t* surv,
                      const uint32_t* surv_target, uint32_t nsurv, uint8_t* pass, cudaStream_t s);
 void launch_surv_targets(const QCOut& q, uint32_t n, uint32_t* surv_target, cudaStream_t s);
@@ -231,11 +242,20 @@ void launch_rule_write_all(const uint32_t* flag, const uint32_t* base, uint32_t 
                            const uint32_t* surv, const uint16_t* sdiff, const uint32_t* surv_target,
                            DevRule* out, cudaStream_t s);
 void launch_rule_count_all(const RoundBuf& R, uint32_t npairs, uint32_t* flag, cudaStream_t s);
-void launch_pair_keys(const DevPool& P, uint32_t dregs, unsigned long long* keys, cudaStream_t s);
+// The steps of a pair index (PairIndex) over the n unpruned pairs `valid`:
+// their sort keys for a dead-register mask; after the sort, which positions
+// begin a group (flag 1); after the flags' inclusive sum, the group records;
+// and the top table.
+void launch_pair_keys(const DevPool& P, const uint4* out, const uint32_t* valid, uint32_t n, uint32_t dregs,
+                      unsigned long long* keys, cudaStream_t s);
+void launch_pair_heads(const uint4* out, const unsigned long long* keys, const uint32_t* members, uint32_t n,
+                       uint32_t dregs, uint32_t* head, cudaStream_t s);
+void launch_pair_groups(const uint4* out, const unsigned long long* keys, const uint32_t* members, uint32_t n,
+                        const uint32_t* gid, uint4* groups, cudaStream_t s);
+void launch_pair_top(const uint4* groups, uint32_t n_groups, uint32_t* top, cudaStream_t s);
 void launch_pair_lanes_init(const DevTargets& T, const Lanes& L1, const QCOut& q1, const Lanes& L2,
                             const PairScan& ps, cudaStream_t s);
-void launch_pair_scan(const DevTargets& T, const DevPool& P, const QCOut& q1, const Lanes& L2, const PairScan& ps,
-                      cudaStream_t s);
+void launch_pair_scan(const DevTargets& T, const QCOut& q1, const Lanes& L2, const PairScan& ps, cudaStream_t s);
 void launch_pair_round_build(const DevTargets& T, const DevPool& P, const QCOut& q1, const Lanes& L2,
                              const PairScan& ps, const RoundBuf& R, cudaStream_t s);
 void launch_verify_small(const uint32_t* tgt, const uint8_t* tlens, const uint32_t* cand,
