@@ -532,55 +532,6 @@ __device__ __forceinline__ void put_window(const RoundBuf& R, uint32_t p0, uint3
   }
 }
 
-// Plans the round's pairs (z80_plan.cuh), one thread each: compared outputs,
-// swept fields, class and chunks.  A pair that its programs prove equivalent
-// gets no chunk and keeps its zero flag; the pairs after it in its window
-// cannot win and are cancelled.  Bound by latency (table loads and local
-// arrays; a few microseconds a pair, thousands of pairs side by side): with
-// the plans made in the round build, windows in one thread, 100,003 masked
-// targets spent 3.4 ms in their 11 rounds, here 0.9 ms.
-__global__ void __launch_bounds__(128) k_pair_plan(DevTargets T, DevPool P, QCOut q, RoundBuf R) {
-  const uint32_t np = min(*R.npairs, R.cap);
-  unsigned long long proven_states = 0;
-  for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < np; p += gridDim.x * blockDim.x) {
-    PairRec pr = R.pairs[p];
-    const uint32_t t = pr.target, c = pr.cand;
-    const bool masked = (pr.keepR & 0x80u) != 0;
-    const uint32_t reads = q.meta[t].reads | P.reads[c];
-    pr.keepF = masked ? uint8_t(~target_dead(T, t)) : uint8_t(0xFFu);
-    pr.keepR = masked ? uint8_t((~target_dead_regs(T, t) & 0x3Fu) | 0x80u) : uint8_t(0x3Fu);
-    const PairPlan pl = plan_pair(g_flow, T.insn + (size_t)t * T.stride, target_len(T, t),
-                                  P.insn + (size_t)c * P.stride, pool_len(P, c), reads, pr.keepF, pr.keepR);
-    pr.reads = pl.reads;
-    pr.sweepf = pl.sweepf;
-    pr.nblocks = pl.nblocks;
-    pr.cmap = 0;
-    if (pl.proven) {
-      pr.nblocks = 0;  // no chunk in any class
-      proven_states += 256ull * plan_blocks(reads, false);
-      if (R.wend)
-        for (uint32_t i = p + 1; i < R.wend[p]; i++) R.rejected[i] = 2;
-    } else {
-      if (pl.a_free || pair_xindep(T, t, P, c)) pr.keepR |= uint8_t(kXIndep);
-      // compact classes: A-dependent pairs, and A-independent ones when those
-      // are swept bit-sliced (units of kXBitsBlocks); the narrow state first
-      if (!(pr.keepR & kXIndep) || R.xunit == kXBitsBlocks) {
-        if (R.compact) pr.cmap = pair_cmap(T, t, P, c);
-        // the wide state: A-dependent pairs only
-        if (!pr.cmap && R.wide && !(pr.keepR & kXIndep)) pr.cmap = pair_wmap(T, t, P, c);
-        // the register state: the rest that name neither SP nor the memory byte
-        if (!pr.cmap && R.wide && pair_regstate(T, t, P, c)) pr.cmap = kRegClass;
-      }
-    }
-    R.pairs[p] = pr;
-    set_chunks(R, p, pr);
-  }
-  __syncwarp();
-#pragma unroll
-  for (int o = 16; o; o >>= 1) proven_states += __shfl_xor_sync(kFull, proven_states, o);
-  if (lane_id() == 0 && proven_states) atomicAdd(R.states, proven_states);
-}
-
 // Lane 0, after a warp's chunk of pair p ran to its end without a mismatch:
 // counts the chunk; the warp that counts the last one of a pair that still
 // stands (its whole sweep passed) cancels the pairs after it in its survivor
@@ -754,6 +705,140 @@ __device__ __forceinline__ bool run_compare(const Init& init, const bool (&valid
     bad = bad || (valid[q] && ((d0 & keep0) | (d1 & keep1) | d2) != 0);
   }
   return bad;
+}
+
+// Runs both programs of a pair on 512 states of its sweep -- every value of A
+// twice, each with a block of its own spread over the sweep -- and tells
+// whether one of them differs.  Warp-wide, the same pair in every lane.
+__device__ __forceinline__ bool probe_pair(const DevTargets& T, const DevPool& P, uint32_t target, uint32_t cand,
+                                           unsigned long long nblocks, uint32_t reads, uint32_t sweepf, uint32_t keepF,
+                                           uint32_t keepR) {
+  const unsigned lane = lane_id();
+  const uint32_t tl = target_len(T, target), cl = pool_len(P, cand);
+  uint32_t pw = 0;
+  if (lane < tl) pw = T.insn[(size_t)target * T.stride + lane];
+  else if (lane < tl + cl) pw = P.insn[(size_t)cand * P.stride + (lane - tl)];
+  const uint32_t ext = reads & (kRegB | kRegC | kRegD | kRegE | kRegH | kRegL | kRegM);
+  const bool spw = (reads & kRegSP) != 0;
+  const int nx = __popc(ext);
+  const bool reduced = spw || nx > 2 || (sweepf & 0x80u) != 0;
+  int slot[7];
+  {
+    int k = 0;
+    const uint32_t bits[7] = {kRegB, kRegC, kRegD, kRegE, kRegH, kRegL, kRegM};
+#pragma unroll
+    for (int r = 0; r < 7; r++) slot[r] = (ext & bits[r]) ? k++ : -1;
+  }
+  const BDec bd = bdec_make(spw, reduced, nx, reduced ? 5 : 8, slot);
+  const uint32_t keep0 = 0xFFu | (keepF << 8) | ((keepR & 1u) ? 0xFF0000u : 0u) | ((keepR & 2u) ? 0xFF000000u : 0u);
+  const uint32_t keep1 = ((keepR & 4u) ? 0xFFu : 0u) | ((keepR & 8u) ? 0xFF00u : 0u) |
+                         ((keepR & 16u) ? 0xFF0000u : 0u) | ((keepR & 32u) ? 0xFF000000u : 0u);
+  bool bad = false;
+#pragma unroll 1
+  for (uint32_t i = 0; i < 4u && !__any_sync(kFull, bad); i++) {
+    uint32_t W[4][3];
+    const bool valid[4] = {true, true, true, true};
+#pragma unroll
+    for (uint32_t q = 0; q < 4; q++) {
+      const uint32_t n = (i * 4u + q) * 32u + lane;  // 0..511
+      unsigned long long h = (n + 1ull) * 0x9E3779B97F4A7C15ull;
+      h ^= h >> 29;
+      h *= 0xBF58476D1CE4E5B9ull;
+      h ^= h >> 32;
+      Z80S x = bdec_state(bd, h & (nblocks - 1ull), g_rep, g_repsp);  // nblocks is a power of two
+      x.a = (n * 37u) & 0xFFu;
+      z_pack(x, W[q]);
+    }
+    auto init = [&](int q, Z80S& x) { x = z_unpack(W[q][0], W[q][1], W[q][2]); };
+    bad = run_compare<4>(init, valid, pw, int(tl), int(cl), keep0, keep1);
+  }
+  return __any_sync(kFull, bad);
+}
+
+// Plans the round's pairs (z80_plan.cuh), one lane each: compared outputs,
+// swept fields, class and chunks.  A pair that its programs prove equivalent
+// gets no chunk and keeps its zero flag; the pairs after it in its window
+// cannot win and are cancelled.  A pair whose sweep takes more than one chunk
+// is probed first by the whole warp: nearly all long sweeps belong to pairs
+// that passed the eight QuickCheck vectors and are no equivalences, and such
+// a sweep draws every resident warp into one pair before its first mismatch
+// is seen, one pair after the other.
+// Bound by latency (table loads and local arrays, a few microseconds a pair,
+// thousands of pairs side by side; a small round spreads its pairs over the
+// warps).  Planned in the round build, a window's up to 64 pairs in one
+// thread, 100,003 masked targets spent 3.4 ms in their 11 rounds, here
+// 0.9 ms.  The probe and the polls between units: 40,009 uneven targets
+// evaluate 4.5e8 states where it was 1.6e10 (84 -> 43 ms of sweeps), the
+// 9.4M length-2 targets 2.7e8 where it was 1.3e9 (3.2 -> 2.05 ms).
+__global__ void __launch_bounds__(128) k_pair_plan(DevTargets T, DevPool P, QCOut q, RoundBuf R) {
+  const uint32_t np = min(*R.npairs, R.cap);
+  const unsigned lane = lane_id();
+  const uint32_t nw = gridDim.x * (blockDim.x >> 5);
+  const uint32_t gw = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const uint32_t per = min(32u, (np + nw - 1u) / nw);
+  unsigned long long covered = 0;  // reference states that proofs and probes answer for
+  uint32_t probes = 0;
+  for (uint32_t base = gw * per; base < np; base += nw * per) {
+    const uint32_t p = base + lane;
+    const bool mine = lane < per && p < np;
+    PairRec pr{};
+    bool large = false;
+    if (mine) {
+      pr = R.pairs[p];
+      const uint32_t t = pr.target, c = pr.cand;
+      const bool masked = (pr.keepR & 0x80u) != 0;
+      const uint32_t reads = q.meta[t].reads | P.reads[c];
+      pr.keepF = masked ? uint8_t(~target_dead(T, t)) : uint8_t(0xFFu);
+      pr.keepR = masked ? uint8_t((~target_dead_regs(T, t) & 0x3Fu) | 0x80u) : uint8_t(0x3Fu);
+      const PairPlan pl = plan_pair(g_flow, T.insn + (size_t)t * T.stride, target_len(T, t),
+                                    P.insn + (size_t)c * P.stride, pool_len(P, c), reads, pr.keepF, pr.keepR);
+      pr.reads = pl.reads;
+      pr.sweepf = pl.sweepf;
+      pr.nblocks = pl.nblocks;
+      pr.cmap = 0;
+      if (pl.proven) {
+        pr.nblocks = 0;  // no chunk in any class
+        covered += 256ull * plan_blocks(reads, false);
+        if (R.wend)
+          for (uint32_t i = p + 1; i < R.wend[p]; i++) R.rejected[i] = 2;
+      } else {
+        if (pl.a_free || pair_xindep(T, t, P, c)) pr.keepR |= uint8_t(kXIndep);
+        // compact classes: A-dependent pairs, and A-independent ones when
+        // those are swept bit-sliced (units of kXBitsBlocks); the narrow
+        // state first
+        if (!(pr.keepR & kXIndep) || R.xunit == kXBitsBlocks) {
+          if (R.compact) pr.cmap = pair_cmap(T, t, P, c);
+          // the wide state: A-dependent pairs only
+          if (!pr.cmap && R.wide && !(pr.keepR & kXIndep)) pr.cmap = pair_wmap(T, t, P, c);
+          // the register state: the rest that name neither SP nor the memory byte
+          if (!pr.cmap && R.wide && pair_regstate(T, t, P, c)) pr.cmap = kRegClass;
+        }
+        large = pair_units(pr.nblocks, pr.keepR, R.xunit) > R.chunk_blocks;
+      }
+    }
+    for (unsigned b = __ballot_sync(kFull, large); b; b &= b - 1) {
+      const int j = __ffs(b) - 1;
+      const uint32_t masks = __shfl_sync(kFull, uint32_t(pr.keepF) | uint32_t(pr.keepR) << 8 | uint32_t(pr.sweepf) << 16, j);
+      const bool bad = probe_pair(T, P, __shfl_sync(kFull, pr.target, j), __shfl_sync(kFull, pr.cand, j),
+                                  __shfl_sync(kFull, pr.nblocks, j), __shfl_sync(kFull, uint32_t(pr.reads), j),
+                                  masks >> 16, masks & 0xFFu, (masks >> 8) & 0xFFu);
+      probes++;
+      if (bad && int(lane) == j) {
+        pr.nblocks = 0;
+        R.rejected[p] = 1;
+      }
+    }
+    if (mine) {
+      R.pairs[p] = pr;
+      set_chunks(R, p, pr);
+    }
+  }
+#pragma unroll
+  for (int o = 16; o; o >>= 1) covered += __shfl_xor_sync(kFull, covered, o);
+  if (lane == 0 && (covered || probes)) {
+    atomicAdd(R.states, covered + 512ull * probes);
+    if (probes) atomicAdd(R.states + 1, 512ull * probes);
+  }
 }
 
 // Planes of the 32 states A = a0 .. a0+31 (a0 a multiple of 32) with the
@@ -1366,6 +1451,7 @@ __global__ void __launch_bounds__(kBlock, CLS == 3 ? 3 : (CLS == 4 ? 2 : (CLS ==
   constexpr bool XI = CLS != 0;
   const unsigned long long* __restrict__ cbase =
       CLS == 5 ? R.cbase_r : (CLS == 4 ? R.cbase_w : (CLS == 3 ? R.cbase_c : (XI ? R.cbase_x : R.cbase)));
+  unsigned long long* const dispenser = R.counter + (CLS >= 3 ? CLS - 1 : (XI ? 1 : 0));
   const unsigned lane = lane_id();
   unsigned long long my_states = 0, my_eval = 0;
   // At most kChunksPerWarp chunks per warp, then the block retires: the grid
@@ -1373,15 +1459,22 @@ __global__ void __launch_bounds__(kBlock, CLS == 3 ? 3 : (CLS == 4 ? 2 : (CLS ==
   // priority) get SMs as soon as blocks of a long sweep retire.
   for (int taken = 0; taken < chunks_per_warp; taken++) {
     unsigned long long k = 0;
-    if (lane == 0) k = atomicAdd(R.counter + (CLS >= 3 ? CLS - 1 : (XI ? 1 : 0)), 1ull);
+    if (lane == 0) k = atomicAdd(dispenser, 1ull);
     k = __shfl_sync(kFull, k, 0);
     if (k >= total) break;
     // pair p: cbase[p] <= k < cbase[p + 1]
     const uint32_t p = chunk_pair(cbase, npairs, k, lane);
     // lane 0 reads the flag and the warp acts on one value, so the
     // shuffles below always see all 32 lanes
-    if (__shfl_sync(kFull, lane == 0 ? *reinterpret_cast<volatile uint32_t*>(&R.rejected[p]) : 0u, 0))
+    if (__shfl_sync(kFull, lane == 0 ? *reinterpret_cast<volatile uint32_t*>(&R.rejected[p]) : 0u, 0)) {
+      // The pair is settled: the dispenser jumps over what is left of its
+      // chunks.  A pair of 2^20 chunks that fails in its first ones had them
+      // all drawn one by one (1 ns each: 2 ms a round for two such pairs;
+      // 40,009 uneven targets, 243 rounds: 196 ms of sweeps, with the jump
+      // 84 ms).
+      if (lane == 0) atomicMax(dispenser, p + 1 < npairs ? cbase[p + 1] : total);
       continue;
+    }
     const PairRec pr = R.pairs[p];
     const unsigned long long nunits = pair_units(pr.nblocks, pr.keepR, R.xunit);
     const unsigned long long nch = (p + 1 < npairs ? cbase[p + 1] : total) - cbase[p];
@@ -1419,6 +1512,10 @@ __global__ void __launch_bounds__(kBlock, CLS == 3 ? 3 : (CLS == 4 ? 2 : (CLS ==
                            ((pr.keepR & 16u) ? 0xFF0000u : 0u) | ((pr.keepR & 32u) ? 0xFF000000u : 0u);
 
     bool bad = false;
+    // The pair's flag, asked for before a unit and looked at after it, so
+    // that the read's latency passes behind the unit: a rejected pair costs
+    // each warp one unit, not a batch of them between two polls.
+    auto poll = [&]() { return lane == 0 ? *reinterpret_cast<volatile uint32_t*>(&R.rejected[p]) : 0u; };
     bool stopped = false;  // left the loop on the pair's flag (rejected or cancelled elsewhere)
     if constexpr (CLS == 5) {
       // the register state (A, F, B..L), programs as they are
@@ -1430,6 +1527,7 @@ __global__ void __launch_bounds__(kBlock, CLS == 3 ? 3 : (CLS == 4 ? 2 : (CLS ==
         for (int r = 0; r < 6; r++)
           if (slot[r] == nx - 1) rlast = r;
         for (unsigned long long u = u0; u < u1; u++) {
+          const uint32_t settled = poll();
           const unsigned long long first = u * kXBitsBlocks;
           const unsigned long long nb = (pr.nblocks - first < kXBitsBlocks) ? pr.nblocks - first : kXBitsBlocks;
           bad = rxbits_unit(u, pr.nblocks, reduced, nx, rlast, bd, pw, int(tl), int(cl), pr.keepF, pr.keepR, sm) ||
@@ -1437,21 +1535,21 @@ __global__ void __launch_bounds__(kBlock, CLS == 3 ? 3 : (CLS == 4 ? 2 : (CLS ==
           my_states += (256ull * nb) << xs;
           my_eval += 2ull * nb;
           if (__any_sync(kFull, bad)) break;
-          if (__shfl_sync(kFull, lane == 0 ? *reinterpret_cast<volatile uint32_t*>(&R.rejected[p]) : 0u, 0)) {
+          if (__shfl_sync(kFull, settled, 0)) {
             stopped = true;
             break;
           }
         }
       } else {
         for (unsigned long long u = u0; u < u1; u++) {
+          const uint32_t settled = poll();
           const unsigned long long first = u * kBitsBlocks;
           const unsigned long long nb = (pr.nblocks - first < kBitsBlocks) ? pr.nblocks - first : kBitsBlocks;
           bad = rbits_unit(u, pr.nblocks, bd, pw, int(tl), int(cl), pr.keepF, pr.keepR, sm) || bad;
           my_states += (256ull * nb) << xs;
           my_eval += 256ull * nb;
           if (__any_sync(kFull, bad)) break;
-          if ((u & 15ull) == 15ull &&
-              __shfl_sync(kFull, lane == 0 ? *reinterpret_cast<volatile uint32_t*>(&R.rejected[p]) : 0u, 0)) {
+          if (__shfl_sync(kFull, settled, 0)) {
             stopped = true;
             break;
           }
@@ -1472,14 +1570,14 @@ __global__ void __launch_bounds__(kBlock, CLS == 3 ? 3 : (CLS == 4 ? 2 : (CLS ==
       uint32_t* sm = zsm + (threadIdx.x >> 5) * (kWideWords * 32) + lane;
       const WDec dec = wdec_make(nx, reduced, slot, o);
       for (unsigned long long u = u0; u < u1; u++) {
+        const uint32_t settled = poll();
         const unsigned long long first = u * kBitsBlocks;
         const unsigned long long nb = (pr.nblocks - first < kBitsBlocks) ? pr.nblocks - first : kBitsBlocks;
         bad = wbits_unit(u, pr.nblocks, dec, pw, int(tl), int(cl), pr.keepF, cmp, sm) || bad;
         my_states += (256ull * nb) << xs;
         my_eval += 256ull * nb;
         if (__any_sync(kFull, bad)) break;
-        if ((u & 15ull) == 15ull &&
-            __shfl_sync(kFull, lane == 0 ? *reinterpret_cast<volatile uint32_t*>(&R.rejected[p]) : 0u, 0)) {
+        if (__shfl_sync(kFull, settled, 0)) {
           stopped = true;
           break;
         }
@@ -1499,6 +1597,7 @@ __global__ void __launch_bounds__(kBlock, CLS == 3 ? 3 : (CLS == 4 ? 2 : (CLS ==
         for (int r = 0; r < 7; r++)
           if (slot[r] == nx - 1) rlast = r;
         for (unsigned long long u = u0; u < u1; u++) {
+          const uint32_t settled = poll();
           const unsigned long long first = u * kXBitsBlocks;
           const unsigned long long nb = (pr.nblocks - first < kXBitsBlocks) ? pr.nblocks - first : kXBitsBlocks;
           bad = cxbits_unit(u, pr.nblocks, nx, dec, rlast, pw, int(tl), int(cl), pr.keepF, pr.keepR, o0, o1, sm) ||
@@ -1506,25 +1605,24 @@ __global__ void __launch_bounds__(kBlock, CLS == 3 ? 3 : (CLS == 4 ? 2 : (CLS ==
           my_states += (256ull * nb) << xs;
           my_eval += 2ull * nb;
           if (__any_sync(kFull, bad)) break;
-          if (__shfl_sync(kFull, lane == 0 ? *reinterpret_cast<volatile uint32_t*>(&R.rejected[p]) : 0u, 0)) {
-          stopped = true;
-          break;
-        }
+          if (__shfl_sync(kFull, settled, 0)) {
+            stopped = true;
+            break;
+          }
         }
       } else {
         for (unsigned long long u = u0; u < u1; u++) {
+          const uint32_t settled = poll();
           const unsigned long long first = u * kBitsBlocks;
           const unsigned long long nb = (pr.nblocks - first < kBitsBlocks) ? pr.nblocks - first : kBitsBlocks;
           bad = cbits_unit(u, pr.nblocks, dec, pw, int(tl), int(cl), pr.keepF, pr.keepR, o0, o1, sm) || bad;
           my_states += (256ull * nb) << xs;
           my_eval += 256ull * nb;
           if (__any_sync(kFull, bad)) break;
-          if ((u & 15ull) == 15ull &&
-              __shfl_sync(kFull, lane == 0 ? *reinterpret_cast<volatile uint32_t*>(&R.rejected[p]) : 0u, 0))
-            {
-              stopped = true;
-              break;
-            }
+          if (__shfl_sync(kFull, settled, 0)) {
+            stopped = true;
+            break;
+          }
         }
       }
     } else if constexpr (!XI) {
@@ -1536,18 +1634,17 @@ __global__ void __launch_bounds__(kBlock, CLS == 3 ? 3 : (CLS == 4 ? 2 : (CLS ==
       extern __shared__ uint32_t zsm[];
       uint32_t* sm = zsm + (threadIdx.x >> 5) * (kBitsWords * 32) + lane;
       for (unsigned long long u = u0; u < u1; u++) {
+        const uint32_t settled = poll();
         const unsigned long long first = u * kBitsBlocks;
         const unsigned long long nb = (pr.nblocks - first < kBitsBlocks) ? pr.nblocks - first : kBitsBlocks;
         bad = bits_unit(u, pr.nblocks, bd, pw, int(tl), int(cl), pr.keepF, pr.keepR, sm) || bad;
         my_states += (256ull * nb) << xs;
         my_eval += 256ull * nb;
         if (__any_sync(kFull, bad)) break;
-        if ((u & 15ull) == 15ull &&
-            __shfl_sync(kFull, lane == 0 ? *reinterpret_cast<volatile uint32_t*>(&R.rejected[p]) : 0u, 0))
-          {
-            stopped = true;
-            break;
-          }
+        if (__shfl_sync(kFull, settled, 0)) {
+          stopped = true;
+          break;
+        }
       }
     } else if constexpr (CLS == 2) {
       // Unit = 1,024 A-blocks, 32 per lane, each at A = 0 and A = 1.
@@ -1558,6 +1655,7 @@ __global__ void __launch_bounds__(kBlock, CLS == 3 ? 3 : (CLS == 4 ? 2 : (CLS ==
       for (int r = 0; r < 7; r++)
         if (slot[r] == nx - 1) rlast = r;
       for (unsigned long long u = u0; u < u1; u++) {
+        const uint32_t settled = poll();
         const unsigned long long first = u * kXBitsBlocks;
         const unsigned long long nb = (pr.nblocks - first < kXBitsBlocks) ? pr.nblocks - first : kXBitsBlocks;
         bad = xbits_unit(u, pr.nblocks, spw, reduced, nx, fw, slot, rlast, pw, int(tl), int(cl), pr.keepF,
@@ -1566,7 +1664,7 @@ __global__ void __launch_bounds__(kBlock, CLS == 3 ? 3 : (CLS == 4 ? 2 : (CLS ==
         my_states += (256ull * nb) << xs;
         my_eval += 2ull * nb;
         if (__any_sync(kFull, bad)) break;
-        if (__shfl_sync(kFull, lane == 0 ? *reinterpret_cast<volatile uint32_t*>(&R.rejected[p]) : 0u, 0)) {
+        if (__shfl_sync(kFull, settled, 0)) {
           stopped = true;
           break;
         }
@@ -1576,18 +1674,17 @@ __global__ void __launch_bounds__(kBlock, CLS == 3 ? 3 : (CLS == 4 ? 2 : (CLS ==
       // of the warp (s = (i*K + q)*32 + lane) takes block unit*128 + s/2 with
       // A = s & 1.
       for (unsigned long long u = u0; u < u1; u++) {
+        const uint32_t settled = poll();
         const unsigned long long first = u * kUnitBlocks;
         const unsigned long long nb = (pr.nblocks - first < kUnitBlocks) ? pr.nblocks - first : kUnitBlocks;
         bad = xindep_unit<K>(first, nb, bd, pw, int(tl), int(cl), keep0, keep1) || bad;
         my_states += (256ull * nb) << xs;
         my_eval += 2ull * nb;
         if (__any_sync(kFull, bad)) break;
-        if ((u & 3ull) == 3ull &&
-            __shfl_sync(kFull, lane == 0 ? *reinterpret_cast<volatile uint32_t*>(&R.rejected[p]) : 0u, 0))
-          {
-            stopped = true;
-            break;
-          }
+        if (__shfl_sync(kFull, settled, 0)) {
+          stopped = true;
+          break;
+        }
       }
     }
     const bool any_bad = __any_sync(kFull, bad);
