@@ -109,6 +109,7 @@ struct PipeOpts {
   uint32_t mode = Z80B_MODE_FIRST;
   uint32_t max_cand = 1;        // longest candidate (1 or 2 instructions)
   uint64_t dreg_masks = 1;      // bit m: dead-register mask m occurs in a masked pass (bit 0 always)
+  bool plain = false;           // one target per launch (Z80B_PATH_PLAIN)
   bool no_exhaustive = false;   // all-hits mode: MidCheck survivors are the rules (Z80B_JOB_NO_EXHAUSTIVE)
   Reporter* rep = nullptr;      // per-target answers as they become final (first-found mode)
   // Targets uploaded in chunks on the copy stream (z80b_search on large
@@ -198,8 +199,8 @@ struct z80b_ctx {
   DBuf cnt_f, cnt_m, cnt_all, base, meta, surv, sdiff, checks;
   DBuf qc_tmp, qc_over;       // single-pass QuickCheck: kept survivors, targets with more
   DBuf next, win, windiff, spec, spec2, wlen, wend, cdone;
-  DBuf pairs, pair_src, nchunks, cbase, nchunks_x, cbase_x, nchunks_c, cbase_c, nchunks_w, cbase_w, nchunks_r,
-      cbase_r, rejected, npairs, counter, states;
+  DBuf pairs, pair_src, cbase[kClasses], cpair[kClasses], rejected, states;
+  DBuf roundctl, roundargs;   // RoundCtl; RoundArgs of the two passes
   DBuf rcnt, rbase, rules, checked, surv_target, midpass, flag;
   HBuf h_rules;               // pinned staging of the device rules read back
   DBuf cub_tmp;
@@ -209,7 +210,7 @@ struct z80b_ctx {
   // length-2 candidates: the pair pool and its indexes, shared by the
   // contexts of a device; the per-lane pass state is per context
   std::shared_ptr<PairShared> pairpool;
-  DBuf next2, win2, windiff2, cnt2, resume2, surv2, sdiff2, refill2;
+  DBuf next2, win2, windiff2, cnt2, resume2, surv2, sdiff2, scan2;
   uint64_t n_rules_dev = 0;
   uint32_t launches = 0;
   int exh_k = 4;              // ExhaustiveCheck states per lane per dispatch (z80b_set_option)
@@ -231,7 +232,6 @@ struct z80b_ctx {
   // that orders the copies after the context stream's earlier work
   cudaStream_t copy_stream = nullptr;
   cudaEvent_t up_ev[kUpChunks + 1] = {};
-  DBuf roundctl;              // RoundCtl of the device-driven rounds
   RoundGraph rg1, rg2;        // instantiated round loops: length-1 and length-2 candidate passes
 };
 
@@ -660,41 +660,65 @@ struct Reporter {
              bool last);
 };
 
-// ExhaustiveCheck of the np pairs of a round: chunk prefixes of both pair
-// classes, then the sweep kernel of each class that has chunks.
-int sweep_round(z80b_ctx* ctx, const DevTargets& T, const DevPool& P, const RoundBuf& R, uint32_t np) {
+// Buffers of a round's pairs (cap slots; windows: first-found passes).
+int ensure_round(z80b_ctx* ctx, uint64_t cap, bool windows, RoundBuf* R) {
+  cap = std::min<uint64_t>(std::max<uint64_t>(cap, 1), kMaxRoundPairs);
+  CK(ctx->pairs.ensure(sizeof(PairRec) * cap));
+  CK(ctx->pair_src.ensure(4 * cap));
+  CK(ctx->rejected.ensure(4 * cap));
+  CK(ctx->states.ensure(16));
+  CK(ctx->roundctl.ensure(sizeof(RoundCtl)));
+  CK(ctx->roundargs.ensure(2 * sizeof(RoundArgs)));
+  *R = RoundBuf{};
+  R->compact = ctx->compact ? 1u : 0u;
+  R->wide = ctx->wide ? 1u : 0u;
+  for (int c = 0; c < kClasses; c++) {
+    if ((c == 2 && !R->compact) || (c >= 3 && !R->wide)) continue;
+    CK(ctx->cbase[c].ensure(8 * cap));
+    CK(ctx->cpair[c].ensure(4 * cap));
+    R->cbase[c] = ctx->cbase[c].as<unsigned long long>();
+    R->cpair[c] = ctx->cpair[c].as<uint32_t>();
+  }
+  R->pairs = ctx->pairs.as<PairRec>();
+  R->pair_src = ctx->pair_src.as<uint32_t>();
+  R->rejected = ctx->rejected.as<uint32_t>();
+  R->states = ctx->states.as<unsigned long long>();
+  R->ctl = ctx->roundctl.as<RoundCtl>();
+  if (windows) {
+    CK(ctx->wlen.ensure(cap));
+    CK(ctx->wend.ensure(4 * cap));
+    CK(ctx->cdone.ensure(4 * cap));
+    R->wlen = ctx->wlen.as<uint8_t>();
+    R->wend = ctx->wend.as<uint32_t>();
+    R->cdone = ctx->cdone.as<uint32_t>();
+  }
+  R->cap = uint32_t(cap);
+  R->max_chunks = max_chunks(cap);
+  R->chunk_blocks = uint32_t(ctx->chunk_blocks);
+  R->xunit = ctx->xbits ? kXBitsBlocks : kXScalarBlocks;
+  return Z80B_OK;
+}
+
+// Jobs of at most this many targets take the launch shapes for few lanes.
+constexpr uint32_t kSmallJob = 4096;
+
+// Plans the round's pairs, reads its counters and sweeps them, the grids by
+// the chunks there are (their blocks retire every few chunks).  h_args: the
+// arguments that a holds on the device.
+int sweep_round(z80b_ctx* ctx, const RoundArgs* a, const RoundArgs& h_args, bool small, uint32_t* np) {
+  const RoundBuf& R = h_args.R;
   cudaStream_t s = ctx->stream;
-  CKR(scan(ctx, R.nchunks, R.cbase, np));
-  CKR(scan(ctx, R.nchunks_x, R.cbase_x, np));
-  if (R.compact) CKR(scan(ctx, R.nchunks_c, R.cbase_c, np));
-  if (R.wide) {
-    CKR(scan(ctx, R.nchunks_w, R.cbase_w, np));
-    CKR(scan(ctx, R.nchunks_r, R.cbase_r, np));
-  }
-  unsigned long long last[10] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
-  CK(cudaMemcpyAsync(&last[0], R.cbase + (np - 1), 8, cudaMemcpyDeviceToHost, s));
-  CK(cudaMemcpyAsync(&last[1], R.nchunks + (np - 1), 8, cudaMemcpyDeviceToHost, s));
-  CK(cudaMemcpyAsync(&last[2], R.cbase_x + (np - 1), 8, cudaMemcpyDeviceToHost, s));
-  CK(cudaMemcpyAsync(&last[3], R.nchunks_x + (np - 1), 8, cudaMemcpyDeviceToHost, s));
-  if (R.compact) {
-    CK(cudaMemcpyAsync(&last[4], R.cbase_c + (np - 1), 8, cudaMemcpyDeviceToHost, s));
-    CK(cudaMemcpyAsync(&last[5], R.nchunks_c + (np - 1), 8, cudaMemcpyDeviceToHost, s));
-  }
-  if (R.wide) {
-    CK(cudaMemcpyAsync(&last[6], R.cbase_w + (np - 1), 8, cudaMemcpyDeviceToHost, s));
-    CK(cudaMemcpyAsync(&last[7], R.nchunks_w + (np - 1), 8, cudaMemcpyDeviceToHost, s));
-    CK(cudaMemcpyAsync(&last[8], R.cbase_r + (np - 1), 8, cudaMemcpyDeviceToHost, s));
-    CK(cudaMemcpyAsync(&last[9], R.nchunks_r + (np - 1), 8, cudaMemcpyDeviceToHost, s));
-  }
-  CK(cudaStreamSynchronize(s));
-  CK(cudaMemsetAsync(R.counter, 0, 40, s));
-  trace("sweep: %u pairs, %llu + %llu + %llu + %llu + %llu chunks", np, last[0] + last[1], last[2] + last[3],
-        last[4] + last[5], last[6] + last[7], last[8] + last[9]);
+  launch_pair_plan(a, small, s);
+  CKR(check_launch(ctx, "pair_plan"));
+  RoundCtl h;
+  CKR(fetch(ctx, &h, R.ctl));
+  *np = std::min(h.npairs, R.cap);
+  trace("sweep: %u pairs, %llu + %llu + %llu + %llu + %llu chunks", *np, h.alloc[0] & kChunkMask,
+        h.alloc[1] & kChunkMask, h.alloc[2] & kChunkMask, h.alloc[3] & kChunkMask, h.alloc[4] & kChunkMask);
   int ke = kbegin(ctx, 1);
-  const int nl = launch_exhaustive(T, P, R, np, last[0] + last[1], last[2] + last[3], last[4] + last[5],
-                                   last[6] + last[7], last[8] + last[9], ctx->exh_k, s, &ctx->sweep_kernels);
+  const int nl = launch_exhaustive(sweep_args(h_args), h.alloc, ctx->exh_k, s, &ctx->sweep_kernels);
   kend(ctx, ke);
-  CKR(check_launch(ctx, "exhaustive"));
+  if (nl) CKR(check_launch(ctx, "exhaustive"));
   if (nl > 1) ctx->launches += uint32_t(nl - 1);
   return Z80B_OK;
 }
@@ -706,37 +730,31 @@ void key_put(std::vector<unsigned char>& k, const V& v) {
 }
 
 // The rounds of one first-found pass driven by the device: one CUDA graph
-// whose WHILE node repeats the round body -- clear the pair counter (and the
-// rescan counter), build the round's pairs, scan their chunk counts and set
-// the loop condition (k_round_scan), [rescan the length-2 buckets of lanes
-// whose slots ran out, only after an empty round], the sweep kernels of
-// every class on persistent grids, resolve -- until a round is empty with no
-// rescan pending.  The same work and order as the host loop of
-// run_pipeline, without a host round trip per round.  The graph is
-// captured once per set of launch arguments and replayed.
-int rounds_on_device(z80b_ctx* ctx, RoundGraph& g, const DevTargets& T, const DevPool& P, const QCOut& q,
-                     const Lanes& L, const RoundBuf& R, uint32_t max_spec, const PairScan* ps, const QCOut* qres,
+// whose WHILE node repeats the round body -- [rescan the length-2 lanes whose
+// slots ran out,] build the round's pairs, plan them, the sweep kernels of
+// every class on persistent grids, resolve, and the round's end, which sets
+// the loop condition -- until no lane has anything left.  The same work and
+// order as rounds_on_host, without a host round trip per round.  The kernels
+// read the job from RoundArgs in device memory (the sweeps what does not
+// depend on its size by value), so a captured graph is replayed for jobs of
+// any size until a buffer grows: a capture costs about 0.9 ms, which every
+// job of another size used to pay.
+int rounds_on_device(z80b_ctx* ctx, RoundGraph& g, const RoundArgs* a, const RoundArgs& h_args, bool pair, bool small,
                      uint32_t* rounds, uint64_t* pairs) {
   cudaStream_t s = ctx->stream;
-  CK(ctx->roundctl.ensure(sizeof(RoundCtl)));
-  RoundCtl* ctl = ctx->roundctl.as<RoundCtl>();
+  const RoundBuf& R = h_args.R;
+  const SweepArgs sweep = sweep_args(h_args);
   std::vector<unsigned char> key;
-  key_put(key, T);
-  key_put(key, P);
-  key_put(key, q);
-  key_put(key, L);
-  key_put(key, R);
-  key_put(key, max_spec);
+  key_put(key, a);
+  key_put(key, sweep);
+  key_put(key, small);
+  key_put(key, R.compact);
+  key_put(key, R.wide);
   key_put(key, ctx->exh_k);
-  key_put(key, ctl);
-  if (ps) {
-    key_put(key, *ps);
-    key_put(key, *qres);
-  }
   key_put(key, ctx->concurrent_sweeps);
   if (!g.exec || g.key != key) {
     g.reset();
-    warm_exhaustive_dev(R, ctx->exh_k);
+    warm_exhaustive_dev(R.compact, R.wide, R.xunit, ctx->exh_k);
     if (ctx->concurrent_sweeps && !ctx->side[0]) {
       CK(cudaEventCreateWithFlags(&ctx->fork_ev, cudaEventDisableTiming));
       for (int i = 0; i < 4; i++) {
@@ -756,16 +774,9 @@ int rounds_on_device(z80b_ctx* ctx, RoundGraph& g, const DevTargets& T, const De
     CK(cudaGraphAddNode(&node, g.graph, nullptr, 0, &cp));
     cudaGraph_t body = cp.conditional.phGraph_out[0];
     CK(cudaStreamBeginCaptureToGraph(s, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
-    cudaMemsetAsync(R.npairs, 0, 4, s);
-    if (ps) {
-      cudaMemsetAsync(ps->refill, 0, 4, s);
-      launch_pair_round_build(T, P, q, L, *ps, R, s);
-      launch_round_scan(R, ctl, ps->refill, loop, s);
-      launch_pair_scan_gated(T, q, L, *ps, ctl, s);
-    } else {
-      launch_round_build(T, P, q, L, R, s);
-      launch_round_scan(R, ctl, nullptr, loop, s);
-    }
+    if (pair) launch_pair_scan(a, 0, false, small, s);
+    launch_round_build(a, pair, small, s);
+    launch_pair_plan(a, small, s);
     {
       // the classes' sweeps on parallel branches of the body graph
       cudaStream_t ss[5] = {s, s, s, s, s};
@@ -776,14 +787,15 @@ int rounds_on_device(z80b_ctx* ctx, RoundGraph& g, const DevTargets& T, const De
           ss[i + 1] = ctx->side[i];
         }
       }
-      launch_exhaustive_dev(T, P, R, ctl, ctx->exh_k, ss);
+      launch_exhaustive_dev(sweep, R.compact, R.wide, ctx->exh_k, ss);
       if (ctx->concurrent_sweeps)
         for (int i = 0; i < 4; i++) {
           cudaEventRecord(ctx->join_ev[i], ctx->side[i]);
           cudaStreamWaitEvent(s, ctx->join_ev[i], 0);
         }
     }
-    launch_round_resolve_dev(R, ctl, ps ? *qres : q, L, max_spec, s);
+    launch_round_resolve(a, pair, small, s);
+    launch_round_end(a, true, loop, s);
     cudaGraph_t captured = nullptr;
     const cudaError_t ce = cudaStreamEndCapture(s, &captured);
     if (ce != cudaSuccess) {
@@ -793,18 +805,16 @@ int rounds_on_device(z80b_ctx* ctx, RoundGraph& g, const DevTargets& T, const De
     }
     CK(cudaGraphInstantiate(&g.exec, g.graph, 0));
     g.key = key;
-    trace("round loop captured (%s pass)", ps ? "length-2" : "length-1");
+    trace("round loop captured (%s pass)", pair ? "length-2" : "length-1");
   }
-  // build, plan, scan (3), [rescan], sweeps, resolve
-  const int per_iter = (ps ? 6 : 5) + 1 + 2 + (R.compact ? 1 : 0) + (R.wide ? 2 : 0);
-  CK(cudaMemsetAsync(ctl, 0, sizeof(RoundCtl), s));
+  // [rescan], build, plan, sweeps, resolve, end
+  const int per_iter = (pair ? 5 : 4) + 2 + (R.compact ? 1 : 0) + (R.wide ? 2 : 0);
   int ke = kbegin(ctx, 1);
   CK(cudaGraphLaunch(g.exec, s));
   kend(ctx, ke);
   CKR(check_launch(ctx, "round loop"));
   RoundCtl h{};
-  CK(cudaMemcpyAsync(&h, ctl, offsetof(RoundCtl, bsum), cudaMemcpyDeviceToHost, s));  // the counters
-  CK(cudaStreamSynchronize(s));
+  CKR(fetch(ctx, &h, R.ctl));
   if (h.overrun) return fail(ctx, Z80B_ETIMEOUT, "device round loop did not end within %u iterations", kMaxRoundIters);
   *rounds += h.rounds;
   *pairs += h.pairs;
@@ -815,6 +825,39 @@ int rounds_on_device(z80b_ctx* ctx, RoundGraph& g, const DevTargets& T, const De
   ctx->sweep_kernels |= mask;
   trace("device rounds: %u rounds, %u iterations, %llu pairs", h.rounds, h.iters, (unsigned long long)h.pairs);
   return Z80B_OK;
+}
+
+// The same rounds driven from the host; after_round runs behind each one.
+template <class AfterRound>
+int rounds_on_host(z80b_ctx* ctx, const RoundArgs* a, const RoundArgs& h_args, bool pair, bool small, uint32_t* rounds,
+                   uint64_t* pairs, AfterRound after_round) {
+  cudaStream_t s = ctx->stream;
+  for (uint32_t it = 0;; it++) {
+    if (pair && it) {
+      int kr = kbegin(ctx, 0);
+      launch_pair_scan(a, 0, false, small, s);
+      kend(ctx, kr);
+      CKR(check_launch(ctx, "pair_scan"));
+    }
+    launch_round_build(a, pair, small, s);
+    CKR(check_launch(ctx, "round_build"));
+    uint32_t np = 0;
+    CKR(sweep_round(ctx, a, h_args, small, &np));
+    launch_round_resolve(a, pair, small, s);
+    CKR(check_launch(ctx, "round_resolve"));
+    launch_round_end(a, false, cudaGraphConditionalHandle{}, s);
+    CKR(check_launch(ctx, "round_end"));
+    RoundCtl h;
+    CKR(fetch(ctx, &h, h_args.R.ctl));
+    trace("%s round %u: %u pairs", pair ? "length-2" : "length-1", *rounds, np);
+    if (np) {
+      *rounds += 1;
+      *pairs += np;
+      CKR(after_round());
+    }
+    if (h.overrun) return fail(ctx, Z80B_ETIMEOUT, "round loop did not end within %u iterations", kMaxRoundIters);
+    if (!h.more) return Z80B_OK;
+  }
 }
 
 // Runs the pipeline on device-resident targets.  Rules stay in ctx->rules
@@ -847,8 +890,6 @@ int run_pipeline(z80b_ctx* ctx, const DevTargets& T, const PipeOpts& opts, z80b_
   CK(ctx->checks.ensure(8));
   CK(ctx->checked.ensure(8));
   CK(ctx->states.ensure(16));
-  CK(ctx->npairs.ensure(4));
-  CK(ctx->counter.ensure(40));
   CK(cudaMemsetAsync(ctx->checks.p, 0, 8, s));
   CK(cudaMemsetAsync(ctx->checked.p, 0, 8, s));
   CK(cudaMemsetAsync(ctx->states.p, 0, 16, s));
@@ -955,79 +996,36 @@ int run_pipeline(z80b_ctx* ctx, const DevTargets& T, const PipeOpts& opts, z80b_
     CK(ctx->next.ensure(8ull * n));
     CK(ctx->win.ensure(8ull * n));
     CK(ctx->windiff.ensure(4ull * n));
-    // pair slots per round: every lane once, and room for survivor windows
-    const uint64_t cap = std::max<uint64_t>(2ull * n, std::min<uint64_t>(128ull * n, 1ull << 20));
-    CK(ctx->pairs.ensure(sizeof(PairRec) * cap));
-    CK(ctx->pair_src.ensure(4 * cap));
-    CK(ctx->nchunks.ensure(8 * cap));
-    CK(ctx->cbase.ensure(8 * cap));
-    CK(ctx->nchunks_x.ensure(8 * cap));
-    CK(ctx->cbase_x.ensure(8 * cap));
-    if (ctx->compact) {
-      CK(ctx->nchunks_c.ensure(8 * cap));
-      CK(ctx->cbase_c.ensure(8 * cap));
-    }
-    if (ctx->wide) {
-      CK(ctx->nchunks_w.ensure(8 * cap));
-      CK(ctx->cbase_w.ensure(8 * cap));
-      CK(ctx->nchunks_r.ensure(8 * cap));
-      CK(ctx->cbase_r.ensure(8 * cap));
-    }
-    CK(ctx->rejected.ensure(4 * cap));
-    CK(ctx->wlen.ensure(cap));
-    CK(ctx->wend.ensure(4 * cap));
-    CK(ctx->cdone.ensure(4 * cap));
     CK(ctx->spec.ensure(2ull * n));
     CK(cudaMemsetAsync(ctx->spec.p, 0, 2ull * n, s));
     CK(cudaMemsetAsync(ctx->next.p, 0, 8ull * n, s));
     CK(cudaMemsetAsync(ctx->win.p, 0xFF, 8ull * n, s));
     Lanes L{ctx->next.as<uint32_t>(), ctx->win.as<uint32_t>(), ctx->windiff.as<uint16_t>(), ctx->spec.as<uint8_t>()};
-    R.pairs = ctx->pairs.as<PairRec>();
-    R.pair_src = ctx->pair_src.as<uint32_t>();
-    R.nchunks = ctx->nchunks.as<unsigned long long>();
-    R.cbase = ctx->cbase.as<unsigned long long>();
-    R.nchunks_x = ctx->nchunks_x.as<unsigned long long>();
-    R.cbase_x = ctx->cbase_x.as<unsigned long long>();
-    R.rejected = ctx->rejected.as<uint32_t>();
-    R.wlen = ctx->wlen.as<uint8_t>();
-    R.wend = ctx->wend.as<uint32_t>();
-    R.cdone = ctx->cdone.as<uint32_t>();
-    R.cap = uint32_t(cap);
-    R.npairs = ctx->npairs.as<uint32_t>();
-    R.counter = ctx->counter.as<unsigned long long>();
-    R.states = ctx->states.as<unsigned long long>();
-    R.chunk_blocks = uint32_t(ctx->chunk_blocks);
-    R.xunit = ctx->xbits ? kXBitsBlocks : kXScalarBlocks;
-    R.compact = mode == Z80B_MODE_FIRST && ctx->compact ? 1u : 0u;
-    R.nchunks_c = R.compact ? ctx->nchunks_c.as<unsigned long long>() : nullptr;
-    R.cbase_c = R.compact ? ctx->cbase_c.as<unsigned long long>() : nullptr;
-    R.wide = mode == Z80B_MODE_FIRST && ctx->wide ? 1u : 0u;
-    R.nchunks_w = R.wide ? ctx->nchunks_w.as<unsigned long long>() : nullptr;
-    R.cbase_w = R.wide ? ctx->cbase_w.as<unsigned long long>() : nullptr;
-    R.nchunks_r = R.wide ? ctx->nchunks_r.as<unsigned long long>() : nullptr;
-    R.cbase_r = R.wide ? ctx->cbase_r.as<unsigned long long>() : nullptr;
+    // pair slots per round: every lane once, and room for survivor windows
+    CKR(ensure_round(ctx, std::max<uint64_t>(2ull * n, std::min<uint64_t>(128ull * n, 1ull << 20)), true, &R));
+    RoundArgs* const args = ctx->roundargs.as<RoundArgs>();
     // rounds on the device (one graph) unless the caller takes answers
-    // round by round (streaming callbacks)
-    const bool dev_rounds = ctx->graph_rounds && !opts.rep;
-    if (nsurv && dev_rounds) {
-      CKR(rounds_on_device(ctx, ctx->rg1, T, P, q, L, R, kMaxSpec1, nullptr, nullptr, &rounds, &exh_pairs));
-    } else if (nsurv) {
-      for (;;) {
-        CK(cudaMemsetAsync(R.npairs, 0, 4, s));
-        launch_round_build(T, P, q, L, R, s);
-        CKR(check_launch(ctx, "round_build"));
-        uint32_t np = 0;
-        CKR(fetch(ctx, &np, R.npairs));
-        np = std::min(np, R.cap);
-        trace("round %u: %u pairs", rounds, np);
-        if (np == 0) break;
-        rounds++;
-        exh_pairs += np;
-        CKR(sweep_round(ctx, T, P, R, np));
-        launch_round_resolve(R, np, q, L, kMaxSpec1, s);
-        CKR(check_launch(ctx, "round_resolve"));
-        if (opts.rep) CKR(opts.rep->update(ctx, n, L, Lanes{}, opts.max_cand, false, false));
-      }
+    // round by round (streaming callbacks) or each target is a job of its
+    // own (its address would be another graph)
+    const bool dev_rounds = ctx->graph_rounds && !opts.rep && !opts.plain;
+    const bool small = n <= kSmallJob;
+    RoundArgs ra{};
+    ra.T = T;
+    ra.P = P;
+    ra.q = q;
+    ra.L = L;
+    ra.R = R;
+    ra.sdiff = q.sdiff;
+    ra.max_spec = kMaxSpec1;
+    if (nsurv) {
+      launch_round_args(ra, args, s);
+      CKR(check_launch(ctx, "round_args"));
+      if (dev_rounds)
+        CKR(rounds_on_device(ctx, ctx->rg1, args, ra, false, small, &rounds, &exh_pairs));
+      else
+        CKR(rounds_on_host(ctx, args, ra, false, small, &rounds, &exh_pairs, [&] {
+          return opts.rep ? opts.rep->update(ctx, n, L, Lanes{}, opts.max_cand, false, false) : Z80B_OK;
+        }));
     }
     Lanes L2{};
     unsigned long long pool2_enum = 0;
@@ -1047,7 +1045,7 @@ int run_pipeline(z80b_ctx* ctx, const DevTargets& T, const PipeOpts& opts, z80b_
       CK(ctx->resume2.ensure(8ull * n));
       CK(ctx->surv2.ensure(8ull * n * kSlots2));
       CK(ctx->sdiff2.ensure(4ull * n * kSlots2));
-      CK(ctx->refill2.ensure(4));
+      CK(ctx->scan2.ensure(8ull * n));
       CK(ctx->spec2.ensure(2ull * n));
       L2 = Lanes{ctx->next2.as<uint32_t>(), ctx->win2.as<uint32_t>(), ctx->windiff2.as<uint16_t>(),
                  ctx->spec2.as<uint8_t>()};
@@ -1058,45 +1056,28 @@ int run_pipeline(z80b_ctx* ctx, const DevTargets& T, const PipeOpts& opts, z80b_
       ps.resume = ctx->resume2.as<uint32_t>();
       ps.surv = ctx->surv2.as<uint32_t>();
       ps.sdiff = ctx->sdiff2.as<uint16_t>();
-      ps.refill = ctx->refill2.as<uint32_t>();
+      ps.scan = ctx->scan2.as<uint32_t>();
       ps.eligible = PS.eligible_dev.as<unsigned long long>();
       ps.checks = ctx->checks.as<unsigned long long>();
-      QCOut q2 = q;
-      q2.sdiff = ps.sdiff;
       launch_pair_lanes_init(T, L, q, L2, ps, s);
       CKR(check_launch(ctx, "pair_lanes_init"));
+      ra.P = P2;
+      ra.L = L2;
+      ra.ps = ps;
+      ra.sdiff = ps.sdiff;
+      ra.max_spec = kMaxSpec2;
+      launch_round_args(ra, args + 1, s);
+      CKR(check_launch(ctx, "round_args"));
       int kq2 = kbegin(ctx, 0);
-      launch_pair_scan(T, q, L2, ps, s);
+      launch_pair_scan(args + 1, n, true, small, s);
       kend(ctx, kq2);
       CKR(check_launch(ctx, "pair_scan"));
       if (dev_rounds)
-        CKR(rounds_on_device(ctx, ctx->rg2, T, P2, q, L2, R, kMaxSpec2, &ps, &q2, &rounds, &exh_pairs));
-      for (; !dev_rounds;) {
-        CK(cudaMemsetAsync(R.npairs, 0, 4, s));
-        CK(cudaMemsetAsync(ps.refill, 0, 4, s));
-        launch_pair_round_build(T, P2, q, L2, ps, R, s);
-        CKR(check_launch(ctx, "pair_round_build"));
-        uint32_t np = 0, nref = 0;
-        CK(cudaMemcpyAsync(&np, R.npairs, 4, cudaMemcpyDeviceToHost, s));
-        CK(cudaMemcpyAsync(&nref, ps.refill, 4, cudaMemcpyDeviceToHost, s));
-        CK(cudaStreamSynchronize(s));
-        np = std::min(np, R.cap);
-        trace("length-2 round %u: %u pairs, %u lanes to rescan", rounds, np, nref);
-        if (np == 0) {
-          if (nref == 0) break;
-          int kr = kbegin(ctx, 0);
-          launch_pair_scan(T, q, L2, ps, s);
-          kend(ctx, kr);
-          CKR(check_launch(ctx, "pair_scan"));
-          continue;
-        }
-        rounds++;
-        exh_pairs += np;
-        CKR(sweep_round(ctx, T, P2, R, np));
-        launch_round_resolve(R, np, q2, L2, kMaxSpec2, s);
-        CKR(check_launch(ctx, "round_resolve"));
-        if (opts.rep) CKR(opts.rep->update(ctx, n, L, L2, opts.max_cand, true, false));
-      }
+        CKR(rounds_on_device(ctx, ctx->rg2, args + 1, ra, true, small, &rounds, &exh_pairs));
+      else
+        CKR(rounds_on_host(ctx, args + 1, ra, true, small, &rounds, &exh_pairs, [&] {
+          return opts.rep ? opts.rep->update(ctx, n, L, L2, opts.max_cand, true, false) : Z80B_OK;
+        }));
     }
     if (opts.rep) CKR(opts.rep->update(ctx, n, L, L2, opts.max_cand, opts.max_cand >= 2, true));
     CK(ctx->rcnt.ensure(4ull * n));
@@ -1120,51 +1101,41 @@ int run_pipeline(z80b_ctx* ctx, const DevTargets& T, const PipeOpts& opts, z80b_
     CK(ctx->midpass.ensure(std::max<uint32_t>(S, 1)));
     CK(ctx->flag.ensure(4ull * std::max<uint32_t>(S, 1)));
     CK(ctx->rbase.ensure(4ull * std::max<uint32_t>(S, 1)));
-    CK(ctx->pairs.ensure(sizeof(PairRec) * std::max<uint32_t>(S, 1)));
-    CK(ctx->pair_src.ensure(4ull * std::max<uint32_t>(S, 1)));
-    CK(ctx->nchunks.ensure(8ull * std::max<uint32_t>(S, 1)));
-    CK(ctx->cbase.ensure(8ull * std::max<uint32_t>(S, 1)));
-    CK(ctx->nchunks_x.ensure(8ull * std::max<uint32_t>(S, 1)));
-    CK(ctx->cbase_x.ensure(8ull * std::max<uint32_t>(S, 1)));
-    CK(ctx->rejected.ensure(4ull * std::max<uint32_t>(S, 1)));
-    R.pairs = ctx->pairs.as<PairRec>();
-    R.pair_src = ctx->pair_src.as<uint32_t>();
-    R.nchunks = ctx->nchunks.as<unsigned long long>();
-    R.cbase = ctx->cbase.as<unsigned long long>();
-    R.nchunks_x = ctx->nchunks_x.as<unsigned long long>();
-    R.cbase_x = ctx->cbase_x.as<unsigned long long>();
-    R.rejected = ctx->rejected.as<uint32_t>();
-    R.npairs = ctx->npairs.as<uint32_t>();
-    R.counter = ctx->counter.as<unsigned long long>();
-    R.states = ctx->states.as<unsigned long long>();
-    R.chunk_blocks = uint32_t(ctx->chunk_blocks);
-    R.xunit = ctx->xbits ? kXBitsBlocks : kXScalarBlocks;
-    R.compact = mode == Z80B_MODE_FIRST && ctx->compact ? 1u : 0u;
-    R.nchunks_c = R.compact ? ctx->nchunks_c.as<unsigned long long>() : nullptr;
-    R.cbase_c = R.compact ? ctx->cbase_c.as<unsigned long long>() : nullptr;
-    R.wide = mode == Z80B_MODE_FIRST && ctx->wide ? 1u : 0u;
-    R.nchunks_w = R.wide ? ctx->nchunks_w.as<unsigned long long>() : nullptr;
-    R.cbase_w = R.wide ? ctx->cbase_w.as<unsigned long long>() : nullptr;
-    R.nchunks_r = R.wide ? ctx->nchunks_r.as<unsigned long long>() : nullptr;
-    R.cbase_r = R.wide ? ctx->cbase_r.as<unsigned long long>() : nullptr;
+    CKR(ensure_round(ctx, S, false, &R));
     if (S) {
       launch_surv_targets(q, n, ctx->surv_target.as<uint32_t>(), s);
       CKR(check_launch(ctx, "surv_targets"));
       launch_midcheck(T, P, q.surv, ctx->surv_target.as<uint32_t>(), S, ctx->midpass.as<uint8_t>(), s);
       CKR(check_launch(ctx, "midcheck"));
-      CK(cudaMemsetAsync(R.npairs, 0, 4, s));
-      launch_pairs_from_survivors(T, P, q, ctx->midpass.as<uint8_t>(), S, ctx->surv_target.as<uint32_t>(), R, s);
-      CKR(check_launch(ctx, "pairs"));
-      uint32_t np = 0;
-      CKR(fetch(ctx, &np, R.npairs));
-      mid_surv = np;
-      exh_pairs = np;
+      RoundArgs* const args = ctx->roundargs.as<RoundArgs>();
+      RoundArgs ra{};
+      ra.T = T;
+      ra.P = P;
+      ra.q = q;
+      ra.R = R;
       CK(cudaMemsetAsync(ctx->flag.p, 0, 4ull * S, s));
-      if (np) {
-        rounds = 1;
+      // all survivors at once, up to the pair slots
+      for (uint64_t lo = 0; lo < S; lo += R.cap) {
+        const uint32_t hi = uint32_t(std::min<uint64_t>(S, lo + R.cap));
+        launch_round_args(ra, args, s);
+        CKR(check_launch(ctx, "round_args"));
+        launch_pairs_from_survivors(q, ctx->midpass.as<uint8_t>(), uint32_t(lo), hi, ctx->surv_target.as<uint32_t>(), R,
+                                    s);
+        CKR(check_launch(ctx, "pairs"));
+        uint32_t np = 0;
         // without the ExhaustiveCheck tier every pair keeps the zero
         // rejection flag its build wrote
-        if (!opts.no_exhaustive) CKR(sweep_round(ctx, T, P, R, np));
+        if (opts.no_exhaustive) {
+          RoundCtl h;
+          CKR(fetch(ctx, &h, R.ctl));
+          np = std::min(h.npairs, R.cap);
+        } else {
+          CKR(sweep_round(ctx, args, ra, S <= kSmallJob, &np));
+        }
+        mid_surv += np;
+        exh_pairs += np;
+        if (!np) continue;
+        rounds = 1;
         launch_rule_count_all(R, np, ctx->flag.as<uint32_t>(), s);
         CKR(check_launch(ctx, "rule_count_all"));
       }
@@ -1429,6 +1400,8 @@ int run_staged(z80b_ctx* ctx, z80b_stats* st, uint64_t* nr, std::vector<z80b_rul
   // plain: one target per pipeline launch, synchronizing in between
   uint64_t total = 0;
   std::vector<DevRule> dr;
+  PipeOpts opts = S.opts;
+  opts.plain = true;
   for (uint32_t i = 0; i < T.n; i++) {
     DevTargets one = T;
     one.insn = T.insn + (size_t)i * T.stride;
@@ -1437,7 +1410,7 @@ int run_staged(z80b_ctx* ctx, z80b_stats* st, uint64_t* nr, std::vector<z80b_rul
     if (T.dead) one.dead = T.dead + i;
     if (T.dead_regs) one.dead_regs = T.dead_regs + i;
     uint64_t k = 0;
-    CKR(run_pipeline(ctx, one, S.opts, st, &k));
+    CKR(run_pipeline(ctx, one, opts, st, &k));
     if (k) {
       dr.resize(k);
       CK(cudaMemcpyAsync(dr.data(), ctx->rules.p, sizeof(DevRule) * k, cudaMemcpyDeviceToHost, ctx->stream));
@@ -1684,57 +1657,32 @@ int z80b_verify_pairs(z80b_ctx* ctx, const uint32_t* tgt, const uint8_t* tlens, 
     P.lens = ctx->v_cl.as<uint8_t>();
     P.n = n;
     P.stride = stride;
-    std::vector<PairRec> pr(n);
-    std::vector<unsigned long long> cb(n), cbx(n);
-    unsigned long long tot = 0, totx = 0;  // chunks of the bit-sliced / A-independent pairs
-    for (uint32_t i = 0; i < n; i++) {
-      uint16_t rd = uint16_t(seq_reads(tgt + (size_t)i * stride, tlens[i]) | seq_reads(cand + (size_t)i * stride, clens[i]));
-      Sweep w = sweep_for(rd);
-      pr[i] = PairRec{};
-      pr[i].target = i;
-      pr[i].cand = i;
-      pr[i].reads = rd;
-      pr[i].nblocks = w.states / 256;
-      pr[i].keepF = uint8_t(~(dead ? dead[i] : 0u));
-      pr[i].keepR = 0x3F;
-      // sweep units (see the sweep kernel): 128 A-blocks for A-independent
-      // pairs, 4 A-blocks (bit-sliced) for the others
-      unsigned long long units = (pr[i].nblocks + 3) / 4;
-      if (seq_aflow(tgt + (size_t)i * stride, tlens[i]) && seq_aflow(cand + (size_t)i * stride, clens[i])) {
-        pr[i].keepR |= 0x40;
-        units = (pr[i].nblocks + 127) / 128;
-      }
-      unsigned long long c = (units + ctx->chunk_blocks - 1) / uint64_t(ctx->chunk_blocks);
-      if (c > (1ull << 20)) c = 1ull << 20;
-      cb[i] = tot;
-      cbx[i] = totx;
-      if (pr[i].keepR & 0x40) totx += c;
-      else tot += c;
-    }
-    CK(ctx->pairs.ensure(sizeof(PairRec) * n));
-    CK(ctx->cbase.ensure(8ull * n));
-    CK(ctx->cbase_x.ensure(8ull * n));
-    CK(ctx->rejected.ensure(4ull * n));
-    CK(ctx->counter.ensure(40));
-    CK(ctx->states.ensure(16));
-    CK(cudaMemcpyAsync(ctx->pairs.p, pr.data(), sizeof(PairRec) * n, cudaMemcpyHostToDevice, s));
-    CK(cudaMemcpyAsync(ctx->cbase.p, cb.data(), 8ull * n, cudaMemcpyHostToDevice, s));
-    CK(cudaMemcpyAsync(ctx->cbase_x.p, cbx.data(), 8ull * n, cudaMemcpyHostToDevice, s));
-    CK(cudaMemsetAsync(ctx->rejected.p, 0, 4ull * n, s));
-    CK(cudaMemsetAsync(ctx->counter.p, 0, 16, s));
     RoundBuf R{};
-    R.pairs = ctx->pairs.as<PairRec>();
-    R.cbase = ctx->cbase.as<unsigned long long>();
-    R.cbase_x = ctx->cbase_x.as<unsigned long long>();
-    R.rejected = ctx->rejected.as<uint32_t>();
-    R.counter = ctx->counter.as<unsigned long long>();
-    R.states = ctx->states.as<unsigned long long>();
-    const int nl = launch_exhaustive(T, P, R, n, tot, totx, 0, 0, 0, ctx->exh_k, s);
-    CKR(check_launch(ctx, "exhaustive"));
-    if (nl > 1) ctx->launches += uint32_t(nl - 1);
+    CKR(ensure_round(ctx, n, false, &R));
+    RoundArgs* const args = ctx->roundargs.as<RoundArgs>();
     std::vector<uint32_t> rej(n);
-    CK(cudaMemcpyAsync(rej.data(), ctx->rejected.p, 4ull * n, cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamSynchronize(s));
+    for (uint64_t lo = 0; lo < n; lo += R.cap) {  // once, up to the pair slots
+      const uint32_t m = uint32_t(std::min<uint64_t>(n - lo, R.cap));
+      RoundArgs ra{};
+      ra.T = T;
+      ra.T.insn += lo * stride;
+      ra.T.len += lo;
+      ra.T.dead += lo;
+      ra.T.n = m;
+      ra.P = P;
+      ra.P.insn += lo * stride;
+      ra.P.lens += lo;
+      ra.P.n = m;
+      ra.R = R;
+      launch_round_args(ra, args, s);
+      CKR(check_launch(ctx, "round_args"));
+      launch_pairs_identity(m, R, s);
+      CKR(check_launch(ctx, "pairs"));
+      uint32_t np = 0;
+      CKR(sweep_round(ctx, args, ra, m <= kSmallJob, &np));
+      CK(cudaMemcpyAsync(rej.data() + lo, ctx->rejected.p, 4ull * m, cudaMemcpyDeviceToHost, s));
+      CK(cudaStreamSynchronize(s));
+    }
     for (uint32_t i = 0; i < n; i++)
       if (!rej[i]) res[i] |= 4;
   }

@@ -201,30 +201,18 @@ __device__ __forceinline__ unsigned long long pair_units(unsigned long long nblo
   const unsigned long long xu = xunit ? xunit : kUnitBlocks;
   return (keepR & kXIndep) ? (nblocks + xu - 1) / xu : (nblocks + kBitsBlocks - 1) / kBitsBlocks;
 }
-constexpr unsigned long long kMaxChunks = 1ull << 20;
 constexpr int kChunksPerWarp = 16;
-// Work chunks of a sweep: cb A-blocks each (cb is the tuning option), at
-// most kMaxChunks per pair.
-__device__ __forceinline__ unsigned long long chunks_for(unsigned long long nb, uint32_t cb);
-// Chunks of pair p in the numbering of its class (zero in the other one).
-__device__ __forceinline__ void set_chunks(const RoundBuf& R, uint32_t p, const PairRec& pr) {
-  const unsigned long long c = chunks_for(pair_units(pr.nblocks, pr.keepR, R.xunit), R.chunk_blocks);
-  const bool xind = (pr.keepR & kXIndep) != 0;
-  const bool wide = (pr.cmap & kWideClass) != 0;     // only set when R.wide
-  const bool regs = pr.cmap == kRegClass;            // only set when R.wide
-  const bool comp = pr.cmap != 0 && !wide && !regs;  // only set when R.compact
-  const bool other = comp || wide || regs;
-  R.nchunks[p] = (xind || other) ? 0ull : c;
-  R.nchunks_x[p] = (xind && !other) ? c : 0ull;
-  if (R.compact) R.nchunks_c[p] = comp ? c : 0ull;
-  if (R.wide) {
-    R.nchunks_w[p] = wide ? c : 0ull;
-    R.nchunks_r[p] = regs ? c : 0ull;
-  }
+// Work chunks of a sweep: chunk_blocks units each (the tuning option).
+__device__ __forceinline__ uint32_t chunks_for(const RoundBuf& R, unsigned long long units) {
+  const unsigned long long c = (units + R.chunk_blocks - 1) / R.chunk_blocks;
+  return c > R.max_chunks ? R.max_chunks : uint32_t(c);
 }
-__device__ __forceinline__ unsigned long long chunks_for(unsigned long long nb, uint32_t cb) {
-  unsigned long long c = (nb + cb - 1) / cb;
-  return c > kMaxChunks ? kMaxChunks : c;
+// The class of a pair (kClasses).
+__device__ __forceinline__ int pair_class(const PairRec& pr) {
+  if (pr.cmap & kWideClass) return 3;    // only set when R.wide
+  if (pr.cmap == kRegClass) return 4;    // only set when R.wide
+  if (pr.cmap != 0) return 2;            // only set when R.compact
+  return (pr.keepR & kXIndep) ? 1 : 0;
 }
 
 // ------------------------------------------------------------------ kernels
@@ -514,7 +502,7 @@ __device__ __forceinline__ uint32_t alloc_pairs(uint32_t* counter, uint32_t w) {
 // microseconds: planned here, one thread would plan a window's pairs one
 // after the other).
 __device__ __forceinline__ void put_window(const RoundBuf& R, uint32_t p0, uint32_t w, uint32_t t, uint32_t kind,
-                                           const uint32_t* __restrict__ surv, uint32_t sbase) {
+                                           const uint32_t* __restrict__ surv, unsigned long long sbase) {
   for (uint32_t j = 0; j < w; j++) {
     const uint32_t p = p0 + j;
     PairRec pr{};
@@ -522,7 +510,7 @@ __device__ __forceinline__ void put_window(const RoundBuf& R, uint32_t p0, uint3
     pr.cand = surv[sbase + j];
     pr.keepR = kind ? 0x80u : 0u;
     R.pairs[p] = pr;
-    R.pair_src[p] = sbase + j;
+    R.pair_src[p] = uint32_t(sbase + j);
     R.rejected[p] = 0;
     R.wlen[p] = j == 0 ? uint8_t(w) : uint8_t(0);
     if (R.wend) {
@@ -554,69 +542,71 @@ __device__ __forceinline__ void chunk_passed(uint32_t* rejected, const uint32_t*
     if (p + i < e) atomicCAS(&rejected[p + i], 0u, 2u);
 }
 
-// One round of the length-1 pass: each unresolved (target, kind) lane puts
-// its window of next survivors into the round (pairs past the buffer's
-// capacity wait for the next round).
-__global__ void k_round_build(DevTargets T, QCOut q, Lanes L, RoundBuf R) {
-  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-#pragma unroll 1
-  for (uint32_t kind = 0; kind < 2; kind++) {
-    uint32_t w = 0, nx = 0, sbase = 0;
-    if (t < T.n) {
-      const uint32_t cf = q.cnt_f[t], cm = q.cnt_m[t];
-      const uint32_t idx = 2 * t + kind;
-      nx = L.next[idx];
+// One round's pairs: each unresolved (target, kind) lane puts its window of
+// next survivors into the round (pairs past the buffer's capacity wait for
+// the next round).  PAIR: the length-2 pass, whose survivors are in slots.
+template <bool PAIR>
+__global__ void __launch_bounds__(256) k_round_build(const RoundArgs* __restrict__ A) {
+  const RoundBuf& R = A->R;
+  const uint32_t lanes = 2u * A->T.n;
+  const uint32_t stride = gridDim.x * blockDim.x;
+  for (uint32_t base = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); base < lanes; base += stride) {
+    const uint32_t idx = base + lane_id();
+    const uint32_t t = idx >> 1, kind = idx & 1u;
+    uint32_t w = 0;
+    unsigned long long sbase = 0;
+    if (idx < lanes) {
+      const uint32_t nx = A->L.next[idx];
       if (!(nx & kResolved)) {
-        const uint32_t cnt = kind ? cm : cf;
-        if (nx >= cnt) {
-          L.next[idx] = nx | kResolved;
+        uint32_t cnt;
+        if constexpr (PAIR) {
+          cnt = A->ps.cnt[idx];
+          sbase = (unsigned long long)idx * kSlots2 + nx;
         } else {
-          w = min(1u << L.spec[idx], cnt - nx);
-          sbase = q.base[t] + (kind ? cf : 0u) + nx;
+          const uint32_t cf = A->q.cnt_f[t];
+          cnt = kind ? A->q.cnt_m[t] : cf;
+          sbase = cnt ? A->q.base[t] + (kind ? cf : 0u) + nx : 0u;
         }
+        if (nx < cnt) w = min(1u << A->L.spec[idx], cnt - nx);
+        else A->L.next[idx] = nx | kResolved;  // no survivor (left): resolved without a winner
       }
     }
     if (!__any_sync(kFull, w != 0)) continue;
-    const uint32_t p0 = alloc_pairs(R.npairs, w);
+    const uint32_t p0 = alloc_pairs(&R.ctl->npairs, w);
     const uint32_t fit = p0 >= R.cap ? 0u : min(w, R.cap - p0);
-    put_window(R, p0, fit, t, kind, q.surv, sbase);
+    if (fit < w) R.ctl->active = 1;
+    put_window(R, p0, fit, t, kind, PAIR ? A->ps.surv : A->q.surv, sbase);
   }
 }
 
 // pkg/gpu semantics: one pair per MidCheck survivor (all survivors when
-// midpass is null).
-__global__ void k_pairs_from_survivors(DevTargets T, DevPool P, QCOut q, const uint8_t* __restrict__ midpass,
-                                       uint32_t nsurv, const uint32_t* __restrict__ surv_target,
-                                       RoundBuf R) {
-  uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  bool have = false;
-  PairRec pr;
-  if (i < nsurv && (!midpass || midpass[i])) {
-    const uint32_t t = surv_target[i], c = q.surv[i];
-    const uint32_t reads = q.meta[t].reads | P.reads[c];
-    pr.target = t;
-    pr.cand = c;
-    pr.reads = uint16_t(reads);
-    pr.nblocks = plan_blocks(reads, false);
-    pr.keepF = uint8_t(~target_dead(T, t));
-    pr.keepR = uint8_t(~target_dead_regs(T, t) & 0x3Fu);
-    if (pair_xindep(T, t, P, c)) pr.keepR |= uint8_t(kXIndep);
-    pr.cmap = 0;
-    pr.sweepf = 0;
-    have = true;
-  }
-  unsigned b = __ballot_sync(kFull, have);
-  if (!b) return;
-  uint32_t base = 0;
-  if (lane_id() == 0) base = atomicAdd(R.npairs, (uint32_t)__popc(b));
-  base = __shfl_sync(kFull, base, 0);
-  if (have) {
-    uint32_t p = base + __popc(b & lanemask_lt());
-    R.pairs[p] = pr;
-    R.pair_src[p] = i;
-    set_chunks(R, p, pr);
-    R.rejected[p] = 0;
-  }
+// midpass is null) of [lo, hi).
+__global__ void k_pairs_from_survivors(QCOut q, const uint8_t* __restrict__ midpass, uint32_t lo, uint32_t hi,
+                                       const uint32_t* __restrict__ surv_target, RoundBuf R) {
+  const uint32_t i = lo + blockIdx.x * blockDim.x + threadIdx.x;
+  const bool have = i < hi && (!midpass || midpass[i]);
+  if (!__any_sync(kFull, have)) return;
+  const uint32_t p = alloc_pairs(&R.ctl->npairs, have ? 1u : 0u);
+  if (!have || p >= R.cap) return;
+  PairRec pr{};
+  pr.target = surv_target[i];
+  pr.cand = q.surv[i];
+  pr.keepR = 0x80u;  // compared under the target's dead masks
+  R.pairs[p] = pr;
+  R.pair_src[p] = i;
+  R.rejected[p] = 0;
+}
+// Independent pairs (i, i) of a target batch and a pool of as many.
+__global__ void k_pairs_identity(uint32_t n, RoundBuf R) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i == 0) R.ctl->npairs = n;
+  if (i >= n) return;
+  PairRec pr{};
+  pr.target = i;
+  pr.cand = i;
+  pr.keepR = 0x80u;
+  R.pairs[i] = pr;
+  R.rejected[i] = 0;
 }
 
 // K = states per lane per dispatch ("vectors per lane").  One warp
@@ -770,8 +760,14 @@ __device__ __forceinline__ bool probe_pair(const DevTargets& T, const DevPool& P
 // 0.9 ms.  The probe and the polls between units: 40,009 uneven targets
 // evaluate 4.5e8 states where it was 1.6e10 (84 -> 43 ms of sweeps), the
 // 9.4M length-2 targets 2.7e8 where it was 1.3e9 (3.2 -> 2.05 ms).
-__global__ void __launch_bounds__(128) k_pair_plan(DevTargets T, DevPool P, QCOut q, RoundBuf R) {
-  const uint32_t np = min(*R.npairs, R.cap);
+// The chunks of a pair go to its class's list (RoundCtl::alloc), one atomic
+// per warp and class.
+__global__ void __launch_bounds__(128) k_pair_plan(const RoundArgs* __restrict__ A) {
+  const RoundBuf& R = A->R;
+  const DevTargets& T = A->T;
+  const DevPool& P = A->P;
+  const uint32_t np = min(R.ctl->npairs, R.cap);
+  if (blockIdx.x == 0 && threadIdx.x == 0) R.ctl->nscan = 0;  // the rescan before this round has read it
   const unsigned lane = lane_id();
   const uint32_t nw = gridDim.x * (blockDim.x >> 5);
   const uint32_t gw = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -787,11 +783,19 @@ __global__ void __launch_bounds__(128) k_pair_plan(DevTargets T, DevPool P, QCOu
       pr = R.pairs[p];
       const uint32_t t = pr.target, c = pr.cand;
       const bool masked = (pr.keepR & 0x80u) != 0;
-      const uint32_t reads = q.meta[t].reads | P.reads[c];
+      const uint32_t* tw = T.insn + (size_t)t * T.stride;
+      const uint32_t* cw = P.insn + (size_t)c * P.stride;
+      const uint32_t tl = target_len(T, t), cl = pool_len(P, c);
+      uint32_t reads = 0;
+      if (P.reads) {
+        reads = A->q.meta[t].reads | P.reads[c];
+      } else {
+        for (uint32_t i = 0; i < tl; i++) reads |= g_ops[tw[i] & 0xFFFFu].reads;
+        for (uint32_t i = 0; i < cl; i++) reads |= g_ops[cw[i] & 0xFFFFu].reads;
+      }
       pr.keepF = masked ? uint8_t(~target_dead(T, t)) : uint8_t(0xFFu);
       pr.keepR = masked ? uint8_t((~target_dead_regs(T, t) & 0x3Fu) | 0x80u) : uint8_t(0x3Fu);
-      const PairPlan pl = plan_pair(g_flow, T.insn + (size_t)t * T.stride, target_len(T, t),
-                                    P.insn + (size_t)c * P.stride, pool_len(P, c), reads, pr.keepF, pr.keepR);
+      const PairPlan pl = plan_pair(g_flow, tw, tl, cw, cl, reads, pr.keepF, pr.keepR);
       pr.reads = pl.reads;
       pr.sweepf = pl.sweepf;
       pr.nblocks = pl.nblocks;
@@ -828,9 +832,28 @@ __global__ void __launch_bounds__(128) k_pair_plan(DevTargets T, DevPool P, QCOu
         R.rejected[p] = 1;
       }
     }
-    if (mine) {
-      R.pairs[p] = pr;
-      set_chunks(R, p, pr);
+    if (mine) R.pairs[p] = pr;
+    // chunk lists
+    const uint32_t ch = mine && pr.nblocks ? chunks_for(R, pair_units(pr.nblocks, pr.keepR, R.xunit)) : 0u;
+    const int cls = ch ? pair_class(pr) : -1;
+    for (int c = 0; c < kClasses; c++) {
+      const unsigned b = __ballot_sync(kFull, cls == c);
+      if (!b) continue;
+      uint32_t incl = cls == c ? ch : 0u;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t v = __shfl_up_sync(kFull, incl, o);
+        if (lane >= unsigned(o)) incl += v;
+      }
+      unsigned long long at = 0;
+      if (lane == 31)
+        at = atomicAdd(&R.ctl->alloc[c], (unsigned long long)__popc(b) << kChunkBits | incl);
+      at = __shfl_sync(kFull, at, 31);
+      if (cls == c) {
+        const uint32_t e = uint32_t(at >> kChunkBits) + __popc(b & lanemask_lt());
+        R.cbase[c][e] = (at & kChunkMask) + incl - ch;
+        R.cpair[c][e] = p;
+      }
     }
   }
 #pragma unroll
@@ -1412,21 +1435,19 @@ __device__ __noinline__ bool xindep_unit(unsigned long long first, unsigned long
 // 5 the rest that name neither SP nor the memory byte, on A, F and B..L; each class
 // draws chunks from its own numbering and dispenser.  Kept apart so that
 // neither path's registers weigh on the other.
-// dev_total / dev_np (device-driven rounds): the class's chunk total and the
-// round's pair count are read from the device instead of total / npairs.
 // chunks_per_warp: chunks a warp takes before its block retires.
 #ifndef Z80B_REG_BLOCKS
 #define Z80B_REG_BLOCKS 2
 #endif
-// The pair whose chunk range holds chunk k: the last p with cbase[p] <= k
-// (cbase ascending from cbase[0] = 0; pairs without chunks in the class
-// repeat their successor's base).  Warp-wide, k the same in every lane: each
-// step the 32 lanes probe 32 evenly spaced pairs of the range left and a
-// ballot keeps the span after the last probe that is <= k, so a round of n
-// pairs takes ceil(log32 n) dependent loads instead of log2 n.
-__device__ __forceinline__ uint32_t chunk_pair(const unsigned long long* __restrict__ cbase, uint32_t npairs,
-                                               unsigned long long k, unsigned lane) {
-  uint32_t lo = 0, n = npairs;  // the answer lies in [lo, lo + n); cbase[lo] <= k
+// The entry of a class's chunk list whose range holds chunk k: the last e
+// with cbase[e] <= k (cbase ascending from cbase[0] = 0).  Warp-wide, k the
+// same in every lane: each step the 32 lanes probe 32 evenly spaced entries
+// of the range left and a ballot keeps the span after the last probe that is
+// <= k, so a list of n entries takes ceil(log32 n) dependent loads instead
+// of log2 n.
+__device__ __forceinline__ uint32_t chunk_entry(const unsigned long long* __restrict__ cbase, uint32_t n,
+                                                unsigned long long k, unsigned lane) {
+  uint32_t lo = 0;  // the answer lies in [lo, lo + n); cbase[lo] <= k
   while (n > 1) {
     const uint32_t step = (n + 31u) / 32u;
     const uint32_t off = lane * step;
@@ -1440,62 +1461,61 @@ __device__ __forceinline__ uint32_t chunk_pair(const unsigned long long* __restr
 }
 template <int K, int CLS>
 __global__ void __launch_bounds__(kBlock, CLS == 3 ? 3 : (CLS == 4 ? 2 : (CLS == 5 ? Z80B_REG_BLOCKS : 1)))
-    k_exhaustive(DevTargets T, DevPool P, RoundBuf R, uint32_t npairs, unsigned long long total,
-                 const unsigned long long* __restrict__ dev_total, const uint32_t* __restrict__ dev_np,
-                 int chunks_per_warp) {
+    k_exhaustive(const __grid_constant__ SweepArgs A, int chunks_per_warp) {
   static_assert(K == 1 || K == 2 || K == 4 || K == 8, "K divides 8");
-  if (dev_total) {
-    total = *dev_total;
-    npairs = *dev_np;
-  }
   constexpr bool XI = CLS != 0;
-  const unsigned long long* __restrict__ cbase =
-      CLS == 5 ? R.cbase_r : (CLS == 4 ? R.cbase_w : (CLS == 3 ? R.cbase_c : (XI ? R.cbase_x : R.cbase)));
-  unsigned long long* const dispenser = R.counter + (CLS >= 3 ? CLS - 1 : (XI ? 1 : 0));
+  constexpr int kList = CLS >= 3 ? CLS - 1 : (XI ? 1 : 0);
+  const unsigned long long alloc = A.ctl->alloc[kList], total = alloc & kChunkMask;
+  const uint32_t entries = uint32_t(alloc >> kChunkBits);
   const unsigned lane = lane_id();
-  unsigned long long my_states = 0, my_eval = 0;
+  __shared__ unsigned long long tally[kBlock / 32][2];  // per warp: reference states covered, states evaluated
+  if (lane < 2) tally[threadIdx.x >> 5][lane] = 0;
+  __syncwarp();
   // At most kChunksPerWarp chunks per warp, then the block retires: the grid
   // covers all chunks, and blocks of kernels on other streams (with a higher
   // priority) get SMs as soon as blocks of a long sweep retire.
   for (int taken = 0; taken < chunks_per_warp; taken++) {
     unsigned long long k = 0;
-    if (lane == 0) k = atomicAdd(dispenser, 1ull);
+    if (lane == 0) k = atomicAdd(&A.ctl->counter[kList], 1ull);
     k = __shfl_sync(kFull, k, 0);
     if (k >= total) break;
-    // pair p: cbase[p] <= k < cbase[p + 1]
-    const uint32_t p = chunk_pair(cbase, npairs, k, lane);
+    const uint32_t e = chunk_entry(A.cbase[kList], entries, k, lane);
+    const uint32_t p = A.cpair[kList] ? A.cpair[kList][e] : e;
+    const unsigned long long c0 = A.cbase[kList][e];
+    const uint32_t nch = uint32_t((e + 1 < entries ? A.cbase[kList][e + 1] : total) - c0);
+    volatile uint32_t* const flag = A.rejected + p;
     // lane 0 reads the flag and the warp acts on one value, so the
     // shuffles below always see all 32 lanes
-    if (__shfl_sync(kFull, lane == 0 ? *reinterpret_cast<volatile uint32_t*>(&R.rejected[p]) : 0u, 0)) {
+    if (__shfl_sync(kFull, lane == 0 ? *flag : 0u, 0)) {
       // The pair is settled: the dispenser jumps over what is left of its
       // chunks.  A pair of 2^20 chunks that fails in its first ones had them
       // all drawn one by one (1 ns each: 2 ms a round for two such pairs;
       // 40,009 uneven targets, 243 rounds: 196 ms of sweeps, with the jump
       // 84 ms).
-      if (lane == 0) atomicMax(dispenser, p + 1 < npairs ? cbase[p + 1] : total);
+      if (lane == 0) atomicMax(&A.ctl->counter[kList], c0 + nch);
       continue;
     }
-    const PairRec pr = R.pairs[p];
-    const unsigned long long nunits = pair_units(pr.nblocks, pr.keepR, R.xunit);
-    const unsigned long long nch = (p + 1 < npairs ? cbase[p + 1] : total) - cbase[p];
-    const unsigned long long upc = (nunits + nch - 1) / nch;
-    const unsigned long long j = k - cbase[p];
-    const unsigned long long u0 = j * upc;
-    unsigned long long u1 = u0 + upc;
-    if (u1 > nunits) u1 = nunits;
+    const PairRec pr = A.pairs[p];
+    unsigned long long u0;
+    uint32_t units;
+    {
+      const unsigned long long nunits = pair_units(pr.nblocks, pr.keepR, A.xunit);
+      const unsigned long long upc = (nunits + nch - 1) / nch;
+      u0 = (k - c0) * upc;
+      units = u0 < nunits ? uint32_t(min(upc, nunits - u0)) : 0u;
+    }
 
     // programs: lanes 0..tl-1 target, tl..tl+cl-1 candidate
-    const uint32_t tl = target_len(T, pr.target), cl = pool_len(P, pr.cand);
+    const uint32_t tl = A.tlens ? A.tlens[pr.target] : A.tlen, cl = A.plens ? A.plens[pr.cand] : A.plen;
     uint32_t pw = 0;
-    if (lane < tl) pw = T.insn[(size_t)pr.target * T.stride + lane];
-    else if (lane < tl + cl) pw = P.insn[(size_t)pr.cand * P.stride + (lane - tl)];
+    if (lane < tl) pw = A.tinsn[(size_t)pr.target * A.tstride + lane];
+    else if (lane < tl + cl) pw = A.pinsn[(size_t)pr.cand * A.pstride + (lane - tl)];
 
     // sweep shape (verifier.go:428-476): extra registers in B,C,D,E,H,L,M order
     const uint32_t ext = pr.reads & (kRegB | kRegC | kRegD | kRegE | kRegH | kRegL | kRegM);
     const int nx = __popc(ext);
     const bool spw = (pr.reads & kRegSP) != 0;
     const bool reduced = spw || nx > 2 || (pr.sweepf & 0x80u) != 0;
-    const uint32_t xs = pr.sweepf & 0x3Fu;  // reference states per evaluated state, log2
     const int fw = reduced ? 5 : 8;  // bits per swept register in the block index
     int slot[7];
     {
@@ -1506,124 +1526,84 @@ __global__ void __launch_bounds__(kBlock, CLS == 3 ? 3 : (CLS == 4 ? 2 : (CLS ==
     }
     const BDec bd = bdec_make(spw, reduced, nx, fw, slot);
     // compared bytes of the packed words (A F B C / D E H L / SP M)
-    const uint32_t keep0 = 0xFFu | (uint32_t(pr.keepF) << 8) | ((pr.keepR & 1u) ? 0xFF0000u : 0u) |
+    [[maybe_unused]] const uint32_t keep0 = 0xFFu | (uint32_t(pr.keepF) << 8) | ((pr.keepR & 1u) ? 0xFF0000u : 0u) |
                            ((pr.keepR & 2u) ? 0xFF000000u : 0u);
-    const uint32_t keep1 = ((pr.keepR & 4u) ? 0xFFu : 0u) | ((pr.keepR & 8u) ? 0xFF00u : 0u) |
-                           ((pr.keepR & 16u) ? 0xFF0000u : 0u) | ((pr.keepR & 32u) ? 0xFF000000u : 0u);
+    [[maybe_unused]] const uint32_t keep1 =
+        ((pr.keepR & 4u) ? 0xFFu : 0u) | ((pr.keepR & 8u) ? 0xFF00u : 0u) | ((pr.keepR & 16u) ? 0xFF0000u : 0u) |
+        ((pr.keepR & 32u) ? 0xFF000000u : 0u);
 
-    bool bad = false;
-    // The pair's flag, asked for before a unit and looked at after it, so
+    bool bad = false;      // a unit of this chunk has a mismatch
+    bool stopped = false;  // left the chunk on the pair's flag (rejected or cancelled elsewhere)
+    uint32_t done = 0;     // units swept
+    // The pair's flag is asked for before a unit and looked at after it, so
     // that the read's latency passes behind the unit: a rejected pair costs
     // each warp one unit, not a batch of them between two polls.
-    auto poll = [&]() { return lane == 0 ? *reinterpret_cast<volatile uint32_t*>(&R.rejected[p]) : 0u; };
-    bool stopped = false;  // left the loop on the pair's flag (rejected or cancelled elsewhere)
-    if constexpr (CLS == 5) {
-      // the register state (A, F, B..L), programs as they are
-      extern __shared__ uint32_t zsm[];
-      uint32_t* sm = zsm + (threadIdx.x >> 5) * (kRegWords * 32) + lane;
-      if (pr.keepR & kXIndep) {
-        int rlast = -1;  // the register of the last swept field (the fastest)
-#pragma unroll
-        for (int r = 0; r < 6; r++)
-          if (slot[r] == nx - 1) rlast = r;
-        for (unsigned long long u = u0; u < u1; u++) {
-          const uint32_t settled = poll();
-          const unsigned long long first = u * kXBitsBlocks;
-          const unsigned long long nb = (pr.nblocks - first < kXBitsBlocks) ? pr.nblocks - first : kXBitsBlocks;
-          bad = rxbits_unit(u, pr.nblocks, reduced, nx, rlast, bd, pw, int(tl), int(cl), pr.keepF, pr.keepR, sm) ||
-                bad;
-          my_states += (256ull * nb) << xs;
-          my_eval += 2ull * nb;
-          if (__any_sync(kFull, bad)) break;
-          if (__shfl_sync(kFull, settled, 0)) {
-            stopped = true;
-            break;
-          }
-        }
-      } else {
-        for (unsigned long long u = u0; u < u1; u++) {
-          const uint32_t settled = poll();
-          const unsigned long long first = u * kBitsBlocks;
-          const unsigned long long nb = (pr.nblocks - first < kBitsBlocks) ? pr.nblocks - first : kBitsBlocks;
-          bad = rbits_unit(u, pr.nblocks, bd, pw, int(tl), int(cl), pr.keepF, pr.keepR, sm) || bad;
-          my_states += (256ull * nb) << xs;
-          my_eval += 256ull * nb;
-          if (__any_sync(kFull, bad)) break;
-          if (__shfl_sync(kFull, settled, 0)) {
-            stopped = true;
-            break;
-          }
-        }
-      }
-    } else if constexpr (CLS == 4) {
-      // the wide compact state, the programs renamed onto B, C, H and L
-      const uint32_t e = (pr.cmap & ~uint32_t(kWideClass)) - 1u;
-      if (lane < tl + cl) pw = (uint32_t(uint16_t(g_wren[e][pw & 0xFFFFu]))) | (pw & 0xFFFF0000u);
-      int o[4];
-      uint32_t cmp = 0;
-#pragma unroll
-      for (int f = 0; f < 4; f++) {
-        o[f] = g_worig[e][f];
-        if (o[f] >= 0 && ((pr.keepR >> o[f]) & 1u)) cmp |= 1u << f;
-      }
-      extern __shared__ uint32_t zsm[];
-      uint32_t* sm = zsm + (threadIdx.x >> 5) * (kWideWords * 32) + lane;
-      const WDec dec = wdec_make(nx, reduced, slot, o);
-      for (unsigned long long u = u0; u < u1; u++) {
-        const uint32_t settled = poll();
-        const unsigned long long first = u * kBitsBlocks;
-        const unsigned long long nb = (pr.nblocks - first < kBitsBlocks) ? pr.nblocks - first : kBitsBlocks;
-        bad = wbits_unit(u, pr.nblocks, dec, pw, int(tl), int(cl), pr.keepF, cmp, sm) || bad;
-        my_states += (256ull * nb) << xs;
-        my_eval += 256ull * nb;
-        if (__any_sync(kFull, bad)) break;
+    auto sweep = [&](auto unit) {
+      while (done < units) {
+        const uint32_t settled = lane == 0 ? *flag : 0u;
+        bad = __any_sync(kFull, unit(u0 + done));
+        done++;
+        if (bad) break;
         if (__shfl_sync(kFull, settled, 0)) {
           stopped = true;
           break;
         }
       }
+    };
+    extern __shared__ uint32_t zsm[];  // the candidate's output planes, a column per lane
+    const bool xind = (pr.keepR & kXIndep) != 0;
+    if constexpr (CLS == 5) {
+      // the register state (A, F, B..L), programs as they are
+      uint32_t* sm = zsm + (threadIdx.x >> 5) * (kRegWords * 32) + lane;
+      if (xind) {
+        int rlast = -1;  // the register of the last swept field (the fastest)
+#pragma unroll
+        for (int r = 0; r < 6; r++)
+          if (slot[r] == nx - 1) rlast = r;
+        sweep([&](unsigned long long u) {
+          return rxbits_unit(u, pr.nblocks, reduced, nx, rlast, bd, pw, int(tl), int(cl), pr.keepF, pr.keepR, sm);
+        });
+      } else {
+        sweep([&](unsigned long long u) {
+          return rbits_unit(u, pr.nblocks, bd, pw, int(tl), int(cl), pr.keepF, pr.keepR, sm);
+        });
+      }
+    } else if constexpr (CLS == 4) {
+      // the wide compact state, the programs renamed onto B, C, H and L
+      const uint32_t set = (pr.cmap & ~uint32_t(kWideClass)) - 1u;
+      if (lane < tl + cl) pw = (uint32_t(uint16_t(g_wren[set][pw & 0xFFFFu]))) | (pw & 0xFFFF0000u);
+      int o[4];
+      uint32_t cmp = 0;
+#pragma unroll
+      for (int f = 0; f < 4; f++) {
+        o[f] = g_worig[set][f];
+        if (o[f] >= 0 && ((pr.keepR >> o[f]) & 1u)) cmp |= 1u << f;
+      }
+      uint32_t* sm = zsm + (threadIdx.x >> 5) * (kWideWords * 32) + lane;
+      const WDec dec = wdec_make(nx, reduced, slot, o);
+      sweep([&](unsigned long long u) {
+        return wbits_unit(u, pr.nblocks, dec, pw, int(tl), int(cl), pr.keepF, cmp, sm);
+      });
     } else if constexpr (CLS == 3) {
       // the compact state, the programs renamed onto B and C
-      const uint32_t e = pr.cmap - 1u;
-      if (lane < tl + cl) pw = (uint32_t(uint16_t(g_cren[e][pw & 0xFFFFu]))) | (pw & 0xFFFF0000u);
-      const int o0 = g_corig[e][0], o1 = g_corig[e][1];
-      extern __shared__ uint32_t zsm[];
+      const uint32_t set = pr.cmap - 1u;
+      if (lane < tl + cl) pw = (uint32_t(uint16_t(g_cren[set][pw & 0xFFFFu]))) | (pw & 0xFFFF0000u);
+      const int o0 = g_corig[set][0], o1 = g_corig[set][1];
       uint32_t* sm = zsm + (threadIdx.x >> 5) * (kCompactWords * 32) + lane;
       const CDec dec = cdec_make(nx, slot, o0, o1);
-      if (pr.keepR & kXIndep) {
+      if (xind) {
         // A-independent: units of 1,024 A-blocks, each at A = 0 and 1
         int rlast = -1;
 #pragma unroll
         for (int r = 0; r < 7; r++)
           if (slot[r] == nx - 1) rlast = r;
-        for (unsigned long long u = u0; u < u1; u++) {
-          const uint32_t settled = poll();
-          const unsigned long long first = u * kXBitsBlocks;
-          const unsigned long long nb = (pr.nblocks - first < kXBitsBlocks) ? pr.nblocks - first : kXBitsBlocks;
-          bad = cxbits_unit(u, pr.nblocks, nx, dec, rlast, pw, int(tl), int(cl), pr.keepF, pr.keepR, o0, o1, sm) ||
-                bad;
-          my_states += (256ull * nb) << xs;
-          my_eval += 2ull * nb;
-          if (__any_sync(kFull, bad)) break;
-          if (__shfl_sync(kFull, settled, 0)) {
-            stopped = true;
-            break;
-          }
-        }
+        sweep([&](unsigned long long u) {
+          return cxbits_unit(u, pr.nblocks, nx, dec, rlast, pw, int(tl), int(cl), pr.keepF, pr.keepR, o0, o1, sm);
+        });
       } else {
-        for (unsigned long long u = u0; u < u1; u++) {
-          const uint32_t settled = poll();
-          const unsigned long long first = u * kBitsBlocks;
-          const unsigned long long nb = (pr.nblocks - first < kBitsBlocks) ? pr.nblocks - first : kBitsBlocks;
-          bad = cbits_unit(u, pr.nblocks, dec, pw, int(tl), int(cl), pr.keepF, pr.keepR, o0, o1, sm) || bad;
-          my_states += (256ull * nb) << xs;
-          my_eval += 256ull * nb;
-          if (__any_sync(kFull, bad)) break;
-          if (__shfl_sync(kFull, settled, 0)) {
-            stopped = true;
-            break;
-          }
-        }
+        sweep([&](unsigned long long u) {
+          return cbits_unit(u, pr.nblocks, dec, pw, int(tl), int(cl), pr.keepF, pr.keepR, o0, o1, sm);
+        });
       }
     } else if constexpr (!XI) {
       // Unit = 4 A-blocks, bit-sliced (256 states of each block in 8 lanes).
@@ -1631,98 +1611,123 @@ __global__ void __launch_bounds__(kBlock, CLS == 3 ? 3 : (CLS == 4 ? 2 : (CLS ==
       // last register, SP (verifier.go:498-531,578-610); the block index
       // varies SP and the last register fastest, so a sweep the reference
       // abandons early is abandoned early here too.
-      extern __shared__ uint32_t zsm[];
       uint32_t* sm = zsm + (threadIdx.x >> 5) * (kBitsWords * 32) + lane;
-      for (unsigned long long u = u0; u < u1; u++) {
-        const uint32_t settled = poll();
-        const unsigned long long first = u * kBitsBlocks;
-        const unsigned long long nb = (pr.nblocks - first < kBitsBlocks) ? pr.nblocks - first : kBitsBlocks;
-        bad = bits_unit(u, pr.nblocks, bd, pw, int(tl), int(cl), pr.keepF, pr.keepR, sm) || bad;
-        my_states += (256ull * nb) << xs;
-        my_eval += 256ull * nb;
-        if (__any_sync(kFull, bad)) break;
-        if (__shfl_sync(kFull, settled, 0)) {
-          stopped = true;
-          break;
-        }
-      }
+      sweep([&](unsigned long long u) {
+        return bits_unit(u, pr.nblocks, bd, pw, int(tl), int(cl), pr.keepF, pr.keepR, sm);
+      });
     } else if constexpr (CLS == 2) {
       // Unit = 1,024 A-blocks, 32 per lane, each at A = 0 and A = 1.
-      extern __shared__ uint32_t zsm[];
       uint32_t* sm = zsm + (threadIdx.x >> 5) * (kBitsWords * 32) + lane;
       int rlast = -1;  // the register of the last swept field (the fastest)
 #pragma unroll
       for (int r = 0; r < 7; r++)
         if (slot[r] == nx - 1) rlast = r;
-      for (unsigned long long u = u0; u < u1; u++) {
-        const uint32_t settled = poll();
-        const unsigned long long first = u * kXBitsBlocks;
-        const unsigned long long nb = (pr.nblocks - first < kXBitsBlocks) ? pr.nblocks - first : kXBitsBlocks;
-        bad = xbits_unit(u, pr.nblocks, spw, reduced, nx, fw, slot, rlast, pw, int(tl), int(cl), pr.keepF,
-                         pr.keepR, sm) ||
-              bad;
-        my_states += (256ull * nb) << xs;
-        my_eval += 2ull * nb;
-        if (__any_sync(kFull, bad)) break;
-        if (__shfl_sync(kFull, settled, 0)) {
-          stopped = true;
-          break;
-        }
-      }
+      sweep([&](unsigned long long u) {
+        return xbits_unit(u, pr.nblocks, spw, reduced, nx, fw, slot, rlast, pw, int(tl), int(cl), pr.keepF, pr.keepR,
+                          sm);
+      });
     } else {
       // Unit = 128 A-blocks, each evaluated at A = 0 and A = 1: state slot s
       // of the warp (s = (i*K + q)*32 + lane) takes block unit*128 + s/2 with
       // A = s & 1.
-      for (unsigned long long u = u0; u < u1; u++) {
-        const uint32_t settled = poll();
+      sweep([&](unsigned long long u) {
         const unsigned long long first = u * kUnitBlocks;
         const unsigned long long nb = (pr.nblocks - first < kUnitBlocks) ? pr.nblocks - first : kUnitBlocks;
-        bad = xindep_unit<K>(first, nb, bd, pw, int(tl), int(cl), keep0, keep1) || bad;
-        my_states += (256ull * nb) << xs;
-        my_eval += 2ull * nb;
-        if (__any_sync(kFull, bad)) break;
-        if (__shfl_sync(kFull, settled, 0)) {
-          stopped = true;
-          break;
-        }
-      }
+        return xindep_unit<K>(first, nb, bd, pw, int(tl), int(cl), keep0, keep1);
+      });
     }
-    const bool any_bad = __any_sync(kFull, bad);
     if (lane == 0) {
-      if (any_bad) atomicExch(&R.rejected[p], 1u);
-      else if (!stopped && R.wend)
-        chunk_passed(R.rejected, R.wend, R.cdone, p,
-                     uint32_t((p + 1 < npairs ? cbase[p + 1] : total) - cbase[p]));
+      const unsigned long long per = xind ? (A.xunit ? A.xunit : kUnitBlocks) : kBitsBlocks;
+      const unsigned long long lo = u0 * per, hi = min(pr.nblocks, (u0 + done) * per);
+      tally[threadIdx.x >> 5][0] += ((hi - lo) * 256ull) << (pr.sweepf & 0x3Fu);
+      tally[threadIdx.x >> 5][1] += (hi - lo) * (xind ? 2ull : 256ull);
+      if (bad) *flag = 1u;
+      else if (!stopped && A.wend) chunk_passed(A.rejected, A.wend, A.cdone, p, nch);
     }
   }
-  if (lane == 0 && my_states) {
-    atomicAdd(R.states, my_states);
-    atomicAdd(R.states + 1, my_eval);
+  if (lane == 0 && tally[threadIdx.x >> 5][0]) {
+    atomicAdd(A.states, tally[threadIdx.x >> 5][0]);
+    atomicAdd(A.states + 1, tally[threadIdx.x >> 5][1]);
   }
 }
 // Window heads settle their lane: the first pair of the window that passed
-// wins; if none did, the lane moves past the window and the next window
-// doubles (up to 2^max_spec).
-__global__ void k_round_resolve(RoundBuf R, uint32_t npairs, QCOut q, Lanes L, uint32_t max_spec,
-                                const uint32_t* __restrict__ dev_np) {
-  const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (dev_np) npairs = *dev_np;
-  if (p >= npairs) return;
-  const uint32_t w = R.wlen[p];
-  if (w == 0) return;
-  const PairRec pr = R.pairs[p];
-  const uint32_t idx = 2 * pr.target + ((pr.keepR & 0x80u) ? 1u : 0u);
-  for (uint32_t j = 0; j < w; j++) {
-    if (R.rejected[p + j] == 0) {
+// wins; if none did, the lane moves past the window, the next window doubles
+// (up to 2^max_spec), and a lane with nothing left is resolved without a
+// winner.  PAIR: a lane whose slots are used up but not its pairs waits for a
+// rescan.
+template <bool PAIR>
+__global__ void __launch_bounds__(256) k_round_resolve(const RoundArgs* __restrict__ A) {
+  const RoundBuf& R = A->R;
+  const Lanes& L = A->L;
+  const uint32_t np = min(R.ctl->npairs, R.cap);
+  for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < np; p += gridDim.x * blockDim.x) {
+    const uint32_t w = R.wlen[p];
+    if (w == 0) continue;
+    const PairRec pr = R.pairs[p];
+    const uint32_t kind = (pr.keepR & 0x80u) ? 1u : 0u;
+    const uint32_t idx = 2 * pr.target + kind;
+    uint32_t j = 0;
+    while (j < w && R.rejected[p + j] != 0) j++;
+    if (j < w) {
       L.win[idx] = R.pairs[p + j].cand;
-      L.windiff[idx] = q.sdiff[R.pair_src[p + j]];
+      L.windiff[idx] = A->sdiff[R.pair_src[p + j]];
       L.next[idx] = (L.next[idx] + j) | kResolved;
-      return;
+      continue;
     }
+    const uint32_t nx = L.next[idx] + w;
+    if (L.spec[idx] < A->max_spec) L.spec[idx] += 1;
+    bool left;
+    if constexpr (PAIR) {
+      left = nx < A->ps.cnt[idx];
+      if (!left && A->ps.resume[idx] != kNone) {
+        left = true;
+        A->ps.scan[atomicAdd(&R.ctl->nscan, 1u)] = idx;
+      }
+    } else {
+      left = nx < (kind ? A->q.cnt_m[pr.target] : A->q.cnt_f[pr.target]);
+    }
+    L.next[idx] = left ? nx : nx | kResolved;
+    if (left) R.ctl->active = 1;
   }
-  L.next[idx] += w;
-  if (L.spec[idx] < max_spec) L.spec[idx] += 1;
 }
+// The counters of the round that ended and a clean slate for the next one;
+// in a loop, its condition.
+template <bool LOOP>
+__global__ void k_round_end(const RoundArgs* __restrict__ A, cudaGraphConditionalHandle loop) {
+  RoundCtl& c = *A->R.ctl;
+  const unsigned lane = lane_id();
+  if (lane < kClasses) {
+    c.alloc[lane] = 0;
+    c.counter[lane] = 0;
+  }
+  if (lane != 0) return;
+  const uint32_t np = min(c.npairs, A->R.cap);
+  c.iters += 1;
+  c.np = np;
+  if (np) {
+    c.rounds += 1;
+    c.pairs += np;
+  }
+  uint32_t more = c.active;
+  if (more && c.iters >= kMaxRoundIters) {
+    // the loop has run far past any legitimate number of rounds: end it and
+    // let the host report the error
+    c.overrun = 1;
+    more = 0;
+  }
+  c.more = more;
+  c.npairs = 0;
+  c.active = 0;
+  if (LOOP && !more) cudaGraphSetConditional(loop, 0);
+}
+__global__ void k_round_args(RoundArgs a, RoundArgs* __restrict__ dst) {
+  const uint32_t* s = reinterpret_cast<const uint32_t*>(&a);
+  uint32_t* d = reinterpret_cast<uint32_t*>(dst);
+  for (uint32_t i = threadIdx.x; i < sizeof(RoundArgs) / 4; i += blockDim.x) d[i] = s[i];
+  uint32_t* c = reinterpret_cast<uint32_t*>(a.R.ctl);
+  for (uint32_t i = threadIdx.x; i < sizeof(RoundCtl) / 4; i += blockDim.x) c[i] = 0u;
+}
+static_assert(sizeof(RoundArgs) % 4 == 0 && sizeof(RoundCtl) % 4 == 0, "copied by words");
 
 __global__ void k_midcheck(DevTargets T, DevPool P, const uint32_t* __restrict__ surv,
                            const uint32_t* __restrict__ surv_target, uint32_t nsurv, uint8_t* __restrict__ pass) {
@@ -2263,16 +2268,17 @@ __device__ __forceinline__ uint32_t warp_sort(uint32_t x) {
 // the groups of one large bucket.  A walk over the bucket's pairs instead
 // (20.5M pairs, one output compared at a time, one warp per target) took
 // 147 ms for 10,007 uneven targets.
-__global__ void __launch_bounds__(kBlock) k_pair_scan(DevTargets T, QCOut q1, Lanes L2, PairScan ps,
-                                                      const RoundCtl* __restrict__ gate) {
-  if (gate && gate->np != 0) return;  // device-driven rounds: rescan only after an empty round
+__global__ void __launch_bounds__(kBlock) k_pair_scan(const RoundArgs* __restrict__ A, bool all) {
+  const DevTargets& T = A->T;
+  const PairScan& ps = A->ps;
   const unsigned lane = lane_id();
   const uint32_t gw = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const uint32_t nw = gridDim.x * (blockDim.x >> 5);
-  for (uint32_t idx = gw; idx < 2u * T.n; idx += nw) {
+  const uint32_t lanes = all ? 2u * T.n : A->R.ctl->nscan;
+  for (uint32_t i = gw; i < lanes; i += nw) {
+    const uint32_t idx = all ? i : ps.scan[i];
     const uint32_t resume = ps.resume[idx];
-    const uint32_t nx = L2.next[idx];
-    if ((nx & kResolved) || nx < ps.cnt[idx] || resume == kNone) continue;
+    if ((A->L.next[idx] & kResolved) || resume == kNone) continue;
     const uint32_t t = idx >> 1, kind = idx & 1u;
     const uint32_t tl = target_len(T, t);
     const uint32_t pw = lane < tl ? T.insn[(size_t)t * T.stride + lane] : 0u;
@@ -2280,7 +2286,7 @@ __global__ void __launch_bounds__(kBlock) k_pair_scan(DevTargets T, QCOut q1, La
     run_lanes(st, pw, 0, int(tl));
     uint32_t w[3];  // the target's output on vector lane & 7
     z_pack(st, w);
-    const uint32_t tb = q1.meta[t].bytes;
+    const uint32_t tb = A->q.meta[t].bytes;
     const uint32_t dead = kind ? target_dead(T, t) & 0xFFu : 0u;
     const uint32_t dregs = kind ? target_dead_regs(T, t) & 0x3Fu : 0u;
     const uint32_t k0 = key_keep0(dregs), k1 = key_keep1(dregs);
@@ -2383,39 +2389,12 @@ __global__ void __launch_bounds__(kBlock) k_pair_scan(DevTargets T, QCOut q1, La
     const uint32_t found = __popc(__ballot_sync(kFull, best != kNone));
     if (lane == 0) {
       ps.cnt[idx] = found;
-      L2.next[idx] = 0;
+      A->L.next[idx] = 0;
       ps.resume[idx] = worst == kNone ? kNone : worst + 1u;
     }
   }
 }
 static_assert(kSlots2 == 32, "one slot per thread of the warp");
-
-// One pair per length-2 lane with an untried survivor; lanes with no slot
-// left either end without a winner (bucket exhausted) or wait for a rescan.
-// One round of the length-2 pass: windows over the lane's slots; a lane
-// with its slots used up and its bucket not exhausted asks for a rescan.
-__global__ void k_pair_round_build(DevTargets T, Lanes L2, PairScan ps, RoundBuf R) {
-  const uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x;
-  uint32_t w = 0, sbase = 0;
-  if (idx < 2 * T.n) {
-    const uint32_t nx = L2.next[idx];
-    if (!(nx & kResolved)) {
-      if (nx < ps.cnt[idx]) {
-        w = min(1u << L2.spec[idx], ps.cnt[idx] - nx);
-        sbase = idx * kSlots2 + nx;
-      } else if (ps.resume[idx] == kNone) {
-        L2.next[idx] = nx | kResolved;
-      } else {
-        atomicAdd(ps.refill, 1u);
-      }
-    }
-  }
-  if (!__any_sync(kFull, w != 0)) return;
-  const uint32_t p0 = alloc_pairs(R.npairs, w);
-  const uint32_t fit = p0 >= R.cap ? 0u : min(w, R.cap - p0);
-  put_window(R, p0, fit, idx >> 1, idx & 1u, ps.surv, sbase);
-}
-
 
 unsigned grid_for(uint32_t n, unsigned block) { return (n + block - 1) / block; }
 
@@ -2572,23 +2551,57 @@ void launch_qc_bucket(const DevTargets& T, const DevPool& P, const QCConfig& cfg
   else if (keep) k_qc_bucket<false, true><<<grid, kBlock, 0, s>>>(T, P, cfg, ix, o);
   else k_qc_bucket<false, false><<<grid, kBlock, 0, s>>>(T, P, cfg, ix, o);
 }
-// The pair count is on the device: a grid-stride launch of up to 16 blocks
-// per SM (the pair slots bound it for small jobs).
-static void launch_pair_plan(const DevTargets& T, const DevPool& P, const QCOut& q, const RoundBuf& R, cudaStream_t s) {
-  const unsigned grid = std::min<unsigned>(grid_for(R.cap, 128), unsigned(dev_num_sms() * 16));
-  k_pair_plan<<<grid, 128, 0, s>>>(T, P, q, R);
+SweepArgs sweep_args(const RoundArgs& a) {
+  SweepArgs w{};
+  w.tinsn = a.T.insn;
+  w.tlens = a.T.len;
+  w.tlen = a.T.len ? 0u : a.T.fixed_len;
+  w.tstride = a.T.stride;
+  w.pinsn = a.P.insn;
+  w.plens = a.P.lens;
+  w.plen = a.P.lens ? 0u : a.P.len;
+  w.pstride = a.P.stride;
+  w.pairs = a.R.pairs;
+  w.rejected = a.R.rejected;
+  w.wend = a.R.wend;
+  w.cdone = a.R.cdone;
+  for (int c = 0; c < kClasses; c++) {
+    w.cbase[c] = a.R.cbase[c];
+    w.cpair[c] = a.R.cpair[c];
+  }
+  w.states = a.R.states;
+  w.ctl = a.R.ctl;
+  w.xunit = a.R.xunit;
+  return w;
 }
-void launch_round_build(const DevTargets& T, const DevPool& P, const QCOut& q, const Lanes& L,
-                        const RoundBuf& R, cudaStream_t s) {
-  if (!T.n) return;
-  k_round_build<<<grid_for(T.n, 256), 256, 0, s>>>(T, q, L, R);
-  launch_pair_plan(T, P, q, R, s);
+void launch_round_args(const RoundArgs& a, RoundArgs* dst, cudaStream_t s) { k_round_args<<<1, 256, 0, s>>>(a, dst); }
+// The work of a round's kernels is known on the device only: grid-stride
+// launches, of a few blocks for small jobs (whose rounds are launch latency)
+// and of every SM's blocks for the others.
+void launch_round_build(const RoundArgs* a, bool pair, bool small, cudaStream_t s) {
+  const unsigned grid = small ? 32u : unsigned(dev_num_sms() * 8);
+  if (pair) k_round_build<true><<<grid, 256, 0, s>>>(a);
+  else k_round_build<false><<<grid, 256, 0, s>>>(a);
 }
-void launch_pairs_from_survivors(const DevTargets& T, const DevPool& P, const QCOut& q,
-                                 const uint8_t* midpass, uint32_t nsurv, const uint32_t* surv_target,
-                                 const RoundBuf& R, cudaStream_t s) {
-  if (!nsurv) return;
-  k_pairs_from_survivors<<<grid_for(nsurv, 256), 256, 0, s>>>(T, P, q, midpass, nsurv, surv_target, R);
+void launch_pair_plan(const RoundArgs* a, bool small, cudaStream_t s) {
+  k_pair_plan<<<unsigned(dev_num_sms() * (small ? 2 : 16)), 128, 0, s>>>(a);
+}
+void launch_round_resolve(const RoundArgs* a, bool pair, bool small, cudaStream_t s) {
+  const unsigned grid = small ? 32u : unsigned(dev_num_sms() * 8);
+  if (pair) k_round_resolve<true><<<grid, 256, 0, s>>>(a);
+  else k_round_resolve<false><<<grid, 256, 0, s>>>(a);
+}
+void launch_round_end(const RoundArgs* a, bool in_loop, cudaGraphConditionalHandle loop, cudaStream_t s) {
+  if (in_loop) k_round_end<true><<<1, 32, 0, s>>>(a, loop);
+  else k_round_end<false><<<1, 32, 0, s>>>(a, loop);
+}
+void launch_pairs_identity(uint32_t n, const RoundBuf& R, cudaStream_t s) {
+  if (n) k_pairs_identity<<<grid_for(n, 256), 256, 0, s>>>(n, R);
+}
+void launch_pairs_from_survivors(const QCOut& q, const uint8_t* midpass, uint32_t lo, uint32_t hi,
+                                 const uint32_t* surv_target, const RoundBuf& R, cudaStream_t s) {
+  if (hi <= lo) return;
+  k_pairs_from_survivors<<<grid_for(hi - lo, 256), 256, 0, s>>>(q, midpass, lo, hi, surv_target, R);
 }
 // Shared memory of a sweep kernel (bit-sliced classes): the candidate's
 // output planes, one column of words per lane.
@@ -2605,8 +2618,7 @@ int exhaustive_blocks_per_sm() {
   return blocks_per_sm(occ, k_exhaustive<K, CLS>, kBlock, smem, smem);
 }
 template <int K, int CLS>
-void launch_exhaustive_k(const DevTargets& T, const DevPool& P, const RoundBuf& R, uint32_t npairs,
-                         unsigned long long total, cudaStream_t s) {
+void launch_exhaustive_k(const SweepArgs& a, unsigned long long total, cudaStream_t s) {
   constexpr int smem = exhaustive_smem(CLS);
   const int per_sm = exhaustive_blocks_per_sm<K, CLS>();
   // resident blocks, or more when the chunks exceed kChunksPerWarp per warp
@@ -2617,58 +2629,55 @@ void launch_exhaustive_k(const DevTargets& T, const DevPool& P, const RoundBuf& 
   const unsigned long long cover = (total + wpb * kChunksPerWarp - 1) / (wpb * kChunksPerWarp);
   if (grid < cover) grid = cover;
   if (grid > 0x7FFFFFFFull) grid = 0x7FFFFFFFull;
-  k_exhaustive<K, CLS><<<unsigned(grid), kBlock, smem, s>>>(T, P, R, npairs, total, nullptr, nullptr,
-                                                               kChunksPerWarp);
+  k_exhaustive<K, CLS><<<unsigned(grid), kBlock, smem, s>>>(a, kChunksPerWarp);
 }
 
 // The same kernel on a persistent grid (resident blocks on every SM) whose
-// blocks take chunks until the class's device-side total is spent.
+// blocks take chunks until the class's total is spent.
 template <int K, int CLS>
-void launch_exhaustive_dev_k(const DevTargets& T, const DevPool& P, const RoundBuf& R, const unsigned long long* total,
-                             const uint32_t* np, cudaStream_t s) {
+void launch_exhaustive_dev_k(const SweepArgs& a, cudaStream_t s) {
   constexpr int smem = exhaustive_smem(CLS);
   const int per_sm = exhaustive_blocks_per_sm<K, CLS>();
   const unsigned grid = unsigned(dev_num_sms() * per_sm);
-  k_exhaustive<K, CLS><<<grid, kBlock, smem, s>>>(T, P, R, 0u, 0ull, total, np, 0x7FFFFFFF);
+  k_exhaustive<K, CLS><<<grid, kBlock, smem, s>>>(a, 0x7FFFFFFF);
 }
 
-int launch_exhaustive(const DevTargets& T, const DevPool& P, const RoundBuf& R, uint32_t npairs,
-                      unsigned long long total_b, unsigned long long total_x, unsigned long long total_c,
-                      unsigned long long total_w, unsigned long long total_r, int k, cudaStream_t s,
+int launch_exhaustive(const SweepArgs& a, const unsigned long long* alloc, int k, cudaStream_t s,
                       uint32_t* kernels) {
-  if (!npairs) return 0;
   int n = 0;
   uint32_t mask = 0;
-  if (total_r) {
-    launch_exhaustive_k<1, 5>(T, P, R, npairs, total_r, s);
+  unsigned long long total[kClasses];
+  for (int c = 0; c < kClasses; c++) total[c] = alloc[c] & kChunkMask;
+  if (total[4]) {
+    launch_exhaustive_k<1, 5>(a, total[4], s);
     mask |= kSweepRegs;
     n++;
   }
-  if (total_w) {
-    launch_exhaustive_k<1, 4>(T, P, R, npairs, total_w, s);
+  if (total[3]) {
+    launch_exhaustive_k<1, 4>(a, total[3], s);
     mask |= kSweepWide;
     n++;
   }
-  if (total_c) {
-    launch_exhaustive_k<1, 3>(T, P, R, npairs, total_c, s);
+  if (total[2]) {
+    launch_exhaustive_k<1, 3>(a, total[2], s);
     mask |= kSweepCompact;
     n++;
   }
-  if (total_b) {
-    launch_exhaustive_k<1, 0>(T, P, R, npairs, total_b, s);
+  if (total[0]) {
+    launch_exhaustive_k<1, 0>(a, total[0], s);
     mask |= kSweepBits;
     n++;
   }
-  if (total_x) {
-    if (R.xunit == kXBitsBlocks) {
-      launch_exhaustive_k<1, 2>(T, P, R, npairs, total_x, s);
+  if (total[1]) {
+    if (a.xunit == kXBitsBlocks) {
+      launch_exhaustive_k<1, 2>(a, total[1], s);
       mask |= kSweepXBits;
     } else {
       switch (k) {
-        case 1: launch_exhaustive_k<1, 1>(T, P, R, npairs, total_x, s); mask |= kSweepScalarK1; break;
-        case 2: launch_exhaustive_k<2, 1>(T, P, R, npairs, total_x, s); mask |= kSweepScalarK1 << 1; break;
-        case 8: launch_exhaustive_k<8, 1>(T, P, R, npairs, total_x, s); mask |= kSweepScalarK1 << 3; break;
-        default: launch_exhaustive_k<4, 1>(T, P, R, npairs, total_x, s); mask |= kSweepScalarK1 << 2; break;
+        case 1: launch_exhaustive_k<1, 1>(a, total[1], s); mask |= kSweepScalarK1; break;
+        case 2: launch_exhaustive_k<2, 1>(a, total[1], s); mask |= kSweepScalarK1 << 1; break;
+        case 8: launch_exhaustive_k<8, 1>(a, total[1], s); mask |= kSweepScalarK1 << 3; break;
+        default: launch_exhaustive_k<4, 1>(a, total[1], s); mask |= kSweepScalarK1 << 2; break;
       }
     }
     n++;
@@ -2676,193 +2685,50 @@ int launch_exhaustive(const DevTargets& T, const DevPool& P, const RoundBuf& R, 
   if (kernels) *kernels |= mask;
   return n;
 }
-void launch_round_resolve(const RoundBuf& R, uint32_t npairs, const QCOut& q, const Lanes& L, uint32_t max_spec,
-                          cudaStream_t s) {
-  if (!npairs) return;
-  k_round_resolve<<<grid_for(npairs, 256), 256, 0, s>>>(R, npairs, q, L, max_spec, nullptr);
-}
-
-// The round's chunk prefixes on the device, in three launches: every block
-// of k_round_scan_sum sums its contiguous segment of each class's chunk
-// counts (coalesced tiles), k_round_scan_write rescans its segment from the
-// sum of the blocks before it, and k_round_scan_ctl takes the totals, clears
-// the dispensers, keeps the loop's counters and sets its condition.  The
-// first two only read RoundCtl; the third alone writes it.
-constexpr int kRScanThreads = 256;
-static_assert(kRScanThreads == kRScanBlocks, "one block sum per thread in the offset reduction");
-
-__device__ __forceinline__ bool rscan_on(const RoundBuf& R, int c) { return !((c == 2 && !R.compact) || (c >= 3 && !R.wide)); }
-__device__ __forceinline__ const unsigned long long* rscan_in(const RoundBuf& R, int c) {
-  return c == 0 ? R.nchunks : (c == 1 ? R.nchunks_x : (c == 2 ? R.nchunks_c : (c == 3 ? R.nchunks_w : R.nchunks_r)));
-}
-__device__ __forceinline__ unsigned long long* rscan_out(const RoundBuf& R, int c) {
-  return c == 0 ? R.cbase : (c == 1 ? R.cbase_x : (c == 2 ? R.cbase_c : (c == 3 ? R.cbase_w : R.cbase_r)));
-}
-// The pairs to scan: the build's count, or 0 once the loop is past its bound.
-__device__ __forceinline__ uint32_t rscan_np(const RoundBuf& R, const RoundCtl* ctl) {
-  const uint32_t np = min(*R.npairs, R.cap);
-  return ctl->iters + 1 >= kMaxRoundIters ? 0u : np;
-}
-// Block-wide sum, the result in every thread (red: kRScanThreads / 32 slots).
-__device__ __forceinline__ unsigned long long rscan_block_sum(unsigned long long v, unsigned long long* red) {
-#pragma unroll
-  for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(kFull, v, o);
-  __syncthreads();  // red is free (an earlier call has been read)
-  if (lane_id() == 0) red[threadIdx.x >> 5] = v;
-  __syncthreads();
-  unsigned long long t = 0;
-#pragma unroll
-  for (int w = 0; w < kRScanThreads / 32; w++) t += red[w];
-  return t;
-}
-
-__global__ void __launch_bounds__(kRScanThreads) k_round_scan_sum(RoundBuf R, RoundCtl* __restrict__ ctl) {
-  __shared__ unsigned long long red[kRScanThreads / 32];
-  const uint32_t np = rscan_np(R, ctl);
-  if (np == 0) return;
-  const uint32_t per = (np + kRScanBlocks - 1) / kRScanBlocks;
-  const uint32_t lo = uint32_t(min((unsigned long long)blockIdx.x * per, (unsigned long long)np));
-  const uint32_t hi = lo + min(per, np - lo);
-  for (int c = 0; c < 5; c++) {
-    if (!rscan_on(R, c)) continue;  // the same for every block
-    const unsigned long long* __restrict__ in = rscan_in(R, c);
-    unsigned long long v = 0;
-    for (uint32_t i = lo + threadIdx.x; i < hi; i += kRScanThreads) v += in[i];
-    v = rscan_block_sum(v, red);
-    if (threadIdx.x == 0) ctl->bsum[c][blockIdx.x] = v;  // 0 for an empty segment
-  }
-}
-
-__global__ void __launch_bounds__(kRScanThreads) k_round_scan_write(RoundBuf R, const RoundCtl* __restrict__ ctl) {
-  __shared__ unsigned long long red[kRScanThreads / 32];
-  const uint32_t np = rscan_np(R, ctl);
-  if (np == 0) return;
-  const uint32_t per = (np + kRScanBlocks - 1) / kRScanBlocks;
-  const uint32_t lo = uint32_t(min((unsigned long long)blockIdx.x * per, (unsigned long long)np));
-  const uint32_t hi = lo + min(per, np - lo);
-  const unsigned lane = lane_id(), warp = threadIdx.x >> 5;
-  for (int c = 0; c < 5; c++) {
-    if (!rscan_on(R, c)) continue;
-    const unsigned long long* __restrict__ in = rscan_in(R, c);
-    unsigned long long* __restrict__ out = rscan_out(R, c);
-    // chunks of the blocks before this one
-    unsigned long long run = rscan_block_sum(threadIdx.x < blockIdx.x ? ctl->bsum[c][threadIdx.x] : 0ull, red);
-    for (uint32_t base = lo; base < hi; base += kRScanThreads) {
-      const uint32_t i = base + threadIdx.x;
-      const unsigned long long v = i < hi ? in[i] : 0ull;
-      // inclusive warp scan, then the warps' totals
-      unsigned long long x = v;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const unsigned long long y = __shfl_up_sync(kFull, x, o);
-        if (lane >= unsigned(o)) x += y;
-      }
-      __syncthreads();  // red is free
-      if (lane == 31) red[warp] = x;
-      __syncthreads();
-      unsigned long long before = 0, tile = 0;
-#pragma unroll
-      for (int w = 0; w < kRScanThreads / 32; w++) {
-        before += unsigned(w) < warp ? red[w] : 0ull;
-        tile += red[w];
-      }
-      if (i < hi) out[i] = run + before + x - v;
-      run += tile;
-    }
-  }
-}
-
-__global__ void k_round_scan_ctl(RoundBuf R, RoundCtl* __restrict__ ctl, const uint32_t* __restrict__ refill,
-                                 cudaGraphConditionalHandle loop) {
-  const unsigned lane = lane_id();
-  const uint32_t np = min(*R.npairs, R.cap);
-  const bool over = ctl->iters + 1 >= kMaxRoundIters;
-  const bool empty = np == 0 || over;
-  unsigned long long tot[5];
-#pragma unroll
-  for (int c = 0; c < 5; c++) {
-    unsigned long long v = 0;
-    if (!empty && rscan_on(R, c))
-      for (int b = lane; b < kRScanBlocks; b += 32) v += ctl->bsum[c][b];
-#pragma unroll
-    for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(kFull, v, o);
-    tot[c] = v;
-  }
-  if (lane != 0) return;
-  ctl->iters += 1;
-  if (over) {
-    // the loop has run far past any legitimate number of rounds: end it,
-    // sweep nothing more, and let the host report the error
-    ctl->overrun = 1;
-    cudaGraphSetConditional(loop, 0);
-  }
-  ctl->np = over ? 0u : np;
-  if (!empty) {
-    ctl->rounds += 1;
-    ctl->pairs += np;
-  }
-  R.counter[0] = R.counter[1] = R.counter[2] = R.counter[3] = R.counter[4] = 0;
-#pragma unroll
-  for (int c = 0; c < 5; c++) ctl->totals[c] = tot[c];
-  if (empty && (!refill || *refill == 0)) cudaGraphSetConditional(loop, 0);
-}
-
-void launch_round_scan(const RoundBuf& R, RoundCtl* ctl, const uint32_t* refill, cudaGraphConditionalHandle loop,
-                       cudaStream_t s) {
-  k_round_scan_sum<<<kRScanBlocks, kRScanThreads, 0, s>>>(R, ctl);
-  k_round_scan_write<<<kRScanBlocks, kRScanThreads, 0, s>>>(R, ctl);
-  k_round_scan_ctl<<<1, 32, 0, s>>>(R, ctl, refill, loop);
-}
 
 template <int K, int CLS>
 void warm_exhaustive_k() {
   (void)exhaustive_blocks_per_sm<K, CLS>();
 }
-void warm_exhaustive_dev(const RoundBuf& R, int k) {
+void warm_exhaustive_dev(bool compact, bool wide, uint32_t xunit, int k) {
   (void)dev_num_sms();
-  if (R.wide) {
+  if (wide) {
     warm_exhaustive_k<1, 4>();
     warm_exhaustive_k<1, 5>();
   }
-  if (R.compact) warm_exhaustive_k<1, 3>();
+  if (compact) warm_exhaustive_k<1, 3>();
   warm_exhaustive_k<1, 0>();
-  if (R.xunit == kXBitsBlocks) warm_exhaustive_k<1, 2>();
+  if (xunit == kXBitsBlocks) warm_exhaustive_k<1, 2>();
   else if (k == 1) warm_exhaustive_k<1, 1>();
   else if (k == 2) warm_exhaustive_k<2, 1>();
   else if (k == 8) warm_exhaustive_k<8, 1>();
   else warm_exhaustive_k<4, 1>();
 }
 
-int launch_exhaustive_dev(const DevTargets& T, const DevPool& P, const RoundBuf& R, const RoundCtl* ctl, int k,
-                          const cudaStream_t* ss) {
+int launch_exhaustive_dev(const SweepArgs& a, bool compact, bool wide, int k, const cudaStream_t* ss) {
   int n = 0;
-  if (R.wide) {
-    launch_exhaustive_dev_k<1, 5>(T, P, R, &ctl->totals[4], &ctl->np, ss[0]);
-    launch_exhaustive_dev_k<1, 4>(T, P, R, &ctl->totals[3], &ctl->np, ss[1]);
+  if (wide) {
+    launch_exhaustive_dev_k<1, 5>(a, ss[0]);
+    launch_exhaustive_dev_k<1, 4>(a, ss[1]);
     n += 2;
   }
-  if (R.compact) {
-    launch_exhaustive_dev_k<1, 3>(T, P, R, &ctl->totals[2], &ctl->np, ss[2]);
+  if (compact) {
+    launch_exhaustive_dev_k<1, 3>(a, ss[2]);
     n++;
   }
-  launch_exhaustive_dev_k<1, 0>(T, P, R, &ctl->totals[0], &ctl->np, ss[3]);
+  launch_exhaustive_dev_k<1, 0>(a, ss[3]);
   const cudaStream_t sx = ss[4];
-  if (R.xunit == kXBitsBlocks) {
-    launch_exhaustive_dev_k<1, 2>(T, P, R, &ctl->totals[1], &ctl->np, sx);
+  if (a.xunit == kXBitsBlocks) {
+    launch_exhaustive_dev_k<1, 2>(a, sx);
   } else {
     switch (k) {
-      case 1: launch_exhaustive_dev_k<1, 1>(T, P, R, &ctl->totals[1], &ctl->np, sx); break;
-      case 2: launch_exhaustive_dev_k<2, 1>(T, P, R, &ctl->totals[1], &ctl->np, sx); break;
-      case 8: launch_exhaustive_dev_k<8, 1>(T, P, R, &ctl->totals[1], &ctl->np, sx); break;
-      default: launch_exhaustive_dev_k<4, 1>(T, P, R, &ctl->totals[1], &ctl->np, sx); break;
+      case 1: launch_exhaustive_dev_k<1, 1>(a, sx); break;
+      case 2: launch_exhaustive_dev_k<2, 1>(a, sx); break;
+      case 8: launch_exhaustive_dev_k<8, 1>(a, sx); break;
+      default: launch_exhaustive_dev_k<4, 1>(a, sx); break;
     }
   }
   return n + 2;
-}
-
-void launch_round_resolve_dev(const RoundBuf& R, const RoundCtl* ctl, const QCOut& q, const Lanes& L,
-                              uint32_t max_spec, cudaStream_t s) {
-  k_round_resolve<<<grid_for(R.cap, 256), 256, 0, s>>>(R, R.cap, q, L, max_spec, &ctl->np);
 }
 
 void launch_midcheck(const DevTargets& T, const DevPool& P, const uint32_t* surv,
@@ -2929,25 +2795,16 @@ void launch_pair_lanes_init(const DevTargets& T, const Lanes& L1, const QCOut& q
   if (!T.n) return;
   k_pair_lanes_init<<<grid_for(T.n, 256), 256, 0, s>>>(T, L1, q1, L2, ps);
 }
-// A warp per lane and no more blocks than that needs; the blocks of a large
-// job retire as their lanes are done, which evens out the few long walks.
-void launch_pair_scan(const DevTargets& T, const QCOut& q1, const Lanes& L2, const PairScan& ps, cudaStream_t s) {
-  if (!T.n) return;
-  k_pair_scan<<<grid_for(T.n, kBlock / 64), kBlock, 0, s>>>(T, q1, L2, ps, nullptr);
+// All lanes: a warp each and no more blocks than that needs; the blocks of a
+// large job retire as their lanes are done, which evens out the few long
+// walks.  The lanes that wait (their number is on the device, mostly none):
+// a resident grid.
+void launch_pair_scan(const RoundArgs* a, uint32_t n, bool all, bool small, cudaStream_t s) {
+  if (all) {
+    if (n) k_pair_scan<<<grid_for(n, kBlock / 64), kBlock, 0, s>>>(a, true);
+  } else {
+    k_pair_scan<<<unsigned(dev_num_sms() * (small ? 1 : 8)), kBlock, 0, s>>>(a, false);
+  }
 }
-// Inside a round graph most launches find nothing to do: a resident grid.
-void launch_pair_scan_gated(const DevTargets& T, const QCOut& q1, const Lanes& L2, const PairScan& ps,
-                            const RoundCtl* ctl, cudaStream_t s) {
-  if (!T.n) return;
-  unsigned grid = std::min<unsigned>(grid_for(T.n, kBlock / 64), unsigned(dev_num_sms() * 8));
-  k_pair_scan<<<grid, kBlock, 0, s>>>(T, q1, L2, ps, ctl);
-}
-void launch_pair_round_build(const DevTargets& T, const DevPool& P, const QCOut& q1, const Lanes& L2,
-                             const PairScan& ps, const RoundBuf& R, cudaStream_t s) {
-  if (!T.n) return;
-  k_pair_round_build<<<grid_for(2 * T.n, 256), 256, 0, s>>>(T, L2, ps, R);
-  launch_pair_plan(T, P, q1, R, s);
-}
-
 
 }  // namespace z80b

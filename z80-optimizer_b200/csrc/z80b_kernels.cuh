@@ -67,29 +67,49 @@ constexpr uint32_t kXScalarBlocks = 128, kXBitsBlocks = 1024;
 constexpr uint32_t kMaxSpec1 = 6;  // length-1 pass: windows up to 64
 constexpr uint32_t kMaxSpec2 = 5;  // length-2 pass: windows up to 32 (the lane's slots)
 
+// The sweep classes: 0 full state, A-dependent; 1 A-independent; 2 compact;
+// 3 wide compact; 4 register state.
+constexpr int kClasses = 5;
+
+// Device-side state of a round and of its loop.
+struct RoundCtl {
+  // Chunk lists of the classes: entries << kChunkBits | chunks, so that one
+  // atomic hands a pair both its entry and its first chunk, and the entries
+  // of a class ascend by first chunk.
+  unsigned long long alloc[kClasses];
+  unsigned long long counter[kClasses];  // chunk dispensers
+  unsigned long long pairs;              // pairs swept, all rounds
+  uint32_t npairs;                       // slots handed out in this round (may exceed the capacity)
+  uint32_t active;                       // set when a lane has something left after this round
+  uint32_t nscan;                        // length-2 pass: lanes that wait for a rescan
+  uint32_t more;                         // the last round's active
+  uint32_t np;                           // the last round's pairs
+  uint32_t rounds;                       // rounds with pairs
+  uint32_t iters;                        // loop iterations
+  uint32_t overrun;                      // set when the loop stopped at kMaxRoundIters (an error)
+};
+constexpr int kChunkBits = 39;
+constexpr unsigned long long kChunkMask = (1ull << kChunkBits) - 1;
+// Most pair slots of a round (an entry number takes the bits above
+// kChunkBits) and most chunks of a pair, so that the chunks of a full round
+// stay below 2^kChunkBits.
+constexpr unsigned long long kMaxRoundPairs = (1ull << (64 - kChunkBits)) - 1;
+inline uint32_t max_chunks(unsigned long long pairs) {
+  unsigned long long c = (1ull << kChunkBits) / (pairs ? pairs : 1ull);
+  if (c > (1ull << 20)) c = 1ull << 20;
+  return uint32_t(c > 1 ? c - 1 : 1);
+}
+
 struct RoundBuf {
   PairRec* pairs;
   uint32_t* pair_src;              // index of the (target, kind) lane or survivor
-  // Two sweep kernels share a round: one runs the bit-sliced pairs (outputs
-  // depend on A), the other the A-independent ones; each class has its own
-  // chunk numbering (pairs of the other class count zero chunks in it).
-  unsigned long long* nchunks;     // per pair (scan input), bit-sliced class
-  unsigned long long* cbase;       // exclusive prefix of nchunks
-  unsigned long long* nchunks_x;   // per pair, A-independent class
-  unsigned long long* cbase_x;     // exclusive prefix of nchunks_x
-  unsigned long long* nchunks_c;   // per pair, compact class (with compact set; else unused)
-  unsigned long long* cbase_c;     // exclusive prefix of nchunks_c
-  uint32_t compact;                // A-dependent pairs whose registers fit the compact state get
-                                   // their own class and kernel
-  unsigned long long* nchunks_w;   // per pair, wide compact class (with wide set; else unused)
-  unsigned long long* cbase_w;     // exclusive prefix of nchunks_w
-  unsigned long long* nchunks_r;   // per pair, register-state class (with wide set; else unused)
-  unsigned long long* cbase_r;     // exclusive prefix of nchunks_r
-  uint32_t wide;                   // pairs whose registers fit the wide compact state (and not
-                                   // the compact one) get their own class and kernel, and so do
-                                   // the rest that name neither SP nor the memory byte
-                                   // (register-state class)
-  uint32_t* rejected;              // per pair
+  // Per class, the pairs that have chunks in it: first chunk and pair index
+  // of each entry (cpair null: entry i is pair i).
+  unsigned long long* cbase[kClasses];
+  uint32_t* cpair[kClasses];
+  uint32_t compact;                // pairs whose registers fit the compact state get that class
+  uint32_t wide;                   // the wide compact and the register-state classes are in use
+  uint32_t* rejected;              // per pair: 1 a mismatch was found, 2 cancelled
   uint8_t* wlen;                   // per pair: survivors in the window it heads (0: not a head)
   // First-found windows (null for independent pairs): per pair the end
   // (exclusive) of its survivor window, and the chunks of its sweep that
@@ -99,13 +119,12 @@ struct RoundBuf {
   uint32_t* wend;
   uint32_t* cdone;
   uint32_t cap;                    // pair slots of the buffers
-  uint32_t* npairs;                // device counter
-  unsigned long long* counter;     // chunk dispensers: [0] bit-sliced, [1] A-independent, [2] compact,
-                                   // [3] wide compact, [4] register-state class
+  uint32_t max_chunks;             // chunks of one pair at most
   unsigned long long* states;      // [2]: states of the reference's sweeps covered, states evaluated
-  uint32_t chunk_blocks;           // A-blocks per work chunk
+  uint32_t chunk_blocks;           // sweep units per work chunk
   uint32_t xunit;                  // A-blocks per unit of an A-independent sweep: kXBitsBlocks
                                    // (bit-sliced kernel), else (0 too) the scalar kernel's 128
+  RoundCtl* ctl;
 };
 
 // Length-2 candidate pass (pair pool): indexes and per-lane slots.
@@ -132,7 +151,7 @@ struct PairScan {
   uint32_t* resume;                      // [2n] pair index to go on from; kNone: exhausted
   uint32_t* surv;                        // [2n * kSlots2] pair-pool indices
   uint16_t* sdiff;                       // [2n * kSlots2]
-  uint32_t* refill;                      // lanes waiting for a rescan (round build)
+  uint32_t* scan;                        // [2n] the lanes waiting for a rescan (ctl->nscan of them)
   const unsigned long long* eligible;    // [16] unpruned pairs shorter than b bytes
   unsigned long long* checks;            // QuickCheck units (eligible pairs per target)
 };
@@ -167,67 +186,77 @@ void launch_qc_keys(const DevPool& P, uint32_t w2mask, unsigned long long* keys,
 void launch_qc_top(const unsigned long long* keys, uint32_t nv, uint32_t* top, cudaStream_t s);
 void launch_qc_bucket(const DevTargets& T, const DevPool& P, const QCConfig& cfg, const QCIndex& ix,
                       const QCOut& o, bool collect, cudaStream_t s);
-void launch_round_build(const DevTargets& T, const DevPool& P, const QCOut& q, const Lanes& L,
-                        const RoundBuf& R, cudaStream_t s);
-void launch_pairs_from_survivors(const DevTargets& T, const DevPool& P, const QCOut& q,
-                                 const uint8_t* midpass, uint32_t nsurv, const uint32_t* surv_target,
-                                 const RoundBuf& R, cudaStream_t s);
-// k = states per lane per dispatch: 1, 2, 4 or 8.
-// Launches the sweep kernel of each class that has chunks (total_b
-// bit-sliced, total_x A-independent, total_c compact); returns the number of
-// launches and ORs the launched instantiations into *kernels (may be NULL):
-// kSweep* bits.
-constexpr uint32_t kSweepBits = 1u, kSweepXBits = 2u, kSweepCompact = 4u;
-constexpr uint32_t kSweepScalarK1 = 8u;  // scalar A-independent kernel, K = 1, 2, 4, 8: bits 3..6
-constexpr uint32_t kSweepWide = 128u, kSweepRegs = 256u;
-int launch_exhaustive(const DevTargets& T, const DevPool& P, const RoundBuf& R, uint32_t npairs,
-                      unsigned long long total_b, unsigned long long total_x, unsigned long long total_c,
-                      unsigned long long total_w, unsigned long long total_r, int k, cudaStream_t s,
-                      uint32_t* kernels = nullptr);
-void launch_round_resolve(const RoundBuf& R, uint32_t npairs, const QCOut& q, const Lanes& L, uint32_t max_spec,
-                          cudaStream_t s);
-
-// ---- device-driven rounds (one CUDA graph, a WHILE node over the round body)
-// The round's pair count and chunk totals stay on the device: the round
-// scan (three launches) takes the count the build left in R.npairs, scans
-// the chunk counts of the five classes (per-block segment sums in bsum, then
-// each segment from its blocks' offset), clears the dispensers and ends the
-// loop (sets the graph's condition to 0) when the round is empty and no lane
-// waits for a rescan.
-constexpr int kRScanBlocks = 256;
-struct RoundCtl {
-  unsigned long long totals[5];  // chunks of the current round: bit-sliced, A-independent, compact, wide,
-                                 // register state
-  unsigned long long pairs;      // pairs swept, all rounds
-  uint32_t rounds;               // rounds with pairs
-  uint32_t iters;                // loop iterations (rounds, rescans, the last empty one)
-  uint32_t np;                   // pairs of the current round
-  uint32_t overrun;              // set when the loop stopped at kMaxRoundIters (an error)
-  unsigned long long bsum[5][kRScanBlocks];  // the current round's chunks per class and scan block
+// Everything the kernels of a round need, in device memory: a captured round
+// graph reads the job at hand from here, so a job of another size replays the
+// same graph (the sweeps' own share: SweepArgs).
+struct RoundArgs {
+  DevTargets T;
+  DevPool P;
+  QCOut q;              // survivors and metadata of the length-1 QuickCheck
+  Lanes L;              // the lanes of this pass
+  RoundBuf R;
+  PairScan ps;          // length-2 pass only
+  const uint16_t* sdiff;  // per survivor: FlagDiff | differing registers << 8
+  uint32_t max_spec;    // windows of up to 2^max_spec survivors
 };
+// Writes a to *dst and clears a.R.ctl.
+void launch_round_args(const RoundArgs& a, RoundArgs* dst, cudaStream_t s);
+
+// One round, in stream order: [rescan,] build, plan, sweeps, resolve, end.
+// `small`: launch shapes for jobs of few targets (any job may use either).
+void launch_round_build(const RoundArgs* a, bool pair, bool small, cudaStream_t s);
+void launch_pair_plan(const RoundArgs* a, bool small, cudaStream_t s);
+void launch_round_resolve(const RoundArgs* a, bool pair, bool small, cudaStream_t s);
+// The counters for the next round, and the loop's condition (in_loop).
+void launch_round_end(const RoundArgs* a, bool in_loop, cudaGraphConditionalHandle loop, cudaStream_t s);
 // Bound on the iterations of one device-driven loop: a loop that has not
 // ended by then stops and reports an error instead of running on.
 constexpr uint32_t kMaxRoundIters = 1u << 20;
-void launch_round_scan(const RoundBuf& R, RoundCtl* ctl, const uint32_t* refill, cudaGraphConditionalHandle loop,
-                       cudaStream_t s);
-// The sweep kernels of the configured classes on persistent grids, the
-// chunk totals and pair count read from ctl; returns the launches per round.
-// ss[0..4]: the streams of the register-state, wide, compact, bit-sliced
-// and A-independent classes (the classes share no chunk, pair or
-// dispenser, so their launches may run side by side: one class's blocks
-// take the SMs that another's finished blocks leave).
-int launch_exhaustive_dev(const DevTargets& T, const DevPool& P, const RoundBuf& R, const RoundCtl* ctl, int k,
-                          const cudaStream_t* ss);
+
+// What the sweep kernels read, by value: their registers are all taken by the
+// states, and a field in the kernel's parameters costs none (the same fields
+// behind a pointer made every class spill, 100 to 400 bytes a thread).  None
+// of it depends on the number of targets, so a captured graph holds for jobs
+// of any size until a buffer grows or the form of the targets changes.
+struct SweepArgs {
+  const uint32_t *tinsn, *pinsn;
+  const uint8_t *tlens, *plens;   // null: tlen / plen
+  uint32_t tlen, tstride, plen, pstride;
+  const PairRec* pairs;
+  uint32_t* rejected;
+  const uint32_t* wend;           // null: independent pairs
+  uint32_t* cdone;
+  const unsigned long long* cbase[kClasses];
+  const uint32_t* cpair[kClasses];
+  unsigned long long* states;
+  RoundCtl* ctl;
+  uint32_t xunit, pad;
+};
+SweepArgs sweep_args(const RoundArgs& a);
+
+// k = states per lane per dispatch: 1, 2, 4 or 8.
+// Launches the sweep kernel of each class that has chunks (alloc: the round's
+// RoundCtl::alloc on the host); returns the number of launches and ORs the
+// launched instantiations into *kernels (may be NULL): kSweep* bits.
+constexpr uint32_t kSweepBits = 1u, kSweepXBits = 2u, kSweepCompact = 4u;
+constexpr uint32_t kSweepScalarK1 = 8u;  // scalar A-independent kernel, K = 1, 2, 4, 8: bits 3..6
+constexpr uint32_t kSweepWide = 128u, kSweepRegs = 256u;
+int launch_exhaustive(const SweepArgs& a, const unsigned long long* alloc, int k, cudaStream_t s,
+                      uint32_t* kernels = nullptr);
+// The sweep kernels of the configured classes on persistent grids, the chunk
+// totals read on the device.  ss[0..4]: the streams of the register-state,
+// wide, compact, bit-sliced and A-independent classes (the classes share no
+// chunk, pair or dispenser, so their launches may run side by side: one
+// class's blocks take the SMs that another's finished blocks leave).
+int launch_exhaustive_dev(const SweepArgs& a, bool compact, bool wide, int k, const cudaStream_t* ss);
 // Sets up (outside any stream capture) the launch facts of the kernels
-// launch_exhaustive_dev will launch for R and k.
-void warm_exhaustive_dev(const RoundBuf& R, int k);
-// k_round_resolve over the pair slots, the pair count read from ctl.
-void launch_round_resolve_dev(const RoundBuf& R, const RoundCtl* ctl, const QCOut& q, const Lanes& L,
-                              uint32_t max_spec, cudaStream_t s);
-// k_pair_scan that does its work only when the current round is empty (the
-// rescan step of the length-2 pass).
-void launch_pair_scan_gated(const DevTargets& T, const QCOut& q1, const Lanes& L2, const PairScan& ps,
-                            const RoundCtl* ctl, cudaStream_t s);
+// launch_exhaustive_dev will launch.
+void warm_exhaustive_dev(bool compact, bool wide, uint32_t xunit, int k);
+// Pairs (i, i) of n independent pairs.
+void launch_pairs_identity(uint32_t n, const RoundBuf& R, cudaStream_t s);
+// One pair per MidCheck survivor among survivors [lo, hi).
+void launch_pairs_from_survivors(const QCOut& q, const uint8_t* midpass, uint32_t lo, uint32_t hi,
+                                 const uint32_t* surv_target, const RoundBuf& R, cudaStream_t s);
 void launch_midcheck(const DevTargets& T, const DevPool& P, const uint32_t* surv,
                      const uint32_t* surv_target, uint32_t nsurv, uint8_t* pass, cudaStream_t s);
 void launch_surv_targets(const QCOut& q, uint32_t n, uint32_t* surv_target, cudaStream_t s);
@@ -255,9 +284,9 @@ void launch_pair_groups(const uint4* out, const unsigned long long* keys, const 
 void launch_pair_top(const uint4* groups, uint32_t n_groups, uint32_t* top, cudaStream_t s);
 void launch_pair_lanes_init(const DevTargets& T, const Lanes& L1, const QCOut& q1, const Lanes& L2,
                             const PairScan& ps, cudaStream_t s);
-void launch_pair_scan(const DevTargets& T, const QCOut& q1, const Lanes& L2, const PairScan& ps, cudaStream_t s);
-void launch_pair_round_build(const DevTargets& T, const DevPool& P, const QCOut& q1, const Lanes& L2,
-                             const PairScan& ps, const RoundBuf& R, cudaStream_t s);
+// Fills the slots of the lanes that have none left: every lane of a job
+// (all), or those in PairScan::scan.
+void launch_pair_scan(const RoundArgs* a, uint32_t n, bool all, bool small, cudaStream_t s);
 void launch_verify_small(const uint32_t* tgt, const uint8_t* tlens, const uint32_t* cand,
                          const uint8_t* clens, uint32_t stride, uint32_t n, const uint8_t* dead,
                          uint32_t tiers, uint8_t* out, uint8_t* flagdiff, cudaStream_t s);

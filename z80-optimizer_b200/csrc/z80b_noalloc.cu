@@ -37,8 +37,8 @@ constexpr size_t kOffPairs = align256(kOffDead + kMaxPairs);
 constexpr size_t kOffCbase = align256(kOffPairs + sizeof(PairRec) * kMaxPairs);
 constexpr size_t kOffCbaseX = align256(kOffCbase + 8ull * kMaxPairs);
 constexpr size_t kOffRej = align256(kOffCbaseX + 8ull * kMaxPairs);
-constexpr size_t kOffCounter = align256(kOffRej + 4ull * kMaxPairs);
-constexpr size_t kOffStates = kOffCounter + 16;
+constexpr size_t kOffCtl = align256(kOffRej + 4ull * kMaxPairs);
+constexpr size_t kOffStates = kOffCtl + sizeof(RoundCtl);
 constexpr size_t kNoAllocBytes = align256(kOffStates + 16);
 static_assert(kNoAllocBytes <= 320 * 1024, "the scratch stays modest");
 
@@ -49,6 +49,8 @@ std::mutex g_mu;
 uint32_t h_tgt[kStride * kMaxPairs], h_cand[kStride * kMaxPairs], h_rej[kMaxPairs];
 PairRec h_pairs[kMaxPairs];
 unsigned long long h_cbase[kMaxPairs], h_cbase_x[kMaxPairs];  // chunk prefixes: bit-sliced / A-independent pairs
+
+RoundCtl h_ctl;
 
 constexpr int kMaxDevices = 64;
 unsigned char* g_dev_ptr[kMaxDevices] = {};  // device address of the scratch on each device
@@ -90,7 +92,7 @@ int run_on_device(int device, uint32_t n, const uint8_t* tlens, const uint8_t* c
             cudaMemcpyAsync(base + kOffCbase, h_cbase, 8ull * n, cudaMemcpyHostToDevice, s) == cudaSuccess &&
             cudaMemcpyAsync(base + kOffCbaseX, h_cbase_x, 8ull * n, cudaMemcpyHostToDevice, s) == cudaSuccess &&
             cudaMemsetAsync(base + kOffRej, 0, 4ull * n, s) == cudaSuccess &&
-            cudaMemsetAsync(base + kOffCounter, 0, 32, s) == cudaSuccess;
+            cudaMemsetAsync(base + kOffStates, 0, 16, s) == cudaSuccess;
   if (dead) ok = ok && cudaMemcpyAsync(base + kOffDead, dead, n, cudaMemcpyHostToDevice, s) == cudaSuccess;
   else ok = ok && cudaMemsetAsync(base + kOffDead, 0, n, s) == cudaSuccess;
   if (!ok) return Z80B_ECUDA;
@@ -108,13 +110,23 @@ int run_on_device(int device, uint32_t n, const uint8_t* tlens, const uint8_t* c
   P.stride = kStride;
   RoundBuf R{};
   R.pairs = reinterpret_cast<PairRec*>(base + kOffPairs);
-  R.cbase = reinterpret_cast<unsigned long long*>(base + kOffCbase);
-  R.cbase_x = reinterpret_cast<unsigned long long*>(base + kOffCbaseX);
+  R.cbase[0] = reinterpret_cast<unsigned long long*>(base + kOffCbase);
+  R.cbase[1] = reinterpret_cast<unsigned long long*>(base + kOffCbaseX);
   R.rejected = reinterpret_cast<uint32_t*>(base + kOffRej);
-  R.counter = reinterpret_cast<unsigned long long*>(base + kOffCounter);
+  R.ctl = reinterpret_cast<RoundCtl*>(base + kOffCtl);
   R.states = reinterpret_cast<unsigned long long*>(base + kOffStates);
   R.chunk_blocks = 32;
-  launch_exhaustive(T, P, R, n, total, total_x, 0, 0, 0, 4, s);
+  RoundArgs a{};
+  a.T = T;
+  a.P = P;
+  a.R = R;
+  // the chunk lists made by the host: entry i is pair i (no chunks: its
+  // successor's first chunk again)
+  h_ctl = RoundCtl{};
+  h_ctl.alloc[0] = (unsigned long long)n << kChunkBits | total;
+  h_ctl.alloc[1] = (unsigned long long)n << kChunkBits | total_x;
+  if (cudaMemcpyAsync(R.ctl, &h_ctl, sizeof h_ctl, cudaMemcpyHostToDevice, s) != cudaSuccess) return Z80B_ECUDA;
+  launch_exhaustive(sweep_args(a), h_ctl.alloc, 4, s);
   if (cudaGetLastError() != cudaSuccess) return Z80B_ECUDA;
   if (cudaMemcpyAsync(h_rej, base + kOffRej, 4ull * n, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
       cudaStreamSynchronize(s) != cudaSuccess)
@@ -174,7 +186,7 @@ extern "C" int z80b_exhaustive_noalloc(int device, const uint32_t* tgt, const ui
       units = (p.nblocks + 127) / 128;
     }
     unsigned long long ch = (units + 31) / 32;
-    if (ch > (1ull << 20)) ch = 1ull << 20;
+    if (ch > max_chunks(kMaxPairs)) ch = max_chunks(kMaxPairs);
     h_cbase[i] = total;
     h_cbase_x[i] = total_x;
     if (p.keepR & 0x40) total_x += ch;
