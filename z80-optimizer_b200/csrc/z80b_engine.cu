@@ -91,10 +91,12 @@ struct HBuf {
 
 struct PoolBufs {
   DBuf insn, qc, mid, size, prune, reads, lens;
-  // QuickCheck bucket index (pools of at most kQCIndexMax candidates)
+  // QuickCheck bucket index (ensure_qc_index)
   DBuf qkeys, qkeys_tmp, qtop, qelig, qsort_tmp;
   int qstate = 0;          // 0 not built, 1 built, -1 pool too large
   uint32_t qw2 = 0;        // word-2 mask the index hashes
+  uint32_t qvalid = 0;     // unpruned candidates
+  uint64_t qmasks = 0;     // dead-register masks indexed
   DevPool dev{};
   std::vector<uint32_t> host_insn;
   std::vector<uint8_t> host_lens;
@@ -479,52 +481,67 @@ int ensure_pair_index(z80b_ctx* ctx, uint32_t m) {
   return Z80B_OK;
 }
 
-// QuickCheck bucket index of a pool: every candidate's (dead-register mask,
-// hash of its masked vector-0 output, index) key for all 64 masks in one
-// sort, the per-mask top tables, and the eligible-candidate counts by
-// target size.  Pools above kQCIndexMax candidates keep the full scan.
-int ensure_qc_index(z80b_ctx* ctx, PoolBufs& P, uint32_t w2mask) {
+// QuickCheck bucket index of a pool (QCIndex) for the dead-register masks in
+// `masks`.  Pools of at most kQCAllMasksMax candidates get all 64 masks in one
+// sort; larger ones (the 266,675 first-op instructions of an all-hits search)
+// each mask when it first occurs, a sort of its own: 0.2 ms, where the scan
+// of all candidates that such pools took cost every target 1.6 us (48 ms for
+// 30,011 targets).  Pools above kQCIndexMax candidates keep the full scan.
+int ensure_qc_index(z80b_ctx* ctx, PoolBufs& P, uint32_t w2mask, uint64_t masks) {
   if (P.qstate == -1) return Z80B_OK;
-  if (P.qstate == 1 && P.qw2 == w2mask) return Z80B_OK;
   const uint32_t n = P.dev.n;
   if (n == 0 || n > kQCIndexMax) {
     P.qstate = -1;
     return Z80B_OK;
   }
   cudaStream_t s = ctx->stream;
-  std::vector<uint8_t> size(n), prune(n);
-  CK(cudaMemcpyAsync(size.data(), P.size.p, n, cudaMemcpyDeviceToHost, s));
-  CK(cudaMemcpyAsync(prune.data(), P.prune.p, n, cudaMemcpyDeviceToHost, s));
-  CK(cudaStreamSynchronize(s));
-  std::vector<uint32_t> by_size(257, 0), elig(256, 0);
-  uint32_t nv = 0;
-  for (uint32_t q = 0; q < n; q++)
-    if (!prune[q]) {
-      nv++;
-      by_size[size[q]]++;
-    }
-  for (int b = 1; b < 256; b++) elig[size_t(b)] = elig[size_t(b - 1)] + by_size[size_t(b - 1)];
-  const size_t nk = 64ull * n;
-  CK(P.qkeys_tmp.ensure(nk * 8));
-  CK(P.qkeys.ensure(nk * 8));
-  CK(P.qtop.ensure(64ull * (kQCTop + 1) * 4));
-  CK(P.qelig.ensure(256 * 4));
-  launch_qc_keys(P.dev, w2mask, P.qkeys_tmp.as<unsigned long long>(), s);
-  CKR(check_launch(ctx, "qc_keys"));
-  size_t tmp = 0;
-  CK(cub::DeviceRadixSort::SortKeys(nullptr, tmp, P.qkeys_tmp.as<unsigned long long>(),
-                                    P.qkeys.as<unsigned long long>(), int(nk), 0, 64, s));
-  CK(P.qsort_tmp.ensure(tmp));
-  CK(cub::DeviceRadixSort::SortKeys(P.qsort_tmp.p, tmp, P.qkeys_tmp.as<unsigned long long>(),
-                                    P.qkeys.as<unsigned long long>(), int(nk), 0, 64, s));
-  launch_qc_top(P.qkeys.as<unsigned long long>(), nv, P.qtop.as<uint32_t>(), s);
-  CKR(check_launch(ctx, "qc_top"));
-  CK(cudaMemcpyAsync(P.qelig.p, elig.data(), 256 * 4, cudaMemcpyHostToDevice, s));
-  CK(cudaStreamSynchronize(s));
-  ctx->launches += 3;
-  P.qstate = 1;
-  P.qw2 = w2mask;
-  trace("QuickCheck index: %u candidates, %u unpruned, 64 masks", n, nv);
+  const uint32_t bits = qc_top_bits(n);
+  const bool all = n <= kQCAllMasksMax;
+  if (P.qstate != 1 || P.qw2 != w2mask) {
+    P.qstate = 0;
+    P.qmasks = 0;
+    std::vector<uint8_t> size(n), prune(n);
+    CK(cudaMemcpyAsync(size.data(), P.size.p, n, cudaMemcpyDeviceToHost, s));
+    CK(cudaMemcpyAsync(prune.data(), P.prune.p, n, cudaMemcpyDeviceToHost, s));
+    CK(cudaStreamSynchronize(s));
+    std::vector<uint32_t> by_size(257, 0), elig(256, 0);
+    P.qvalid = 0;
+    for (uint32_t q = 0; q < n; q++)
+      if (!prune[q]) {
+        P.qvalid++;
+        by_size[size[q]]++;
+      }
+    for (int b = 1; b < 256; b++) elig[size_t(b)] = elig[size_t(b - 1)] + by_size[size_t(b - 1)];
+    CK(P.qkeys.ensure(64ull * n * 8));
+    CK(P.qkeys_tmp.ensure((all ? 64ull : 1ull) * n * 8));
+    CK(P.qtop.ensure(64ull * ((1ull << bits) + 1) * 4));
+    CK(P.qelig.ensure(256 * 4));
+    CK(cudaMemcpyAsync(P.qelig.p, elig.data(), 256 * 4, cudaMemcpyHostToDevice, s));
+    CK(cudaStreamSynchronize(s));
+    P.qstate = 1;
+    P.qw2 = w2mask;
+  }
+  if (all) masks = ~0ull;
+  for (uint32_t m = 0; m < 64; m += all ? 64 : 1) {
+    if (!((masks & ~P.qmasks) >> m & 1u)) continue;
+    const uint32_t nm = all ? 64 : 1;
+    // all masks: one sort leaves the segments of P.qvalid keys one behind the
+    // other; one mask: its own segment of n slots
+    const size_t nk = size_t(nm) * n, first = all ? 0 : size_t(m) * n;
+    launch_qc_keys(P.dev, w2mask, m, nm, P.qkeys_tmp.as<unsigned long long>(), s);
+    CKR(check_launch(ctx, "qc_keys"));
+    size_t tmp = 0;
+    CK(cub::DeviceRadixSort::SortKeys(nullptr, tmp, P.qkeys_tmp.as<unsigned long long>(),
+                                      P.qkeys.as<unsigned long long>() + first, int(nk), 0, 64, s));
+    CK(P.qsort_tmp.ensure(tmp));
+    CK(cub::DeviceRadixSort::SortKeys(P.qsort_tmp.p, tmp, P.qkeys_tmp.as<unsigned long long>(),
+                                      P.qkeys.as<unsigned long long>() + first, int(nk), 0, 64, s));
+    launch_qc_top(P.qkeys.as<unsigned long long>(), P.qvalid, uint32_t(first), m, nm, bits, P.qtop.as<uint32_t>(), s);
+    CKR(check_launch(ctx, "qc_top"));
+    ctx->launches += 3;
+    P.qmasks |= all ? ~0ull : 1ull << m;
+  }
+  trace("QuickCheck index: %u candidates, %u unpruned, masks %016llx", n, P.qvalid, (unsigned long long)P.qmasks);
   return Z80B_OK;
 }
 
@@ -897,12 +914,13 @@ int run_pipeline(z80b_ctx* ctx, const DevTargets& T, const PipeOpts& opts, z80b_
   QCIndex qix{};
   bool use_ix = false;
   if (ctx->qc_index) {
-    CKR(ensure_qc_index(ctx, *pool, cfg.w2mask));
+    CKR(ensure_qc_index(ctx, *pool, cfg.w2mask, opts.dreg_masks));
     if (pool->qstate == 1) {
       use_ix = true;
       qix.keys = pool->qkeys.as<unsigned long long>();
       qix.top = pool->qtop.as<uint32_t>();
       qix.elig_lt = pool->qelig.as<uint32_t>();
+      qix.top_bits = qc_top_bits(P.n);
     }
   }
   trace("pipeline: %u targets, mode %u, pool %u", n, mode, P.n);
@@ -912,8 +930,9 @@ int run_pipeline(z80b_ctx* ctx, const DevTargets& T, const PipeOpts& opts, z80b_
   q.cnt_all = ctx->cnt_all.as<uint32_t>();
   q.meta = ctx->meta.as<TargetMeta>();
   q.checks = ctx->checks.as<unsigned long long>();
-  if (use_ix && ctx->qc_single) {
+  if (use_ix && ctx->qc_single && P.n <= 65536) {
     // single pass: the count pass keeps the survivors of targets with few
+    // (16-bit candidate indices)
     CK(ctx->qc_tmp.ensure(4ull * kQCSlots * n));
     CK(ctx->qc_over.ensure(4));
     CK(cudaMemsetAsync(ctx->qc_over.p, 0, 4, s));
@@ -1308,6 +1327,8 @@ int upload_targets(z80b_ctx* ctx, Staged& S, const z80b_job* job, DevTargets* T,
   S.opts.mode = job->mode;
   S.opts.max_cand = job->max_cand_len;
   S.opts.no_exhaustive = (job->flags & Z80B_JOB_NO_EXHAUSTIVE) != 0;
+  if (job->mode == Z80B_MODE_ALL && job->dead_regs)
+    for (uint32_t i = 0; i < n; i++) S.opts.dreg_masks |= 1ull << (job->dead_regs[i] & 0x3Fu);
   if (job->max_cand_len >= 2)
     for (uint32_t i = 0; i < n; i++) {
       const uint32_t dr = job->dead_regs ? job->dead_regs[i] & 0x3Fu : 0u;

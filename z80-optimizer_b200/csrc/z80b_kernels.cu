@@ -2023,30 +2023,30 @@ __device__ __forceinline__ uint32_t lower_bound_u64(const unsigned long long* a,
   return lo;
 }
 
-// QuickCheck bucket index of a candidate pool (at most 65,536 entries): one
-// segment per dead-register mask m, keys m << 48 | bucket hash << 16 | index
-// sorted, pruned candidates left out (their keys sort past the last
-// segment); a top table per segment holds the first entry of each 4,096th of
-// the hash range.
-__global__ void k_qc_keys(DevPool P, uint32_t w2mask, unsigned long long* __restrict__ keys) {
+// QuickCheck bucket index of a candidate pool (QCIndex): pruned candidates'
+// keys sort past every real one.
+__global__ void k_qc_keys(DevPool P, uint32_t w2mask, uint32_t m0, uint32_t nm, unsigned long long* __restrict__ keys) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= 64u * P.n) return;
-  const uint32_t m = i / P.n, q = i - m * P.n;
+  if (i >= nm * P.n) return;
+  const uint32_t m = m0 + i / P.n, q = i % P.n;
   if (P.prune[q]) {
     keys[i] = ~0ull;
     return;
   }
   const uint4 o = P.qc[q];
   const uint32_t h = bucket_hash(o.x & key_keep0(m), o.y & key_keep1(m), o.z & w2mask);
-  keys[i] = ((unsigned long long)m << 48) | ((unsigned long long)h << 16) | q;
+  keys[i] = ((unsigned long long)m << 58) | ((unsigned long long)h << kQCIndexBits) | q;
 }
-__global__ void k_qc_top(const unsigned long long* __restrict__ keys, uint32_t nv, uint32_t* __restrict__ top) {
+__global__ void k_qc_top(const unsigned long long* __restrict__ keys, uint32_t nv, uint32_t first, uint32_t m0,
+                         uint32_t nm, uint32_t top_bits, uint32_t* __restrict__ top) {
+  const uint32_t per = (1u << top_bits) + 1u;
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= 64u * (kQCTop + 1)) return;
-  const uint32_t m = i / (kQCTop + 1), b = i - m * (kQCTop + 1);
-  top[i] = b == kQCTop ? (m + 1) * nv
-                       : m * nv + lower_bound_u64(keys + (size_t)m * nv, nv,
-                                                  ((unsigned long long)m << 48) | ((unsigned long long)b << 36));
+  if (i >= nm * per) return;
+  const uint32_t j = i / per, b = i - j * per, m = m0 + j;
+  const uint32_t seg = first + j * nv;
+  const unsigned long long lo =
+      ((unsigned long long)m << 58) | ((unsigned long long)b << (32u - top_bits + kQCIndexBits));
+  top[m * per + b] = b == per - 1u ? seg + nv : seg + lower_bound_u64(keys + seg, nv, lo);
 }
 
 // QuickCheck through the bucket index: a target only meets the candidates
@@ -2136,7 +2136,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_qc_bucket(DevTargets T, DevPool P
     const uint32_t h = bucket_hash(g.tw[0][0] & key_keep0(m), g.tw[0][1] & key_keep1(m), g.tw[0][2] & cfg.w2mask);
     uint32_t r0 = 0, r1 = 0;
     if (work) {
-      const uint32_t* top = ix.top + m * (kQCTop + 1) + (h >> (32 - kQCTopBits));
+      const uint32_t* top = ix.top + m * ((1u << ix.top_bits) + 1u) + (h >> (32u - ix.top_bits));
       r0 = top[0];
       r1 = top[1];
     }
@@ -2150,8 +2150,8 @@ __global__ void __launch_bounds__(kBlock, 4) k_qc_bucket(DevTargets T, DevPool P
       uint32_t diff = 0, c = 0;
       if (i < r1) {
         const unsigned long long key = ix.keys[i];
-        c = uint32_t(key) & 0xFFFFu;
-        if (uint32_t(key >> 16) == h && P.size[c] < g.tb)
+        c = uint32_t(key) & ((1u << kQCIndexBits) - 1u);
+        if (uint32_t(key >> kQCIndexBits) == h && P.size[c] < g.tb)
           qc_candidate(P, P.qc[c], c, g, cfg.w2mask, cfg.all_hits != 0, fp, mp, diff);
       }
       if constexpr (!COLLECT) {
@@ -2523,13 +2523,15 @@ void launch_qc_scan(const DevTargets& T, const DevPool& P, const QCConfig& cfg, 
   if (collect) k_qc_scan<true><<<grid, kBlock, smem, s>>>(T, P, cfg, o);
   else k_qc_scan<false><<<grid, kBlock, smem, s>>>(T, P, cfg, o);
 }
-void launch_qc_keys(const DevPool& P, uint32_t w2mask, unsigned long long* keys, cudaStream_t s) {
-  const uint32_t n = 64u * P.n;
-  if (n) k_qc_keys<<<grid_for(n, 256), 256, 0, s>>>(P, w2mask, keys);
+void launch_qc_keys(const DevPool& P, uint32_t w2mask, uint32_t m0, uint32_t nm, unsigned long long* keys,
+                    cudaStream_t s) {
+  const uint32_t n = nm * P.n;
+  if (n) k_qc_keys<<<grid_for(n, 256), 256, 0, s>>>(P, w2mask, m0, nm, keys);
 }
-void launch_qc_top(const unsigned long long* keys, uint32_t nv, uint32_t* top, cudaStream_t s) {
-  const uint32_t n = 64u * (kQCTop + 1);
-  k_qc_top<<<grid_for(n, 256), 256, 0, s>>>(keys, nv, top);
+void launch_qc_top(const unsigned long long* keys, uint32_t nv, uint32_t first, uint32_t m0, uint32_t nm,
+                   uint32_t top_bits, uint32_t* top, cudaStream_t s) {
+  const uint32_t n = nm * ((1u << top_bits) + 1u);
+  k_qc_top<<<grid_for(n, 256), 256, 0, s>>>(keys, nv, first, m0, nm, top_bits, top);
 }
 void launch_qc_compact(const QCOut& q, uint32_t n, cudaStream_t s) {
   if (!n) return;
