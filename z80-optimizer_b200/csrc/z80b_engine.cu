@@ -208,7 +208,12 @@ struct z80b_ctx {
   DBuf cub_tmp;
   DBuf hits, nhits, fpq;
   DBuf v_tgt, v_cand, v_tl, v_cl, v_dead, v_out, v_fd, v_in, v_outs;
-  DBuf mul_best, mul_stats;   // constant-multiply search: best key per K, counters
+  DBuf mul_best, mul_stats;   // constant-multiply search: best key per length and K, counters
+  DBuf mul_hash[mul::kMaxLen], mul_key[mul::kMaxLen];  // prefixes with distinct states per length
+  DBuf mul_child, mul_tab_hash, mul_tab_key, mul_count;
+  DBuf mul_words[mul::kNumPools][2][mul::kMaxInner + 1];  // the walk's suffixes (WordBufs), by min_len 1 or not
+  uint32_t mul_first_ops[mul::kNumPools][2][mul::kMaxInner + 1] = {};
+  HBuf h_mul;
   // length-2 candidates: the pair pool and its indexes, shared by the
   // contexts of a device; the per-lane pass state is per context
   std::shared_ptr<PairShared> pairpool;
@@ -876,6 +881,179 @@ int rounds_on_host(z80b_ctx* ctx, const RoundArgs* a, const RoundArgs& h_args, b
     if (!h.more) return Z80B_OK;
   }
 }
+
+// One constant-multiply search.  The short lengths (up to kDirect sequences)
+// are walked one behind the other without a host round trip, each launch
+// leaving out the constants that shorter ones have answered.  The longer ones
+// take their prefixes from the levels of distinct states
+// (z80b_mulopt.cuh), extended by a level per length, and walk the last
+// kSuffix instructions; a level of more than kMaxChildren children is not
+// built, the walk then takes longer suffixes.
+struct MulSearch {
+  z80b_ctx* ctx;
+  mul::SearchArgs a;
+  int n_ops, sms;
+  z80b_mul_stats& st;
+  // 21 ops to length 6 and 14 ops to length 7 (25 and 16 us a length); a
+  // level of states costs about 40 us of launches and a wait
+  static constexpr double kDirect = 1.5e8;
+  static constexpr double kShort = 1e6;  // all in one launch
+  static constexpr int kSuffix = mul::kMaxInner + 1;
+  static constexpr uint64_t kMaxChildren = 1ull << 24;  // at most 1.6 GB of scratch
+  uint32_t count[mul::kMaxLen] = {};  // prefixes per level
+  int built = -1;                     // levels built
+  bool plain = false;                 // walk every prefix (two states shared a hash)
+
+  // a level's children fit the scratch and their odometer indices 32 bits
+  bool can_extend() const {
+    if (built < 0) return true;
+    double v = 1;
+    for (int i = 0; i <= built; i++) v *= n_ops;
+    return uint64_t(count[built]) * uint64_t(n_ops) <= kMaxChildren && v < 4294967296.0;
+  }
+
+  int extend() {
+    cudaStream_t s = ctx->stream;
+    const int l = built;
+    if (l < 0) {
+      CK(ctx->mul_hash[0].ensure(8));
+      CK(ctx->mul_key[0].ensure(8));
+      CK(mul::launch_root(a, ctx->mul_hash[0].as<unsigned long long>(), ctx->mul_key[0].as<unsigned long long>(), s));
+      st.launches++;
+      count[0] = 1;
+      built = 0;
+      return Z80B_OK;
+    }
+    const uint64_t children = uint64_t(count[l]) * uint64_t(n_ops);
+    uint64_t known = 0, slots = 1024;
+    for (int i = 0; i <= l; i++) known += count[i];
+    while (slots < 2 * (children + known)) slots *= 2;
+    CK(ctx->mul_tab_hash.ensure(8 * slots));
+    CK(ctx->mul_tab_key.ensure(8 * slots));
+    CK(ctx->mul_child.ensure(8 * std::max<uint64_t>(children, 1)));
+    CK(ctx->mul_hash[l + 1].ensure(8 * std::max<uint64_t>(children, 1)));
+    CK(ctx->mul_key[l + 1].ensure(8 * std::max<uint64_t>(children, 1)));
+    CK(ctx->mul_count.ensure(8));
+    CK(cudaMemsetAsync(ctx->mul_tab_hash.p, 0, 8 * slots, s));
+    CK(cudaMemsetAsync(ctx->mul_tab_key.p, 0xFF, 8 * slots, s));
+    CK(cudaMemsetAsync(ctx->mul_count.p, 0, 8, s));
+    const mul::StateTable t{ctx->mul_tab_hash.as<unsigned long long>(), ctx->mul_tab_key.as<unsigned long long>(),
+                            slots - 1};
+    for (int i = 0; i <= l; i++) {
+      CK(mul::launch_enter(t, ctx->mul_hash[i].as<unsigned long long>(), ctx->mul_key[i].as<unsigned long long>(),
+                           count[i], s));
+      st.launches++;
+    }
+    const unsigned long long* key = ctx->mul_key[l].as<unsigned long long>();
+    CK(mul::launch_children(a, t, key, count[l], l, ctx->mul_child.as<unsigned long long>(), sms, s));
+    CK(mul::launch_select(a, t, key, count[l], l, ctx->mul_child.as<unsigned long long>(),
+                          ctx->mul_hash[l + 1].as<unsigned long long>(), ctx->mul_key[l + 1].as<unsigned long long>(),
+                          ctx->mul_count.as<uint32_t>(), sms, s));
+    st.launches += 2;
+    uint32_t c[2] = {0, 0};
+    CKR(fetch(ctx, c, ctx->mul_count.as<uint32_t>(), 2));
+    count[l + 1] = c[0];
+    built = l + 1;
+    if (c[1]) plain = true;
+    trace("mulopt level %d: %llu children, %u new states", l + 1, (unsigned long long)children, c[0]);
+    return Z80B_OK;
+  }
+
+  int walk(int len, const unsigned long long* reps, uint32_t n, int rep_len) {
+    const int inner = (reps ? len - rep_len : mul::plain_suffix(a.pool, len)) - 1;
+    const int sh = a.min_len == 1 ? 1 : 0;
+    DBuf& w = ctx->mul_words[a.pool][sh][inner];
+    size_t masks = 0, leaves = 1;
+    for (int i = 0; i < inner; i++) {
+      masks += leaves;
+      leaves *= size_t(n_ops);
+    }
+    if (!w.p) {
+      const mul::WordImage im = mul::word_image(a.pool, inner, sh != 0);
+      CK(w.ensure(4 * masks + leaves));
+      CK(cudaMemcpy(w.p, im.mask.data(), 4 * masks, cudaMemcpyHostToDevice));
+      CK(cudaMemcpy(w.as<uint8_t>() + 4 * masks, im.leaf.data(), leaves, cudaMemcpyHostToDevice));
+      ctx->mul_first_ops[a.pool][sh][inner] = im.first_ops;
+    }
+    const mul::WordBufs words{w.as<uint32_t>(), w.as<uint8_t>() + 4 * masks, ctx->mul_first_ops[a.pool][sh][inner]};
+    cudaError_t e = mul::launch_length(a, len, reps, n, rep_len, words, ctx->mul_best.as<unsigned long long>(),
+                                       ctx->mul_stats.as<mul::LenStats>(), sms, ctx->stream);
+    if (e != cudaSuccess) return fail(ctx, Z80B_ECUDA, "mulopt length %d launch: %s", len, cudaGetErrorString(e));
+    st.launches++;
+    return Z80B_OK;
+  }
+
+  int run(int* found_len, unsigned long long* found_key) {
+    cudaStream_t s = ctx->stream;
+    const size_t row = 256 * sizeof(unsigned long long);
+    CK(ctx->mul_best.ensure(mul::kMaxLen * row));
+    CK(ctx->mul_stats.ensure(sizeof(mul::LenStats)));
+    CK(ctx->h_mul.ensure(mul::kMaxLen * row + sizeof(mul::LenStats)));
+    unsigned long long* const best = ctx->h_mul.as<unsigned long long>();
+    mul::LenStats* const ls = reinterpret_cast<mul::LenStats*>(best + mul::kMaxLen * 256);
+    CK(cudaMemsetAsync(ctx->mul_best.p, 0xFF, mul::kMaxLen * row, s));
+    CK(cudaMemsetAsync(ctx->mul_stats.p, 0, sizeof(mul::LenStats), s));
+    Timer tm{ctx, 0, 1};
+    tm.start();
+    double nl = 1;  // sequences of the current length
+    for (int i = 0; i < a.min_len; i++) nl *= n_ops;
+    int len = a.min_len;
+    while (len <= a.max_len) {
+      // the lengths of this turn: the short ones together, or one long one
+      const int first = len;
+      double v = nl;  // sequences of length len
+      for (; len <= a.max_len && v <= kShort; v *= n_ops) len++;
+      if (len > first) {
+        const cudaError_t e = mul::launch_short(a, first, len - first, ctx->mul_best.as<unsigned long long>(),
+                                                ctx->mul_stats.as<mul::LenStats>(), sms, s);
+        if (e != cudaSuccess) return fail(ctx, Z80B_ECUDA, "mulopt lengths %d.. launch: %s", first, cudaGetErrorString(e));
+        st.launches++;
+      }
+      for (; len <= a.max_len && v <= kDirect; len++, v *= n_ops) CKR(walk(len, nullptr, 0, 0));
+      if (len == first) {
+        int p = std::max(1, len - kSuffix);
+        while (!plain && built < p && can_extend()) CKR(extend());
+        p = std::min(p, built);
+        if (plain || len - p > kSuffix) CKR(walk(len, nullptr, 0, 0));
+        else CKR(walk(len, ctx->mul_key[p].as<unsigned long long>(), count[p], p));
+        len++;
+      }
+      tm.stop();
+      CK(cudaMemcpyAsync(best + first * 256, ctx->mul_best.as<unsigned long long>() + first * 256,
+                         size_t(len - first) * row, cudaMemcpyDeviceToHost, s));
+      CK(cudaMemcpyAsync(ls, ctx->mul_stats.p, sizeof *ls, cudaMemcpyDeviceToHost, s));
+      CK(cudaStreamSynchronize(s));
+      // the answers of these lengths, in order; what a length searched is
+      // what the shorter ones left
+      for (int l = first; l < len; l++, nl *= n_ops) {
+        bool any = false;
+        for (int w = 0; w < 8; w++) any = any || a.want[w];
+        if (!any) break;
+        st.lengths++;
+        st.sequences += (uint64_t)nl;
+        for (int k = 2; k < 256; k++) {
+          if (!((a.want[k >> 5] >> (k & 31)) & 1u)) continue;
+          st.per_k_sequences += (uint64_t)nl;
+          if (best[l * 256 + k] != mul::kNoKey) {
+            found_len[k] = l;
+            found_key[k] = best[l * 256 + k];
+            a.want[k >> 5] &= ~(1u << (k & 31));
+          }
+        }
+      }
+      bool any = false;
+      for (int w = 0; w < 8; w++) any = any || a.want[w];
+      trace("mulopt pool %d lengths %d..%d: %llu nodes filtered, %llu full checks", a.pool, first, len - 1,
+            ls->filter_nodes, ls->full_checks);
+      if (!any) break;
+    }
+    st.filter_nodes = ls->filter_nodes;
+    st.full_checks = ls->full_checks;
+    st.full_pass = ls->full_pass;
+    st.device_ms = tm.ms();
+    return Z80B_OK;
+  }
+};
 
 // Runs the pipeline on device-resident targets.  Rules stay in ctx->rules
 // (DevRule), count in *nr.
@@ -2028,8 +2206,6 @@ int z80b_mul_search(z80b_ctx* ctx, int pool, uint8_t init_b, uint8_t init_c, uin
   cudaSetDevice(ctx->device);
   int sms = 0;
   CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device));
-  CK(ctx->mul_best.ensure(256 * sizeof(unsigned long long)));
-  CK(ctx->mul_stats.ensure(sizeof(mul::LenStats)));
   mul::SearchArgs a{};
   a.pool = pool;
   a.b = init_b;
@@ -2045,44 +2221,9 @@ int z80b_mul_search(z80b_ctx* ctx, int pool, uint8_t init_b, uint8_t init_c, uin
   z80b_mul_stats st{};
   int found_len[256] = {};
   unsigned long long found_key[256] = {};
-  double nl = 1;
-  for (int i = 0; i < min_len - 1; i++) nl *= pi.n;
-  for (int len = min_len; len <= max_len; len++) {
-    nl *= pi.n;
-    bool any = false;
-    for (int w = 0; w < 8; w++) any = any || a.want[w];
-    if (!any) break;
-    CK(cudaMemsetAsync(ctx->mul_best.p, 0xFF, 256 * sizeof(unsigned long long), ctx->stream));
-    CK(cudaMemsetAsync(ctx->mul_stats.p, 0, sizeof(mul::LenStats), ctx->stream));
-    Timer tm{ctx, 0, 1};
-    tm.start();
-    cudaError_t e = mul::launch_length(a, len, ctx->mul_best.as<unsigned long long>(),
-                                       ctx->mul_stats.as<mul::LenStats>(), sms, ctx->stream);
-    if (e != cudaSuccess) return fail(ctx, Z80B_ECUDA, "mulopt length %d launch: %s", len, cudaGetErrorString(e));
-    tm.stop();
-    st.launches++;
-    unsigned long long best[256];
-    mul::LenStats ls{};
-    CK(cudaMemcpyAsync(best, ctx->mul_best.p, sizeof best, cudaMemcpyDeviceToHost, ctx->stream));
-    CK(cudaMemcpyAsync(&ls, ctx->mul_stats.p, sizeof ls, cudaMemcpyDeviceToHost, ctx->stream));
-    CK(cudaStreamSynchronize(ctx->stream));
-    st.device_ms += tm.ms();
-    st.lengths++;
-    st.sequences += (uint64_t)nl;
-    st.filter_nodes += ls.filter_nodes;
-    st.full_checks += ls.full_checks;
-    st.full_pass += ls.full_pass;
-    for (int k = 2; k < 256; k++) {
-      if (!((a.want[k >> 5] >> (k & 31)) & 1u)) continue;
-      st.per_k_sequences += (uint64_t)nl;
-      if (best[k] != mul::kNoKey) {
-        found_len[k] = len;
-        found_key[k] = best[k];
-        a.want[k >> 5] &= ~(1u << (k & 31));
-      }
-    }
-    trace("mulopt pool %d length %d: %.3f ms, %llu nodes filtered, %llu full checks", pool, len, st.device_ms,
-          (unsigned long long)ls.filter_nodes, (unsigned long long)ls.full_checks);
+  if (!kl.empty()) {
+    MulSearch ms{ctx, a, pi.n, sms, st};
+    CKR(ms.run(found_len, found_key));
   }
   for (size_t i = 0; i < kl.size(); i++) {
     const int k = kl[i];
