@@ -92,7 +92,7 @@ struct HBuf {
 struct PoolBufs {
   DBuf insn, qc, mid, size, prune, reads, lens;
   // QuickCheck bucket index (ensure_qc_index)
-  DBuf qkeys, qkeys_tmp, qtop, qelig, qsort_tmp;
+  DBuf qkeys, qkeys_tmp, qentries, qhash2, qtop, qelig, qsort_tmp, qclash;
   int qstate = 0;          // 0 not built, 1 built, -1 pool too large
   uint32_t qw2 = 0;        // word-2 mask the index hashes
   uint32_t qvalid = 0;     // unpruned candidates
@@ -486,12 +486,13 @@ int ensure_pair_index(z80b_ctx* ctx, uint32_t m) {
   return Z80B_OK;
 }
 
-// QuickCheck bucket index of a pool (QCIndex) for the dead-register masks in
+// QuickCheck index of a pool (QCIndex) for the dead-register masks in
 // `masks`.  Pools of at most kQCAllMasksMax candidates get all 64 masks in one
 // sort; larger ones (the 266,675 first-op instructions of an all-hits search)
 // each mask when it first occurs, a sort of its own: 0.2 ms, where the scan
 // of all candidates that such pools took cost every target 1.6 us (48 ms for
-// 30,011 targets).  Pools above kQCIndexMax candidates keep the full scan.
+// 30,011 targets).  Pools above kQCIndexMax candidates keep the full scan, and
+// so does a pool in which two different outputs share both hashes.
 int ensure_qc_index(z80b_ctx* ctx, PoolBufs& P, uint32_t w2mask, uint64_t masks) {
   if (P.qstate == -1) return Z80B_OK;
   const uint32_t n = P.dev.n;
@@ -502,6 +503,9 @@ int ensure_qc_index(z80b_ctx* ctx, PoolBufs& P, uint32_t w2mask, uint64_t masks)
   cudaStream_t s = ctx->stream;
   const uint32_t bits = qc_top_bits(n);
   const bool all = n <= kQCAllMasksMax;
+  if (all) masks = ~0ull;
+  if (P.qstate == 1 && P.qw2 == w2mask && !(masks & ~P.qmasks)) return Z80B_OK;
+  const uint32_t nm = all ? 64 : 1;
   if (P.qstate != 1 || P.qw2 != w2mask) {
     P.qstate = 0;
     P.qmasks = 0;
@@ -517,36 +521,43 @@ int ensure_qc_index(z80b_ctx* ctx, PoolBufs& P, uint32_t w2mask, uint64_t masks)
         by_size[size[q]]++;
       }
     for (int b = 1; b < 256; b++) elig[size_t(b)] = elig[size_t(b - 1)] + by_size[size_t(b - 1)];
-    CK(P.qkeys.ensure(64ull * n * 8));
-    CK(P.qkeys_tmp.ensure((all ? 64ull : 1ull) * n * 8));
+    const size_t ne = std::max<size_t>(64ull * P.qvalid, 1);
+    CK(P.qkeys.ensure(size_t(nm) * n * 8));
+    CK(P.qkeys_tmp.ensure(size_t(nm) * n * 8));
+    CK(P.qentries.ensure(ne * 16));
+    CK(P.qhash2.ensure(ne * 4));
     CK(P.qtop.ensure(64ull * ((1ull << bits) + 1) * 4));
     CK(P.qelig.ensure(256 * 4));
+    CK(P.qclash.ensure(4));
     CK(cudaMemcpyAsync(P.qelig.p, elig.data(), 256 * 4, cudaMemcpyHostToDevice, s));
+    CK(cudaMemsetAsync(P.qclash.p, 0, 4, s));
     CK(cudaStreamSynchronize(s));
     P.qstate = 1;
     P.qw2 = w2mask;
   }
-  if (all) masks = ~0ull;
-  for (uint32_t m = 0; m < 64; m += all ? 64 : 1) {
+  for (uint32_t m = 0; m < 64; m += nm) {
     if (!((masks & ~P.qmasks) >> m & 1u)) continue;
-    const uint32_t nm = all ? 64 : 1;
-    // all masks: one sort leaves the segments of P.qvalid keys one behind the
-    // other; one mask: its own segment of n slots
-    const size_t nk = size_t(nm) * n, first = all ? 0 : size_t(m) * n;
+    const size_t nk = size_t(nm) * n;
     launch_qc_keys(P.dev, w2mask, m, nm, P.qkeys_tmp.as<unsigned long long>(), s);
     CKR(check_launch(ctx, "qc_keys"));
     size_t tmp = 0;
     CK(cub::DeviceRadixSort::SortKeys(nullptr, tmp, P.qkeys_tmp.as<unsigned long long>(),
-                                      P.qkeys.as<unsigned long long>() + first, int(nk), 0, 64, s));
+                                      P.qkeys.as<unsigned long long>(), int(nk), 0, 64, s));
     CK(P.qsort_tmp.ensure(tmp));
     CK(cub::DeviceRadixSort::SortKeys(P.qsort_tmp.p, tmp, P.qkeys_tmp.as<unsigned long long>(),
-                                      P.qkeys.as<unsigned long long>() + first, int(nk), 0, 64, s));
-    launch_qc_top(P.qkeys.as<unsigned long long>(), P.qvalid, uint32_t(first), m, nm, bits, P.qtop.as<uint32_t>(), s);
-    CKR(check_launch(ctx, "qc_top"));
-    ctx->launches += 3;
+                                      P.qkeys.as<unsigned long long>(), int(nk), 0, 64, s));
+    launch_qc_entries(P.dev, w2mask, P.qkeys.as<unsigned long long>(), P.qvalid, m * P.qvalid, m, nm, bits,
+                      P.qentries.as<uint4>(), P.qhash2.as<uint32_t>(), P.qtop.as<uint32_t>(), P.qclash.as<uint32_t>(),
+                      s);
+    CKR(check_launch(ctx, "qc_entries"));
+    ctx->launches += 5;
     P.qmasks |= all ? ~0ull : 1ull << m;
   }
-  trace("QuickCheck index: %u candidates, %u unpruned, masks %016llx", n, P.qvalid, (unsigned long long)P.qmasks);
+  uint32_t clash = 0;
+  CKR(fetch(ctx, &clash, P.qclash.as<uint32_t>()));
+  if (clash) P.qstate = -1;
+  trace("QuickCheck index: %u candidates, %u unpruned, masks %016llx, clash %u", n, P.qvalid,
+        (unsigned long long)P.qmasks, clash);
   return Z80B_OK;
 }
 
@@ -1095,7 +1106,8 @@ int run_pipeline(z80b_ctx* ctx, const DevTargets& T, const PipeOpts& opts, z80b_
     CKR(ensure_qc_index(ctx, *pool, cfg.w2mask, opts.dreg_masks));
     if (pool->qstate == 1) {
       use_ix = true;
-      qix.keys = pool->qkeys.as<unsigned long long>();
+      qix.entries = pool->qentries.as<uint4>();
+      qix.hash2 = pool->qhash2.as<uint32_t>();
       qix.top = pool->qtop.as<uint32_t>();
       qix.elig_lt = pool->qelig.as<uint32_t>();
       qix.top_bits = qc_top_bits(P.n);

@@ -1884,18 +1884,6 @@ __device__ __forceinline__ uint32_t key_keep1(uint32_t dregs) {
   return ((dregs & 4u) ? 0u : 0xFFu) | ((dregs & 8u) ? 0u : 0xFF00u) | ((dregs & 16u) ? 0u : 0xFF0000u) |
          ((dregs & 32u) ? 0u : 0xFF000000u);
 }
-// 32-bit bucket hash of a masked output (splitmix64 finalizer).
-__device__ __forceinline__ uint32_t bucket_hash(uint32_t w0, uint32_t w1, uint32_t w2) {
-  unsigned long long h = ((unsigned long long)w0 << 32) | w1;
-  h ^= (unsigned long long)w2 * 0x9E3779B97F4A7C15ull;
-  h ^= h >> 30;
-  h *= 0xBF58476D1CE4E5B9ull;
-  h ^= h >> 27;
-  h *= 0x94D049BB133111EBull;
-  h ^= h >> 31;
-  return uint32_t(h >> 32);
-}
-
 // Hash of one vector's output (A, live registers, SP, M); the hash of a
 // sequence is the sum over the eight vectors, so that the lanes of a warp can
 // each hash one.
@@ -2023,8 +2011,23 @@ __device__ __forceinline__ uint32_t lower_bound_u64(const unsigned long long* a,
   return lo;
 }
 
-// QuickCheck bucket index of a candidate pool (QCIndex): pruned candidates'
-// keys sort past every real one.
+// The two hashes of one vector's compared output; an output's hash is the sum
+// over the eight vectors, so that lanes can each hash one.
+__device__ __forceinline__ uint32_t qc_mix(uint32_t a, uint32_t b, uint32_t c) {
+  uint32_t h = a * 0x9E3779B1u;
+  h = (h ^ (h >> 15)) + b;
+  h *= 0x85EBCA6Bu;
+  h = (h ^ (h >> 13)) + c;
+  h *= 0xC2B2AE35u;
+  return h ^ (h >> 16);
+}
+__device__ __forceinline__ uint32_t qc_hash(uint32_t w0, uint32_t w1, uint32_t w2, uint32_t v) {
+  return qc_mix(w0, w1, w2 + (v << 27));
+}
+__device__ __forceinline__ uint32_t qc_hash2(uint32_t w0, uint32_t w1, uint32_t w2, uint32_t v) {
+  return qc_mix(w1 ^ 0x5BD1E995u, w2 + (v << 24), w0 + 0x27D4EB2Fu);
+}
+// Index build (QCIndex): pruned candidates' keys sort past every real one.
 __global__ void k_qc_keys(DevPool P, uint32_t w2mask, uint32_t m0, uint32_t nm, unsigned long long* __restrict__ keys) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nm * P.n) return;
@@ -2033,9 +2036,50 @@ __global__ void k_qc_keys(DevPool P, uint32_t w2mask, uint32_t m0, uint32_t nm, 
     keys[i] = ~0ull;
     return;
   }
-  const uint4 o = P.qc[q];
-  const uint32_t h = bucket_hash(o.x & key_keep0(m), o.y & key_keep1(m), o.z & w2mask);
+  uint32_t h = 0;
+#pragma unroll
+  for (uint32_t v = 0; v < 8; v++) {
+    const uint4 o = P.qc[(size_t)v * P.n + q];
+    h += qc_hash(o.x & key_keep0(m), o.y & key_keep1(m), o.z & w2mask, v);
+  }
   keys[i] = ((unsigned long long)m << 58) | ((unsigned long long)h << kQCIndexBits) | q;
+}
+__global__ void k_qc_entries(DevPool P, uint32_t w2mask, const unsigned long long* __restrict__ keys, uint32_t n,
+                             uint4* __restrict__ entries, uint32_t* __restrict__ hash2) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const unsigned long long key = keys[i];
+  const uint32_t m = uint32_t(key >> 58), c = uint32_t(key) & ((1u << kQCIndexBits) - 1u);
+  uint32_t h2 = 0, f[2] = {0u, 0u};
+#pragma unroll
+  for (uint32_t v = 0; v < 8; v++) {
+    const uint4 o = P.qc[(size_t)v * P.n + c];
+    h2 += qc_hash2(o.x & key_keep0(m), o.y & key_keep1(m), o.z & w2mask, v);
+    f[v >> 2] |= ((o.x >> 8) & 0xFFu) << (8 * (v & 3u));
+  }
+  entries[i] = make_uint4(uint32_t(key >> kQCIndexBits), c | uint32_t(P.size[c]) << kQCIndexBits, f[0], f[1]);
+  hash2[i] = h2;
+}
+// Every entry against the nearest one before it with both hashes equal.
+__global__ void k_qc_check(DevPool P, uint32_t w2mask, const unsigned long long* __restrict__ keys,
+                           const uint32_t* __restrict__ hash2, uint32_t n, uint32_t* __restrict__ clash) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const unsigned long long run = keys[i] >> kQCIndexBits;
+  const uint32_t m = uint32_t(keys[i] >> 58), c = uint32_t(keys[i]) & ((1u << kQCIndexBits) - 1u);
+  uint32_t j = i;
+  do {
+    if (j == 0 || (keys[j - 1] >> kQCIndexBits) != run) return;
+    j--;
+  } while (hash2[j] != hash2[i]);
+  const uint32_t e = uint32_t(keys[j]) & ((1u << kQCIndexBits) - 1u);
+  uint32_t d = 0;
+#pragma unroll
+  for (uint32_t v = 0; v < 8; v++) {
+    const uint4 x = P.qc[(size_t)v * P.n + c], y = P.qc[(size_t)v * P.n + e];
+    d |= ((x.x ^ y.x) & key_keep0(m)) | ((x.y ^ y.y) & key_keep1(m)) | ((x.z ^ y.z) & w2mask);
+  }
+  if (d) *clash = 1;
 }
 __global__ void k_qc_top(const unsigned long long* __restrict__ keys, uint32_t nv, uint32_t first, uint32_t m0,
                          uint32_t nm, uint32_t top_bits, uint32_t* __restrict__ top) {
@@ -2043,67 +2087,27 @@ __global__ void k_qc_top(const unsigned long long* __restrict__ keys, uint32_t n
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nm * per) return;
   const uint32_t j = i / per, b = i - j * per, m = m0 + j;
-  const uint32_t seg = first + j * nv;
+  const uint32_t seg = j * nv;
   const unsigned long long lo =
       ((unsigned long long)m << 58) | ((unsigned long long)b << (32u - top_bits + kQCIndexBits));
-  top[m * per + b] = b == per - 1u ? seg + nv : seg + lower_bound_u64(keys + seg, nv, lo);
+  top[m * per + b] = first + (b == per - 1u ? seg + nv : seg + lower_bound_u64(keys + seg, nv, lo));
 }
 
-// QuickCheck through the bucket index: a target only meets the candidates
-// whose vector-0 output agrees with its own on A, the live registers and
-// word 2 (the flags are compared per candidate, under the dead flags), which
-// is every candidate that can pass.  Entries of a bucket are in pool order,
-// so survivors come out in enumeration order as in the full scan.
-// Four targets per warp, eight lanes each: lane 8g + v runs target t0 + g on
-// vector v, so one pass of the dispatch loop, the output shuffles and the
-// bucket loop serve four targets (the buckets hold a candidate or two; a
-// warp per target left three quarters of its lanes idle).  Lanes of a group
-// that has no target (past the end) take part in the warp's collectives
-// with nothing to do.
-__device__ __forceinline__ void qc_target4(const DevTargets& T, uint32_t t, bool valid, QCTarget& g) {
-  const unsigned lane = lane_id();
-  const unsigned sub = lane & 7u;
-  const uint32_t tl = valid ? target_len(T, t) : 0u;
-  const uint32_t pw = sub < tl ? T.insn[(size_t)t * T.stride + sub] : 0u;
-  uint32_t sz = 0, ts = 0, rd = 0;
-  if (sub < tl) {
-    const OpInfo oi = g_ops[pw & 0xFFFFu];
-    sz = oi.size;
-    ts = oi.tstates;
-    rd = oi.reads;
-  }
-#pragma unroll
-  for (int off = 2; off >= 1; off >>= 1) {
-    sz += __shfl_down_sync(kFull, sz, off, 8);
-    ts += __shfl_down_sync(kFull, ts, off, 8);
-    rd |= __shfl_down_sync(kFull, rd, off, 8);
-  }
-  g.tl = tl;
-  g.tb = __shfl_sync(kFull, sz, 0, 8);
-  g.tts = __shfl_sync(kFull, ts, 0, 8);
-  g.trd = __shfl_sync(kFull, rd, 0, 8);
-  Z80S s = vec_state(int(sub));
-  const uint32_t steps = __reduce_max_sync(kFull, tl);
-#pragma unroll 1
-  for (uint32_t i = 0; i < steps; i++) {
-    const uint32_t w = __shfl_sync(kFull, pw, int(i), 8);
-    if (i < tl) z_step(s, w & 0xFFFFu, w >> 16);
-  }
-  uint32_t w[3];
-  z_pack(s, w);
-#pragma unroll
-  for (int v = 0; v < 8; v++) {
-    g.tw[v][0] = __shfl_sync(kFull, w[0], v, 8);
-    g.tw[v][1] = __shfl_sync(kFull, w[1], v, 8);
-    g.tw[v][2] = __shfl_sync(kFull, w[2], v, 8);
-  }
-  const uint32_t dead = valid ? target_dead(T, t) & 0xFFu : 0u;
-  const uint32_t dregs = valid ? target_dead_regs(T, t) & 0x3Fu : 0u;
-  g.keep0 = 0xFFu | ((~dead & 0xFFu) << 8) | ((dregs & 1u) ? 0u : 0xFF0000u) | ((dregs & 2u) ? 0u : 0xFF000000u);
-  g.keep1 = ((dregs & 4u) ? 0u : 0xFFu) | ((dregs & 8u) ? 0u : 0xFF00u) | ((dregs & 16u) ? 0u : 0xFF0000u) |
-            ((dregs & 32u) ? 0u : 0xFF000000u);
-}
-
+// QuickCheck through the index: a target only meets the candidates whose
+// compared outputs hash like its own.  Eight lanes per target, four targets
+// per warp: lane 8g + v runs target t0 + g on vector v and hashes its output;
+// the hash's range is read eight entries at a time.  A target with an entry
+// of its hash (one in fourteen of the length-2 enumeration) goes on: the
+// second hash, its outputs against the first such entry's, and F under the
+// dead flags entry by entry, from the entries themselves.  Entries of a hash
+// are in pool order, so survivors come out in enumeration order as in the
+// full scan.  Lanes of a group that has no target (past the end) take part in
+// the warp's collectives with nothing to do.
+// Bound by issue and by the chain program - table - entry.  Hashing the first
+// vector alone, gathering all eight outputs of every candidate that agreed on
+// it and broadcasting the target's eight outputs to every lane took 5.1 ms for
+// 9.4M length-2 targets and 1.0 ms for 100,003 targets with every flag dead,
+// this 1.9 and 0.15 ms (of the 1.9, the targets' upload 1.4).
 // COLLECT: the collect pass; else the count pass, which with KEEP also keeps
 // the survivors of targets with at most kQCSlots (single pass).
 template <bool COLLECT, bool KEEP>
@@ -2113,6 +2117,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_qc_bucket(DevTargets T, DevPool P
   const unsigned group_lt = lanemask_lt() & (0xFFu << gshift);
   const uint32_t gw = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const uint32_t nw = gridDim.x * (blockDim.x >> 5);
+  const uint32_t per_mask = (1u << ix.top_bits) + 1u, top_shift = 32u - ix.top_bits;
   unsigned long long my_checks = 0;
   for (uint32_t t0 = gw * 4u; t0 < T.n; t0 += nw * 4u) {
     const uint32_t t = t0 + (lane >> 3);
@@ -2130,39 +2135,107 @@ __global__ void __launch_bounds__(kBlock, 4) k_qc_bucket(DevTargets T, DevPool P
       }
       if (!__any_sync(kFull, work)) continue;
     }
-    QCTarget g;
-    qc_target4(T, t, valid, g);
+    // the target on vector `sub`; every lane reads the program itself
+    const uint32_t tl = valid ? target_len(T, t) : 0u;
+    const uint32_t* prog = T.insn + (size_t)t * T.stride;
+    uint32_t size = 0, tstates = 0, reads = 0;
+    Z80S st = vec_state(int(sub));
+    const uint32_t steps = __reduce_max_sync(kFull, tl);
+#pragma unroll 1
+    for (uint32_t i = 0; i < steps; i++) {
+      if (i < tl) {
+        const uint32_t w = prog[i];
+        const OpInfo oi = g_ops[w & 0xFFFFu];
+        size += oi.size;
+        tstates += oi.tstates;
+        reads |= oi.reads;
+        z_step(st, w & 0xFFFFu, w >> 16);
+      }
+    }
+    uint32_t w[3];
+    z_pack(st, w);
+    const uint32_t dead = valid ? target_dead(T, t) & 0xFFu : 0u;
     const uint32_t m = valid ? target_dead_regs(T, t) & 0x3Fu : 0u;
-    const uint32_t h = bucket_hash(g.tw[0][0] & key_keep0(m), g.tw[0][1] & key_keep1(m), g.tw[0][2] & cfg.w2mask);
+    const uint32_t k0 = key_keep0(m), k1 = key_keep1(m);
+    uint32_t h = qc_hash(w[0] & k0, w[1] & k1, w[2] & cfg.w2mask, sub);
+#pragma unroll
+    for (int off = 4; off >= 1; off >>= 1) h += __shfl_xor_sync(kFull, h, off);
     uint32_t r0 = 0, r1 = 0;
     if (work) {
-      const uint32_t* top = ix.top + m * ((1u << ix.top_bits) + 1u) + (h >> (32u - ix.top_bits));
+      const uint32_t* top = ix.top + m * per_mask + (h >> top_shift);
       r0 = top[0];
       r1 = top[1];
     }
     const uint32_t iters = (__reduce_max_sync(kFull, r1 - r0) + 7u) / 8u;
     uint32_t nf = 0, nm = 0, lf = 0, lm = 0;
     uint32_t nk = 0;  // this group's survivors so far (count pass, single pass)
+    uint32_t h2 = 0, flo = 0, fhi = 0;
+    bool hashed = false;             // h2, flo, fhi are there (warp-uniform)
+    uint32_t same = 2;               // this group's outputs against an entry's: 2 not compared yet
     uint32_t* const keep = KEEP ? o.tmp + (size_t)t * kQCSlots : nullptr;
     for (uint32_t k = 0; k < iters; k++) {
       const uint32_t i = r0 + 8u * k + sub;
-      bool fp = false, mp = false;
-      uint32_t diff = 0, c = 0;
-      if (i < r1) {
-        const unsigned long long key = ix.keys[i];
-        c = uint32_t(key) & ((1u << kQCIndexBits) - 1u);
-        if (uint32_t(key >> kQCIndexBits) == h && P.size[c] < g.tb)
-          qc_candidate(P, P.qc[c], c, g, cfg.w2mask, cfg.all_hits != 0, fp, mp, diff);
+      uint4 e = make_uint4(0u, 0u, 0u, 0u);
+      bool hit = i < r1;
+      if (hit) {
+        e = ix.entries[i];
+        hit = e.x == h;
       }
+      if (!__any_sync(kFull, hit)) continue;  // most steps find nothing
+      if (!hashed) {
+        hashed = true;
+        h2 = qc_hash2(w[0] & k0, w[1] & k1, w[2] & cfg.w2mask, sub);
+        const uint32_t f = ((w[0] >> 8) & 0xFFu) << (8u * (sub & 3u));
+        flo = sub < 4u ? f : 0u;
+        fhi = sub < 4u ? 0u : f;
+#pragma unroll
+        for (int off = 4; off >= 1; off >>= 1) {
+          h2 += __shfl_xor_sync(kFull, h2, off);
+          flo |= __shfl_xor_sync(kFull, flo, off);
+          fhi |= __shfl_xor_sync(kFull, fhi, off);
+        }
+      }
+      if (hit) hit = ix.hash2[i] == h2;
+      const uint32_t c = e.y & ((1u << kQCIndexBits) - 1u);
+      // the outputs themselves, once per target: entries of equal hashes have
+      // equal outputs
+      const unsigned ghit = (__ballot_sync(kFull, hit) >> gshift) & 0xFFu;
+      const uint32_t c0 = __shfl_sync(kFull, c, ghit ? __ffs(int(ghit)) - 1 : 0, 8);
+      bool differs = false;
+      if (same == 2 && ghit) {
+        const uint4 q = P.qc[(size_t)sub * P.n + c0];
+        differs = (((q.x ^ w[0]) & k0) | ((q.y ^ w[1]) & k1) | ((q.z ^ w[2]) & cfg.w2mask)) != 0;
+      }
+      const unsigned gdiff = (__ballot_sync(kFull, differs) >> gshift) & 0xFFu;
+      if (same == 2 && ghit) same = gdiff ? 0u : 1u;
+      const uint32_t live = (~dead & 0xFFu) * 0x01010101u;
+      const bool pass = hit && same == 1u && (e.y >> kQCIndexBits) < size &&
+                        (((e.z ^ flo) | (e.w ^ fhi)) & live) == 0;
+      uint32_t fd = (e.z ^ flo) | (e.w ^ fhi);
+      fd |= fd >> 16;
+      fd = (fd | (fd >> 8)) & 0xFFu;
+      uint32_t rdf = 0;
+      if (__any_sync(kFull, pass && m != 0)) {
+        // dead registers: which of them differ, on the candidate itself
+#pragma unroll 1
+        for (int v = 0; v < 8; v++) {
+          const uint32_t x = __shfl_sync(kFull, w[0], v, 8), y = __shfl_sync(kFull, w[1], v, 8);
+          if (pass && m != 0) {
+            const uint4 q = P.qc[(size_t)v * P.n + c];
+            rdf |= reg_diff(q.x ^ x, q.y ^ y);
+          }
+        }
+      }
+      const uint32_t diff = fd | (rdf << 8);
+      const bool fp = pass && (cfg.all_hits != 0 || diff == 0), mp = pass && !fp;
       if constexpr (!COLLECT) {
         lf += fp ? 1u : 0u;
         lm += mp ? 1u : 0u;
         if constexpr (KEEP) {
-          const bool sv = fp || mp;
-          const unsigned bs = __ballot_sync(kFull, sv);
-          if (bs) {  // most steps find nothing
+          const unsigned bs = __ballot_sync(kFull, pass);
+          if (bs) {
             const uint32_t rank = nk + __popc(bs & group_lt);
-            if (sv && rank < kQCSlots) keep[rank] = c | (diff << 16) | (mp ? 0x80000000u : 0u);
+            if (pass && rank < kQCSlots) keep[rank] = c | (diff << 16) | (mp ? 0x80000000u : 0u);
             nk += __popc((bs >> gshift) & 0xFFu);
           }
         }
@@ -2184,13 +2257,20 @@ __global__ void __launch_bounds__(kBlock, 4) k_qc_bucket(DevTargets T, DevPool P
       }
     }
     if constexpr (!COLLECT) {
+      if (hashed) {
 #pragma unroll
-      for (int off = 4; off >= 1; off >>= 1) {
-        lf += __shfl_xor_sync(kFull, lf, off);
-        lm += __shfl_xor_sync(kFull, lm, off);
+        for (int off = 4; off >= 1; off >>= 1) {
+          lf += __shfl_xor_sync(kFull, lf, off);
+          lm += __shfl_xor_sync(kFull, lm, off);
+        }
       }
       if (sub == 0 && valid) {
-        my_checks += ix.elig_lt[g.tb < 255u ? g.tb : 255u];
+        my_checks += ix.elig_lt[size < 255u ? size : 255u];
+        QCTarget g;
+        g.tb = size;
+        g.tts = tstates;
+        g.trd = reads;
+        g.tl = tl;
         qc_count_out(o, t, g, lf, lm);
         if (KEEP && lf + lm > kQCSlots) atomicAdd(o.over, 1u);
       }
@@ -2528,10 +2608,16 @@ void launch_qc_keys(const DevPool& P, uint32_t w2mask, uint32_t m0, uint32_t nm,
   const uint32_t n = nm * P.n;
   if (n) k_qc_keys<<<grid_for(n, 256), 256, 0, s>>>(P, w2mask, m0, nm, keys);
 }
-void launch_qc_top(const unsigned long long* keys, uint32_t nv, uint32_t first, uint32_t m0, uint32_t nm,
-                   uint32_t top_bits, uint32_t* top, cudaStream_t s) {
-  const uint32_t n = nm * ((1u << top_bits) + 1u);
-  k_qc_top<<<grid_for(n, 256), 256, 0, s>>>(keys, nv, first, m0, nm, top_bits, top);
+void launch_qc_entries(const DevPool& P, uint32_t w2mask, const unsigned long long* keys, uint32_t nv, uint32_t first,
+                       uint32_t m0, uint32_t nm, uint32_t top_bits, uint4* entries, uint32_t* hash2, uint32_t* top,
+                       uint32_t* clash, cudaStream_t s) {
+  const uint32_t n = nm * nv;
+  if (n) {
+    k_qc_entries<<<grid_for(n, 256), 256, 0, s>>>(P, w2mask, keys, n, entries + first, hash2 + first);
+    k_qc_check<<<grid_for(n, 256), 256, 0, s>>>(P, w2mask, keys, hash2 + first, n, clash);
+  }
+  const uint32_t nt = nm * ((1u << top_bits) + 1u);
+  k_qc_top<<<grid_for(nt, 256), 256, 0, s>>>(keys, nv, first, m0, nm, top_bits, top);
 }
 void launch_qc_compact(const QCOut& q, uint32_t n, cudaStream_t s) {
   if (!n) return;

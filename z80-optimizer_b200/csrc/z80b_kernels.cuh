@@ -35,20 +35,25 @@ struct QCConfig {
   int use_smem;      // pool QC0 staged in shared memory
 };
 
-// QuickCheck bucket index of a candidate pool: per dead-register mask in use
-// the unpruned candidates' keys m << 58 | hash << 26 | index, sorted, and a
-// table of the first entry of each range of the top hash bits; and the
-// unpruned candidates shorter than b bytes (the count of QuickCheck units a
-// target of b bytes evaluates).  Ranges of about one key for the 4,531
+// QuickCheck index of a candidate pool: per dead-register mask in use the
+// unpruned candidates by a hash of what QuickCheck compares whatever the dead
+// flags are (A, the live registers, SP and, where compared, M, on all eight
+// vectors), in pool order within a hash, each with its eight F bytes; a table
+// of the first entry of each range of the top hash bits; and the unpruned
+// candidates shorter than b bytes (the count of QuickCheck units a target of b
+// bytes evaluates).  Two entries with both hashes equal have equal outputs
+// (the build checks it), so a target compares its outputs with one of them
+// and its F bytes with each.  Ranges of about one entry for the 4,531
 // instructions (12 bits) and four for the 266,675 first-op instructions (16
-// bits): a target reads its range eight keys at a time.
-constexpr uint32_t kQCIndexBits = 26;
-constexpr uint32_t kQCIndexMax = 1u << 20;      // a key and its scratch: 16 bytes per candidate and mask in use
+// bits): a target reads its range eight entries at a time.
+constexpr uint32_t kQCIndexBits = 26;           // candidate number in a sort key and an entry
+constexpr uint32_t kQCIndexMax = 1u << 20;      // an entry and its scratch: 36 bytes per candidate and mask in use
 constexpr uint32_t kQCAllMasksMax = 65536;      // pools up to here: all 64 masks in one sort
 inline uint32_t qc_top_bits(uint32_t n) { return n <= kQCAllMasksMax ? 12u : 16u; }
 struct QCIndex {
-  const unsigned long long* keys;
-  const uint32_t* top;             // [64 * ((1 << top_bits) + 1)] positions in keys
+  const uint4* entries;            // {hash, candidate | bytes << kQCIndexBits, F of vectors 0-3, F of vectors 4-7}
+  const uint32_t* hash2;           // per entry a second hash
+  const uint32_t* top;             // [64 * ((1 << top_bits) + 1)] positions in entries
   const uint32_t* elig_lt;         // [256]
   uint32_t top_bits;
 };
@@ -187,12 +192,15 @@ void launch_qc_scan(const DevTargets& T, const DevPool& P, const QCConfig& cfg, 
                     bool collect, cudaStream_t s);
 void launch_fp_query(const DevPool& P, const uint32_t* fp3x8, uint32_t dead, uint32_t* hits,
                      uint32_t* nhits, uint32_t cap, cudaStream_t s);
-// Keys of masks [m0, m0 + nm): keys[i * P.n + c] for mask m0 + i.
+// Sort keys of masks [m0, m0 + nm): keys[i * P.n + c] for mask m0 + i.
 void launch_qc_keys(const DevPool& P, uint32_t w2mask, uint32_t m0, uint32_t nm, unsigned long long* keys,
                     cudaStream_t s);
-// Top tables of masks [m0, m0 + nm), whose nv keys each begin at keys[first + i * nv].
-void launch_qc_top(const unsigned long long* keys, uint32_t nv, uint32_t first, uint32_t m0, uint32_t nm,
-                   uint32_t top_bits, uint32_t* top, cudaStream_t s);
+// From the nm * nv sorted keys at keys[0]: the entries at positions first on,
+// and their masks' top tables; *clash is set when two entries of equal hashes
+// differ in their outputs.
+void launch_qc_entries(const DevPool& P, uint32_t w2mask, const unsigned long long* keys, uint32_t nv, uint32_t first,
+                       uint32_t m0, uint32_t nm, uint32_t top_bits, uint4* entries, uint32_t* hash2, uint32_t* top,
+                       uint32_t* clash, cudaStream_t s);
 void launch_qc_bucket(const DevTargets& T, const DevPool& P, const QCConfig& cfg, const QCIndex& ix,
                       const QCOut& o, bool collect, cudaStream_t s);
 // Everything the kernels of a round need, in device memory: a captured round
