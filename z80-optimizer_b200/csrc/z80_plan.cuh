@@ -1,6 +1,8 @@
 // z80_plan.cuh -- what decides the ExhaustiveCheck of a (target, candidate)
-// pair, worked out from its two programs before anything is swept.  Plain
-// C++ shared by the kernels that build pairs and by the host tests.
+// pair, worked out from its two programs before anything is swept.  plan_pair
+// is the rule in plain C++ (checked against the oracle on the host); the
+// kernel that plans pairs (plan_pair_warp in z80b_kernels.cu) is the same with
+// a lane per field, and shares plan_from below.
 //
 // Value numbers.  Both programs run on names instead of values: a field (A,
 // a register, SP, the memory byte, a flag bit) holds the name of an input
@@ -41,6 +43,11 @@ struct OpFlow {
   uint16_t cst[kFlowFields];   // output g is this constant; kFlowImmLo / kFlowImmHi: a byte of the
                                // immediate; kFlowNoConst: not a constant
 };
+// One field of OpFlow in 64 bits, as the kernels read it: dep (24 bits), src
+// (8), cst (16), changed (1).
+inline uint64_t flow_word(const OpFlow& f, int g) {
+  return uint64_t(f.dep[g]) | uint64_t(f.src[g]) << 24 | uint64_t(f.cst[g]) << 32 | uint64_t(f.changed >> g & 1u) << 48;
+}
 constexpr uint16_t kFlowImmLo = 0x100, kFlowImmHi = 0x101, kFlowNoConst = 0xFFFF;
 constexpr uint32_t kFlowCarry = 1u << 16;
 
@@ -159,20 +166,15 @@ Z80B_PLAN_HD unsigned long long plan_blocks(uint32_t reads, bool reduced) {
   return (2ull << (5 * n)) * (sp ? 16ull : 1ull);
 }
 
-// reads: the union of the programs' read masks; keepF: compared flag bits;
-// keepR: compared registers (bits 0..5 = B..L).  A, SP and the memory byte
-// are always compared.
-Z80B_PLAN_HD PairPlan plan_pair(const OpFlow* F, const uint32_t* tw, uint32_t tl, const uint32_t* cw, uint32_t cl,
-                                uint32_t reads, uint32_t keepF, uint32_t keepR) {
+// The plan from the open outputs: rest, what those other than A can depend on;
+// at / ac, what A can (where it is open) in either program; keeps_t / keeps_c:
+// the program leaves A as it was.
+Z80B_PLAN_HD PairPlan plan_from(uint32_t reads, uint32_t open, uint32_t rest, uint32_t at, uint32_t ac, bool keeps_t,
+                                bool keeps_c) {
   PairPlan r;
-  const uint32_t cmp = kRegA | kRegSP | kRegM | ((keepR & 0x3Fu) << 2) | ((keepF & 0xFFu) << 16);
   const uint32_t ext = reads & (kRegB | kRegC | kRegD | kRegE | kRegH | kRegL | kRegM);
   const uint32_t sp = reads & kRegSP;
-  const uint32_t open = open_outputs(F, tw, tl, cw, cl, ext | sp | kRegA | kFlowCarry, cmp);
   r.proven = open == 0;
-  // what the open outputs other than A, and A itself, depend on
-  const uint32_t rest = flow_relevant(F, tw, tl, open & ~uint32_t(kRegA)) | flow_relevant(F, cw, cl, open & ~uint32_t(kRegA));
-  const uint32_t at = flow_relevant(F, tw, tl, open & kRegA), ac = flow_relevant(F, cw, cl, open & kRegA);
   const uint32_t rel = rest | at | ac;
   const uint32_t drop = (ext | sp) & ~rel;
   const bool red = sp != 0 || plan_popc(ext) > 2;
@@ -189,8 +191,25 @@ Z80B_PLAN_HD PairPlan plan_pair(const OpFlow* F, const uint32_t* tw, uint32_t tl
   }
   // Two values of A decide when no open output but A depends on the input A
   // and each program keeps A or computes its A from other inputs.
-  r.a_free = !(rest & kRegA) && (!(at & kRegA) || flow_keeps_a(F, tw, tl)) && (!(ac & kRegA) || flow_keeps_a(F, cw, cl));
+  r.a_free = !(rest & kRegA) && (!(at & kRegA) || keeps_t) && (!(ac & kRegA) || keeps_c);
   return r;
+}
+// Compared outputs and varying inputs of a pair.  reads: the union of the
+// programs' read masks; keepF: compared flag bits; keepR: compared registers
+// (bits 0..5 = B..L).  A, SP and the memory byte are always compared.
+Z80B_PLAN_HD uint32_t plan_compared(uint32_t keepF, uint32_t keepR) {
+  return kRegA | kRegSP | kRegM | ((keepR & 0x3Fu) << 2) | ((keepF & 0xFFu) << 16);
+}
+Z80B_PLAN_HD uint32_t plan_varying(uint32_t reads) {
+  return (reads & (kRegB | kRegC | kRegD | kRegE | kRegH | kRegL | kRegM | kRegSP)) | kRegA | kFlowCarry;
+}
+
+Z80B_PLAN_HD PairPlan plan_pair(const OpFlow* F, const uint32_t* tw, uint32_t tl, const uint32_t* cw, uint32_t cl,
+                                uint32_t reads, uint32_t keepF, uint32_t keepR) {
+  const uint32_t open = open_outputs(F, tw, tl, cw, cl, plan_varying(reads), plan_compared(keepF, keepR));
+  const uint32_t rest = flow_relevant(F, tw, tl, open & ~uint32_t(kRegA)) | flow_relevant(F, cw, cl, open & ~uint32_t(kRegA));
+  return plan_from(reads, open, rest, flow_relevant(F, tw, tl, open & kRegA), flow_relevant(F, cw, cl, open & kRegA),
+                   flow_keeps_a(F, tw, tl), flow_keeps_a(F, cw, cl));
 }
 
 }  // namespace z80b

@@ -97,6 +97,7 @@ struct PoolBufs {
   uint32_t qw2 = 0;        // word-2 mask the index hashes
   uint32_t qvalid = 0;     // unpruned candidates
   uint64_t qmasks = 0;     // dead-register masks indexed
+  bool qmixed = false;     // QCIndex::check_h2
   DevPool dev{};
   std::vector<uint32_t> host_insn;
   std::vector<uint8_t> host_lens;
@@ -200,6 +201,7 @@ struct z80b_ctx {
   // pipeline scratch
   DBuf cnt_f, cnt_m, cnt_all, base, meta, surv, sdiff, checks;
   DBuf qc_tmp, qc_over;       // single-pass QuickCheck: kept survivors, targets with more
+  DBuf qc_longs, qc_nlong;    // targets with long ranges in the index, per chunk of targets and pass
   DBuf next, win, windiff, spec, spec2, wlen, wend, cdone;
   DBuf pairs, pair_src, cbase[kClasses], cpair[kClasses], rejected, states;
   DBuf roundctl, roundargs;   // RoundCtl; RoundArgs of the two passes
@@ -528,9 +530,9 @@ int ensure_qc_index(z80b_ctx* ctx, PoolBufs& P, uint32_t w2mask, uint64_t masks)
     CK(P.qhash2.ensure(ne * 4));
     CK(P.qtop.ensure(64ull * ((1ull << bits) + 1) * 4));
     CK(P.qelig.ensure(256 * 4));
-    CK(P.qclash.ensure(4));
+    CK(P.qclash.ensure(8));
     CK(cudaMemcpyAsync(P.qelig.p, elig.data(), 256 * 4, cudaMemcpyHostToDevice, s));
-    CK(cudaMemsetAsync(P.qclash.p, 0, 4, s));
+    CK(cudaMemsetAsync(P.qclash.p, 0, 8, s));
     CK(cudaStreamSynchronize(s));
     P.qstate = 1;
     P.qw2 = w2mask;
@@ -553,11 +555,12 @@ int ensure_qc_index(z80b_ctx* ctx, PoolBufs& P, uint32_t w2mask, uint64_t masks)
     ctx->launches += 5;
     P.qmasks |= all ? ~0ull : 1ull << m;
   }
-  uint32_t clash = 0;
-  CKR(fetch(ctx, &clash, P.qclash.as<uint32_t>()));
-  if (clash) P.qstate = -1;
-  trace("QuickCheck index: %u candidates, %u unpruned, masks %016llx, clash %u", n, P.qvalid,
-        (unsigned long long)P.qmasks, clash);
+  uint32_t clash[2] = {0, 0};
+  CKR(fetch(ctx, clash, P.qclash.as<uint32_t>(), 2));
+  if (clash[0]) P.qstate = -1;
+  P.qmixed = clash[1] != 0;
+  trace("QuickCheck index: %u candidates, %u unpruned, masks %016llx, clash %u, mixed %u", n,
+        P.qvalid, (unsigned long long)P.qmasks, clash[0], clash[1]);
   return Z80B_OK;
 }
 
@@ -1111,6 +1114,7 @@ int run_pipeline(z80b_ctx* ctx, const DevTargets& T, const PipeOpts& opts, z80b_
       qix.top = pool->qtop.as<uint32_t>();
       qix.elig_lt = pool->qelig.as<uint32_t>();
       qix.top_bits = qc_top_bits(P.n);
+      qix.check_h2 = pool->qmixed ? 1u : 0u;
     }
   }
   trace("pipeline: %u targets, mode %u, pool %u", n, mode, P.n);
@@ -1129,8 +1133,16 @@ int run_pipeline(z80b_ctx* ctx, const DevTargets& T, const PipeOpts& opts, z80b_
     q.tmp = ctx->qc_tmp.as<uint32_t>();
     q.over = ctx->qc_over.as<uint32_t>();
   }
-  // the count over targets [lo, hi) (every per-target array offset by lo)
-  auto qc_count = [&](uint32_t lo, uint32_t hi) {
+  if (use_ix) {
+    CK(ctx->qc_longs.ensure(4ull * n));
+    CK(ctx->qc_nlong.ensure(4 * (kUpChunks + 1)));
+    CK(cudaMemsetAsync(ctx->qc_nlong.p, 0, 4 * (kUpChunks + 1), s));
+    q.longs = ctx->qc_longs.as<uint32_t>();
+    q.nlong = ctx->qc_nlong.as<uint32_t>();
+  }
+  // the count over targets [lo, hi) (every per-target array offset by lo),
+  // chunk number k
+  auto qc_count = [&](uint32_t lo, uint32_t hi, int k) {
     DevTargets Tc = T;
     QCOut qc = q;
     if (lo) {
@@ -1143,10 +1155,13 @@ int run_pipeline(z80b_ctx* ctx, const DevTargets& T, const PipeOpts& opts, z80b_
       qc.cnt_all += lo;
       qc.meta += lo;
       if (qc.tmp) qc.tmp += (size_t)lo * kQCSlots;
+      if (use_ix) qc.longs += lo;
     }
+    if (use_ix) qc.nlong += k;
     Tc.n = hi - lo;
     if (use_ix) launch_qc_bucket(Tc, P, cfg, qix, qc, false, s);
     else launch_qc_scan(Tc, P, cfg, qc, false, s);
+    if (use_ix) ctx->launches++;
     return check_launch(ctx, "qc_count");
   };
   // chunked upload: the first chunk is on the device before the clock starts
@@ -1160,11 +1175,11 @@ int run_pipeline(z80b_ctx* ctx, const DevTargets& T, const PipeOpts& opts, z80b_
     for (int k = 0; k < opts.up_chunks; k++) {
       const uint32_t hi = opts.up_hi[k];
       if (k) CK(cudaStreamWaitEvent(s, ctx->up_ev[k], 0));
-      if (hi > lo) CKR(qc_count(lo, hi));
+      if (hi > lo) CKR(qc_count(lo, hi, k));
       lo = hi;
     }
   } else {
-    CKR(qc_count(0, n));
+    CKR(qc_count(0, n, 0));
   }
   kend(ctx, kq);
   CKR(scan(ctx, ctx->cnt_all.as<uint32_t>(), ctx->base.as<uint32_t>(), n));
@@ -1192,8 +1207,14 @@ int run_pipeline(z80b_ctx* ctx, const DevTargets& T, const PipeOpts& opts, z80b_
     // every target (two passes), or those with more survivors than the
     // count pass kept
     int kc = kbegin(ctx, 0);
-    if (use_ix) launch_qc_bucket(T, P, cfg, qix, q, true, s);
-    else launch_qc_scan(T, P, cfg, q, true, s);
+    QCOut qc = q;
+    if (use_ix) {
+      qc.nlong += kUpChunks;
+      ctx->launches++;
+      launch_qc_bucket(T, P, cfg, qix, qc, true, s);
+    } else {
+      launch_qc_scan(T, P, cfg, qc, true, s);
+    }
     kend(ctx, kc);
     CKR(check_launch(ctx, "qc_collect"));
   }
@@ -2114,8 +2135,10 @@ static int search_impl(z80b_ctx* ctx, const z80b_job* job, z80b_rule* out, uint6
   cudaSetDevice(ctx->device);
   if (stats) std::memset(stats, 0, sizeof *stats);
   ctx->launches = 0;
+  trace("search of %u targets", job->n_targets);
   DevTargets T;
   CKR(upload_targets(ctx, ctx->staged, job, &T, false));
+  trace("upload queued");
   ctx->staged.valid = false;  // this job's targets are not kept for z80b_fetch_rules
   {
     // the host scan of the targets runs while their copy is in flight; on
@@ -2127,6 +2150,7 @@ static int search_impl(z80b_ctx* ctx, const z80b_job* job, z80b_rule* out, uint6
       return v;
     }
   }
+  trace("targets checked");
   uint64_t nr = 0;
   if (job->path == Z80B_PATH_PLAIN) {
     std::vector<z80b_rule> hr;
@@ -2165,7 +2189,9 @@ static int search_impl(z80b_ctx* ctx, const z80b_job* job, z80b_rule* out, uint6
   if (nr && !out) return fail(ctx, Z80B_EINVAL, "null output");
   const DevRule* dr = nullptr;
   CKR(rules_to_host(ctx, nr, &dr));
+  trace("rules read");
   to_rules(ctx, dr, nr, job->targets, job->target_lens, job->target_len, job->target_stride, job->mode, 0, out);
+  trace("rules written");
   return Z80B_OK;
 }
 

@@ -24,6 +24,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <mutex>
 
 #include "z80_bits.cuh"
 #include "z80_tables.h"
@@ -62,8 +63,8 @@ __device__ uint8_t g_cid[64];
 __device__ uint8_t g_opregs[kNumOps];
 // wide compact sweep: the same per register set of at most four registers
 // (wide_tables)
-// what each opcode's outputs are computed from (z80_plan.cuh)
-__device__ OpFlow g_flow[kNumOps];
+// what each opcode's outputs are computed from (flow_word of z80_plan.cuh)
+__device__ unsigned long long g_flow[kNumOps][kFlowFields];
 __device__ int16_t g_wren[kWideSets][kNumOps];
 __device__ int8_t g_worig[kWideSets][4];
 __device__ uint8_t g_wid[64];
@@ -130,67 +131,56 @@ __device__ __forceinline__ uint32_t reg_diff(uint32_t d0, uint32_t d1) {
 // 32,768.  PairRec.keepR bit 6 marks it.
 constexpr uint32_t kXIndep = 0x40u;
 constexpr unsigned long long kUnitBlocks = 128;
-__device__ __forceinline__ uint32_t dev_seq_aflow(const uint32_t* w, uint32_t n) {
-  bool a_is_x = true;
-  for (uint32_t i = 0; i < n; i++) {
-    const uint32_t k = g_aclass[w[i] & 0xFFFFu];
-    if (k == 0u && a_is_x) return 0u;
-    if (k == 2u) a_is_x = false;
-  }
-  return a_is_x ? 3u : 1u;
+// A pair's two programs, one instruction per lane: lanes 0..tl-1 the target,
+// lanes tl..tl+cl-1 the candidate.
+struct PairWords {
+  uint32_t w;        // this lane's instruction (0 past the programs)
+  uint32_t tl, cl;
+  __device__ __forceinline__ bool mine() const { return lane_id() < tl + cl; }
+};
+__device__ __forceinline__ PairWords pair_words(const DevTargets& T, uint32_t t, const DevPool& P, uint32_t c) {
+  PairWords p;
+  p.tl = target_len(T, t);
+  p.cl = pool_len(P, c);
+  const unsigned lane = lane_id();
+  p.w = 0;
+  if (lane < p.tl) p.w = T.insn[(size_t)t * T.stride + lane];
+  else if (lane < p.tl + p.cl) p.w = P.insn[(size_t)c * P.stride + (lane - p.tl)];
+  return p;
 }
-__device__ __forceinline__ bool pair_xindep(const DevTargets& T, uint32_t t, const DevPool& P, uint32_t c) {
-  return dev_seq_aflow(T.insn + (size_t)t * T.stride, target_len(T, t)) != 0u &&
-         dev_seq_aflow(P.insn + (size_t)c * P.stride, pool_len(P, c)) != 0u;
+// The fold of the AClass table over both programs: true when no output of
+// either depends on the input A but A passing through (an A-dependent
+// instruction only after one that overwrites A).
+__device__ __forceinline__ bool pair_xindep(const PairWords& p) {
+  const uint32_t k = p.mine() ? g_aclass[p.w & 0xFFFFu] : 1u;
+  const unsigned dep = __ballot_sync(kFull, k == 0u), over = __ballot_sync(kFull, k == 2u);
+  const unsigned tm = (1u << p.tl) - 1u, cm = ((1u << p.cl) - 1u) << p.tl;
+  auto free_of = [&](unsigned m) {
+    const unsigned d = dep & m, o = over & m;
+    return d == 0u || (o != 0u && __ffs(int(o)) < __ffs(int(d)));
+  };
+  return free_of(tm) && free_of(cm);
 }
-// Compact sweep: 1 + the register-set entry when the pair's instructions
-// name at most two of B..L, neither SP nor the memory byte, and all rename
-// onto B and C (compact_map); 0 otherwise.
-__device__ __forceinline__ uint8_t pair_cmap(const DevTargets& T, uint32_t t, const DevPool& P, uint32_t c) {
-  const uint32_t tl = target_len(T, t), cl = pool_len(P, c);
-  const uint32_t* tw = T.insn + (size_t)t * T.stride;
-  const uint32_t* cw = P.insn + (size_t)c * P.stride;
-  uint32_t fp = 0;
-  for (uint32_t i = 0; i < tl; i++) fp |= g_opregs[tw[i] & 0xFFFFu];
-  for (uint32_t i = 0; i < cl; i++) fp |= g_opregs[cw[i] & 0xFFFFu];
-  if (fp & 0xC0u) return 0;
-  const uint32_t id = g_cid[fp & 0x3Fu];
-  if (!id) return 0;
-  for (uint32_t i = 0; i < tl; i++)
-    if (g_cren[id - 1][tw[i] & 0xFFFFu] < 0) return 0;
-  for (uint32_t i = 0; i < cl; i++)
-    if (g_cren[id - 1][cw[i] & 0xFFFFu] < 0) return 0;
-  return uint8_t(id);
-}
-// Wide compact sweep: kWideClass | (1 + the register-set entry) when the
-// pair's instructions name at most four of B..L and not SP, and all rename
-// onto B, C, H and L (wide_map); 0 otherwise.
+// The sweep class of a pair (PairRec::cmap) by the registers its
+// instructions name (fp, op_regs): 1 + the register-set entry when they name
+// at most two of B..L, neither SP nor the memory byte, and all rename onto B
+// and C (compact_map); kWideClass | (1 + the entry) for A-dependent pairs that
+// name at most four and not SP and rename onto B, C, H and L (wide_map);
+// kRegClass for the rest that name neither SP nor the memory byte; else 0.
 constexpr uint8_t kWideClass = 0x80u;
-// Register-state sweep: the pair's instructions name neither SP nor the
-// memory byte.
 constexpr uint8_t kRegClass = 0x40u;
-__device__ __forceinline__ bool pair_regstate(const DevTargets& T, uint32_t t, const DevPool& P, uint32_t c) {
-  const uint32_t tl = target_len(T, t), cl = pool_len(P, c);
-  uint32_t fp = 0;
-  for (uint32_t i = 0; i < tl; i++) fp |= g_opregs[T.insn[(size_t)t * T.stride + i] & 0xFFFFu];
-  for (uint32_t i = 0; i < cl; i++) fp |= g_opregs[P.insn[(size_t)c * P.stride + i] & 0xFFFFu];
-  return (fp & 0xC0u) == 0u;
-}
-__device__ __forceinline__ uint8_t pair_wmap(const DevTargets& T, uint32_t t, const DevPool& P, uint32_t c) {
-  const uint32_t tl = target_len(T, t), cl = pool_len(P, c);
-  const uint32_t* tw = T.insn + (size_t)t * T.stride;
-  const uint32_t* cw = P.insn + (size_t)c * P.stride;
-  uint32_t fp = 0;
-  for (uint32_t i = 0; i < tl; i++) fp |= g_opregs[tw[i] & 0xFFFFu];
-  for (uint32_t i = 0; i < cl; i++) fp |= g_opregs[cw[i] & 0xFFFFu];
-  if (fp & 0x80u) return 0;
-  const uint32_t id = g_wid[fp & 0x3Fu];
-  if (!id) return 0;
-  for (uint32_t i = 0; i < tl; i++)
-    if (g_wren[id - 1][tw[i] & 0xFFFFu] < 0) return 0;
-  for (uint32_t i = 0; i < cl; i++)
-    if (g_wren[id - 1][cw[i] & 0xFFFFu] < 0) return 0;
-  return uint8_t(kWideClass | id);
+__device__ __forceinline__ uint8_t pair_cmap(const PairWords& p, bool compact, bool wide, bool xindep) {
+  const uint32_t op = p.w & 0xFFFFu;
+  const uint32_t fp = __reduce_or_sync(kFull, p.mine() ? uint32_t(g_opregs[op]) : 0u);
+  if (compact && !(fp & 0xC0u)) {
+    const uint32_t id = g_cid[fp & 0x3Fu];
+    if (id && __all_sync(kFull, !p.mine() || g_cren[id - 1][op] >= 0)) return uint8_t(id);
+  }
+  if (wide && !xindep && !(fp & 0x80u)) {
+    const uint32_t id = g_wid[fp & 0x3Fu];
+    if (id && __all_sync(kFull, !p.mine() || g_wren[id - 1][op] >= 0)) return uint8_t(kWideClass | id);
+  }
+  return wide && !(fp & 0xC0u) ? kRegClass : uint8_t(0);
 }
 // A-dependent pairs run bit-sliced (z80_bits.cuh): a unit is 4 A-blocks, a
 // lane takes 32 consecutive values of A of one block.
@@ -700,14 +690,9 @@ __device__ __forceinline__ bool run_compare(const Init& init, const bool (&valid
 // Runs both programs of a pair on 512 states of its sweep -- every value of A
 // twice, each with a block of its own spread over the sweep -- and tells
 // whether one of them differs.  Warp-wide, the same pair in every lane.
-__device__ __forceinline__ bool probe_pair(const DevTargets& T, const DevPool& P, uint32_t target, uint32_t cand,
-                                           unsigned long long nblocks, uint32_t reads, uint32_t sweepf, uint32_t keepF,
-                                           uint32_t keepR) {
+__device__ __forceinline__ bool probe_pair(const PairWords& words, unsigned long long nblocks, uint32_t reads,
+                                           uint32_t sweepf, uint32_t keepF, uint32_t keepR) {
   const unsigned lane = lane_id();
-  const uint32_t tl = target_len(T, target), cl = pool_len(P, cand);
-  uint32_t pw = 0;
-  if (lane < tl) pw = T.insn[(size_t)target * T.stride + lane];
-  else if (lane < tl + cl) pw = P.insn[(size_t)cand * P.stride + (lane - tl)];
   const uint32_t ext = reads & (kRegB | kRegC | kRegD | kRegE | kRegH | kRegL | kRegM);
   const bool spw = (reads & kRegSP) != 0;
   const int nx = __popc(ext);
@@ -725,12 +710,12 @@ __device__ __forceinline__ bool probe_pair(const DevTargets& T, const DevPool& P
                          ((keepR & 16u) ? 0xFF0000u : 0u) | ((keepR & 32u) ? 0xFF000000u : 0u);
   bool bad = false;
 #pragma unroll 1
-  for (uint32_t i = 0; i < 4u && !__any_sync(kFull, bad); i++) {
-    uint32_t W[4][3];
-    const bool valid[4] = {true, true, true, true};
+  for (uint32_t i = 0; i < 8u && !__any_sync(kFull, bad); i++) {
+    uint32_t W[2][3];
+    const bool valid[2] = {true, true};
 #pragma unroll
-    for (uint32_t q = 0; q < 4; q++) {
-      const uint32_t n = (i * 4u + q) * 32u + lane;  // 0..511
+    for (uint32_t q = 0; q < 2; q++) {
+      const uint32_t n = (i * 2u + q) * 32u + lane;  // 0..511
       unsigned long long h = (n + 1ull) * 0x9E3779B97F4A7C15ull;
       h ^= h >> 29;
       h *= 0xBF58476D1CE4E5B9ull;
@@ -740,29 +725,103 @@ __device__ __forceinline__ bool probe_pair(const DevTargets& T, const DevPool& P
       z_pack(x, W[q]);
     }
     auto init = [&](int q, Z80S& x) { x = z_unpack(W[q][0], W[q][1], W[q][2]); };
-    bad = run_compare<4>(init, valid, pw, int(tl), int(cl), keep0, keep1);
+    bad = run_compare<2>(init, valid, words.w, int(words.tl), int(words.cl), keep0, keep1);
   }
   return __any_sync(kFull, bad);
 }
 
-// Plans the round's pairs (z80_plan.cuh), one lane each: compared outputs,
+// plan_pair (z80_plan.cuh) by a warp, lane g on field g: the names of the
+// fields are in the lanes, an instruction's dependency sets are met by ballots.
+__device__ __forceinline__ PairPlan plan_pair_warp(const PairWords& p, uint32_t reads, uint32_t keepF, uint32_t keepR) {
+  const unsigned lane = lane_id();
+  const uint32_t n = p.tl + p.cl;
+  unsigned long long row[kPlanMaxInsn];
+  uint32_t word[kPlanMaxInsn], in[kPlanMaxInsn], out[kPlanMaxInsn];
+#pragma unroll
+  for (int i = 0; i < kPlanMaxInsn; i++) {
+    word[i] = __shfl_sync(kFull, p.w, i);
+    row[i] = 0;
+    in[i] = out[i] = 0;
+    if (uint32_t(i) < n && lane < kFlowFields) row[i] = g_flow[word[i] & 0xFFFFu][lane];
+  }
+  const uint32_t varying = plan_varying(reads), cmp = plan_compared(keepF, keepR);
+  const uint32_t first = ((varying >> lane) & 1u) ? 256u + lane : 0u;
+  uint32_t cur = first, end_t = 0;
+#pragma unroll
+  for (int i = 0; i < kPlanMaxInsn; i++) {
+    if (uint32_t(i) >= n) break;
+    if (uint32_t(i) == p.tl) {
+      end_t = cur;
+      cur = first;
+    }
+    in[i] = cur;
+    const uint32_t dep = uint32_t(row[i]) & 0xFFFFFFu, src = uint32_t(row[i] >> 24) & 0xFFu;
+    const uint32_t cst = uint32_t(row[i] >> 32) & 0xFFFFu;
+    const uint32_t copy = __shfl_sync(kFull, cur, int(src & 31u));
+    uint32_t id;
+    if (!((row[i] >> 48) & 1u)) id = cur;
+    else if (src != 0xFFu) id = copy;
+    else if (cst < 256u) id = cst;
+    else if (cst == kFlowImmLo) id = (word[i] >> 16) & 0xFFu;
+    else if (cst == kFlowImmHi) id = word[i] >> 24;
+    else id = 280u + 24u * i + lane;
+    const bool computed = id == 280u + 24u * i + lane;
+    bool found = false;
+#pragma unroll
+    for (int j = 0; j < i; j++) {
+      if (word[j] != word[i]) continue;
+      const unsigned same = __ballot_sync(kFull, in[j] == in[i]);
+      if (computed && !found && (dep & ~same) == 0) {
+        id = out[j];
+        found = true;
+      }
+    }
+    out[i] = id;
+    cur = id;
+  }
+  if (p.cl == 0) end_t = cur;
+  const uint32_t open = __ballot_sync(kFull, end_t != cur) & cmp;
+  // what outputs can depend on, walked backwards over lanes [lo, hi)
+  auto relevant = [&](uint32_t lo, uint32_t hi, uint32_t o) {
+#pragma unroll
+    for (int i = kPlanMaxInsn - 1; i >= 0; i--) {
+      if (uint32_t(i) < lo || uint32_t(i) >= hi) continue;
+      const bool on = (o >> lane) & 1u, changed = (row[i] >> 48) & 1u;
+      o = __reduce_or_sync(kFull, !on ? 0u : (changed ? uint32_t(row[i]) & 0xFFFFFFu : 1u << lane));
+    }
+    return o;
+  };
+  bool keeps_t = true, keeps_c = true;
+#pragma unroll
+  for (int i = 0; i < kPlanMaxInsn; i++) {
+    const bool ch = __shfl_sync(kFull, uint32_t(row[i] >> 48) & 1u, 0) != 0u;
+    if (uint32_t(i) < p.tl) keeps_t = keeps_t && !ch;
+    else if (uint32_t(i) < n) keeps_c = keeps_c && !ch;
+  }
+  const uint32_t rest = open & ~uint32_t(kRegA), a = open & kRegA;
+  return plan_from(reads, open, relevant(0, p.tl, rest) | relevant(p.tl, n, rest), a ? relevant(0, p.tl, a) : 0u,
+                   a ? relevant(p.tl, n, a) : 0u, keeps_t, keeps_c);
+}
+
+// Plans the round's pairs (z80_plan.cuh), a warp each: compared outputs,
 // swept fields, class and chunks.  A pair that its programs prove equivalent
 // gets no chunk and keeps its zero flag; the pairs after it in its window
 // cannot win and are cancelled.  A pair whose sweep takes more than one chunk
-// is probed first by the whole warp: nearly all long sweeps belong to pairs
-// that passed the eight QuickCheck vectors and are no equivalences, and such
-// a sweep draws every resident warp into one pair before its first mismatch
-// is seen, one pair after the other.
-// Bound by latency (table loads and local arrays, a few microseconds a pair,
-// thousands of pairs side by side; a small round spreads its pairs over the
-// warps).  Planned in the round build, a window's up to 64 pairs in one
-// thread, 100,003 masked targets spent 3.4 ms in their 11 rounds, here
-// 0.9 ms.  The probe and the polls between units: 40,009 uneven targets
-// evaluate 4.5e8 states where it was 1.6e10 (84 -> 43 ms of sweeps), the
-// 9.4M length-2 targets 2.7e8 where it was 1.3e9 (3.2 -> 2.05 ms).
-// The chunks of a pair go to its class's list (RoundCtl::alloc), one atomic
-// per warp and class.
-__global__ void __launch_bounds__(128) k_pair_plan(const RoundArgs* __restrict__ A) {
+// is probed first: nearly all long sweeps belong to pairs that passed the
+// eight QuickCheck vectors and are no equivalences, and such a sweep draws
+// every resident warp into one pair before its first mismatch is seen, one
+// pair after the other.  The chunks of a pair go to its class's list
+// (RoundCtl::alloc), one atomic each.
+// Bound by latency (some ten dependent loads and a few hundred instructions a
+// pair).  A lane per pair, each running plan_pair on arrays in local memory,
+// took 26 us a round however few its pairs (200 uneven targets: 1.75 ms a
+// search, 0.95 ms with this and k_qc_long; the 818,000 pairs of the 9.4M
+// length-2 targets' rounds pay for it with 0.4 ms of 5); in the round build, a
+// window's up to 64 pairs in one thread, 0.3 ms a round.  The probe and the polls between units:
+// 40,009 uneven targets evaluate 4.5e8 states where it was 1.6e10 (84 -> 43 ms
+// of sweeps), the 9.4M length-2 targets 2.7e8 where it was 1.3e9 (3.2 ->
+// 2.05 ms).
+__global__ void __launch_bounds__(128, 8) k_pair_plan(const RoundArgs* __restrict__ A) {
   const RoundBuf& R = A->R;
   const DevTargets& T = A->T;
   const DevPool& P = A->P;
@@ -770,94 +829,53 @@ __global__ void __launch_bounds__(128) k_pair_plan(const RoundArgs* __restrict__
   if (blockIdx.x == 0 && threadIdx.x == 0) R.ctl->nscan = 0;  // the rescan before this round has read it
   const unsigned lane = lane_id();
   const uint32_t nw = gridDim.x * (blockDim.x >> 5);
-  const uint32_t gw = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  const uint32_t per = min(32u, (np + nw - 1u) / nw);
   unsigned long long covered = 0;  // reference states that proofs and probes answer for
   uint32_t probes = 0;
-  for (uint32_t base = gw * per; base < np; base += nw * per) {
-    const uint32_t p = base + lane;
-    const bool mine = lane < per && p < np;
-    PairRec pr{};
-    bool large = false;
-    if (mine) {
-      pr = R.pairs[p];
-      const uint32_t t = pr.target, c = pr.cand;
-      const bool masked = (pr.keepR & 0x80u) != 0;
-      const uint32_t* tw = T.insn + (size_t)t * T.stride;
-      const uint32_t* cw = P.insn + (size_t)c * P.stride;
-      const uint32_t tl = target_len(T, t), cl = pool_len(P, c);
-      uint32_t reads = 0;
-      if (P.reads) {
-        reads = A->q.meta[t].reads | P.reads[c];
-      } else {
-        for (uint32_t i = 0; i < tl; i++) reads |= g_ops[tw[i] & 0xFFFFu].reads;
-        for (uint32_t i = 0; i < cl; i++) reads |= g_ops[cw[i] & 0xFFFFu].reads;
-      }
-      pr.keepF = masked ? uint8_t(~target_dead(T, t)) : uint8_t(0xFFu);
-      pr.keepR = masked ? uint8_t((~target_dead_regs(T, t) & 0x3Fu) | 0x80u) : uint8_t(0x3Fu);
-      const PairPlan pl = plan_pair(g_flow, tw, tl, cw, cl, reads, pr.keepF, pr.keepR);
-      pr.reads = pl.reads;
-      pr.sweepf = pl.sweepf;
-      pr.nblocks = pl.nblocks;
-      pr.cmap = 0;
-      if (pl.proven) {
-        pr.nblocks = 0;  // no chunk in any class
-        covered += 256ull * plan_blocks(reads, false);
-        if (R.wend)
-          for (uint32_t i = p + 1; i < R.wend[p]; i++) R.rejected[i] = 2;
-      } else {
-        if (pl.a_free || pair_xindep(T, t, P, c)) pr.keepR |= uint8_t(kXIndep);
-        // compact classes: A-dependent pairs, and A-independent ones when
-        // those are swept bit-sliced (units of kXBitsBlocks); the narrow
-        // state first
-        if (!(pr.keepR & kXIndep) || R.xunit == kXBitsBlocks) {
-          if (R.compact) pr.cmap = pair_cmap(T, t, P, c);
-          // the wide state: A-dependent pairs only
-          if (!pr.cmap && R.wide && !(pr.keepR & kXIndep)) pr.cmap = pair_wmap(T, t, P, c);
-          // the register state: the rest that name neither SP nor the memory byte
-          if (!pr.cmap && R.wide && pair_regstate(T, t, P, c)) pr.cmap = kRegClass;
+  for (uint32_t p = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); p < np; p += nw) {
+    PairRec pr = R.pairs[p];
+    const uint32_t t = pr.target, c = pr.cand;
+    const bool masked = (pr.keepR & 0x80u) != 0;
+    const PairWords words = pair_words(T, t, P, c);
+    uint32_t reads;
+    if (P.reads) reads = A->q.meta[t].reads | P.reads[c];
+    else reads = __reduce_or_sync(kFull, words.mine() ? uint32_t(g_ops[words.w & 0xFFFFu].reads) : 0u);
+    pr.keepF = masked ? uint8_t(~target_dead(T, t)) : uint8_t(0xFFu);
+    pr.keepR = masked ? uint8_t((~target_dead_regs(T, t) & 0x3Fu) | 0x80u) : uint8_t(0x3Fu);
+    const PairPlan pl = plan_pair_warp(words, reads, pr.keepF, pr.keepR);
+    pr.reads = pl.reads;
+    pr.sweepf = pl.sweepf;
+    pr.nblocks = pl.nblocks;
+    pr.cmap = 0;
+    if (pl.proven) {
+      pr.nblocks = 0;  // no chunk in any class
+      covered += 256ull * plan_blocks(reads, false);
+      if (R.wend)
+        for (uint32_t i = p + 1 + lane; i < R.wend[p]; i += 32) R.rejected[i] = 2;
+    } else {
+      if (pl.a_free || pair_xindep(words)) pr.keepR |= uint8_t(kXIndep);
+      // compact classes: A-dependent pairs, and A-independent ones when
+      // those are swept bit-sliced (units of kXBitsBlocks)
+      const bool xind = (pr.keepR & kXIndep) != 0;
+      if (!xind || R.xunit == kXBitsBlocks) pr.cmap = pair_cmap(words, R.compact != 0, R.wide != 0, xind);
+      if (pair_units(pr.nblocks, pr.keepR, R.xunit) > R.chunk_blocks) {
+        probes++;
+        if (probe_pair(words, pr.nblocks, pr.reads, pr.sweepf, pr.keepF, pr.keepR)) {
+          pr.nblocks = 0;
+          if (lane == 0) R.rejected[p] = 1;
         }
-        large = pair_units(pr.nblocks, pr.keepR, R.xunit) > R.chunk_blocks;
       }
     }
-    for (unsigned b = __ballot_sync(kFull, large); b; b &= b - 1) {
-      const int j = __ffs(b) - 1;
-      const uint32_t masks = __shfl_sync(kFull, uint32_t(pr.keepF) | uint32_t(pr.keepR) << 8 | uint32_t(pr.sweepf) << 16, j);
-      const bool bad = probe_pair(T, P, __shfl_sync(kFull, pr.target, j), __shfl_sync(kFull, pr.cand, j),
-                                  __shfl_sync(kFull, pr.nblocks, j), __shfl_sync(kFull, uint32_t(pr.reads), j),
-                                  masks >> 16, masks & 0xFFu, (masks >> 8) & 0xFFu);
-      probes++;
-      if (bad && int(lane) == j) {
-        pr.nblocks = 0;
-        R.rejected[p] = 1;
-      }
-    }
-    if (mine) R.pairs[p] = pr;
-    // chunk lists
-    const uint32_t ch = mine && pr.nblocks ? chunks_for(R, pair_units(pr.nblocks, pr.keepR, R.xunit)) : 0u;
-    const int cls = ch ? pair_class(pr) : -1;
-    for (int c = 0; c < kClasses; c++) {
-      const unsigned b = __ballot_sync(kFull, cls == c);
-      if (!b) continue;
-      uint32_t incl = cls == c ? ch : 0u;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t v = __shfl_up_sync(kFull, incl, o);
-        if (lane >= unsigned(o)) incl += v;
-      }
-      unsigned long long at = 0;
-      if (lane == 31)
-        at = atomicAdd(&R.ctl->alloc[c], (unsigned long long)__popc(b) << kChunkBits | incl);
-      at = __shfl_sync(kFull, at, 31);
-      if (cls == c) {
-        const uint32_t e = uint32_t(at >> kChunkBits) + __popc(b & lanemask_lt());
-        R.cbase[c][e] = (at & kChunkMask) + incl - ch;
-        R.cpair[c][e] = p;
+    if (lane == 0) {
+      R.pairs[p] = pr;
+      const uint32_t ch = pr.nblocks ? chunks_for(R, pair_units(pr.nblocks, pr.keepR, R.xunit)) : 0u;
+      if (ch) {
+        const int cls = pair_class(pr);
+        const unsigned long long at = atomicAdd(&R.ctl->alloc[cls], 1ull << kChunkBits | ch);
+        R.cbase[cls][at >> kChunkBits] = at & kChunkMask;
+        R.cpair[cls][at >> kChunkBits] = p;
       }
     }
   }
-#pragma unroll
-  for (int o = 16; o; o >>= 1) covered += __shfl_xor_sync(kFull, covered, o);
   if (lane == 0 && (covered || probes)) {
     atomicAdd(R.states, covered + 512ull * probes);
     if (probes) atomicAdd(R.states + 1, 512ull * probes);
@@ -2060,9 +2078,11 @@ __global__ void k_qc_entries(DevPool P, uint32_t w2mask, const unsigned long lon
   entries[i] = make_uint4(uint32_t(key >> kQCIndexBits), c | uint32_t(P.size[c]) << kQCIndexBits, f[0], f[1]);
   hash2[i] = h2;
 }
-// Every entry against the nearest one before it with both hashes equal.
+// Every entry against the nearest one before it with both hashes equal:
+// flags[0] is set where their outputs differ, flags[1] where entries of one
+// first hash have two second ones.
 __global__ void k_qc_check(DevPool P, uint32_t w2mask, const unsigned long long* __restrict__ keys,
-                           const uint32_t* __restrict__ hash2, uint32_t n, uint32_t* __restrict__ clash) {
+                           const uint32_t* __restrict__ hash2, uint32_t n, uint32_t* __restrict__ flags) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const unsigned long long run = keys[i] >> kQCIndexBits;
@@ -2071,6 +2091,7 @@ __global__ void k_qc_check(DevPool P, uint32_t w2mask, const unsigned long long*
   do {
     if (j == 0 || (keys[j - 1] >> kQCIndexBits) != run) return;
     j--;
+    if (hash2[j] != hash2[i]) flags[1] = 1;
   } while (hash2[j] != hash2[i]);
   const uint32_t e = uint32_t(keys[j]) & ((1u << kQCIndexBits) - 1u);
   uint32_t d = 0;
@@ -2079,7 +2100,7 @@ __global__ void k_qc_check(DevPool P, uint32_t w2mask, const unsigned long long*
     const uint4 x = P.qc[(size_t)v * P.n + c], y = P.qc[(size_t)v * P.n + e];
     d |= ((x.x ^ y.x) & key_keep0(m)) | ((x.y ^ y.y) & key_keep1(m)) | ((x.z ^ y.z) & w2mask);
   }
-  if (d) *clash = 1;
+  if (d) flags[0] = 1;
 }
 __global__ void k_qc_top(const unsigned long long* __restrict__ keys, uint32_t nv, uint32_t first, uint32_t m0,
                          uint32_t nm, uint32_t top_bits, uint32_t* __restrict__ top) {
@@ -2093,46 +2114,183 @@ __global__ void k_qc_top(const unsigned long long* __restrict__ keys, uint32_t n
   top[m * per + b] = first + (b == per - 1u ? seg + nv : seg + lower_bound_u64(keys + seg, nv, lo));
 }
 
+// What a target's lanes know of it when they read its range of entries.
+struct QCQuery {
+  uint32_t t;                  // the target
+  uint32_t base;               // lane that ran vector 0 (the others follow it)
+  uint32_t h, h2, flo, fhi;    // hashes, F bytes
+  uint32_t live;               // live flag bits, in every byte
+  uint32_t size, m, k0, k1;    // encoded bytes, dead registers, live bytes of words 0 and 1
+  uint32_t nf_total, obase;    // collect pass: full survivors, first slot
+};
+// Survivors of one target found so far: tallies per lane (count pass), places
+// (collect pass: full, masked), all of them (single pass).
+struct QCFound {
+  uint32_t lf = 0, lm = 0, nf = 0, nm = 0, nk = 0;
+};
+// Reads entries [r0, r1) of a target's range, W at a time (W lanes per target:
+// 8, each group its own target, or 32, the whole warp one), `steps` times.
+// w: this lane's vector's outputs (of its own target).
+// late: fills in what the query does not need before its first hit.
+template <int W, bool COLLECT, bool KEEP, class Late>
+__device__ __forceinline__ void qc_range(QCQuery& q, QCFound& f, uint32_t r0, uint32_t r1, uint32_t steps,
+                                         const uint32_t (&w)[3], const DevPool& P, const QCConfig& cfg,
+                                         const QCIndex& ix, const QCOut& o, Late late) {
+  const unsigned lane = lane_id(), sub = lane & 7u;
+  const unsigned pos = W == 8 ? sub : lane;
+  const unsigned gshift = W == 8 ? (lane & ~7u) : 0u, gmask = W == 8 ? 0xFFu : kFull;
+  const unsigned before = lanemask_lt() & (gmask << gshift);
+  uint32_t same = 2;  // the target's outputs against an entry's: 2 not compared yet
+  for (uint32_t k = 0; k < steps; k++) {
+    const uint32_t i = r0 + uint32_t(W) * k + pos;
+    uint4 e = make_uint4(0u, 0u, 0u, 0u);
+    bool hit = i < r1;
+    if (hit) {
+      e = ix.entries[i];
+      hit = e.x == q.h;
+    }
+    if (!__any_sync(kFull, hit)) continue;  // most steps find nothing
+    late();
+    if (ix.check_h2 && hit) hit = ix.hash2[i] == q.h2;
+    const uint32_t c = e.y & ((1u << kQCIndexBits) - 1u);
+    // the outputs themselves, once per target: entries of equal hashes have
+    // equal outputs
+    const unsigned ghit = (__ballot_sync(kFull, hit) >> gshift) & gmask;
+    const uint32_t c0 = __shfl_sync(kFull, c, int(gshift) + (ghit ? __ffs(int(ghit)) - 1 : 0));
+    const uint32_t x = __shfl_sync(kFull, w[0], int(q.base + sub)), y = __shfl_sync(kFull, w[1], int(q.base + sub));
+    const uint32_t z = __shfl_sync(kFull, w[2], int(q.base + sub));
+    bool differs = false;
+    if (same == 2 && ghit) {
+      const uint4 v = P.qc[(size_t)sub * P.n + c0];
+      differs = (((v.x ^ x) & q.k0) | ((v.y ^ y) & q.k1) | ((v.z ^ z) & cfg.w2mask)) != 0;
+    }
+    const unsigned gdiff = (__ballot_sync(kFull, differs) >> gshift) & gmask;
+    if (same == 2 && ghit) same = gdiff ? 0u : 1u;
+    const bool pass = hit && same == 1u && (e.y >> kQCIndexBits) < q.size &&
+                      (((e.z ^ q.flo) | (e.w ^ q.fhi)) & q.live) == 0;
+    uint32_t fd = (e.z ^ q.flo) | (e.w ^ q.fhi);
+    fd |= fd >> 16;
+    fd = (fd | (fd >> 8)) & 0xFFu;
+    // dead registers that differ, on the candidate itself: to tell full from
+    // masked, and for the survivors that are stored
+    uint32_t rdf = 0;
+    const bool need = pass && q.m != 0 && (COLLECT || fd == 0 || (KEEP && f.nk < kQCSlots));
+    if (__any_sync(kFull, need)) {
+      constexpr int kAhead = W == 8 ? 2 : 8;  // loads in flight
+#pragma unroll 1
+      for (int j0 = 0; j0 < 8; j0 += kAhead) {
+        uint2 v[kAhead];
+#pragma unroll
+        for (int j = 0; j < kAhead; j++)
+          if (need) v[j] = *reinterpret_cast<const uint2*>(&P.qc[(size_t)(j0 + j) * P.n + c]);
+#pragma unroll
+        for (int j = 0; j < kAhead; j++) {
+          const uint32_t a = __shfl_sync(kFull, w[0], int(q.base) + j0 + j);
+          const uint32_t b = __shfl_sync(kFull, w[1], int(q.base) + j0 + j);
+          if (need) rdf |= reg_diff(v[j].x ^ a, v[j].y ^ b);
+        }
+      }
+    }
+    const uint32_t diff = fd | (rdf << 8);
+    const bool fp = pass && (cfg.all_hits != 0 || diff == 0), mp = pass && !fp;
+    if constexpr (!COLLECT) {
+      f.lf += fp ? 1u : 0u;
+      f.lm += mp ? 1u : 0u;
+      if constexpr (KEEP) {
+        const unsigned bs = __ballot_sync(kFull, pass);
+        const uint32_t rank = f.nk + __popc(bs & before);
+        if (pass && rank < kQCSlots)
+          o.tmp[(size_t)q.t * kQCSlots + rank] = c | (diff << 16) | (mp ? 0x80000000u : 0u);
+        f.nk += __popc((bs >> gshift) & gmask);
+      }
+    } else {
+      // this target's survivors of the step, in enumeration order
+      const unsigned bf = __ballot_sync(kFull, fp), bm = __ballot_sync(kFull, mp);
+      if (fp) {
+        const uint32_t idx = q.obase + f.nf + __popc(bf & before);
+        o.surv[idx] = c;
+        o.sdiff[idx] = uint16_t(diff);
+      }
+      if (mp) {
+        const uint32_t idx = q.obase + q.nf_total + f.nm + __popc(bm & before);
+        o.surv[idx] = c;
+        o.sdiff[idx] = uint16_t(diff);
+      }
+      f.nf += __popc((bf >> gshift) & gmask);
+      f.nm += __popc((bm >> gshift) & gmask);
+    }
+  }
+}
+
+// The query of the target in lanes base.. (w: its outputs by vector) short of
+// the second hash and the F bytes.
+__device__ __forceinline__ QCQuery qc_query(const DevTargets& T, const QCConfig& cfg, uint32_t t, bool valid,
+                                            const uint32_t (&w)[3]) {
+  QCQuery q{};
+  q.t = t;
+  q.base = lane_id() & ~7u;
+  q.live = valid ? (~target_dead(T, t) & 0xFFu) * 0x01010101u : 0u;
+  q.m = valid ? target_dead_regs(T, t) & 0x3Fu : 0u;
+  q.k0 = key_keep0(q.m);
+  q.k1 = key_keep1(q.m);
+  q.h = qc_hash(w[0] & q.k0, w[1] & q.k1, w[2] & cfg.w2mask, lane_id() & 7u);
+#pragma unroll
+  for (int off = 4; off >= 1; off >>= 1) q.h += __shfl_xor_sync(kFull, q.h, off);
+  return q;
+}
+__device__ __forceinline__ void qc_late(QCQuery& q, const QCConfig& cfg, const uint32_t (&w)[3]) {
+  const unsigned sub = lane_id() & 7u;
+  const uint32_t fb = ((w[0] >> 8) & 0xFFu) << (8u * (sub & 3u));
+  q.h2 = qc_hash2(w[0] & q.k0, w[1] & q.k1, w[2] & cfg.w2mask, sub);
+  q.flo = sub < 4u ? fb : 0u;
+  q.fhi = sub < 4u ? 0u : fb;
+#pragma unroll
+  for (int off = 4; off >= 1; off >>= 1) {
+    q.h2 += __shfl_xor_sync(kFull, q.h2, off);
+    q.flo |= __shfl_xor_sync(kFull, q.flo, off);
+    q.fhi |= __shfl_xor_sync(kFull, q.fhi, off);
+  }
+}
+__device__ __forceinline__ void qc_bounds(const QCIndex& ix, const QCQuery& q, uint32_t& r0, uint32_t& r1) {
+  const uint32_t* top = ix.top + q.m * ((1u << ix.top_bits) + 1u) + (q.h >> (32u - ix.top_bits));
+  r0 = top[0];
+  r1 = top[1];
+}
+
 // QuickCheck through the index: a target only meets the candidates whose
 // compared outputs hash like its own.  Eight lanes per target, four targets
 // per warp: lane 8g + v runs target t0 + g on vector v and hashes its output;
 // the hash's range is read eight entries at a time.  A target with an entry
-// of its hash (one in fourteen of the length-2 enumeration) goes on: the
-// second hash, its outputs against the first such entry's, and F under the
-// dead flags entry by entry, from the entries themselves.  Entries of a hash
-// are in pool order, so survivors come out in enumeration order as in the
-// full scan.  Lanes of a group that has no target (past the end) take part in
-// the warp's collectives with nothing to do.
-// Bound by issue and by the chain program - table - entry.  Hashing the first
-// vector alone, gathering all eight outputs of every candidate that agreed on
-// it and broadcasting the target's eight outputs to every lane took 5.1 ms for
-// 9.4M length-2 targets and 1.0 ms for 100,003 targets with every flag dead,
-// this 1.9 and 0.15 ms (of the 1.9, the targets' upload 1.4).
+// of its hash (one in fourteen of the length-2 enumeration) goes on: its
+// outputs against the first such entry's, and F under the dead flags entry by
+// entry, from the entries themselves.  Entries of a hash are in pool order, so
+// survivors come out in enumeration order as in the full scan.  Targets with
+// long ranges are left to k_qc_long.  Lanes of a group that has no target
+// (past the end) take part in the warp's collectives with nothing to do.
+// Bound by issue and by the chain program - table - entry (more registers
+// than 64 and it slows with the blocks that go).  Hashing the first vector
+// alone, gathering all eight outputs of every candidate that agreed on it and
+// broadcasting the target's eight outputs to every lane took 5.1 ms for 9.4M
+// length-2 targets and 1.0 ms for 100,003 targets with every flag dead, this
+// 1.9 and 0.13 ms (of the 1.9, the targets' upload 1.4).
 // COLLECT: the collect pass; else the count pass, which with KEEP also keeps
 // the survivors of targets with at most kQCSlots (single pass).
+constexpr uint32_t kQCLong = 64;  // entries: eight steps of a group, two of a warp
 template <bool COLLECT, bool KEEP>
 __global__ void __launch_bounds__(kBlock, 4) k_qc_bucket(DevTargets T, DevPool P, QCConfig cfg, QCIndex ix, QCOut o) {
   const unsigned lane = lane_id();
-  const unsigned sub = lane & 7u, gshift = lane & ~7u;
-  const unsigned group_lt = lanemask_lt() & (0xFFu << gshift);
+  const unsigned sub = lane & 7u;
   const uint32_t gw = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const uint32_t nw = gridDim.x * (blockDim.x >> 5);
-  const uint32_t per_mask = (1u << ix.top_bits) + 1u, top_shift = 32u - ix.top_bits;
   unsigned long long my_checks = 0;
   for (uint32_t t0 = gw * 4u; t0 < T.n; t0 += nw * 4u) {
     const uint32_t t = t0 + (lane >> 3);
     const bool valid = t < T.n;
-    uint32_t nf_total = 0, obase = 0;
     bool work = valid;
     if (COLLECT) {
-      if (valid) {
-        nf_total = o.cnt_f[t];
-        const uint32_t tot = nf_total + o.cnt_m[t];
-        // single pass: the count pass kept the survivors of targets with at
-        // most kQCSlots of them
-        work = o.tmp ? tot > kQCSlots : tot != 0;
-        obase = o.base[t];
-      }
+      // single pass: the count pass kept the survivors of targets with at
+      // most kQCSlots of them
+      if (valid) work = o.cnt_f[t] + o.cnt_m[t] > (o.tmp ? kQCSlots : 0u);
       if (!__any_sync(kFull, work)) continue;
     }
     // the target on vector `sub`; every lane reads the program itself
@@ -2154,114 +2312,31 @@ __global__ void __launch_bounds__(kBlock, 4) k_qc_bucket(DevTargets T, DevPool P
     }
     uint32_t w[3];
     z_pack(st, w);
-    const uint32_t dead = valid ? target_dead(T, t) & 0xFFu : 0u;
-    const uint32_t m = valid ? target_dead_regs(T, t) & 0x3Fu : 0u;
-    const uint32_t k0 = key_keep0(m), k1 = key_keep1(m);
-    uint32_t h = qc_hash(w[0] & k0, w[1] & k1, w[2] & cfg.w2mask, sub);
-#pragma unroll
-    for (int off = 4; off >= 1; off >>= 1) h += __shfl_xor_sync(kFull, h, off);
+    QCQuery q = qc_query(T, cfg, t, valid, w);
+    q.size = size;
+    if (COLLECT && valid) {
+      q.nf_total = o.cnt_f[t];
+      q.obase = o.base[t];
+    }
     uint32_t r0 = 0, r1 = 0;
-    if (work) {
-      const uint32_t* top = ix.top + m * per_mask + (h >> top_shift);
-      r0 = top[0];
-      r1 = top[1];
+    if (work) qc_bounds(ix, q, r0, r1);
+    const bool is_long = r1 - r0 > kQCLong;
+    if (is_long) {
+      if (sub == 0) o.longs[atomicAdd(o.nlong, 1u)] = t;
+      r1 = r0;
     }
-    const uint32_t iters = (__reduce_max_sync(kFull, r1 - r0) + 7u) / 8u;
-    uint32_t nf = 0, nm = 0, lf = 0, lm = 0;
-    uint32_t nk = 0;  // this group's survivors so far (count pass, single pass)
-    uint32_t h2 = 0, flo = 0, fhi = 0;
-    bool hashed = false;             // h2, flo, fhi are there (warp-uniform)
-    uint32_t same = 2;               // this group's outputs against an entry's: 2 not compared yet
-    uint32_t* const keep = KEEP ? o.tmp + (size_t)t * kQCSlots : nullptr;
-    for (uint32_t k = 0; k < iters; k++) {
-      const uint32_t i = r0 + 8u * k + sub;
-      uint4 e = make_uint4(0u, 0u, 0u, 0u);
-      bool hit = i < r1;
-      if (hit) {
-        e = ix.entries[i];
-        hit = e.x == h;
-      }
-      if (!__any_sync(kFull, hit)) continue;  // most steps find nothing
-      if (!hashed) {
-        hashed = true;
-        h2 = qc_hash2(w[0] & k0, w[1] & k1, w[2] & cfg.w2mask, sub);
-        const uint32_t f = ((w[0] >> 8) & 0xFFu) << (8u * (sub & 3u));
-        flo = sub < 4u ? f : 0u;
-        fhi = sub < 4u ? 0u : f;
-#pragma unroll
-        for (int off = 4; off >= 1; off >>= 1) {
-          h2 += __shfl_xor_sync(kFull, h2, off);
-          flo |= __shfl_xor_sync(kFull, flo, off);
-          fhi |= __shfl_xor_sync(kFull, fhi, off);
-        }
-      }
-      if (hit) hit = ix.hash2[i] == h2;
-      const uint32_t c = e.y & ((1u << kQCIndexBits) - 1u);
-      // the outputs themselves, once per target: entries of equal hashes have
-      // equal outputs
-      const unsigned ghit = (__ballot_sync(kFull, hit) >> gshift) & 0xFFu;
-      const uint32_t c0 = __shfl_sync(kFull, c, ghit ? __ffs(int(ghit)) - 1 : 0, 8);
-      bool differs = false;
-      if (same == 2 && ghit) {
-        const uint4 q = P.qc[(size_t)sub * P.n + c0];
-        differs = (((q.x ^ w[0]) & k0) | ((q.y ^ w[1]) & k1) | ((q.z ^ w[2]) & cfg.w2mask)) != 0;
-      }
-      const unsigned gdiff = (__ballot_sync(kFull, differs) >> gshift) & 0xFFu;
-      if (same == 2 && ghit) same = gdiff ? 0u : 1u;
-      const uint32_t live = (~dead & 0xFFu) * 0x01010101u;
-      const bool pass = hit && same == 1u && (e.y >> kQCIndexBits) < size &&
-                        (((e.z ^ flo) | (e.w ^ fhi)) & live) == 0;
-      uint32_t fd = (e.z ^ flo) | (e.w ^ fhi);
-      fd |= fd >> 16;
-      fd = (fd | (fd >> 8)) & 0xFFu;
-      uint32_t rdf = 0;
-      if (__any_sync(kFull, pass && m != 0)) {
-        // dead registers: which of them differ, on the candidate itself
-#pragma unroll 1
-        for (int v = 0; v < 8; v++) {
-          const uint32_t x = __shfl_sync(kFull, w[0], v, 8), y = __shfl_sync(kFull, w[1], v, 8);
-          if (pass && m != 0) {
-            const uint4 q = P.qc[(size_t)v * P.n + c];
-            rdf |= reg_diff(q.x ^ x, q.y ^ y);
-          }
-        }
-      }
-      const uint32_t diff = fd | (rdf << 8);
-      const bool fp = pass && (cfg.all_hits != 0 || diff == 0), mp = pass && !fp;
-      if constexpr (!COLLECT) {
-        lf += fp ? 1u : 0u;
-        lm += mp ? 1u : 0u;
-        if constexpr (KEEP) {
-          const unsigned bs = __ballot_sync(kFull, pass);
-          if (bs) {
-            const uint32_t rank = nk + __popc(bs & group_lt);
-            if (pass && rank < kQCSlots) keep[rank] = c | (diff << 16) | (mp ? 0x80000000u : 0u);
-            nk += __popc((bs >> gshift) & 0xFFu);
-          }
-        }
-      } else {
-        // this group's survivors of the step, in enumeration order
-        const unsigned bf = __ballot_sync(kFull, fp), bm = __ballot_sync(kFull, mp);
-        if (fp) {
-          const uint32_t idx = obase + nf + __popc(bf & group_lt);
-          o.surv[idx] = c;
-          o.sdiff[idx] = uint16_t(diff);
-        }
-        if (mp) {
-          const uint32_t idx = obase + nf_total + nm + __popc(bm & group_lt);
-          o.surv[idx] = c;
-          o.sdiff[idx] = uint16_t(diff);
-        }
-        nf += __popc((bf >> gshift) & 0xFFu);
-        nm += __popc((bm >> gshift) & 0xFFu);
-      }
-    }
+    QCFound f;
+    bool hashed = false;
+    qc_range<8, COLLECT, KEEP>(q, f, r0, r1, (__reduce_max_sync(kFull, r1 - r0) + 7u) / 8u, w, P, cfg, ix, o, [&] {
+      if (!hashed) qc_late(q, cfg, w);
+      hashed = true;
+    });
     if constexpr (!COLLECT) {
       if (hashed) {
 #pragma unroll
         for (int off = 4; off >= 1; off >>= 1) {
-          lf += __shfl_xor_sync(kFull, lf, off);
-          lm += __shfl_xor_sync(kFull, lm, off);
+          f.lf += __shfl_xor_sync(kFull, f.lf, off);
+          f.lm += __shfl_xor_sync(kFull, f.lm, off);
         }
       }
       if (sub == 0 && valid) {
@@ -2271,14 +2346,57 @@ __global__ void __launch_bounds__(kBlock, 4) k_qc_bucket(DevTargets T, DevPool P
         g.tts = tstates;
         g.trd = reads;
         g.tl = tl;
-        qc_count_out(o, t, g, lf, lm);
-        if (KEEP && lf + lm > kQCSlots) atomicAdd(o.over, 1u);
+        qc_count_out(o, t, g, f.lf, f.lm);
+        if (KEEP && f.lf + f.lm > kQCSlots) atomicAdd(o.over, 1u);
       }
     }
   }
   if constexpr (!COLLECT) {
     for (int off = 16; off; off >>= 1) my_checks += __shfl_down_sync(kFull, my_checks, off);
     if (lane == 0 && my_checks) atomicAdd(o.checks, my_checks);
+  }
+}
+// The targets whose range is long (they leave little to compare: A kept,
+// registers dead; up to 3,900 of the 4,523 candidates), a warp each: every
+// eight lanes run the target, the range is read 32 entries at a time.  A
+// kernel of its own, so that its registers do not weigh on the others' warps.
+// Eight entries at a time such targets took 0.5 ms of a search of 200 uneven
+// targets, here 0.15 ms.
+template <bool COLLECT, bool KEEP>
+__global__ void __launch_bounds__(128) k_qc_long(DevTargets T, DevPool P, QCConfig cfg, QCIndex ix, QCOut o) {
+  const unsigned lane = lane_id();
+  const uint32_t gw = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const uint32_t nw = gridDim.x * (blockDim.x >> 5);
+  const uint32_t n = *o.nlong;
+  for (uint32_t i = gw; i < n; i += nw) {
+    const uint32_t t = o.longs[i], tl = target_len(T, t);
+    const uint32_t pw = lane < tl ? T.insn[(size_t)t * T.stride + lane] : 0u;
+    const uint32_t size = __reduce_add_sync(kFull, lane < tl ? uint32_t(g_ops[pw & 0xFFFFu].size) : 0u);
+    Z80S st = vec_state(int(lane & 7u));
+    run_lanes(st, pw, 0, int(tl));
+    uint32_t w[3];
+    z_pack(st, w);
+    QCQuery q = qc_query(T, cfg, t, true, w);
+    qc_late(q, cfg, w);
+    q.size = size;
+    q.base = 0;
+    if (COLLECT) {
+      q.nf_total = o.cnt_f[t];
+      q.obase = o.base[t];
+    }
+    uint32_t r0, r1;
+    qc_bounds(ix, q, r0, r1);
+    QCFound f;
+    qc_range<32, COLLECT, KEEP>(q, f, r0, r1, (r1 - r0 + 31u) / 32u, w, P, cfg, ix, o, [] {});
+    if constexpr (!COLLECT) {
+      const uint32_t lf = __reduce_add_sync(kFull, f.lf), lm = __reduce_add_sync(kFull, f.lm);
+      if (lane == 0) {
+        o.cnt_f[t] = lf;
+        o.cnt_m[t] = lm;
+        o.cnt_all[t] = lf + lm;
+        if (KEEP && lf + lm > kQCSlots) atomicAdd(o.over, 1u);
+      }
+    }
   }
 }
 
@@ -2542,7 +2660,13 @@ void dev_upload_tables(cudaStream_t s) {
   cudaMemcpyToSymbolAsync(g_repsp, rep_sp(), 32, 0, cudaMemcpyHostToDevice, s);
   cudaMemcpyToSymbolAsync(g_aclass, op_aclass(), kNumOps, 0, cudaMemcpyHostToDevice, s);
   {
-    cudaMemcpyToSymbolAsync(g_flow, op_flow(), sizeof(OpFlow) * kNumOps, 0, cudaMemcpyHostToDevice, s);
+    static uint64_t flow[kNumOps][kFlowFields];
+    static std::once_flag once;
+    std::call_once(once, [] {
+      for (int op = 0; op < kNumOps; op++)
+        for (int g = 0; g < kFlowFields; g++) flow[op][g] = flow_word(op_flow()[op], g);
+    });
+    cudaMemcpyToSymbolAsync(g_flow, flow, sizeof flow, 0, cudaMemcpyHostToDevice, s);
     const CompactTables& C = compact_tables();
     cudaMemcpyToSymbolAsync(g_cren, C.ren, sizeof C.ren, 0, cudaMemcpyHostToDevice, s);
     cudaMemcpyToSymbolAsync(g_corig, C.orig, sizeof C.orig, 0, cudaMemcpyHostToDevice, s);
@@ -2610,11 +2734,11 @@ void launch_qc_keys(const DevPool& P, uint32_t w2mask, uint32_t m0, uint32_t nm,
 }
 void launch_qc_entries(const DevPool& P, uint32_t w2mask, const unsigned long long* keys, uint32_t nv, uint32_t first,
                        uint32_t m0, uint32_t nm, uint32_t top_bits, uint4* entries, uint32_t* hash2, uint32_t* top,
-                       uint32_t* clash, cudaStream_t s) {
+                       uint32_t* flags, cudaStream_t s) {
   const uint32_t n = nm * nv;
   if (n) {
     k_qc_entries<<<grid_for(n, 256), 256, 0, s>>>(P, w2mask, keys, n, entries + first, hash2 + first);
-    k_qc_check<<<grid_for(n, 256), 256, 0, s>>>(P, w2mask, keys, hash2 + first, n, clash);
+    k_qc_check<<<grid_for(n, 256), 256, 0, s>>>(P, w2mask, keys, hash2 + first, n, flags);
   }
   const uint32_t nt = nm * ((1u << top_bits) + 1u);
   k_qc_top<<<grid_for(nt, 256), 256, 0, s>>>(keys, nv, first, m0, nm, top_bits, top);
@@ -2635,9 +2759,17 @@ void launch_qc_bucket(const DevTargets& T, const DevPool& P, const QCConfig& cfg
   unsigned need = grid_for((T.n + 3u) / 4u, kBlock / 32);  // four targets per warp
   unsigned grid = unsigned(dev_num_sms() * per_sm);
   if (grid > need) grid = need;
-  if (collect) k_qc_bucket<true, false><<<grid, kBlock, 0, s>>>(T, P, cfg, ix, o);
-  else if (keep) k_qc_bucket<false, true><<<grid, kBlock, 0, s>>>(T, P, cfg, ix, o);
-  else k_qc_bucket<false, false><<<grid, kBlock, 0, s>>>(T, P, cfg, ix, o);
+  const unsigned lgrid = std::min<unsigned>(grid_for(T.n, 4), unsigned(dev_num_sms() * 4));
+  if (collect) {
+    k_qc_bucket<true, false><<<grid, kBlock, 0, s>>>(T, P, cfg, ix, o);
+    k_qc_long<true, false><<<lgrid, 128, 0, s>>>(T, P, cfg, ix, o);
+  } else if (keep) {
+    k_qc_bucket<false, true><<<grid, kBlock, 0, s>>>(T, P, cfg, ix, o);
+    k_qc_long<false, true><<<lgrid, 128, 0, s>>>(T, P, cfg, ix, o);
+  } else {
+    k_qc_bucket<false, false><<<grid, kBlock, 0, s>>>(T, P, cfg, ix, o);
+    k_qc_long<false, false><<<lgrid, 128, 0, s>>>(T, P, cfg, ix, o);
+  }
 }
 SweepArgs sweep_args(const RoundArgs& a) {
   SweepArgs w{};
@@ -2672,7 +2804,7 @@ void launch_round_build(const RoundArgs* a, bool pair, bool small, cudaStream_t 
   else k_round_build<false><<<grid, 256, 0, s>>>(a);
 }
 void launch_pair_plan(const RoundArgs* a, bool small, cudaStream_t s) {
-  k_pair_plan<<<unsigned(dev_num_sms() * (small ? 2 : 16)), 128, 0, s>>>(a);
+  k_pair_plan<<<unsigned(dev_num_sms() * (small ? 4 : 16)), 128, 0, s>>>(a);
 }
 void launch_round_resolve(const RoundArgs* a, bool pair, bool small, cudaStream_t s) {
   const unsigned grid = small ? 32u : unsigned(dev_num_sms() * 8);

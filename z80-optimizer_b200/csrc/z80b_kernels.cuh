@@ -26,6 +26,10 @@ struct QCOut {
   // collect pass runs for the others alone.
   uint32_t* tmp;
   uint32_t* over;
+  // Bucket index: the targets whose range of entries is long (k_qc_long takes
+  // them), and their number.
+  uint32_t* longs;
+  uint32_t* nlong;
 };
 constexpr uint32_t kQCSlots = 8;
 
@@ -56,6 +60,7 @@ struct QCIndex {
   const uint32_t* top;             // [64 * ((1 << top_bits) + 1)] positions in entries
   const uint32_t* elig_lt;         // [256]
   uint32_t top_bits;
+  uint32_t check_h2;               // entries of one hash can have different second ones
 };
 
 // Per-(target, kind) progress of the first-found rounds.
@@ -196,11 +201,12 @@ void launch_fp_query(const DevPool& P, const uint32_t* fp3x8, uint32_t dead, uin
 void launch_qc_keys(const DevPool& P, uint32_t w2mask, uint32_t m0, uint32_t nm, unsigned long long* keys,
                     cudaStream_t s);
 // From the nm * nv sorted keys at keys[0]: the entries at positions first on,
-// and their masks' top tables; *clash is set when two entries of equal hashes
-// differ in their outputs.
+// and their masks' top tables; flags[0] is set when two entries of equal
+// hashes differ in their outputs, flags[1] when two of equal first hashes
+// differ in the second.
 void launch_qc_entries(const DevPool& P, uint32_t w2mask, const unsigned long long* keys, uint32_t nv, uint32_t first,
                        uint32_t m0, uint32_t nm, uint32_t top_bits, uint4* entries, uint32_t* hash2, uint32_t* top,
-                       uint32_t* clash, cudaStream_t s);
+                       uint32_t* flags, cudaStream_t s);
 void launch_qc_bucket(const DevTargets& T, const DevPool& P, const QCConfig& cfg, const QCIndex& ix,
                       const QCOut& o, bool collect, cudaStream_t s);
 // Everything the kernels of a round need, in device memory: a captured round
