@@ -122,7 +122,7 @@ struct PipeOpts {
   int up_chunks = 0;
   const uint32_t* up_hi = nullptr;
 };
-constexpr int kUpChunks = 4;
+constexpr int kUpChunks = kMaxCountParts - 1;
 constexpr uint32_t kUpChunkMin = 1u << 16;  // targets; smaller jobs upload in one copy
 
 // The 4,531^2 pair pool, its QuickCheck outputs and its indexes (one per
@@ -161,6 +161,8 @@ struct Staged {
   z80b_job job{};
   bool valid = false;
   DBuf d_targets, d_lens, d_dead, d_dregs;
+  DBuf d_small;                 // small jobs: lengths, dead flags, dead registers (kSmallJob bytes each), targets
+  DevTargets T{};               // the uploaded targets
   int up_chunks = 0;            // the last upload's chunks (PipeOpts::up_chunks)
   uint32_t up_hi[kUpChunks] = {};
 };
@@ -199,14 +201,17 @@ struct z80b_ctx {
   PoolBufs firstop;  // EnumerateFirstOp pool for all-hits jobs
   Staged staged;
   // pipeline scratch
-  DBuf cnt_f, cnt_m, cnt_all, base, meta, surv, sdiff, checks;
-  DBuf qc_tmp, qc_over;       // single-pass QuickCheck: kept survivors, targets with more
-  DBuf qc_longs, qc_nlong;    // targets with long ranges in the index, per chunk of targets and pass
+  DBuf cnt_f, cnt_m, cnt_all, base, meta, surv, sdiff, tally;
+  DBuf qc_tmp;                // single-pass QuickCheck: kept survivors
+  DBuf qc_longs;              // targets with long ranges in the index
   DBuf next, win, windiff, spec, spec2, wlen, wend, cdone;
-  DBuf pairs, pair_src, cbase[kClasses], cpair[kClasses], rejected, states;
-  DBuf roundctl, roundargs;   // RoundCtl; RoundArgs of the two passes
-  DBuf rcnt, rbase, rules, checked, surv_target, midpass, flag;
+  DBuf pairs, pair_src, cbase[kClasses], cpair[kClasses], rejected;
+  DBuf roundctl, roundargs;   // RoundCtl and RoundArgs of the two passes
+  DBuf rcnt, rbase, rules, surv_target, midpass, flag;
   HBuf h_rules;               // pinned staging of the device rules read back
+  uint64_t rules_on_host = 0; // device rules that the run has already copied there
+  HBuf h_report;              // Report
+  HBuf h_up;                  // small jobs: the host arrays of a search, one copy
   DBuf cub_tmp;
   DBuf hits, nhits, fpq;
   DBuf v_tgt, v_cand, v_tl, v_cl, v_dead, v_out, v_fd, v_in, v_outs;
@@ -241,7 +246,7 @@ struct z80b_ctx {
   // that orders the copies after the context stream's earlier work
   cudaStream_t copy_stream = nullptr;
   cudaEvent_t up_ev[kUpChunks + 1] = {};
-  RoundGraph rg1, rg2;        // instantiated round loops: length-1 and length-2 candidate passes
+  RoundGraph rg[2][2];        // instantiated round loops: length-1 and length-2 candidate passes, small jobs or not
 };
 
 namespace {
@@ -293,10 +298,14 @@ int check_launch(z80b_ctx* ctx, const char* what) {
   return Z80B_OK;
 }
 
-// Exclusive prefix sum (CUB) of n items.
-template <class T>
-int scan(z80b_ctx* ctx, const T* in, T* out, uint32_t n) {
+// Exclusive prefix sum of n items: one block for few, CUB (an init and a scan
+// kernel) above.
+int scan(z80b_ctx* ctx, const uint32_t* in, uint32_t* out, uint32_t n) {
   if (!n) return Z80B_OK;
+  if (n <= kScanSmall) {
+    launch_scan_small(in, out, n, ctx->stream);
+    return check_launch(ctx, "scan");
+  }
   size_t tmp = 0;
   CK(cub::DeviceScan::ExclusiveSum(nullptr, tmp, in, out, n, ctx->stream));
   CK(ctx->cub_tmp.ensure(tmp));
@@ -702,8 +711,8 @@ int ensure_round(z80b_ctx* ctx, uint64_t cap, bool windows, RoundBuf* R) {
   CK(ctx->pairs.ensure(sizeof(PairRec) * cap));
   CK(ctx->pair_src.ensure(4 * cap));
   CK(ctx->rejected.ensure(4 * cap));
-  CK(ctx->states.ensure(16));
-  CK(ctx->roundctl.ensure(sizeof(RoundCtl)));
+  CK(ctx->tally.ensure(sizeof(Tally)));
+  CK(ctx->roundctl.ensure(2 * sizeof(RoundCtl)));
   CK(ctx->roundargs.ensure(2 * sizeof(RoundArgs)));
   *R = RoundBuf{};
   R->compact = ctx->compact ? 1u : 0u;
@@ -718,7 +727,7 @@ int ensure_round(z80b_ctx* ctx, uint64_t cap, bool windows, RoundBuf* R) {
   R->pairs = ctx->pairs.as<PairRec>();
   R->pair_src = ctx->pair_src.as<uint32_t>();
   R->rejected = ctx->rejected.as<uint32_t>();
-  R->states = ctx->states.as<unsigned long long>();
+  R->states = ctx->tally.as<Tally>()->states;
   R->ctl = ctx->roundctl.as<RoundCtl>();
   if (windows) {
     CK(ctx->wlen.ensure(cap));
@@ -735,8 +744,23 @@ int ensure_round(z80b_ctx* ctx, uint64_t cap, bool windows, RoundBuf* R) {
   return Z80B_OK;
 }
 
-// Jobs of at most this many targets take the launch shapes for few lanes.
+// Jobs of at most this many targets take the launch shapes for few lanes and
+// send their host arrays in one copy.
 constexpr uint32_t kSmallJob = 4096;
+// Jobs of at most this many targets are queued as a whole: survivors and rules
+// have room for the most there can be (4,523 survivors, 2 rules a target), so
+// nothing is waited for before the rules are on the host.  A wait and the
+// reads behind it cost 10 to 20 us each, and there were six.
+constexpr uint32_t kQueuedJob = 1024;
+// Jobs of at most this many have room for every rule before they are counted.
+constexpr uint32_t kLazyRules = 1u << 20;
+
+// Waits for the stream and gives what the last report holds.
+int read_report(z80b_ctx* ctx, const Report** out) {
+  CK(cudaStreamSynchronize(ctx->stream));
+  *out = ctx->h_report.as<Report>();
+  return Z80B_OK;
+}
 
 // Plans the round's pairs, reads its counters and sweeps them, the grids by
 // the chunks there are (their blocks retire every few chunks).  h_args: the
@@ -775,8 +799,8 @@ void key_put(std::vector<unsigned char>& k, const V& v) {
 // depend on its size by value), so a captured graph is replayed for jobs of
 // any size until a buffer grows: a capture costs about 0.9 ms, which every
 // job of another size used to pay.
-int rounds_on_device(z80b_ctx* ctx, RoundGraph& g, const RoundArgs* a, const RoundArgs& h_args, bool pair, bool small,
-                     uint32_t* rounds, uint64_t* pairs) {
+// What the loop did is read with the run's report (rounds_done).
+int rounds_on_device(z80b_ctx* ctx, RoundGraph& g, const RoundArgs* a, const RoundArgs& h_args, bool pair, bool small) {
   cudaStream_t s = ctx->stream;
   const RoundBuf& R = h_args.R;
   const SweepArgs sweep = sweep_args(h_args);
@@ -843,14 +867,15 @@ int rounds_on_device(z80b_ctx* ctx, RoundGraph& g, const RoundArgs* a, const Rou
     g.key = key;
     trace("round loop captured (%s pass)", pair ? "length-2" : "length-1");
   }
-  // [rescan], build, plan, sweeps, resolve, end
-  const int per_iter = (pair ? 5 : 4) + 2 + (R.compact ? 1 : 0) + (R.wide ? 2 : 0);
   int ke = kbegin(ctx, 1);
   CK(cudaGraphLaunch(g.exec, s));
   kend(ctx, ke);
-  CKR(check_launch(ctx, "round loop"));
-  RoundCtl h{};
-  CKR(fetch(ctx, &h, R.ctl));
+  return check_launch(ctx, "round loop");
+}
+// Takes the counts of a device-driven loop from its RoundCtl.
+int rounds_done(z80b_ctx* ctx, const RoundCtl& h, const RoundBuf& R, bool pair, uint32_t* rounds, uint64_t* pairs) {
+  // [rescan], build, plan, sweeps, resolve, end
+  const int per_iter = (pair ? 5 : 4) + 2 + (R.compact ? 1 : 0) + (R.wide ? 2 : 0);
   if (h.overrun) return fail(ctx, Z80B_ETIMEOUT, "device round loop did not end within %u iterations", kMaxRoundIters);
   *rounds += h.rounds;
   *pairs += h.pairs;
@@ -1096,12 +1121,14 @@ int run_pipeline(z80b_ctx* ctx, const DevTargets& T, const PipeOpts& opts, z80b_
   CK(ctx->cnt_all.ensure(4ull * n));
   CK(ctx->base.ensure(4ull * n));
   CK(ctx->meta.ensure(sizeof(TargetMeta) * n));
-  CK(ctx->checks.ensure(8));
-  CK(ctx->checked.ensure(8));
-  CK(ctx->states.ensure(16));
-  CK(cudaMemsetAsync(ctx->checks.p, 0, 8, s));
-  CK(cudaMemsetAsync(ctx->checked.p, 0, 8, s));
-  CK(cudaMemsetAsync(ctx->states.p, 0, 16, s));
+  CK(ctx->tally.ensure(sizeof(Tally)));
+  CK(ctx->roundctl.ensure(2 * sizeof(RoundCtl)));
+  CK(ctx->h_report.ensure(sizeof(Report)));
+  ctx->rules_on_host = 0;
+  Tally* const tally = ctx->tally.as<Tally>();
+  Report* const report = ctx->h_report.as<Report>();
+  const Report* rep = nullptr;
+  CK(cudaMemsetAsync(tally, 0, sizeof(Tally), s));
 
   QCIndex qix{};
   bool use_ix = false;
@@ -1123,22 +1150,18 @@ int run_pipeline(z80b_ctx* ctx, const DevTargets& T, const PipeOpts& opts, z80b_
   q.cnt_m = ctx->cnt_m.as<uint32_t>();
   q.cnt_all = ctx->cnt_all.as<uint32_t>();
   q.meta = ctx->meta.as<TargetMeta>();
-  q.checks = ctx->checks.as<unsigned long long>();
+  q.checks = &tally->checks;
   if (use_ix && ctx->qc_single && P.n <= 65536) {
     // single pass: the count pass keeps the survivors of targets with few
     // (16-bit candidate indices)
     CK(ctx->qc_tmp.ensure(4ull * kQCSlots * n));
-    CK(ctx->qc_over.ensure(4));
-    CK(cudaMemsetAsync(ctx->qc_over.p, 0, 4, s));
     q.tmp = ctx->qc_tmp.as<uint32_t>();
-    q.over = ctx->qc_over.as<uint32_t>();
+    q.over = &tally->over;
   }
   if (use_ix) {
     CK(ctx->qc_longs.ensure(4ull * n));
-    CK(ctx->qc_nlong.ensure(4 * (kUpChunks + 1)));
-    CK(cudaMemsetAsync(ctx->qc_nlong.p, 0, 4 * (kUpChunks + 1), s));
     q.longs = ctx->qc_longs.as<uint32_t>();
-    q.nlong = ctx->qc_nlong.as<uint32_t>();
+    q.nlong = tally->nlong;
   }
   // the count over targets [lo, hi) (every per-target array offset by lo),
   // chunk number k
@@ -1183,18 +1206,25 @@ int run_pipeline(z80b_ctx* ctx, const DevTargets& T, const PipeOpts& opts, z80b_
   }
   kend(ctx, kq);
   CKR(scan(ctx, ctx->cnt_all.as<uint32_t>(), ctx->base.as<uint32_t>(), n));
-  uint32_t last[4] = {0, 0, 0, 0};
-  CK(cudaMemcpyAsync(&last[0], ctx->base.as<uint32_t>() + (n - 1), 4, cudaMemcpyDeviceToHost, s));
-  CK(cudaMemcpyAsync(&last[1], ctx->cnt_f.as<uint32_t>() + (n - 1), 4, cudaMemcpyDeviceToHost, s));
-  CK(cudaMemcpyAsync(&last[2], ctx->cnt_m.as<uint32_t>() + (n - 1), 4, cudaMemcpyDeviceToHost, s));
-  if (q.over) CK(cudaMemcpyAsync(&last[3], q.over, 4, cudaMemcpyDeviceToHost, s));
-  CK(cudaStreamSynchronize(s));
-  const uint64_t nsurv = uint64_t(last[0]) + last[1] + last[2];
-  trace("qc count done: %llu survivors", (unsigned long long)nsurv);
+  q.base = ctx->base.as<uint32_t>();
+  // rounds on the device (one graph) unless the caller takes answers round by
+  // round (streaming callbacks) or each target is a job of its own (its
+  // address would be another graph)
+  const bool dev_rounds = mode == Z80B_MODE_FIRST && ctx->graph_rounds && !opts.rep && !opts.plain;
+  const bool queued = dev_rounds && n <= kQueuedJob && use_ix;
+  uint64_t nsurv = 0;
+  if (queued) {
+    nsurv = uint64_t(n) * pool->qvalid;  // at most; the count comes with the report
+  } else {
+    launch_report(tally, q, n, nullptr, nullptr, 0, nullptr, report, s);
+    CKR(check_launch(ctx, "report"));
+    CKR(read_report(ctx, &rep));
+    nsurv = rep->nsurv;
+    trace("qc count done: %llu survivors", (unsigned long long)nsurv);
+  }
   if (nsurv > 0xFFFFFFF0ull) return fail(ctx, Z80B_ECAPACITY, "too many QuickCheck survivors (%llu)", (unsigned long long)nsurv);
   CK(ctx->surv.ensure(4ull * std::max<uint64_t>(nsurv, 1)));
   CK(ctx->sdiff.ensure(2ull * std::max<uint64_t>(nsurv, 1)));
-  q.base = ctx->base.as<uint32_t>();
   q.surv = ctx->surv.as<uint32_t>();
   q.sdiff = ctx->sdiff.as<uint16_t>();
   if (nsurv && q.tmp) {
@@ -1203,7 +1233,7 @@ int run_pipeline(z80b_ctx* ctx, const DevTargets& T, const PipeOpts& opts, z80b_
     kend(ctx, kc);
     CKR(check_launch(ctx, "qc_compact"));
   }
-  if (nsurv && (!q.tmp || last[3])) {
+  if (nsurv && (!q.tmp || queued || rep->tally.over)) {
     // every target (two passes), or those with more survivors than the
     // count pass kept
     int kc = kbegin(ctx, 0);
@@ -1227,17 +1257,12 @@ int run_pipeline(z80b_ctx* ctx, const DevTargets& T, const PipeOpts& opts, z80b_
     CK(ctx->win.ensure(8ull * n));
     CK(ctx->windiff.ensure(4ull * n));
     CK(ctx->spec.ensure(2ull * n));
-    CK(cudaMemsetAsync(ctx->spec.p, 0, 2ull * n, s));
-    CK(cudaMemsetAsync(ctx->next.p, 0, 8ull * n, s));
-    CK(cudaMemsetAsync(ctx->win.p, 0xFF, 8ull * n, s));
     Lanes L{ctx->next.as<uint32_t>(), ctx->win.as<uint32_t>(), ctx->windiff.as<uint16_t>(), ctx->spec.as<uint8_t>()};
+    launch_lanes_init(L, n, s);
+    CKR(check_launch(ctx, "lanes_init"));
     // pair slots per round: every lane once, and room for survivor windows
     CKR(ensure_round(ctx, std::max<uint64_t>(2ull * n, std::min<uint64_t>(128ull * n, 1ull << 20)), true, &R));
     RoundArgs* const args = ctx->roundargs.as<RoundArgs>();
-    // rounds on the device (one graph) unless the caller takes answers
-    // round by round (streaming callbacks) or each target is a job of its
-    // own (its address would be another graph)
-    const bool dev_rounds = ctx->graph_rounds && !opts.rep && !opts.plain;
     const bool small = n <= kSmallJob;
     RoundArgs ra{};
     ra.T = T;
@@ -1251,7 +1276,7 @@ int run_pipeline(z80b_ctx* ctx, const DevTargets& T, const PipeOpts& opts, z80b_
       launch_round_args(ra, args, s);
       CKR(check_launch(ctx, "round_args"));
       if (dev_rounds)
-        CKR(rounds_on_device(ctx, ctx->rg1, args, ra, false, small, &rounds, &exh_pairs));
+        CKR(rounds_on_device(ctx, ctx->rg[0][small], args, ra, false, small));
       else
         CKR(rounds_on_host(ctx, args, ra, false, small, &rounds, &exh_pairs, [&] {
           return opts.rep ? opts.rep->update(ctx, n, L, Lanes{}, opts.max_cand, false, false) : Z80B_OK;
@@ -1288,7 +1313,7 @@ int run_pipeline(z80b_ctx* ctx, const DevTargets& T, const PipeOpts& opts, z80b_
       ps.sdiff = ctx->sdiff2.as<uint16_t>();
       ps.scan = ctx->scan2.as<uint32_t>();
       ps.eligible = PS.eligible_dev.as<unsigned long long>();
-      ps.checks = ctx->checks.as<unsigned long long>();
+      ps.checks = &tally->checks;
       launch_pair_lanes_init(T, L, q, L2, ps, s);
       CKR(check_launch(ctx, "pair_lanes_init"));
       ra.P = P2;
@@ -1296,6 +1321,7 @@ int run_pipeline(z80b_ctx* ctx, const DevTargets& T, const PipeOpts& opts, z80b_
       ra.ps = ps;
       ra.sdiff = ps.sdiff;
       ra.max_spec = kMaxSpec2;
+      ra.R.ctl = R.ctl + 1;
       launch_round_args(ra, args + 1, s);
       CKR(check_launch(ctx, "round_args"));
       int kq2 = kbegin(ctx, 0);
@@ -1303,7 +1329,7 @@ int run_pipeline(z80b_ctx* ctx, const DevTargets& T, const PipeOpts& opts, z80b_
       kend(ctx, kq2);
       CKR(check_launch(ctx, "pair_scan"));
       if (dev_rounds)
-        CKR(rounds_on_device(ctx, ctx->rg2, args + 1, ra, true, small, &rounds, &exh_pairs));
+        CKR(rounds_on_device(ctx, ctx->rg[1][small], args + 1, ra, true, small));
       else
         CKR(rounds_on_host(ctx, args + 1, ra, true, small, &rounds, &exh_pairs, [&] {
           return opts.rep ? opts.rep->update(ctx, n, L, L2, opts.max_cand, true, false) : Z80B_OK;
@@ -1312,18 +1338,36 @@ int run_pipeline(z80b_ctx* ctx, const DevTargets& T, const PipeOpts& opts, z80b_
     if (opts.rep) CKR(opts.rep->update(ctx, n, L, L2, opts.max_cand, opts.max_cand >= 2, true));
     CK(ctx->rcnt.ensure(4ull * n));
     CK(ctx->rbase.ensure(4ull * n));
-    launch_rule_count_first(L, L2, n, ctx->rcnt.as<uint32_t>(), T, ctx->checked.as<unsigned long long>(),
+    launch_rule_count_first(L, L2, n, ctx->rcnt.as<uint32_t>(), T, &tally->checked,
                             uint32_t(pool8().size()), pool2_enum, s);
     CKR(check_launch(ctx, "rule_count"));
     CKR(scan(ctx, ctx->rcnt.as<uint32_t>(), ctx->rbase.as<uint32_t>(), n));
-    uint32_t lb = 0, lc = 0;
-    CK(cudaMemcpyAsync(&lb, ctx->rbase.as<uint32_t>() + (n - 1), 4, cudaMemcpyDeviceToHost, s));
-    CK(cudaMemcpyAsync(&lc, ctx->rcnt.as<uint32_t>() + (n - 1), 4, cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamSynchronize(s));
-    *nr = uint64_t(lb) + lc;
-    CK(ctx->rules.ensure(sizeof(DevRule) * std::max<uint64_t>(*nr, 1)));
+    const RoundCtl* const ctls = ctx->roundctl.as<RoundCtl>();
+    const bool lazy = dev_rounds && n <= kLazyRules;
+    launch_report(tally, q, n, ctx->rbase.as<uint32_t>(), ctx->rcnt.as<uint32_t>(), n, ctls, report, s);
+    CKR(check_launch(ctx, "report"));
+    if (!lazy) {
+      CKR(read_report(ctx, &rep));
+      *nr = rep->nrules;
+    }
+    CK(ctx->rules.ensure(sizeof(DevRule) * std::max<uint64_t>(lazy ? 2ull * n : *nr, 1)));
     launch_rule_write_first(L, L2, n, ctx->rbase.as<uint32_t>(), ctx->rules.as<DevRule>(), s);
     CKR(check_launch(ctx, "rule_write"));
+    if (queued) {
+      CK(ctx->h_rules.ensure(sizeof(DevRule) * 2ull * kQueuedJob));
+      CK(cudaMemcpyAsync(ctx->h_rules.p, ctx->rules.p, sizeof(DevRule) * 2ull * n, cudaMemcpyDeviceToHost, s));
+    }
+    tall.stop();
+    CKR(read_report(ctx, &rep));
+    *nr = rep->nrules;
+    if (queued) {
+      nsurv = rep->nsurv;
+      ctx->rules_on_host = *nr;
+    }
+    if (dev_rounds) {
+      if (nsurv || queued) CKR(rounds_done(ctx, rep->pass[0], R, false, &rounds, &exh_pairs));
+      if (opts.max_cand >= 2) CKR(rounds_done(ctx, rep->pass[1], R, true, &rounds, &exh_pairs));
+    }
   } else {
     // all-hits: MidCheck on every survivor, one ExhaustiveCheck pass
     const uint32_t S = uint32_t(nsurv);
@@ -1370,25 +1414,24 @@ int run_pipeline(z80b_ctx* ctx, const DevTargets& T, const PipeOpts& opts, z80b_
         CKR(check_launch(ctx, "rule_count_all"));
       }
       CKR(scan(ctx, ctx->flag.as<uint32_t>(), ctx->rbase.as<uint32_t>(), S));
-      uint32_t lb = 0, lc = 0;
-      CK(cudaMemcpyAsync(&lb, ctx->rbase.as<uint32_t>() + (S - 1), 4, cudaMemcpyDeviceToHost, s));
-      CK(cudaMemcpyAsync(&lc, ctx->flag.as<uint32_t>() + (S - 1), 4, cudaMemcpyDeviceToHost, s));
-      CK(cudaStreamSynchronize(s));
-      *nr = uint64_t(lb) + lc;
+      launch_report(tally, q, n, ctx->rbase.as<uint32_t>(), ctx->flag.as<uint32_t>(), S, nullptr, report, s);
+      CKR(check_launch(ctx, "report"));
+      CKR(read_report(ctx, &rep));
+      *nr = rep->nrules;
       CK(ctx->rules.ensure(sizeof(DevRule) * std::max<uint64_t>(*nr, 1)));
       launch_rule_write_all(ctx->flag.as<uint32_t>(), ctx->rbase.as<uint32_t>(), S, q.surv, q.sdiff,
                             ctx->surv_target.as<uint32_t>(), ctx->rules.as<DevRule>(), s);
       CKR(check_launch(ctx, "rule_write_all"));
     }
   }
-  tall.stop();
-  CK(cudaStreamSynchronize(s));
+  if (mode == Z80B_MODE_ALL) {
+    tall.stop();
+    CKR(read_report(ctx, &rep));
+  }
   trace("pipeline done: %llu rules, %u rounds", (unsigned long long)*nr, rounds);
   if (st) {
-    unsigned long long checks = 0, checked = 0, states[2] = {0, 0};
-    CKR(fetch(ctx, &checks, ctx->checks.as<unsigned long long>()));
-    CKR(fetch(ctx, &checked, ctx->checked.as<unsigned long long>()));
-    CKR(fetch(ctx, states, ctx->states.as<unsigned long long>(), 2));
+    const unsigned long long checks = rep->tally.checks, checked = rep->tally.checked;
+    const unsigned long long* states = rep->tally.states;
     st->targets += n;
     st->checks += checks;
     st->checked_ref += (mode == Z80B_MODE_FIRST) ? checked : 0;
@@ -1547,8 +1590,36 @@ int upload_targets(z80b_ctx* ctx, Staged& S, const z80b_job* job, DevTargets* T,
       if (dr || df) S.opts.dreg_masks |= 1ull << dr;
     }
   cudaStream_t s = ctx->stream;
-  CK(S.d_targets.ensure(4ull * std::max<size_t>(words, 1)));
   S.up_chunks = 0;
+  if (!keep_host && n <= kSmallJob) {
+    // one copy from page-locked memory, to fixed places (a captured round
+    // graph holds the addresses)
+    const size_t head = 3 * size_t(kSmallJob), bytes = head + 4 * words;
+    CK(S.d_small.ensure(std::max<size_t>(bytes, head + 16 * size_t(kSmallJob))));
+    CK(ctx->h_up.ensure(std::max<size_t>(bytes, head + 16 * size_t(kSmallJob))));
+    uint8_t* const h = ctx->h_up.as<uint8_t>();
+    uint8_t* const d = S.d_small.as<uint8_t>();
+    if (n) {
+      if (job->target_lens) std::memcpy(h, job->target_lens, n);
+      if (job->dead_flags) std::memcpy(h + kSmallJob, job->dead_flags, n);
+      if (job->dead_regs) std::memcpy(h + 2 * kSmallJob, job->dead_regs, n);
+      std::memcpy(h + head, job->targets, 4 * words);
+      CK(cudaMemcpyAsync(d, h, bytes, cudaMemcpyHostToDevice, s));
+    }
+    *T = DevTargets{};
+    T->insn = reinterpret_cast<const uint32_t*>(d + head);
+    T->n = n;
+    T->stride = job->target_stride;
+    T->fixed_len = job->target_len;
+    T->global_dead = job->global_dead_flags;
+    if (job->target_lens) T->len = d;
+    if (job->dead_flags) T->dead = d + kSmallJob;
+    if (job->dead_regs) T->dead_regs = d + 2 * kSmallJob;
+    S.T = *T;
+    S.valid = true;
+    return Z80B_OK;
+  }
+  CK(S.d_targets.ensure(4ull * std::max<size_t>(words, 1)));
   if (!keep_host && n >= kUpChunkMin) {
     // in chunks on the copy stream, so that the QuickCheck count of the
     // first chunks runs while the rest are copied
@@ -1592,6 +1663,7 @@ int upload_targets(z80b_ctx* ctx, Staged& S, const z80b_job* job, DevTargets* T,
     CK(cudaMemcpyAsync(S.d_dregs.p, S.dregs.data(), n, cudaMemcpyHostToDevice, s));
     T->dead_regs = S.d_dregs.as<uint8_t>();
   }
+  S.T = *T;
   S.valid = true;
   return Z80B_OK;
 }
@@ -1601,24 +1673,13 @@ int upload_targets(z80b_ctx* ctx, Staged& S, const z80b_job* job, DevTargets* T,
 int rules_to_host(z80b_ctx* ctx, uint64_t nr, const DevRule** out) {
   *out = nullptr;
   if (!nr) return Z80B_OK;
-  CK(ctx->h_rules.ensure(sizeof(DevRule) * nr));
-  CK(cudaMemcpyAsync(ctx->h_rules.p, ctx->rules.p, sizeof(DevRule) * nr, cudaMemcpyDeviceToHost, ctx->stream));
-  CK(cudaStreamSynchronize(ctx->stream));
+  if (ctx->rules_on_host < nr) {
+    CK(ctx->h_rules.ensure(sizeof(DevRule) * nr));
+    CK(cudaMemcpyAsync(ctx->h_rules.p, ctx->rules.p, sizeof(DevRule) * nr, cudaMemcpyDeviceToHost, ctx->stream));
+    CK(cudaStreamSynchronize(ctx->stream));
+  }
   *out = ctx->h_rules.as<DevRule>();
   return Z80B_OK;
-}
-
-DevTargets staged_targets(Staged& S) {
-  DevTargets T{};
-  T.insn = S.d_targets.as<uint32_t>();
-  T.n = S.job.n_targets;
-  T.stride = S.job.target_stride;
-  T.fixed_len = S.job.target_len;
-  T.global_dead = S.job.global_dead_flags;
-  if (!S.lens.empty()) T.len = S.d_lens.as<uint8_t>();
-  if (!S.dead.empty()) T.dead = S.d_dead.as<uint8_t>();
-  if (!S.dregs.empty()) T.dead_regs = S.d_dregs.as<uint8_t>();
-  return T;
 }
 
 // Runs the staged job (batched or plain path) and leaves rules on the device
@@ -1626,7 +1687,7 @@ DevTargets staged_targets(Staged& S) {
 int run_staged(z80b_ctx* ctx, z80b_stats* st, uint64_t* nr, std::vector<z80b_rule>* host_rules,
                const uint32_t* host_targets) {
   Staged& S = ctx->staged;
-  DevTargets T = staged_targets(S);
+  const DevTargets T = S.T;
   const z80b_job& job = S.job;
   if (job.path == Z80B_PATH_BATCHED) return run_pipeline(ctx, T, S.opts, st, nr);
   // plain: one target per pipeline launch, synchronizing in between

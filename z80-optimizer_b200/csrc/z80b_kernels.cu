@@ -1747,6 +1747,54 @@ __global__ void k_round_args(RoundArgs a, RoundArgs* __restrict__ dst) {
 }
 static_assert(sizeof(RoundArgs) % 4 == 0 && sizeof(RoundCtl) % 4 == 0, "copied by words");
 
+// Lane i copies word i of the counters and the passes' controls; lane 0 adds
+// the totals.
+__global__ void k_report(const Tally* __restrict__ t, QCOut q, uint32_t n, const uint32_t* __restrict__ rbase,
+                         const uint32_t* __restrict__ rcnt, uint32_t nr, const RoundCtl* __restrict__ ctl, Report* out) {
+  static_assert(sizeof(Tally) % 4 == 0 && sizeof(RoundCtl) % 4 == 0, "copied by words");
+  for (uint32_t i = threadIdx.x; i < sizeof(Tally) / 4; i += blockDim.x)
+    reinterpret_cast<uint32_t*>(&out->tally)[i] = reinterpret_cast<const uint32_t*>(t)[i];
+  if (ctl)
+    for (uint32_t i = threadIdx.x; i < 2 * sizeof(RoundCtl) / 4; i += blockDim.x)
+      reinterpret_cast<uint32_t*>(out->pass)[i] = reinterpret_cast<const uint32_t*>(ctl)[i];
+  if (threadIdx.x != 0) return;
+  out->nsurv = (unsigned long long)q.base[n - 1] + q.cnt_f[n - 1] + q.cnt_m[n - 1];
+  out->nrules = nr ? (unsigned long long)rbase[nr - 1] + rcnt[nr - 1] : 0ull;
+}
+__global__ void k_lanes_init(Lanes L, uint32_t lanes) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= lanes) return;
+  L.next[i] = 0;
+  L.win[i] = kNone;
+  L.spec[i] = 0;
+}
+// Thread i takes the i-th run of the items; the runs' sums are scanned by
+// warps, then the warps' totals by the first.
+__global__ void __launch_bounds__(1024) k_scan_small(const uint32_t* __restrict__ in, uint32_t* __restrict__ out,
+                                                     uint32_t n) {
+  __shared__ uint32_t totals[32];
+  const uint32_t per = (n + blockDim.x - 1) / blockDim.x;
+  const uint32_t lo = min(threadIdx.x * per, n), hi = min(lo + per, n);
+  uint32_t sum = 0;
+  for (uint32_t i = lo; i < hi; i++) sum += in[i];
+  uint32_t x = sum;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(kFull, x, o);
+    if (lane_id() >= unsigned(o)) x += y;
+  }
+  if (lane_id() == 31) totals[threadIdx.x >> 5] = x;
+  __syncthreads();
+  uint32_t before = 0;
+  for (uint32_t w = 0; w < (threadIdx.x >> 5); w++) before += totals[w];
+  uint32_t at = before + x - sum;
+  for (uint32_t i = lo; i < hi; i++) {
+    const uint32_t v = in[i];  // in may be out
+    out[i] = at;
+    at += v;
+  }
+}
+
 __global__ void k_midcheck(DevTargets T, DevPool P, const uint32_t* __restrict__ surv,
                            const uint32_t* __restrict__ surv_target, uint32_t nsurv, uint8_t* __restrict__ pass) {
   const unsigned lane = lane_id();
@@ -2951,6 +2999,16 @@ int launch_exhaustive_dev(const SweepArgs& a, bool compact, bool wide, int k, co
   return n + 2;
 }
 
+void launch_report(const Tally* t, const QCOut& q, uint32_t n, const uint32_t* rbase, const uint32_t* rcnt, uint32_t nr,
+                   const RoundCtl* ctl, Report* out, cudaStream_t s) {
+  k_report<<<1, 64, 0, s>>>(t, q, n, rbase, rcnt, nr, ctl, out);
+}
+void launch_lanes_init(const Lanes& L, uint32_t n, cudaStream_t s) {
+  if (n) k_lanes_init<<<grid_for(2 * n, 256), 256, 0, s>>>(L, 2 * n);
+}
+void launch_scan_small(const uint32_t* in, uint32_t* out, uint32_t n, cudaStream_t s) {
+  if (n) k_scan_small<<<1, n > 1024 ? 1024 : (n + 31u) / 32u * 32u, 0, s>>>(in, out, n);
+}
 void launch_midcheck(const DevTargets& T, const DevPool& P, const uint32_t* surv,
                      const uint32_t* surv_target, uint32_t nsurv, uint8_t* pass, cudaStream_t s) {
   if (!nsurv) return;

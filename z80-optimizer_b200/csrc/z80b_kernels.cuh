@@ -209,6 +209,31 @@ void launch_qc_entries(const DevPool& P, uint32_t w2mask, const unsigned long lo
                        uint32_t* flags, cudaStream_t s);
 void launch_qc_bucket(const DevTargets& T, const DevPool& P, const QCConfig& cfg, const QCIndex& ix,
                       const QCOut& o, bool collect, cudaStream_t s);
+// Counters of one pipeline run on the device, cleared before it.
+constexpr int kMaxCountParts = 5;  // chunks of targets in a count pass, and the collect pass
+struct Tally {
+  unsigned long long checks, checked;    // QuickCheck units; the reference's 'checked' counter
+  unsigned long long states[2];          // RoundBuf::states
+  uint32_t over;                         // QCOut::over
+  uint32_t nlong[kMaxCountParts];        // QCOut::nlong
+};
+// What the host reads of a run, written to page-locked host memory by one
+// small kernel where several copies would each cost a few microseconds.
+struct Report {
+  Tally tally;
+  unsigned long long nsurv, nrules;      // totals of the survivor and the rule prefix sums
+  RoundCtl pass[2];                      // the two passes' rounds
+};
+// survivors: base / cnt_f / cnt_m of q over n targets; rules: rbase / rcnt
+// over nr items (nr 0: none yet); ctl: RoundCtl[2] or null.
+void launch_report(const Tally* t, const QCOut& q, uint32_t n, const uint32_t* rbase, const uint32_t* rcnt, uint32_t nr,
+                   const RoundCtl* ctl, Report* out, cudaStream_t s);
+// The lanes of n targets before their first round.
+void launch_lanes_init(const Lanes& L, uint32_t n, cudaStream_t s);
+// Exclusive sum of n <= kScanSmall items in one block.
+constexpr uint32_t kScanSmall = 8192;
+void launch_scan_small(const uint32_t* in, uint32_t* out, uint32_t n, cudaStream_t s);
+
 // Everything the kernels of a round need, in device memory: a captured round
 // graph reads the job at hand from here, so a job of another size replays the
 // same graph (the sweeps' own share: SweepArgs).
