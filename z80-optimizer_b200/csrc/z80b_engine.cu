@@ -213,7 +213,8 @@ struct z80b_ctx {
   HBuf h_report;              // Report
   HBuf h_up;                  // small jobs: the host arrays of a search, one copy
   DBuf cub_tmp;
-  DBuf hits, nhits, fpq;
+  DBuf hits, nhits;           // fingerprint queries: all hits, FpCounters
+  HBuf h_fp;                  // FpAnswer
   DBuf v_tgt, v_cand, v_tl, v_cl, v_dead, v_out, v_fd, v_in, v_outs;
   DBuf mul_best, mul_stats;   // constant-multiply search: best key per length and K, counters
   DBuf mul_hash[mul::kMaxLen], mul_key[mul::kMaxLen];  // prefixes with distinct states per length
@@ -1873,26 +1874,29 @@ int z80b_quickcheck(z80b_ctx* ctx, const uint8_t* fp80, uint32_t dead_flags, uin
   if (!ctx->loaded.loaded) return fail(ctx, Z80B_ESTATE, "z80b_load_candidates has not been called");
   cudaSetDevice(ctx->device);
   // fingerprint bytes -> packed words (F byte masked on the device)
-  uint32_t w[24];
+  FpQuery fq;
   for (int v = 0; v < 8; v++) {
     const uint8_t* p = fp80 + v * 10;
-    w[3 * v] = uint32_t(p[0]) | uint32_t(p[1]) << 8 | uint32_t(p[2]) << 16 | uint32_t(p[3]) << 24;
-    w[3 * v + 1] = uint32_t(p[4]) | uint32_t(p[5]) << 8 | uint32_t(p[6]) << 16 | uint32_t(p[7]) << 24;
-    w[3 * v + 2] = uint32_t(p[8]) << 8 | uint32_t(p[9]);
+    fq.w[3 * v] = uint32_t(p[0]) | uint32_t(p[1]) << 8 | uint32_t(p[2]) << 16 | uint32_t(p[3]) << 24;
+    fq.w[3 * v + 1] = uint32_t(p[4]) | uint32_t(p[5]) << 8 | uint32_t(p[6]) << 16 | uint32_t(p[7]) << 24;
+    fq.w[3 * v + 2] = uint32_t(p[8]) << 8 | uint32_t(p[9]);
   }
-  const uint32_t dev_cap = ctx->loaded.n;
-  CK(ctx->fpq.ensure(sizeof w));
-  CK(ctx->hits.ensure(4ull * std::max<uint32_t>(dev_cap, 1)));
-  CK(ctx->nhits.ensure(4));
-  CK(cudaMemcpyAsync(ctx->fpq.p, w, sizeof w, cudaMemcpyHostToDevice, ctx->stream));
-  CK(cudaMemsetAsync(ctx->nhits.p, 0, 4, ctx->stream));
-  launch_fp_query(ctx->loaded.dev, ctx->fpq.as<uint32_t>(), dead_flags & 0xFFu, ctx->hits.as<uint32_t>(),
-                  ctx->nhits.as<uint32_t>(), dev_cap, ctx->stream);
+  cudaStream_t s = ctx->stream;
+  CK(ctx->hits.ensure(4ull * std::max<uint32_t>(ctx->loaded.n, 1)));
+  CK(ctx->h_fp.ensure(sizeof(FpAnswer)));
+  if (!ctx->nhits.p) {
+    CK(ctx->nhits.ensure(sizeof(FpCounters)));
+    CK(cudaMemsetAsync(ctx->nhits.p, 0, sizeof(FpCounters), s));
+  }
+  FpAnswer* const answer = ctx->h_fp.as<FpAnswer>();
+  launch_fp_query(ctx->loaded.dev, fq, dead_flags & 0xFFu, ctx->hits.as<uint32_t>(), ctx->nhits.as<FpCounters>(),
+                  answer, s);
   CKR(check_launch(ctx, "fp_query"));
-  uint32_t nh = 0;
-  CKR(fetch(ctx, &nh, ctx->nhits.as<uint32_t>()));
+  CK(cudaStreamSynchronize(s));
+  const uint32_t nh = answer->count;
   std::vector<uint32_t> h(nh);
-  if (nh) CKR(fetch(ctx, h.data(), ctx->hits.as<uint32_t>(), nh));
+  if (nh <= kFpHere) std::copy(answer->hits, answer->hits + nh, h.begin());
+  else CKR(fetch(ctx, h.data(), ctx->hits.as<uint32_t>(), nh));
   std::sort(h.begin(), h.end());
   *n_hits = nh;
   for (uint32_t i = 0; i < nh && i < cap; i++) hits[i] = h[i];

@@ -195,8 +195,23 @@ void launch_exec(const uint32_t* in_states, const uint32_t* seqs, const uint8_t*
 void launch_fingerprints(const uint32_t* seqs, uint32_t n, uint32_t len, uint8_t* out, cudaStream_t s);
 void launch_qc_scan(const DevTargets& T, const DevPool& P, const QCConfig& cfg, const QCOut& o,
                     bool collect, cudaStream_t s);
-void launch_fp_query(const DevPool& P, const uint32_t* fp3x8, uint32_t dead, uint32_t* hits,
-                     uint32_t* nhits, uint32_t cap, cudaStream_t s);
+// One fingerprint query: packed words by vector; the counters a query leaves
+// cleared; what the host reads (page-locked memory).
+struct FpQuery {
+  uint32_t w[24];
+};
+struct FpCounters {
+  uint32_t hits, done;
+};
+constexpr uint32_t kFpHere = 2046;
+struct FpAnswer {
+  uint32_t count, pad;
+  uint32_t hits[kFpHere];  // the first of them, in no order
+};
+// Indices of the candidates with the fingerprint, flags in `dead` aside: all
+// of them in hits (P.n slots), their number and the first kFpHere in answer.
+void launch_fp_query(const DevPool& P, const FpQuery& fp, uint32_t dead, uint32_t* hits, FpCounters* ctr,
+                     FpAnswer* answer, cudaStream_t s);
 // Sort keys of masks [m0, m0 + nm): keys[i * P.n + c] for mask m0 + i.
 void launch_qc_keys(const DevPool& P, uint32_t w2mask, uint32_t m0, uint32_t nm, unsigned long long* keys,
                     cudaStream_t s);
