@@ -1863,7 +1863,16 @@ __global__ void k_rule_count_first(Lanes L, Lanes L2, uint32_t n, uint32_t* __re
   for (int off = 16; off; off >>= 1) ch += __shfl_down_sync(kFull, ch, off);
   if (lane_id() == 0 && ch) atomicAdd(checked, ch);
 }
+// What candidate c saves on a target.
+__device__ __forceinline__ void rule_savings(DevRule& r, const TargetMeta& m, const DevPool& P, uint32_t c) {
+  int ts = 0;
+  const uint32_t cl = pool_len(P, c);
+  for (uint32_t i = 0; i < cl; i++) ts += g_ops[P.insn[(size_t)c * P.stride + i] & 0xFFFFu].tstates;
+  r.bytes_saved = int16_t(int(m.bytes) - int(P.size[c]));
+  r.cycles_saved = int16_t(int(m.tstates) - ts);
+}
 __global__ void k_rule_write_first(Lanes L, Lanes L2, uint32_t n, const uint32_t* __restrict__ base,
+                                   const TargetMeta* __restrict__ meta, DevPool P, DevPool P2,
                                    DevRule* __restrict__ out) {
   uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n) return;
@@ -1879,6 +1888,7 @@ __global__ void k_rule_write_first(Lanes L, Lanes L2, uint32_t n, const uint32_t
     r.diff = kind ? (w1 != kNone ? L.windiff[idx] : L2.windiff[idx]) : uint16_t(0);
     r.kind = uint8_t(kind);
     r.clen = w1 != kNone ? 1 : 2;
+    rule_savings(r, meta[t], w1 != kNone ? P : P2, r.cand);
     out[b++] = r;
   }
 }
@@ -1893,7 +1903,7 @@ __global__ void k_rule_count_all(RoundBuf R, uint32_t npairs, uint32_t* __restri
 __global__ void k_rule_write_all(const uint32_t* __restrict__ flag, const uint32_t* __restrict__ base,
                                  uint32_t nsurv, const uint32_t* __restrict__ surv,
                                  const uint16_t* __restrict__ sdiff, const uint32_t* __restrict__ surv_target,
-                                 DevRule* __restrict__ out) {
+                                 const TargetMeta* __restrict__ meta, DevPool P, DevRule* __restrict__ out) {
   uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nsurv || !flag[i]) return;
   DevRule r;
@@ -1902,6 +1912,7 @@ __global__ void k_rule_write_all(const uint32_t* __restrict__ flag, const uint32
   r.diff = sdiff[i];
   r.kind = 2;
   r.clen = 1;
+  rule_savings(r, meta[r.target], P, r.cand);
   out[base[i]] = r;
 }
 
@@ -2366,6 +2377,13 @@ __global__ void __launch_bounds__(kBlock, 4) k_qc_bucket(DevTargets T, DevPool P
     for (uint32_t i = 0; i < steps; i++) {
       if (i < tl) {
         const uint32_t w = prog[i];
+        if ((w & 0xFFFFu) >= uint32_t(kNumOps)) {
+          // (only where the host leaves the check to this kernel) reported,
+          // and nothing more of this target
+          if (cfg.bad) atomicMax(cfg.bad, ~(cfg.first + t));
+          work = false;
+          continue;
+        }
         const OpInfo oi = g_ops[w & 0xFFFFu];
         size += oi.size;
         tstates += oi.tstates;
@@ -3043,20 +3061,20 @@ void launch_rule_count_first(const Lanes& L, const Lanes& L2, uint32_t n, uint32
   if (!n) return;
   k_rule_count_first<<<grid_for(n, 256), 256, 0, s>>>(L, L2, n, cnt, T, checked, pool_enum, pool2_enum);
 }
-void launch_rule_write_first(const Lanes& L, const Lanes& L2, uint32_t n, const uint32_t* base, DevRule* out,
-                             cudaStream_t s) {
+void launch_rule_write_first(const Lanes& L, const Lanes& L2, uint32_t n, const uint32_t* base, const TargetMeta* meta,
+                             const DevPool& P, const DevPool& P2, DevRule* out, cudaStream_t s) {
   if (!n) return;
-  k_rule_write_first<<<grid_for(n, 256), 256, 0, s>>>(L, L2, n, base, out);
+  k_rule_write_first<<<grid_for(n, 256), 256, 0, s>>>(L, L2, n, base, meta, P, P2, out);
 }
 void launch_rule_count_all(const RoundBuf& R, uint32_t npairs, uint32_t* flag, cudaStream_t s) {
   if (!npairs) return;
   k_rule_count_all<<<grid_for(npairs, 256), 256, 0, s>>>(R, npairs, flag);
 }
-void launch_rule_write_all(const uint32_t* flag, const uint32_t* base, uint32_t nsurv,
-                           const uint32_t* surv, const uint16_t* sdiff, const uint32_t* surv_target,
+void launch_rule_write_all(const uint32_t* flag, const uint32_t* base, uint32_t nsurv, const uint32_t* surv,
+                           const uint16_t* sdiff, const uint32_t* surv_target, const TargetMeta* meta, const DevPool& P,
                            DevRule* out, cudaStream_t s) {
   if (!nsurv) return;
-  k_rule_write_all<<<grid_for(nsurv, 256), 256, 0, s>>>(flag, base, nsurv, surv, sdiff, surv_target, out);
+  k_rule_write_all<<<grid_for(nsurv, 256), 256, 0, s>>>(flag, base, nsurv, surv, sdiff, surv_target, meta, P, out);
 }
 void launch_verify_small(const uint32_t* tgt, const uint8_t* tlens, const uint32_t* cand,
                          const uint8_t* clens, uint32_t stride, uint32_t n, const uint8_t* dead,

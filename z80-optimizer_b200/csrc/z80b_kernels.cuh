@@ -37,6 +37,9 @@ struct QCConfig {
   uint32_t w2mask;   // 0xFFFFFFFF: compare SP and M; 0x0000FFFF: fingerprint (SP only)
   int all_hits;      // 1: pkg/gpu semantics (one list: masked-QC passes)
   int use_smem;      // pool QC0 staged in shared memory
+  uint32_t* bad;     // bucket index: the programs' opcodes are checked here, the least bad target
+                     // goes to *bad (null: the host has checked them)
+  uint32_t first;    // index of the launch's first target
 };
 
 // QuickCheck index of a candidate pool: per dead-register mask in use the
@@ -177,6 +180,7 @@ struct DevRule {
   uint16_t diff;   // flag diff | reg diff << 8
   uint8_t kind;    // 0 full, 1 masked, 2 all-hits
   uint8_t clen;    // candidate length: 1 (pool index) or 2 (pair-pool index)
+  int16_t bytes_saved, cycles_saved;
 };
 
 // Moves the survivors the count pass kept (targets with 1..kQCSlots) to
@@ -231,6 +235,7 @@ struct Tally {
   unsigned long long states[2];          // RoundBuf::states
   uint32_t over;                         // QCOut::over
   uint32_t nlong[kMaxCountParts];        // QCOut::nlong
+  uint32_t bad, pad;                     // QCConfig::bad, complemented: 0 none
 };
 // What the host reads of a run, written to page-locked host memory by one
 // small kernel where several copies would each cost a few microseconds.
@@ -328,10 +333,11 @@ void launch_surv_targets(const QCOut& q, uint32_t n, uint32_t* surv_target, cuda
 void launch_rule_count_first(const Lanes& L, const Lanes& L2, uint32_t n, uint32_t* cnt, const DevTargets& T,
                              unsigned long long* checked, uint32_t pool_enum, unsigned long long pool2_enum,
                              cudaStream_t s);
-void launch_rule_write_first(const Lanes& L, const Lanes& L2, uint32_t n, const uint32_t* base, DevRule* out,
-                             cudaStream_t s);
-void launch_rule_write_all(const uint32_t* flag, const uint32_t* base, uint32_t nsurv,
-                           const uint32_t* surv, const uint16_t* sdiff, const uint32_t* surv_target,
+// P / P2: the pools of the two passes; meta: the targets' bytes and T-states.
+void launch_rule_write_first(const Lanes& L, const Lanes& L2, uint32_t n, const uint32_t* base, const TargetMeta* meta,
+                             const DevPool& P, const DevPool& P2, DevRule* out, cudaStream_t s);
+void launch_rule_write_all(const uint32_t* flag, const uint32_t* base, uint32_t nsurv, const uint32_t* surv,
+                           const uint16_t* sdiff, const uint32_t* surv_target, const TargetMeta* meta, const DevPool& P,
                            DevRule* out, cudaStream_t s);
 void launch_rule_count_all(const RoundBuf& R, uint32_t npairs, uint32_t* flag, cudaStream_t s);
 // The steps of a pair index (PairIndex) over the n unpruned pairs `valid`:
