@@ -2547,17 +2547,30 @@ __device__ __forceinline__ uint32_t warp_sort(uint32_t x) {
 // the groups of one large bucket.  A walk over the bucket's pairs instead
 // (20.5M pairs, one output compared at a time, one warp per target) took
 // 147 ms for 10,007 uneven targets.
-__global__ void __launch_bounds__(kBlock) k_pair_scan(const RoundArgs* __restrict__ A, bool all) {
+// W warps per lane.  One suits many lanes; where few lanes are looked at (small
+// jobs, and the lanes that wait for a rescan) a block of 16 shares the groups
+// and merges what its warps found: a rescan of the large bucket that a late
+// round's lanes share took 137 us of one warp, 46 of a block (40,009 uneven
+// targets, 228 rescans: 33 -> 20 ms).  32 warps are no faster (the search for
+// where to go on within each group that passes is a chain of loads), and a
+// bound shared by the warps while they scan gave nothing.
+constexpr int kScanWarps = 16;
+template <int W>
+__global__ void __launch_bounds__(W == 1 ? kBlock : 32 * W) k_pair_scan(const RoundArgs* __restrict__ A, bool all) {
+  __shared__ uint32_t found_by[W][32];
   const DevTargets& T = A->T;
   const PairScan& ps = A->ps;
-  const unsigned lane = lane_id();
-  const uint32_t gw = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  const uint32_t nw = gridDim.x * (blockDim.x >> 5);
+  const unsigned lane = lane_id(), warp = threadIdx.x >> 5;
+  const uint32_t gw = W == 1 ? blockIdx.x * (blockDim.x >> 5) + warp : blockIdx.x;
+  const uint32_t nw = W == 1 ? gridDim.x * (blockDim.x >> 5) : gridDim.x;
+  const uint32_t part = W == 1 ? 0u : warp;  // this warp's share of the groups
   const uint32_t lanes = all ? 2u * T.n : A->R.ctl->nscan;
   for (uint32_t i = gw; i < lanes; i += nw) {
     const uint32_t idx = all ? i : ps.scan[i];
     const uint32_t resume = ps.resume[idx];
-    if ((A->L.next[idx] & kResolved) || resume == kNone) continue;
+    int skip = (A->L.next[idx] & kResolved) || resume == kNone;
+    if constexpr (W > 1) skip = __syncthreads_or(skip);  // one answer for all the warps
+    if (skip) continue;
     const uint32_t t = idx >> 1, kind = idx & 1u;
     const uint32_t tl = target_len(T, t);
     const uint32_t pw = lane < tl ? T.insn[(size_t)t * T.stride + lane] : 0u;
@@ -2591,7 +2604,7 @@ __global__ void __launch_bounds__(kBlock) k_pair_scan(const RoundArgs* __restric
       const uint32_t* top = ix.top + (key >> (32 - kPairTopBits));
       const uint32_t hi = top[1];
       const uint32_t g0 = warp_first(top[0], hi, [&](uint32_t i) { return ix.groups[i].x < key; });
-      for (uint32_t base = g0; base < hi; base += 128) {
+      for (uint32_t base = g0 + 128u * part; base < hi; base += 128u * W) {
         uint4 r[4];
         bool in[4];
 #pragma unroll
@@ -2649,6 +2662,17 @@ __global__ void __launch_bounds__(kBlock) k_pair_scan(const RoundArgs* __restric
         }
         if (!__all_sync(kFull, in[3])) break;
       }
+    }
+    if constexpr (W > 1) {
+      // the smallest of all warps' (the whole block comes here or none of it does)
+      found_by[warp][lane] = best;
+      __syncthreads();
+      if (warp == 0) {
+        for (int k = 1; k < W; k++) best = warp_merge(min(best, found_by[k][31 - lane]));
+        worst = __shfl_sync(kFull, best, 31);
+      }
+      __syncthreads();
+      if (warp != 0) continue;
     }
     // slots, and the outputs in which each survivor differs
     uint32_t fd = 0, rdf = 0;
@@ -3106,15 +3130,17 @@ void launch_pair_lanes_init(const DevTargets& T, const Lanes& L1, const QCOut& q
   if (!T.n) return;
   k_pair_lanes_init<<<grid_for(T.n, 256), 256, 0, s>>>(T, L1, q1, L2, ps);
 }
-// All lanes: a warp each and no more blocks than that needs; the blocks of a
-// large job retire as their lanes are done, which evens out the few long
-// walks.  The lanes that wait (their number is on the device, mostly none):
-// a resident grid.
+// All lanes of a large job: a warp each and no more blocks than that needs;
+// the blocks retire as their lanes are done, which evens out the long walks.
+// A small job's lanes, and the lanes that wait (their number is on the device,
+// mostly none or few): a block each.
 void launch_pair_scan(const RoundArgs* a, uint32_t n, bool all, bool small, cudaStream_t s) {
-  if (all) {
-    if (n) k_pair_scan<<<grid_for(n, kBlock / 64), kBlock, 0, s>>>(a, true);
+  if (all && !small) {
+    if (n) k_pair_scan<1><<<grid_for(n, kBlock / 64), kBlock, 0, s>>>(a, true);
   } else {
-    k_pair_scan<<<unsigned(dev_num_sms() * (small ? 1 : 8)), kBlock, 0, s>>>(a, false);
+    const unsigned most = unsigned(dev_num_sms() * (small ? 1 : 2));
+    const unsigned grid = all ? std::min(2u * n, 4u * most) : most;
+    if (grid) k_pair_scan<kScanWarps><<<grid, 32 * kScanWarps, 0, s>>>(a, all);
   }
 }
 
