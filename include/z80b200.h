@@ -78,8 +78,9 @@ typedef struct z80b_stats {
   double device_ms;         /* whole pipeline, first to last event on the context's stream */
   double qc_ms, exh_ms;     /* summed durations of the QuickCheck scan kernels and of the
                                ExhaustiveCheck kernels (CUDA events around each launch) */
-  uint64_t exhaustive_evaluated; /* states the sweep kernel ran: exhaustive_states less what
-                               the A-independent sweeps skip (2 of 256 values of A decide) */
+  uint64_t exhaustive_evaluated; /* states the sweep kernels ran: exhaustive_states less what
+                               the pair plans show to be decided by others, and less what
+                               a rejected pair's sweep leaves out */
 } z80b_stats;
 
 /* Semantics of a search job. */
@@ -283,7 +284,8 @@ typedef struct z80b_mul_result {   /* MulResult (cmd/mulopt/main.go:162-167) */
 } z80b_mul_result;
 
 typedef struct z80b_mul_stats {
-  uint64_t sequences;      /* sequences walked: sum of pool^L over the lengths searched */
+  uint64_t sequences;      /* sequences covered: sum of pool^L over the lengths searched
+                              (prefixes that reach the same state are walked once) */
   uint64_t per_k_sequences;/* sequences the per-K odometers would test: sum over K of its lengths' pool^L */
   uint64_t filter_nodes;   /* warp-level tree nodes whose leaves passed the x=2/x=255 filter */
   uint64_t full_checks;    /* all-256-input tests run */

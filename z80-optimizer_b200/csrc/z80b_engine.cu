@@ -3,16 +3,21 @@
 //
 // The batched pipeline of one job (first-found semantics, pkg/search
 // worker.go:124-265):
-//   1. QuickCheck count pass   (k_qc_scan<false>)  survivors per target
-//   2. exclusive scan          -> contiguous per-target survivor ranges
-//   3. QuickCheck collect pass (k_qc_scan<true>)   survivors in enumeration order
-//   4. rounds: each unresolved (target, pass) lane offers its next survivor;
-//      ExhaustiveCheck of all offered pairs at once; a passing pair resolves
-//      its lane (first passing survivor in enumeration order = the
-//      reference's first found), a failing one advances it.
+//   1. QuickCheck count pass (k_qc_bucket, or k_qc_scan without an index):
+//      survivors per target, those of most targets kept on the way
+//   2. exclusive scan -> contiguous per-target survivor ranges
+//   3. the kept survivors to their places, a collect pass for the rest
+//   4. rounds: each unresolved (target, pass) lane offers its next survivors;
+//      a warp plans each pair (which inputs its sweep has to vary), the pairs
+//      left are swept by class; a passing pair resolves its lane (first
+//      passing survivor in enumeration order = the reference's first found),
+//      a lane whose survivors all fail moves on.  Candidates of two
+//      instructions: the same rounds on survivors of the pair index
+//      (k_pair_scan).
 //   5. rule compaction in target order.
-// The all-hits pipeline (pkg/gpu/search.go:80-199) replaces 4 by MidCheck on
-// every survivor and one ExhaustiveCheck pass over the MidCheck survivors.
+// A small job is queued as a whole and waited for once (run_pipeline).  The
+// all-hits pipeline (pkg/gpu/search.go:80-199) replaces 4 by MidCheck on every
+// survivor and one planned ExhaustiveCheck pass over the MidCheck survivors.
 #include <cuda_runtime.h>
 
 #include <algorithm>

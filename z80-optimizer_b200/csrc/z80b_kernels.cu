@@ -1,25 +1,26 @@
 // z80b_kernels.cu -- the CUDA kernels of the verification pipeline (sm_100a).
 //
-// Tier 1, QuickCheck (pkg/search/verifier.go:85-94,626-638): one warp per
-// target.  Lanes 0..7 run the target on the eight test vectors (same opcode
-// in every lane), the outputs are broadcast with shuffles, then the warp
-// scans the candidate table 32 candidates at a time.  Candidate outputs are
-// precomputed once (k_pool_outputs), so a check is a compare of vector 0
-// (one 16-byte shared-memory load) and, on the rare match, of vectors 1..7.
+// Tier 1, QuickCheck (pkg/search/verifier.go:85-94,626-638): eight lanes per
+// target run it on the eight test vectors (same opcode in every lane of a
+// warp), hash the outputs and read the candidates filed under the same hash
+// (k_qc_bucket, k_qc_long; k_pair_scan for the candidates of two
+// instructions); pools without an index are scanned 32 candidates at a time
+// (k_qc_scan).  Candidate outputs are precomputed once (k_pool_outputs).
 // __ballot_sync turns the per-lane verdicts into ordered survivor slots.
 //
 // Tier 2, MidCheck (verifier.go:98-123): one warp per pair, lane v runs both
 // sequences on MidCheck vector v, __all_sync decides.
 //
-// Tier 3, ExhaustiveCheck (verifier.go:159-612,642-853): the sweep of a pair
-// is cut into chunks of "A-blocks" (the 256 values of A for one carry and
-// one assignment of the swept registers).  A persistent grid pulls chunks
-// from an atomic dispenser; within a chunk the 32 lanes take 32 consecutive
-// A values, so every lane executes the same opcode and the swept registers
-// are warp-uniform.  A mismatch sets the pair's rejected flag, which the
-// other chunks of the pair poll to stop early.  The reference's sweep order
-// only matters for its early exit; the verdict (all states equal) does not
-// depend on it.
+// Tier 3, ExhaustiveCheck (verifier.go:159-612,642-853): k_pair_plan finds
+// which inputs a pair's verdict depends on (z80_plan.cuh) and tries the pair
+// on 512 states; the sweep of what is left is cut into chunks of "A-blocks"
+// (the 256 values of A for one carry and one assignment of the swept
+// registers).  A persistent grid pulls chunks from an atomic dispenser;
+// within a chunk the 32 lanes take 32 consecutive A values or blocks, so
+// every lane executes the same opcode.  A mismatch sets the pair's rejected
+// flag, which the other chunks of the pair poll to stop early.  The
+// reference's sweep order only matters for its early exit; the verdict (all
+// states equal) does not depend on it.
 #include <cuda_runtime.h>
 
 #include <algorithm>
