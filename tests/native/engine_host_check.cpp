@@ -1,0 +1,54 @@
+// Host checks of the engine's order of work, its behaviour when a call fails
+// and what it keeps, on a CUDA runtime without a device (fake_cudart.h).
+// Usage: engine_host_check <check>; prints "OK <check>".
+#include <cstdio>
+#include <cstring>
+#include <string>
+#include <vector>
+
+#include "../../include/z80b200.h"
+#include "fake_cudart.h"
+
+#define CHECK(x)                                              \
+  do {                                                        \
+    if (!(x)) {                                               \
+      std::printf("FAILED %s:%d: %s\n", __FILE__, __LINE__, #x); \
+      return 1;                                               \
+    }                                                         \
+  } while (0)
+
+static int verify(z80b_ctx* ctx, uint32_t tiers, std::vector<uint8_t>* out = nullptr) {
+  const uint32_t tgt[2] = {0, 1}, cand[2] = {0, 0};
+  const uint8_t len[2] = {1, 1};
+  std::vector<uint8_t> o(2);
+  const int r = z80b_verify_pairs(ctx, tgt, len, cand, len, 1, 2, nullptr, tiers, o.data(), nullptr);
+  if (out) *out = o;
+  return r;
+}
+// An allocation that fails is reported by the call that made it, once.
+static int error_reported_once(z80b_ctx* ctx) {
+  fake::fail_malloc = 1;
+  CHECK(verify(ctx, 7) == Z80B_ENOMEM);
+  CHECK(verify(ctx, 7) == Z80B_OK);
+  return 0;
+}
+
+int main(int argc, char** argv) {
+  const std::string name = argc > 1 ? argv[1] : "";
+  struct {
+    const char* name;
+    int (*run)(z80b_ctx*);
+  } checks[] = {{"error_reported_once", error_reported_once}};
+  for (const auto& c : checks)
+    if (name == c.name) {
+      z80b_ctx* ctx = nullptr;
+      CHECK(z80b_init(0, &ctx) == Z80B_OK);
+      CHECK(fake::unordered == 0);
+      if (c.run(ctx)) return 1;
+      z80b_destroy(ctx);
+      std::printf("OK %s\n", c.name);
+      return 0;
+    }
+  std::printf("unknown check '%s'\n", name.c_str());
+  return 1;
+}

@@ -286,12 +286,16 @@ int fail(z80b_ctx* c, int code, const char* fmt, ...) {
   return code;
 }
 
+// (the runtime keeps a failed call's error until it is asked for: left there,
+// the launch check of the caller's next call would report it again)
 #define CK(call)                                                                       \
   do {                                                                                 \
     cudaError_t e_ = (call);                                                           \
-    if (e_ != cudaSuccess)                                                             \
+    if (e_ != cudaSuccess) {                                                           \
+      cudaGetLastError();                                                              \
       return fail(ctx, e_ == cudaErrorMemoryAllocation ? Z80B_ENOMEM : Z80B_ECUDA,     \
                   "%s: %s (%s:%d)", #call, cudaGetErrorString(e_), __FILE__, __LINE__); \
+    }                                                                                  \
   } while (0)
 
 #define CKR(expr)              \
