@@ -33,12 +33,42 @@ static int error_reported_once(z80b_ctx* ctx) {
   return 0;
 }
 
+static int mul(z80b_ctx* ctx, int min_len, int max_len) {
+  const int32_t k = 37;
+  z80b_mul_result r;
+  return z80b_mul_search(ctx, 0, 0, 0, 0, min_len, max_len, &k, 1, &r, nullptr);
+}
+
+// The suffix tables of a walk are ordered before it, and a table whose copy
+// failed is copied again by the next search.
+static int mul_tables(z80b_ctx* ctx) {
+  CHECK(mul(ctx, 1, 6) == Z80B_OK);
+  CHECK(fake::unordered == 0);
+  const int before = fake::copies_in;
+  CHECK(mul(ctx, 2, 6) == Z80B_OK);  // other tables
+  const int copies = fake::copies_in - before;
+  CHECK(copies > 0 && fake::unordered == 0);
+  CHECK(mul(ctx, 2, 6) == Z80B_OK);
+  CHECK(fake::copies_in == before + copies);  // kept
+  for (int nth = 1; nth <= copies; nth++) {
+    z80b_ctx* c = nullptr;
+    CHECK(z80b_init(0, &c) == Z80B_OK);
+    fake::fail_copy_in = nth;
+    CHECK(mul(c, 2, 6) != Z80B_OK);
+    const int at = fake::copies_in;
+    CHECK(mul(c, 2, 6) == Z80B_OK);
+    CHECK(fake::copies_in == at + copies);
+    z80b_destroy(c);
+  }
+  return 0;
+}
+
 int main(int argc, char** argv) {
   const std::string name = argc > 1 ? argv[1] : "";
   struct {
     const char* name;
     int (*run)(z80b_ctx*);
-  } checks[] = {{"error_reported_once", error_reported_once}};
+  } checks[] = {{"error_reported_once", error_reported_once}, {"mul_tables", mul_tables}};
   for (const auto& c : checks)
     if (name == c.name) {
       z80b_ctx* ctx = nullptr;

@@ -196,6 +196,13 @@ struct RoundGraph {
   }
 };
 
+// The suffixes of a constant-multiply walk on the device (WordBufs).
+struct MulWords {
+  DBuf buf;
+  uint32_t first_ops = 0;
+  bool ready = false;  // the copy has been queued
+};
+
 struct z80b_ctx {
   int device = 0;
   cudaStream_t stream = nullptr;
@@ -227,8 +234,7 @@ struct z80b_ctx {
   DBuf mul_best, mul_stats;   // constant-multiply search: best key per length and K, counters
   DBuf mul_hash[mul::kMaxLen], mul_key[mul::kMaxLen];  // prefixes with distinct states per length
   DBuf mul_child, mul_tab_hash, mul_tab_key, mul_count;
-  DBuf mul_words[mul::kNumPools][2][mul::kMaxInner + 1];  // the walk's suffixes (WordBufs), by min_len 1 or not
-  uint32_t mul_first_ops[mul::kNumPools][2][mul::kMaxInner + 1] = {};
+  MulWords mul_words[mul::kNumPools][2][mul::kMaxInner + 1];  // the walk's suffixes, by min_len 1 or not
   HBuf h_mul;
   // length-2 candidates: the pair pool and its indexes, shared by the
   // contexts of a device; the per-lane pass state is per context
@@ -1021,20 +1027,26 @@ struct MulSearch {
   int walk(int len, const unsigned long long* reps, uint32_t n, int rep_len) {
     const int inner = (reps ? len - rep_len : mul::plain_suffix(a.pool, len)) - 1;
     const int sh = a.min_len == 1 ? 1 : 0;
-    DBuf& w = ctx->mul_words[a.pool][sh][inner];
+    MulWords& w = ctx->mul_words[a.pool][sh][inner];
     size_t masks = 0, leaves = 1;
     for (int i = 0; i < inner; i++) {
       masks += leaves;
       leaves *= size_t(n_ops);
     }
-    if (!w.p) {
+    if (!w.ready) {
       const mul::WordImage im = mul::word_image(a.pool, inner, sh != 0);
-      CK(w.ensure(4 * masks + leaves));
-      CK(cudaMemcpy(w.p, im.mask.data(), 4 * masks, cudaMemcpyHostToDevice));
-      CK(cudaMemcpy(w.as<uint8_t>() + 4 * masks, im.leaf.data(), leaves, cudaMemcpyHostToDevice));
-      ctx->mul_first_ops[a.pool][sh][inner] = im.first_ops;
+      std::vector<uint8_t> image(4 * masks + leaves);
+      if (masks) std::memcpy(image.data(), im.mask.data(), 4 * masks);
+      std::memcpy(image.data() + 4 * masks, im.leaf.data(), leaves);
+      CK(w.buf.ensure(image.size()));
+      // on the stream of the walk that reads it (a plain cudaMemcpy from
+      // pageable memory runs on the legacy stream, which that one is not
+      // ordered behind)
+      CK(cudaMemcpyAsync(w.buf.p, image.data(), image.size(), cudaMemcpyHostToDevice, ctx->stream));
+      w.first_ops = im.first_ops;
+      w.ready = true;
     }
-    const mul::WordBufs words{w.as<uint32_t>(), w.as<uint8_t>() + 4 * masks, ctx->mul_first_ops[a.pool][sh][inner]};
+    const mul::WordBufs words{w.buf.as<uint32_t>(), w.buf.as<uint8_t>() + 4 * masks, w.first_ops};
     cudaError_t e = mul::launch_length(a, len, reps, n, rep_len, words, ctx->mul_best.as<unsigned long long>(),
                                        ctx->mul_stats.as<mul::LenStats>(), sms, ctx->stream);
     if (e != cudaSuccess) return fail(ctx, Z80B_ECUDA, "mulopt length %d launch: %s", len, cudaGetErrorString(e));
