@@ -63,12 +63,35 @@ static int mul_tables(z80b_ctx* ctx) {
   return 0;
 }
 
+// One search with candidates of two instructions.
+static int search2(z80b_ctx* ctx) {
+  const uint32_t targets[4] = {0, 0, 0, 0};
+  z80b_job job{};
+  job.targets = targets;
+  job.n_targets = 1;
+  job.target_len = job.target_stride = 4;
+  job.max_cand_len = 2;
+  job.global_dead_flags = 0x28;
+  job.mode = Z80B_MODE_FIRST;
+  job.path = Z80B_PATH_BATCHED;
+  z80b_rule rules[8];
+  uint64_t n = 0;
+  return z80b_search(ctx, &job, rules, 8, &n, nullptr);
+}
+// What goes up with the pair pool is ordered before the work that reads it.
+static int pair_pool_order(z80b_ctx* ctx) {
+  CHECK(search2(ctx) == Z80B_OK);
+  CHECK(fake::unordered == 0);
+  return 0;
+}
+
 int main(int argc, char** argv) {
   const std::string name = argc > 1 ? argv[1] : "";
   struct {
     const char* name;
     int (*run)(z80b_ctx*);
-  } checks[] = {{"error_reported_once", error_reported_once}, {"mul_tables", mul_tables}};
+  } checks[] = {{"error_reported_once", error_reported_once}, {"mul_tables", mul_tables},
+                {"pair_pool_order", pair_pool_order}};
   for (const auto& c : checks)
     if (name == c.name) {
       z80b_ctx* ctx = nullptr;

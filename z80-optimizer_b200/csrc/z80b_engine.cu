@@ -458,13 +458,17 @@ int ensure_pairpool(z80b_ctx* ctx) {
   for (uint32_t q = 0, k = 0; q < n; q++)
     if (!prune[q]) ids[k++] = q;
   CK(S.valid_ids.ensure(4ull * valid));
-  CK(cudaMemcpy(S.valid_ids.p, ids.data(), 4ull * valid, cudaMemcpyHostToDevice));
+  // on the context's stream: it is not ordered behind the legacy stream, which
+  // plain copies from pageable memory and memsets run on and may outlast
+  cudaStream_t s = ctx->stream;
+  CK(cudaMemcpyAsync(S.valid_ids.p, ids.data(), 4ull * valid, cudaMemcpyHostToDevice, s));
   S.eligible.assign(16, 0);
   for (int b = 1; b < 16; b++) S.eligible[size_t(b)] = S.eligible[size_t(b - 1)] + by_size[size_t(b - 1)];
   CK(S.eligible_dev.ensure(16 * sizeof(unsigned long long)));
-  CK(cudaMemcpy(S.eligible_dev.p, S.eligible.data(), 16 * sizeof(unsigned long long), cudaMemcpyHostToDevice));
+  CK(cudaMemcpyAsync(S.eligible_dev.p, S.eligible.data(), 16 * sizeof(unsigned long long), cudaMemcpyHostToDevice, s));
   CK(S.idx.ensure(64 * sizeof(PairIndex)));
-  CK(cudaMemset(S.idx.p, 0, 64 * sizeof(PairIndex)));
+  CK(cudaMemsetAsync(S.idx.p, 0, 64 * sizeof(PairIndex), s));
+  CK(cudaStreamSynchronize(s));  // other contexts' streams read it too
   trace("pair pool ready: %u unpruned", valid);
   return Z80B_OK;
 }
