@@ -138,6 +138,7 @@ constexpr uint32_t kUpChunkMin = 1u << 16;  // targets; smaller jobs upload in o
 // contexts of a device share one copy; mu serializes the builds.
 struct PairShared {
   std::mutex mu;
+  bool ready = false;                          // all of the below but the indexes is there
   PoolBufs pool;
   uint32_t valid = 0;                          // unpruned pairs
   DBuf valid_ids;                              // [valid] their indices, ascending
@@ -427,7 +428,7 @@ int ensure_pairpool(z80b_ctx* ctx) {
   if (!ctx->pairpool) ctx->pairpool = pair_shared(ctx->device);
   PairShared& S = *ctx->pairpool;
   std::lock_guard<std::mutex> lk(S.mu);
-  if (S.pool.loaded) return Z80B_OK;
+  if (S.ready) return Z80B_OK;  // (not pool.loaded: what follows the outputs can fail too)
   const auto& p8 = pool8();
   const uint32_t n1 = uint32_t(p8.size());
   const uint32_t n = n1 * n1;
@@ -469,6 +470,7 @@ int ensure_pairpool(z80b_ctx* ctx) {
   CK(S.idx.ensure(64 * sizeof(PairIndex)));
   CK(cudaMemsetAsync(S.idx.p, 0, 64 * sizeof(PairIndex), s));
   CK(cudaStreamSynchronize(s));  // other contexts' streams read it too
+  S.ready = true;
   trace("pair pool ready: %u unpruned", valid);
   return Z80B_OK;
 }
