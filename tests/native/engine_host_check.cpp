@@ -7,6 +7,8 @@
 #include <vector>
 
 #include "../../include/z80b200.h"
+#include "../../z80-optimizer_b200/csrc/z80_plan.cuh"
+#include "../../z80-optimizer_b200/csrc/z80b_kernels.cuh"
 #include "fake_cudart.h"
 
 #define CHECK(x)                                              \
@@ -123,6 +125,30 @@ static int pair_pool_retry(z80b_ctx* first) {
   return 0;
 }
 
+// No chunk of a sweep is empty (the sweep kernels count what a chunk covers
+// from its first unit on), the chunks cover the sweep, and those of a full
+// round can be numbered.
+static int chunks(z80b_ctx* ctx) {
+  std::vector<unsigned long long> caps{1, 2, 3, 4096, 1ull << 19, (1ull << 19) + 1, (1ull << 20) - 1, 1ull << 20,
+                                       20000001, z80b::kMaxRoundPairs};
+  for (unsigned long long n = 1; n < 40000000; n = n * 3 / 2 + 1) caps.push_back(n);
+  for (unsigned long long cap : caps) {
+    if (cap > z80b::kMaxRoundPairs) continue;
+    const uint32_t most = z80b::max_chunks(cap);
+    CHECK(cap * most <= z80b::kChunkMask);
+    for (uint32_t blocks : {1u, 2u, 3u, 7u, 8u, 31u, 32u, 33u, 100u, 511u, 512u, 4095u, 4096u})
+      for (int k = 0; k <= 40; k++) {  // a sweep's units are a power of two
+        const unsigned long long units = 1ull << k;
+        const uint32_t n = z80b::chunk_count(units, blocks, most);
+        const unsigned long long per = z80b::chunk_units(units, n);
+        CHECK(n >= 1 && n <= most);
+        CHECK((n - 1ull) * per < units && n * per >= units);
+      }
+  }
+  z80b_destroy(ctx);
+  return 0;
+}
+
 int main(int argc, char** argv) {
   const std::string name = argc > 1 ? argv[1] : "";
   struct {
@@ -130,7 +156,7 @@ int main(int argc, char** argv) {
     int (*run)(z80b_ctx*);
   } checks[] = {{"error_reported_once", error_reported_once}, {"mul_tables", mul_tables},
                 {"pair_pool_order", pair_pool_order},
-                {"pair_pool_retry", pair_pool_retry}};
+                {"pair_pool_retry", pair_pool_retry}, {"chunks", chunks}};
   for (const auto& c : checks)
     if (name == c.name) {
       z80b_ctx* ctx = nullptr;

@@ -166,6 +166,16 @@ Z80B_PLAN_HD unsigned long long plan_blocks(uint32_t reads, bool reduced) {
   return (2ull << (5 * n)) * (sp ? 16ull : 1ull);
 }
 
+// A sweep of `units` units in chunks of chunk_blocks units, at most max_chunks
+// of them: their number, and the units of one.
+Z80B_PLAN_HD uint32_t chunk_count(unsigned long long units, uint32_t chunk_blocks, uint32_t max_chunks) {
+  const unsigned long long c = (units + chunk_blocks - 1) / chunk_blocks;
+  return c > max_chunks ? max_chunks : uint32_t(c);
+}
+Z80B_PLAN_HD unsigned long long chunk_units(unsigned long long units, uint32_t chunks) {
+  return (units + chunks - 1) / chunks;
+}
+
 // The plan from the open outputs: rest, what those other than A can depend on;
 // at / ac, what A can (where it is open) in either program; keeps_t / keeps_c:
 // the program leaves A as it was.

@@ -193,11 +193,6 @@ __device__ __forceinline__ unsigned long long pair_units(unsigned long long nblo
   return (keepR & kXIndep) ? (nblocks + xu - 1) / xu : (nblocks + kBitsBlocks - 1) / kBitsBlocks;
 }
 constexpr int kChunksPerWarp = 16;
-// Work chunks of a sweep: chunk_blocks units each (the tuning option).
-__device__ __forceinline__ uint32_t chunks_for(const RoundBuf& R, unsigned long long units) {
-  const unsigned long long c = (units + R.chunk_blocks - 1) / R.chunk_blocks;
-  return c > R.max_chunks ? R.max_chunks : uint32_t(c);
-}
 // The class of a pair (kClasses).
 __device__ __forceinline__ int pair_class(const PairRec& pr) {
   if (pr.cmap & kWideClass) return 3;    // only set when R.wide
@@ -926,7 +921,8 @@ __global__ void __launch_bounds__(128, 8) k_pair_plan(const RoundArgs* __restric
     }
     if (lane == 0) {
       R.pairs[p] = pr;
-      const uint32_t ch = pr.nblocks ? chunks_for(R, pair_units(pr.nblocks, pr.keepR, R.xunit)) : 0u;
+      const uint32_t ch =
+          pr.nblocks ? chunk_count(pair_units(pr.nblocks, pr.keepR, R.xunit), R.chunk_blocks, R.max_chunks) : 0u;
       if (ch) {
         const int cls = pair_class(pr);
         const unsigned long long at = atomicAdd(&R.ctl->alloc[cls], 1ull << kChunkBits | ch);
@@ -1577,7 +1573,7 @@ __global__ void __launch_bounds__(kBlock, CLS == 3 ? 3 : (CLS == 4 ? 2 : (CLS ==
     uint32_t units;
     {
       const unsigned long long nunits = pair_units(pr.nblocks, pr.keepR, A.xunit);
-      const unsigned long long upc = (nunits + nch - 1) / nch;
+      const unsigned long long upc = chunk_units(nunits, nch);
       u0 = (k - c0) * upc;
       units = u0 < nunits ? uint32_t(min(upc, nunits - u0)) : 0u;
     }

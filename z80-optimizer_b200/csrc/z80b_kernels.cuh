@@ -110,12 +110,14 @@ constexpr int kChunkBits = 39;
 constexpr unsigned long long kChunkMask = (1ull << kChunkBits) - 1;
 // Most pair slots of a round (an entry number takes the bits above
 // kChunkBits) and most chunks of a pair, so that the chunks of a full round
-// stay below 2^kChunkBits.
+// stay below 2^kChunkBits.  A power of two, as the units of every sweep are:
+// any other limit leaves a long sweep's last chunks empty, and the kernels
+// count a chunk from its first unit on.
 constexpr unsigned long long kMaxRoundPairs = (1ull << (64 - kChunkBits)) - 1;
 inline uint32_t max_chunks(unsigned long long pairs) {
-  unsigned long long c = (1ull << kChunkBits) / (pairs ? pairs : 1ull);
-  if (c > (1ull << 20)) c = 1ull << 20;
-  return uint32_t(c > 1 ? c - 1 : 1);
+  uint32_t c = 1u << 20;
+  while (c > 1 && c * pairs > kChunkMask) c >>= 1;
+  return c;
 }
 
 struct RoundBuf {
