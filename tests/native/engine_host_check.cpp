@@ -36,6 +36,17 @@ static int error_reported_once(z80b_ctx* ctx) {
   return 0;
 }
 
+// Verification keeps no events: their number does not grow with the calls.
+static int verify_events(z80b_ctx* ctx) {
+  CHECK(verify(ctx, 7) == Z80B_OK);
+  const int events = fake::events;
+  for (int i = 0; i < 200; i++) CHECK(verify(ctx, 7) == Z80B_OK);
+  CHECK(fake::events == events);
+  z80b_destroy(ctx);
+  CHECK(fake::events == 0);
+  return 0;
+}
+
 static int mul(z80b_ctx* ctx, int min_len, int max_len) {
   const int32_t k = 37;
   z80b_mul_result r;
@@ -156,7 +167,8 @@ int main(int argc, char** argv) {
     int (*run)(z80b_ctx*);
   } checks[] = {{"error_reported_once", error_reported_once}, {"mul_tables", mul_tables},
                 {"pair_pool_order", pair_pool_order},
-                {"pair_pool_retry", pair_pool_retry}, {"chunks", chunks}};
+                {"pair_pool_retry", pair_pool_retry}, {"chunks", chunks},
+                {"verify_events", verify_events}};
   for (const auto& c : checks)
     if (name == c.name) {
       z80b_ctx* ctx = nullptr;

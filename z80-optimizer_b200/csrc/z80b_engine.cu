@@ -796,8 +796,9 @@ int read_report(z80b_ctx* ctx, const Report** out) {
 
 // Plans the round's pairs, reads its counters and sweeps them, the grids by
 // the chunks there are (their blocks retire every few chunks).  h_args: the
-// arguments that a holds on the device.
-int sweep_round(z80b_ctx* ctx, const RoundArgs* a, const RoundArgs& h_args, bool small, uint32_t* np) {
+// arguments that a holds on the device.  timed: the sweeps are bracketed by
+// events, which the caller's ksum reads and gives back.
+int sweep_round(z80b_ctx* ctx, const RoundArgs* a, const RoundArgs& h_args, bool small, bool timed, uint32_t* np) {
   const RoundBuf& R = h_args.R;
   cudaStream_t s = ctx->stream;
   launch_pair_plan(a, small, s);
@@ -807,7 +808,7 @@ int sweep_round(z80b_ctx* ctx, const RoundArgs* a, const RoundArgs& h_args, bool
   *np = std::min(h.npairs, R.cap);
   trace("sweep: %u pairs, %llu + %llu + %llu + %llu + %llu chunks", *np, h.alloc[0] & kChunkMask,
         h.alloc[1] & kChunkMask, h.alloc[2] & kChunkMask, h.alloc[3] & kChunkMask, h.alloc[4] & kChunkMask);
-  int ke = kbegin(ctx, 1);
+  const int ke = timed ? kbegin(ctx, 1) : -1;
   const int nl = launch_exhaustive(sweep_args(h_args), h.alloc, ctx->exh_k, s, &ctx->sweep_kernels);
   kend(ctx, ke);
   if (nl) CKR(check_launch(ctx, "exhaustive"));
@@ -935,7 +936,7 @@ int rounds_on_host(z80b_ctx* ctx, const RoundArgs* a, const RoundArgs& h_args, b
     launch_round_build(a, pair, small, s);
     CKR(check_launch(ctx, "round_build"));
     uint32_t np = 0;
-    CKR(sweep_round(ctx, a, h_args, small, &np));
+    CKR(sweep_round(ctx, a, h_args, small, true, &np));
     launch_round_resolve(a, pair, small, s);
     CKR(check_launch(ctx, "round_resolve"));
     launch_round_end(a, false, cudaGraphConditionalHandle{}, s);
@@ -1450,7 +1451,7 @@ int run_pipeline(z80b_ctx* ctx, const DevTargets& T, const PipeOpts& opts, z80b_
           CKR(fetch(ctx, &h, R.ctl));
           np = std::min(h.npairs, R.cap);
         } else {
-          CKR(sweep_round(ctx, args, ra, S <= kSmallJob, &np));
+          CKR(sweep_round(ctx, args, ra, S <= kSmallJob, true, &np));
         }
         mid_surv += np;
         exh_pairs += np;
@@ -2029,7 +2030,7 @@ int z80b_verify_pairs(z80b_ctx* ctx, const uint32_t* tgt, const uint8_t* tlens, 
       launch_pairs_identity(m, R, s);
       CKR(check_launch(ctx, "pairs"));
       uint32_t np = 0;
-      CKR(sweep_round(ctx, args, ra, m <= kSmallJob, &np));
+      CKR(sweep_round(ctx, args, ra, m <= kSmallJob, false, &np));
       CK(cudaMemcpyAsync(rej.data() + lo, ctx->rejected.p, 4ull * m, cudaMemcpyDeviceToHost, s));
       CK(cudaStreamSynchronize(s));
     }
