@@ -65,6 +65,15 @@ struct DBuf {
     if (e == cudaSuccess) bytes = want;
     return e;
   }
+  void release() {
+    if (p) cudaFree(p);
+    p = nullptr;
+    bytes = 0;
+  }
+  void swap(DBuf& o) {
+    std::swap(p, o.p);
+    std::swap(bytes, o.bytes);
+  }
   template <class T>
   T* as() const {
     return static_cast<T*>(p);
@@ -98,10 +107,11 @@ struct PoolBufs {
   DBuf insn, qc, mid, size, prune, reads, lens;
   // QuickCheck bucket index (ensure_qc_index)
   DBuf qkeys, qkeys_tmp, qentries, qhash2, qtop, qelig, qsort_tmp, qclash;
-  int qstate = 0;          // 0 not built, 1 built, -1 pool too large
+  int qstate = 0;          // 0 not built, 1 built, -1 no index for this pool
   uint32_t qw2 = 0;        // word-2 mask the index hashes
   uint32_t qvalid = 0;     // unpruned candidates
   uint64_t qmasks = 0;     // dead-register masks indexed
+  uint32_t qslots = 0;     // masks that qentries and qhash2 have room for
   bool qmixed = false;     // QCIndex::check_h2
   DevPool dev{};
   std::vector<uint32_t> host_insn;
@@ -522,29 +532,39 @@ int ensure_pair_index(z80b_ctx* ctx, uint32_t m) {
   return Z80B_OK;
 }
 
-// QuickCheck index of a pool (QCIndex) for the dead-register masks in
-// `masks`.  Pools of at most kQCAllMasksMax candidates get all 64 masks in one
-// sort; larger ones (the 266,675 first-op instructions of an all-hits search)
-// each mask when it first occurs, a sort of its own: 0.2 ms, where the scan
-// of all candidates that such pools took cost every target 1.6 us (48 ms for
-// 30,011 targets).  Pools above kQCIndexMax candidates keep the full scan, and
-// so does a pool in which two different outputs share both hashes.
-int ensure_qc_index(z80b_ctx* ctx, PoolBufs& P, uint32_t w2mask, uint64_t masks) {
-  if (P.qstate == -1) return Z80B_OK;
-  const uint32_t n = P.dev.n;
-  if (n == 0 || n > kQCIndexMax) {
-    P.qstate = -1;
-    return Z80B_OK;
+// Room for the entries of `masks` masks; what is there stays.
+int grow_qc_index(z80b_ctx* ctx, PoolBufs& P, uint32_t masks) {
+  if (masks <= P.qslots) return Z80B_OK;
+  masks = std::min(64u, std::max(masks, 2 * P.qslots));
+  const size_t used = size_t(__builtin_popcountll(P.qmasks)) * P.qvalid;
+  const size_t ne = std::max<size_t>(size_t(masks) * P.qvalid, 1);
+  DBuf entries, hash2;
+  CK(entries.ensure(ne * 16));
+  CK(hash2.ensure(ne * 4));
+  if (used) {
+    CK(cudaMemcpyAsync(entries.p, P.qentries.p, used * 16, cudaMemcpyDeviceToDevice, ctx->stream));
+    CK(cudaMemcpyAsync(hash2.p, P.qhash2.p, used * 4, cudaMemcpyDeviceToDevice, ctx->stream));
+    CK(cudaStreamSynchronize(ctx->stream));
   }
+  P.qentries.swap(entries);
+  P.qhash2.swap(hash2);
+  P.qslots = masks;
+  return Z80B_OK;
+}
+void drop_qc_index(PoolBufs& P) {
+  for (DBuf* b : {&P.qkeys, &P.qkeys_tmp, &P.qentries, &P.qhash2, &P.qtop, &P.qsort_tmp}) b->release();
+  P.qslots = 0;
+  P.qmasks = 0;
+}
+int build_qc_index(z80b_ctx* ctx, PoolBufs& P, uint32_t w2mask, uint64_t masks) {
+  const uint32_t n = P.dev.n;
   cudaStream_t s = ctx->stream;
   const uint32_t bits = qc_top_bits(n);
-  const bool all = n <= kQCAllMasksMax;
-  if (all) masks = ~0ull;
-  if (P.qstate == 1 && P.qw2 == w2mask && !(masks & ~P.qmasks)) return Z80B_OK;
-  const uint32_t nm = all ? 64 : 1;
+  const uint32_t nm = n <= kQCAllMasksMax ? 64 : 1;  // masks per sort
   if (P.qstate != 1 || P.qw2 != w2mask) {
     P.qstate = 0;
     P.qmasks = 0;
+    P.qslots = 0;
     std::vector<uint8_t> size(n), prune(n);
     CK(cudaMemcpyAsync(size.data(), P.size.p, n, cudaMemcpyDeviceToHost, s));
     CK(cudaMemcpyAsync(prune.data(), P.prune.p, n, cudaMemcpyDeviceToHost, s));
@@ -557,44 +577,78 @@ int ensure_qc_index(z80b_ctx* ctx, PoolBufs& P, uint32_t w2mask, uint64_t masks)
         by_size[size[q]]++;
       }
     for (int b = 1; b < 256; b++) elig[size_t(b)] = elig[size_t(b - 1)] + by_size[size_t(b - 1)];
-    const size_t ne = std::max<size_t>(64ull * P.qvalid, 1);
     CK(P.qkeys.ensure(size_t(nm) * n * 8));
     CK(P.qkeys_tmp.ensure(size_t(nm) * n * 8));
-    CK(P.qentries.ensure(ne * 16));
-    CK(P.qhash2.ensure(ne * 4));
     CK(P.qtop.ensure(64ull * ((1ull << bits) + 1) * 4));
     CK(P.qelig.ensure(256 * 4));
     CK(P.qclash.ensure(8));
     CK(cudaMemcpyAsync(P.qelig.p, elig.data(), 256 * 4, cudaMemcpyHostToDevice, s));
     CK(cudaMemsetAsync(P.qclash.p, 0, 8, s));
     CK(cudaStreamSynchronize(s));
-    P.qstate = 1;
-    P.qw2 = w2mask;
   }
+  const size_t nk = size_t(nm) * n;
+  size_t tmp = 0;
+  CK(cub::DeviceRadixSort::SortKeys(nullptr, tmp, P.qkeys_tmp.as<unsigned long long>(),
+                                    P.qkeys.as<unsigned long long>(), int(nk), 0, 64, s));
+  CK(P.qsort_tmp.ensure(tmp));
+  const uint64_t add = masks & ~P.qmasks;
+  uint32_t slot = uint32_t(__builtin_popcountll(P.qmasks));
+  CKR(grow_qc_index(ctx, P, slot + uint32_t(__builtin_popcountll(add))));
+  P.qstate = 1;
+  P.qw2 = w2mask;
   for (uint32_t m = 0; m < 64; m += nm) {
-    if (!((masks & ~P.qmasks) >> m & 1u)) continue;
-    const size_t nk = size_t(nm) * n;
+    if (!(add >> m & 1u)) continue;
     launch_qc_keys(P.dev, w2mask, m, nm, P.qkeys_tmp.as<unsigned long long>(), s);
     CKR(check_launch(ctx, "qc_keys"));
-    size_t tmp = 0;
-    CK(cub::DeviceRadixSort::SortKeys(nullptr, tmp, P.qkeys_tmp.as<unsigned long long>(),
-                                      P.qkeys.as<unsigned long long>(), int(nk), 0, 64, s));
-    CK(P.qsort_tmp.ensure(tmp));
     CK(cub::DeviceRadixSort::SortKeys(P.qsort_tmp.p, tmp, P.qkeys_tmp.as<unsigned long long>(),
                                       P.qkeys.as<unsigned long long>(), int(nk), 0, 64, s));
-    launch_qc_entries(P.dev, w2mask, P.qkeys.as<unsigned long long>(), P.qvalid, m * P.qvalid, m, nm, bits,
+    launch_qc_entries(P.dev, w2mask, P.qkeys.as<unsigned long long>(), P.qvalid, slot * P.qvalid, m, nm, bits,
                       P.qentries.as<uint4>(), P.qhash2.as<uint32_t>(), P.qtop.as<uint32_t>(), P.qclash.as<uint32_t>(),
                       s);
     CKR(check_launch(ctx, "qc_entries"));
     ctx->launches += 5;
-    P.qmasks |= all ? ~0ull : 1ull << m;
+    slot += nm;
   }
   uint32_t clash[2] = {0, 0};
   CKR(fetch(ctx, clash, P.qclash.as<uint32_t>(), 2));
-  if (clash[0]) P.qstate = -1;
+  P.qmasks |= masks;
   P.qmixed = clash[1] != 0;
-  trace("QuickCheck index: %u candidates, %u unpruned, masks %016llx, clash %u, mixed %u", n,
-        P.qvalid, (unsigned long long)P.qmasks, clash[0], clash[1]);
+  trace("QuickCheck index: %u candidates, %u unpruned, masks %016llx, room for %u, clash %u, mixed %u", n, P.qvalid,
+        (unsigned long long)P.qmasks, P.qslots, clash[0], clash[1]);
+  if (clash[0]) {
+    drop_qc_index(P);
+    P.qstate = -1;
+  }
+  return Z80B_OK;
+}
+// QuickCheck index of a pool (QCIndex) for the dead-register masks in
+// `masks`.  Pools of at most kQCAllMasksMax candidates get all 64 masks in one
+// sort; larger ones (the 266,675 first-op instructions of an all-hits search)
+// each mask when it first occurs, a sort of its own: 0.2 ms, where the scan
+// of all candidates that such pools took cost every target 1.6 us (48 ms for
+// 30,011 targets).  Pools above kQCIndexMax candidates keep the full scan, and
+// so do a pool in which two different outputs share both hashes and a search
+// whose masks the device has no room for.
+// *usable: the index answers for these masks.
+int ensure_qc_index(z80b_ctx* ctx, PoolBufs& P, uint32_t w2mask, uint64_t masks, bool* usable) {
+  *usable = false;
+  if (P.qstate == -1) return Z80B_OK;
+  const uint32_t n = P.dev.n;
+  if (n == 0 || n > kQCIndexMax) {
+    P.qstate = -1;
+    return Z80B_OK;
+  }
+  if (n <= kQCAllMasksMax) masks = ~0ull;
+  if (P.qstate != 1 || P.qw2 != w2mask || (masks & ~P.qmasks)) {
+    const int r = build_qc_index(ctx, P, w2mask, masks);
+    if (r == Z80B_ENOMEM) {
+      if (P.qstate != 1) drop_qc_index(P);  // what there is stays with the masks it has
+      trace("QuickCheck index: %s", ctx->err.c_str());
+      return Z80B_OK;
+    }
+    CKR(r);
+  }
+  *usable = P.qstate == 1;
   return Z80B_OK;
 }
 
@@ -1172,9 +1226,8 @@ int run_pipeline(z80b_ctx* ctx, const DevTargets& T, const PipeOpts& opts, z80b_
   QCIndex qix{};
   bool use_ix = false;
   if (ctx->qc_index) {
-    CKR(ensure_qc_index(ctx, *pool, cfg.w2mask, opts.dreg_masks));
-    if (pool->qstate == 1) {
-      use_ix = true;
+    CKR(ensure_qc_index(ctx, *pool, cfg.w2mask, opts.dreg_masks, &use_ix));
+    if (use_ix) {
       qix.entries = pool->qentries.as<uint4>();
       qix.hash2 = pool->qhash2.as<uint32_t>();
       qix.top = pool->qtop.as<uint32_t>();

@@ -54,7 +54,10 @@ struct QCConfig {
 // instructions (12 bits) and four for the 266,675 first-op instructions (16
 // bits): a target reads its range eight entries at a time.
 constexpr uint32_t kQCIndexBits = 26;           // candidate number in a sort key and an entry
-constexpr uint32_t kQCIndexMax = 1u << 20;      // an entry and its scratch: 36 bytes per candidate and mask in use
+// Device memory: 20 bytes per candidate and mask, for the masks in use (as
+// much again at most where their room has doubled); 16 bytes per candidate of
+// sort scratch for the masks of one sort; 64 top tables (17 MB at 16 bits).
+constexpr uint32_t kQCIndexMax = 1u << 20;
 constexpr uint32_t kQCAllMasksMax = 65536;      // pools up to here: all 64 masks in one sort
 inline uint32_t qc_top_bits(uint32_t n) { return n <= kQCAllMasksMax ? 12u : 16u; }
 struct QCIndex {
