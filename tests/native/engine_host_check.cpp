@@ -217,6 +217,25 @@ static int qc_index_memory(z80b_ctx* ctx) {
   return 0;
 }
 
+// The counters of fingerprint queries are clear before the first one: where
+// clearing them failed, the next query clears them.
+static int query_counters(z80b_ctx* ctx) {
+  CHECK(load(ctx, 8) == Z80B_OK);
+  const uint8_t fp[80] = {};
+  uint32_t hits[8], n = 0;
+  for (int i = 0; i < 2; i++) {
+    fake::fail_memset = 1;
+    CHECK(z80b_quickcheck(ctx, fp, 0, hits, 8, &n) != Z80B_OK);
+    CHECK(fake::fail_memset == 0);
+  }
+  CHECK(z80b_quickcheck(ctx, fp, 0, hits, 8, &n) == Z80B_OK);
+  fake::fail_memset = 1;
+  CHECK(z80b_quickcheck(ctx, fp, 0, hits, 8, &n) == Z80B_OK);  // a query leaves them clear
+  fake::fail_memset = 0;
+  z80b_destroy(ctx);
+  return 0;
+}
+
 int main(int argc, char** argv) {
   const std::string name = argc > 1 ? argv[1] : "";
   struct {
@@ -225,7 +244,8 @@ int main(int argc, char** argv) {
   } checks[] = {{"error_reported_once", error_reported_once}, {"mul_tables", mul_tables},
                 {"pair_pool_order", pair_pool_order},
                 {"pair_pool_retry", pair_pool_retry}, {"chunks", chunks},
-                {"verify_events", verify_events}, {"qc_index_memory", qc_index_memory}};
+                {"verify_events", verify_events}, {"qc_index_memory", qc_index_memory},
+                {"query_counters", query_counters}};
   for (const auto& c : checks)
     if (name == c.name) {
       z80b_ctx* ctx = nullptr;

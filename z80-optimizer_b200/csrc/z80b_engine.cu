@@ -240,6 +240,7 @@ struct z80b_ctx {
   HBuf h_up;                  // small jobs: the host arrays of a search, one copy
   DBuf cub_tmp;
   DBuf hits, nhits;           // fingerprint queries: all hits, FpCounters
+  bool nhits_clear = false;   // they have been cleared once; each query leaves them so
   HBuf h_fp;                  // FpAnswer
   DBuf v_tgt, v_cand, v_tl, v_cl, v_dead, v_out, v_fd, v_in, v_outs;
   DBuf mul_best, mul_stats;   // constant-multiply search: best key per length and K, counters
@@ -1991,9 +1992,10 @@ int z80b_quickcheck(z80b_ctx* ctx, const uint8_t* fp80, uint32_t dead_flags, uin
   cudaStream_t s = ctx->stream;
   CK(ctx->hits.ensure(4ull * std::max<uint32_t>(ctx->loaded.n, 1)));
   CK(ctx->h_fp.ensure(sizeof(FpAnswer)));
-  if (!ctx->nhits.p) {
+  if (!ctx->nhits_clear) {
     CK(ctx->nhits.ensure(sizeof(FpCounters)));
     CK(cudaMemsetAsync(ctx->nhits.p, 0, sizeof(FpCounters), s));
+    ctx->nhits_clear = true;
   }
   FpAnswer* const answer = ctx->h_fp.as<FpAnswer>();
   launch_fp_query(ctx->loaded.dev, fq, dead_flags & 0xFFu, ctx->hits.as<uint32_t>(), ctx->nhits.as<FpCounters>(),
