@@ -79,6 +79,29 @@ static int mul_tables(z80b_ctx* ctx) {
   return 0;
 }
 
+// A search whose levels of states do not fit the device walks every prefix.
+static int mul_no_room(z80b_ctx* ctx) {
+  z80b_destroy(ctx);
+  int refused = 0, done = 0;
+  for (int nth = 1;; nth++) {
+    z80b_ctx* c = nullptr;
+    CHECK(z80b_init(0, &c) == Z80B_OK);
+    fake::fail_malloc = nth;
+    const int r = mul(c, 1, 9);
+    const bool hit = fake::fail_malloc == 0;
+    fake::fail_malloc = 0;
+    CHECK(r == Z80B_OK || (r == Z80B_ENOMEM && hit));
+    CHECK(mul(c, 1, 9) == Z80B_OK);
+    z80b_destroy(c);
+    if (!hit) break;
+    (r == Z80B_OK ? done : refused)++;
+  }
+  // what any walk takes: the answers, the counters and the suffix tables of
+  // the depths 1 (length 6), 2 (length 7) and 4 (behind the states)
+  CHECK(refused == 5 && done >= 10);
+  return 0;
+}
+
 // One search with candidates of two instructions.
 static int search2(z80b_ctx* ctx) {
   const uint32_t targets[4] = {0, 0, 0, 0};
@@ -241,7 +264,7 @@ int main(int argc, char** argv) {
   struct {
     const char* name;
     int (*run)(z80b_ctx*);
-  } checks[] = {{"error_reported_once", error_reported_once}, {"mul_tables", mul_tables},
+  } checks[] = {{"error_reported_once", error_reported_once}, {"mul_tables", mul_tables}, {"mul_no_room", mul_no_room},
                 {"pair_pool_order", pair_pool_order},
                 {"pair_pool_retry", pair_pool_retry}, {"chunks", chunks},
                 {"verify_events", verify_events}, {"qc_index_memory", qc_index_memory},

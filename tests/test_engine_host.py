@@ -23,7 +23,7 @@ def exe(tmp_path_factory):
     return out
 
 
-@pytest.mark.parametrize("check", ["error_reported_once", "mul_tables", "pair_pool_order", "pair_pool_retry", "chunks",
+@pytest.mark.parametrize("check", ["error_reported_once", "mul_tables", "mul_no_room", "pair_pool_order", "pair_pool_retry", "chunks",
                                    "verify_events", "qc_index_memory", "query_counters"])
 def test_engine_host(exe, check):
     r = subprocess.run([str(exe), check], capture_output=True, text=True, timeout=600)

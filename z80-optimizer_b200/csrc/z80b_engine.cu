@@ -1029,7 +1029,7 @@ struct MulSearch {
   static constexpr uint64_t kMaxChildren = 1ull << 24;  // at most 1.6 GB of scratch
   uint32_t count[mul::kMaxLen] = {};  // prefixes per level
   int built = -1;                     // levels built
-  bool plain = false;                 // walk every prefix (two states shared a hash)
+  bool plain = false;                 // walk every prefix (two states shared a hash, or no room for a level)
 
   // a level's children fit the scratch and their odometer indices 32 bits
   bool can_extend() const {
@@ -1145,7 +1145,16 @@ struct MulSearch {
       for (; len <= a.max_len && v <= kDirect; len++, v *= n_ops) CKR(walk(len, nullptr, 0, 0));
       if (len == first) {
         int p = std::max(1, len - kSuffix);
-        while (!plain && built < p && can_extend()) CKR(extend());
+        while (!plain && built < p && can_extend()) {
+          const int r = extend();
+          if (r == Z80B_ENOMEM) {
+            trace("mulopt: %s", ctx->err.c_str());
+            for (DBuf* b : {&ctx->mul_child, &ctx->mul_tab_hash, &ctx->mul_tab_key}) b->release();
+            plain = true;
+          } else {
+            CKR(r);
+          }
+        }
         p = std::min(p, built);
         if (plain || len - p > kSuffix) CKR(walk(len, nullptr, 0, 0));
         else CKR(walk(len, ctx->mul_key[p].as<unsigned long long>(), count[p], p));
