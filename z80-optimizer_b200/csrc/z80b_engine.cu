@@ -113,6 +113,7 @@ struct PoolBufs {
   uint64_t qmasks = 0;     // dead-register masks indexed
   uint32_t qslots = 0;     // masks that qentries and qhash2 have room for
   bool qmixed = false;     // QCIndex::check_h2
+  double qdebt = 0;        // scans made since for want of an index, in masks of its build
   DevPool dev{};
   std::vector<uint32_t> host_insn;
   std::vector<uint8_t> host_lens;
@@ -359,6 +360,7 @@ int build_pool(z80b_ctx* ctx, PoolBufs& P, const uint32_t* insn, uint32_t n, uin
                const uint8_t* lens, bool with_mid, bool by_pair = false) {
   P.loaded = false;
   P.qstate = 0;  // a QuickCheck index of the previous contents is stale
+  P.qdebt = 0;
   P.n = n;
   P.len = len;
   P.host_insn.assign(insn, insn + (size_t)n * len);
@@ -630,8 +632,15 @@ int build_qc_index(z80b_ctx* ctx, PoolBufs& P, uint32_t w2mask, uint64_t masks) 
 // 30,011 targets).  Pools above kQCIndexMax candidates keep the full scan, and
 // so do a pool in which two different outputs share both hashes and a search
 // whose masks the device has no room for.
+// A search of few targets under many new masks is scanned too: one of 100
+// targets under 64 masks takes 6.3 ms by the scan, and 23 ms where it builds
+// their indexes first.  A scan costs at least what 25 masks do (5 ms: a warp
+// walks the list, twice), and one more mask per 125 targets; the masks are
+// built when the searches that asked for new ones have scanned for as long as
+// that takes.
 // *usable: the index answers for these masks.
-int ensure_qc_index(z80b_ctx* ctx, PoolBufs& P, uint32_t w2mask, uint64_t masks, bool* usable) {
+constexpr double kQCScanMasks = 25, kQCTargetsPerMask = 125;
+int ensure_qc_index(z80b_ctx* ctx, PoolBufs& P, uint32_t w2mask, uint64_t masks, uint32_t targets, bool* usable) {
   *usable = false;
   if (P.qstate == -1) return Z80B_OK;
   const uint32_t n = P.dev.n;
@@ -640,7 +649,15 @@ int ensure_qc_index(z80b_ctx* ctx, PoolBufs& P, uint32_t w2mask, uint64_t masks,
     return Z80B_OK;
   }
   if (n <= kQCAllMasksMax) masks = ~0ull;
-  if (P.qstate != 1 || P.qw2 != w2mask || (masks & ~P.qmasks)) {
+  const bool some = P.qstate == 1 && P.qw2 == w2mask;
+  const uint64_t add = some ? masks & ~P.qmasks : masks;
+  if (!some || add) {
+    const double scan = kQCScanMasks + targets / kQCTargetsPerMask;
+    if (n > kQCAllMasksMax && __builtin_popcountll(add) > P.qdebt + scan) {
+      P.qdebt += scan;
+      return Z80B_OK;
+    }
+    P.qdebt = 0;
     const int r = build_qc_index(ctx, P, w2mask, masks);
     if (r == Z80B_ENOMEM) {
       if (P.qstate != 1) drop_qc_index(P);  // what there is stays with the masks it has
@@ -1236,7 +1253,7 @@ int run_pipeline(z80b_ctx* ctx, const DevTargets& T, const PipeOpts& opts, z80b_
   QCIndex qix{};
   bool use_ix = false;
   if (ctx->qc_index) {
-    CKR(ensure_qc_index(ctx, *pool, cfg.w2mask, opts.dreg_masks, &use_ix));
+    CKR(ensure_qc_index(ctx, *pool, cfg.w2mask, opts.dreg_masks, n, &use_ix));
     if (use_ix) {
       qix.entries = pool->qentries.as<uint4>();
       qix.hash2 = pool->qhash2.as<uint32_t>();
