@@ -48,6 +48,18 @@ static int verify_events(z80b_ctx* ctx) {
   return 0;
 }
 
+// Few pairs go up in one copy, and come back in one where nothing is swept.
+static int verify_copies(z80b_ctx* ctx) {
+  CHECK(verify(ctx, 7) == Z80B_OK);
+  const int in = fake::copies_in, out = fake::copies_out;
+  CHECK(verify(ctx, 7) == Z80B_OK);
+  CHECK(fake::copies_in == in + 1 && fake::copies_out == out + 1);
+  CHECK(verify(ctx, 3) == Z80B_OK);
+  CHECK(fake::copies_in == in + 2 && fake::copies_out == out + 2);
+  z80b_destroy(ctx);
+  return 0;
+}
+
 static int mul(z80b_ctx* ctx, int min_len, int max_len) {
   const int32_t k = 37;
   z80b_mul_result r;
@@ -291,7 +303,7 @@ int main(int argc, char** argv) {
   } checks[] = {{"error_reported_once", error_reported_once}, {"mul_tables", mul_tables}, {"mul_no_room", mul_no_room},
                 {"pair_pool_order", pair_pool_order},
                 {"pair_pool_retry", pair_pool_retry}, {"chunks", chunks},
-                {"verify_events", verify_events}, {"qc_index_memory", qc_index_memory},
+                {"verify_events", verify_events}, {"verify_copies", verify_copies}, {"qc_index_memory", qc_index_memory},
                 {"query_counters", query_counters}, {"qc_index_debt", qc_index_debt}};
   for (const auto& c : checks)
     if (name == c.name) {

@@ -8,7 +8,7 @@
 #include <map>
 
 namespace fake {
-int unordered, copies_in, events, launches, fail_malloc, fail_copy_in, fail_memset;
+int unordered, copies_in, copies_out, events, launches, fail_malloc, fail_copy_in, fail_memset;
 size_t bytes, peak, limit;
 static bool pending;                       // legacy-stream work that may still run
 static cudaError_t last;                   // what cudaGetLastError gives
@@ -76,6 +76,7 @@ static cudaError_t copy(void* d, const void* s, size_t n, cudaMemcpyKind k) {
     if (hit(fail_copy_in)) return ret(cudaErrorInvalidValue);
     copies_in++;
   }
+  if (k == cudaMemcpyDeviceToHost) copies_out++;
   std::memcpy(d, s, n);
   return cudaSuccess;
 }

@@ -10,7 +10,7 @@ namespace fake {
 // done) is not known to have ended: streams made with cudaStreamNonBlocking
 // are not ordered behind it.
 extern int unordered;
-extern int copies_in;        // host-to-device copies
+extern int copies_in, copies_out;  // host-to-device and device-to-host copies
 extern int events;           // events alive
 extern int launches;         // kernels
 extern size_t bytes, peak;   // device memory alive, and the most there was

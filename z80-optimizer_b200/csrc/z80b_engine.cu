@@ -243,7 +243,8 @@ struct z80b_ctx {
   DBuf hits, nhits;           // fingerprint queries: all hits, FpCounters
   bool nhits_clear = false;   // they have been cleared once; each query leaves them so
   HBuf h_fp;                  // FpAnswer
-  DBuf v_tgt, v_cand, v_tl, v_cl, v_dead, v_out, v_fd, v_in, v_outs;
+  DBuf v_tgt, v_tl, v_out, v_in, v_outs;
+  DBuf v_pairs;               // verification: the pairs and their verdicts
   DBuf mul_best, mul_stats;   // constant-multiply search: best key per length and K, counters
   DBuf mul_hash[mul::kMaxLen], mul_key[mul::kMaxLen];  // prefixes with distinct states per length
   DBuf mul_child, mul_tab_hash, mul_tab_key, mul_count;
@@ -866,11 +867,16 @@ int read_report(z80b_ctx* ctx, const Report** out) {
   return Z80B_OK;
 }
 
-// Plans the round's pairs, reads its counters and sweeps them, the grids by
-// the chunks there are (their blocks retire every few chunks).  h_args: the
-// arguments that a holds on the device.  timed: the sweeps are bracketed by
-// events, which the caller's ksum reads and gives back.
-int sweep_round(z80b_ctx* ctx, const RoundArgs* a, const RoundArgs& h_args, bool small, bool timed, uint32_t* np) {
+// Sweeps the chunks there are (alloc: RoundCtl::alloc on the host), the grids
+// by their number (the blocks retire every few chunks); returns the launches.
+int sweep_chunks(z80b_ctx* ctx, const RoundArgs& h_args, const unsigned long long* alloc) {
+  const int nl = launch_exhaustive(sweep_args(h_args), alloc, ctx->exh_k, ctx->stream, &ctx->sweep_kernels);
+  if (nl > 1) ctx->launches += uint32_t(nl - 1);
+  return nl;
+}
+// Plans the round's pairs, reads its counters and sweeps them.  h_args: the
+// arguments that a holds on the device.
+int sweep_round(z80b_ctx* ctx, const RoundArgs* a, const RoundArgs& h_args, bool small, uint32_t* np) {
   const RoundBuf& R = h_args.R;
   cudaStream_t s = ctx->stream;
   launch_pair_plan(a, small, s);
@@ -880,11 +886,10 @@ int sweep_round(z80b_ctx* ctx, const RoundArgs* a, const RoundArgs& h_args, bool
   *np = std::min(h.npairs, R.cap);
   trace("sweep: %u pairs, %llu + %llu + %llu + %llu + %llu chunks", *np, h.alloc[0] & kChunkMask,
         h.alloc[1] & kChunkMask, h.alloc[2] & kChunkMask, h.alloc[3] & kChunkMask, h.alloc[4] & kChunkMask);
-  const int ke = timed ? kbegin(ctx, 1) : -1;
-  const int nl = launch_exhaustive(sweep_args(h_args), h.alloc, ctx->exh_k, s, &ctx->sweep_kernels);
+  int ke = kbegin(ctx, 1);
+  const int nl = sweep_chunks(ctx, h_args, h.alloc);
   kend(ctx, ke);
   if (nl) CKR(check_launch(ctx, "exhaustive"));
-  if (nl > 1) ctx->launches += uint32_t(nl - 1);
   return Z80B_OK;
 }
 
@@ -1008,7 +1013,7 @@ int rounds_on_host(z80b_ctx* ctx, const RoundArgs* a, const RoundArgs& h_args, b
     launch_round_build(a, pair, small, s);
     CKR(check_launch(ctx, "round_build"));
     uint32_t np = 0;
-    CKR(sweep_round(ctx, a, h_args, small, true, &np));
+    CKR(sweep_round(ctx, a, h_args, small, &np));
     launch_round_resolve(a, pair, small, s);
     CKR(check_launch(ctx, "round_resolve"));
     launch_round_end(a, false, cudaGraphConditionalHandle{}, s);
@@ -1531,7 +1536,7 @@ int run_pipeline(z80b_ctx* ctx, const DevTargets& T, const PipeOpts& opts, z80b_
           CKR(fetch(ctx, &h, R.ctl));
           np = std::min(h.npairs, R.cap);
         } else {
-          CKR(sweep_round(ctx, args, ra, S <= kSmallJob, true, &np));
+          CKR(sweep_round(ctx, args, ra, S <= kSmallJob, &np));
         }
         mid_surv += np;
         exh_pairs += np;
@@ -2054,72 +2059,89 @@ int z80b_verify_pairs(z80b_ctx* ctx, const uint32_t* tgt, const uint8_t* tlens, 
   }
   cudaSetDevice(ctx->device);
   cudaStream_t s = ctx->stream;
-  CK(ctx->v_tgt.ensure(4ull * n * stride));
-  CK(ctx->v_cand.ensure(4ull * n * stride));
-  CK(ctx->v_tl.ensure(n));
-  CK(ctx->v_cl.ensure(n));
-  CK(ctx->v_dead.ensure(n));
-  CK(ctx->v_out.ensure(n));
-  CK(ctx->v_fd.ensure(n));
-  CK(cudaMemcpyAsync(ctx->v_tgt.p, tgt, 4ull * n * stride, cudaMemcpyHostToDevice, s));
-  CK(cudaMemcpyAsync(ctx->v_cand.p, cand, 4ull * n * stride, cudaMemcpyHostToDevice, s));
-  CK(cudaMemcpyAsync(ctx->v_tl.p, tlens, n, cudaMemcpyHostToDevice, s));
-  CK(cudaMemcpyAsync(ctx->v_cl.p, clens, n, cudaMemcpyHostToDevice, s));
-  if (dead) CK(cudaMemcpyAsync(ctx->v_dead.p, dead, n, cudaMemcpyHostToDevice, s));
-  else CK(cudaMemsetAsync(ctx->v_dead.p, 0, n, s));
-  launch_verify_small(ctx->v_tgt.as<uint32_t>(), ctx->v_tl.as<uint8_t>(), ctx->v_cand.as<uint32_t>(),
-                      ctx->v_cl.as<uint8_t>(), stride, n, ctx->v_dead.as<uint8_t>(), tiers, ctx->v_out.as<uint8_t>(),
-                      ctx->v_fd.as<uint8_t>(), s);
+  // One block of device memory: the pairs, and behind them all that is read
+  // back.  Few pairs go up in one copy and their verdicts come with the plan's
+  // counters: a call on few pairs is bound by its copies and waits (through the
+  // Python binding 53 us for one pair and 102 for 16; with each of the five
+  // arrays copied and each result waited for on its own 95 and 129).
+  const size_t words = (size_t)n * stride;
+  const size_t o_cand = 4 * words, o_tl = 2 * o_cand, o_cl = o_tl + n, o_dead = o_cl + n, in_bytes = o_dead + n;
+  const size_t o_ctl = (in_bytes + 255) & ~size_t(255), o_rej = o_ctl + sizeof(RoundCtl), o_out = o_rej + 4ull * n;
+  const size_t o_fd = o_out + n, bytes = o_fd + n;
+  static_assert(sizeof(RoundCtl) % 4 == 0, "the flags behind it are words");
+  CK(ctx->v_pairs.ensure(bytes));
+  uint8_t* const d = ctx->v_pairs.as<uint8_t>();
+  const bool small = n <= kSmallJob;
+  std::vector<uint8_t> up, down(bytes - o_ctl);
+  if (small) {
+    up.resize(in_bytes);
+    std::memcpy(up.data(), tgt, 4 * words);
+    std::memcpy(up.data() + o_cand, cand, 4 * words);
+    std::memcpy(up.data() + o_tl, tlens, n);
+    std::memcpy(up.data() + o_cl, clens, n);
+    if (dead) std::memcpy(up.data() + o_dead, dead, n);
+    CK(cudaMemcpyAsync(d, up.data(), in_bytes, cudaMemcpyHostToDevice, s));
+  } else {
+    CK(cudaMemcpyAsync(d, tgt, 4 * words, cudaMemcpyHostToDevice, s));
+    CK(cudaMemcpyAsync(d + o_cand, cand, 4 * words, cudaMemcpyHostToDevice, s));
+    CK(cudaMemcpyAsync(d + o_tl, tlens, n, cudaMemcpyHostToDevice, s));
+    CK(cudaMemcpyAsync(d + o_cl, clens, n, cudaMemcpyHostToDevice, s));
+    if (dead) CK(cudaMemcpyAsync(d + o_dead, dead, n, cudaMemcpyHostToDevice, s));
+    else CK(cudaMemsetAsync(d + o_dead, 0, n, s));
+  }
+  launch_verify_small(reinterpret_cast<uint32_t*>(d), d + o_tl, reinterpret_cast<uint32_t*>(d + o_cand), d + o_cl, stride,
+                      n, d + o_dead, tiers, d + o_out, d + o_fd, s);
   CKR(check_launch(ctx, "verify_small"));
-  std::vector<uint8_t> res(n), fd(n);
-  CK(cudaMemcpyAsync(res.data(), ctx->v_out.p, n, cudaMemcpyDeviceToHost, s));
-  CK(cudaMemcpyAsync(fd.data(), ctx->v_fd.p, n, cudaMemcpyDeviceToHost, s));
-  CK(cudaStreamSynchronize(s));
+  // device block from `from` on to its place in `down`
+  auto fetch_from = [&](size_t from, size_t to) {
+    CK(cudaMemcpyAsync(down.data() + (from - o_ctl), d + from, to - from, cudaMemcpyDeviceToHost, s));
+    CK(cudaStreamSynchronize(s));
+    return int(Z80B_OK);
+  };
+  const RoundCtl* const ctl = reinterpret_cast<const RoundCtl*>(down.data());
+  const uint32_t* const rej = reinterpret_cast<const uint32_t*>(down.data() + (o_rej - o_ctl));
+  bool read = false;  // down holds the results
   if (tiers & 4u) {
     // ExhaustiveCheck of every pair: pairs are (i, i) of a target batch and
     // a candidate pool with per-candidate lengths
-    DevTargets T{};
-    T.insn = ctx->v_tgt.as<uint32_t>();
-    T.len = ctx->v_tl.as<uint8_t>();
-    T.dead = ctx->v_dead.as<uint8_t>();
-    T.n = n;
-    T.stride = stride;
-    DevPool P{};
-    P.insn = ctx->v_cand.as<uint32_t>();
-    P.lens = ctx->v_cl.as<uint8_t>();
-    P.n = n;
-    P.stride = stride;
     RoundBuf R{};
     CKR(ensure_round(ctx, n, false, &R));
+    R.ctl = reinterpret_cast<RoundCtl*>(d + o_ctl);
     RoundArgs* const args = ctx->roundargs.as<RoundArgs>();
-    std::vector<uint32_t> rej(n);
     for (uint64_t lo = 0; lo < n; lo += R.cap) {  // once, up to the pair slots
       const uint32_t m = uint32_t(std::min<uint64_t>(n - lo, R.cap));
       RoundArgs ra{};
-      ra.T = T;
-      ra.T.insn += lo * stride;
-      ra.T.len += lo;
-      ra.T.dead += lo;
+      ra.T.insn = reinterpret_cast<uint32_t*>(d) + lo * stride;
+      ra.T.len = d + o_tl + lo;
+      ra.T.dead = d + o_dead + lo;
       ra.T.n = m;
-      ra.P = P;
-      ra.P.insn += lo * stride;
-      ra.P.lens += lo;
+      ra.T.stride = stride;
+      ra.P.insn = reinterpret_cast<uint32_t*>(d + o_cand) + lo * stride;
+      ra.P.lens = d + o_cl + lo;
       ra.P.n = m;
+      ra.P.stride = stride;
       ra.R = R;
+      ra.R.rejected = reinterpret_cast<uint32_t*>(d + o_rej) + lo;
       launch_round_args(ra, args, s);
       CKR(check_launch(ctx, "round_args"));
-      launch_pairs_identity(m, R, s);
+      launch_pairs_identity(m, ra.R, s);
       CKR(check_launch(ctx, "pairs"));
-      uint32_t np = 0;
-      CKR(sweep_round(ctx, args, ra, m <= kSmallJob, false, &np));
-      CK(cudaMemcpyAsync(rej.data() + lo, ctx->rejected.p, 4ull * m, cudaMemcpyDeviceToHost, s));
-      CK(cudaStreamSynchronize(s));
+      launch_pair_plan(args, small, s);
+      CKR(check_launch(ctx, "pair_plan"));
+      CKR(fetch_from(o_ctl, small ? bytes : o_rej));
+      read = small;
+      if (sweep_chunks(ctx, ra, ctl->alloc)) {
+        CKR(check_launch(ctx, "exhaustive"));
+        read = false;
+      }
     }
-    for (uint32_t i = 0; i < n; i++)
-      if (!rej[i]) res[i] |= 4;
+    if (!read) CKR(fetch_from(o_rej, bytes));
+  } else {
+    CKR(fetch_from(o_out, bytes));
   }
-  std::memcpy(out, res.data(), n);
-  if (flagdiff) std::memcpy(flagdiff, fd.data(), n);
+  const uint8_t* const res = down.data() + (o_out - o_ctl);
+  for (uint32_t i = 0; i < n; i++) out[i] = uint8_t(res[i] | ((tiers & 4u) && !rej[i] ? 4 : 0));
+  if (flagdiff) std::memcpy(flagdiff, down.data() + (o_fd - o_ctl), n);
   return Z80B_OK;
 }
 
