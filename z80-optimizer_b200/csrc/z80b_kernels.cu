@@ -28,6 +28,7 @@
 #include <mutex>
 
 #include "z80_bits.cuh"
+#include "z80_plan_warp.cuh"
 #include "z80_tables.h"
 #include "z80b_kernels.cuh"
 
@@ -132,13 +133,6 @@ __device__ __forceinline__ uint32_t reg_diff(uint32_t d0, uint32_t d1) {
 // 32,768.  PairRec.keepR bit 6 marks it.
 constexpr uint32_t kXIndep = 0x40u;
 constexpr unsigned long long kUnitBlocks = 128;
-// A pair's two programs, one instruction per lane: lanes 0..tl-1 the target,
-// lanes tl..tl+cl-1 the candidate.
-struct PairWords {
-  uint32_t w;        // this lane's instruction (0 past the programs)
-  uint32_t tl, cl;
-  __device__ __forceinline__ bool mine() const { return lane_id() < tl + cl; }
-};
 __device__ __forceinline__ PairWords pair_words(const DevTargets& T, uint32_t t, const DevPool& P, uint32_t c) {
   PairWords p;
   p.tl = target_len(T, t);
@@ -153,7 +147,7 @@ __device__ __forceinline__ PairWords pair_words(const DevTargets& T, uint32_t t,
 // either depends on the input A but A passing through (an A-dependent
 // instruction only after one that overwrites A).
 __device__ __forceinline__ bool pair_xindep(const PairWords& p) {
-  const uint32_t k = p.mine() ? g_aclass[p.w & 0xFFFFu] : 1u;
+  const uint32_t k = p.mine(lane_id()) ? g_aclass[p.w & 0xFFFFu] : 1u;
   const unsigned dep = __ballot_sync(kFull, k == 0u), over = __ballot_sync(kFull, k == 2u);
   const unsigned tm = (1u << p.tl) - 1u, cm = ((1u << p.cl) - 1u) << p.tl;
   auto free_of = [&](unsigned m) {
@@ -172,14 +166,14 @@ constexpr uint8_t kWideClass = 0x80u;
 constexpr uint8_t kRegClass = 0x40u;
 __device__ __forceinline__ uint8_t pair_cmap(const PairWords& p, bool compact, bool wide, bool xindep) {
   const uint32_t op = p.w & 0xFFFFu;
-  const uint32_t fp = __reduce_or_sync(kFull, p.mine() ? uint32_t(g_opregs[op]) : 0u);
+  const uint32_t fp = __reduce_or_sync(kFull, p.mine(lane_id()) ? uint32_t(g_opregs[op]) : 0u);
   if (compact && !(fp & 0xC0u)) {
     const uint32_t id = g_cid[fp & 0x3Fu];
-    if (id && __all_sync(kFull, !p.mine() || g_cren[id - 1][op] >= 0)) return uint8_t(id);
+    if (id && __all_sync(kFull, !p.mine(lane_id()) || g_cren[id - 1][op] >= 0)) return uint8_t(id);
   }
   if (wide && !xindep && !(fp & 0x80u)) {
     const uint32_t id = g_wid[fp & 0x3Fu];
-    if (id && __all_sync(kFull, !p.mine() || g_wren[id - 1][op] >= 0)) return uint8_t(kWideClass | id);
+    if (id && __all_sync(kFull, !p.mine(lane_id()) || g_wren[id - 1][op] >= 0)) return uint8_t(kWideClass | id);
   }
   return wide && !(fp & 0xC0u) ? kRegClass : uint8_t(0);
 }
@@ -784,79 +778,6 @@ __device__ __forceinline__ bool probe_pair(const PairWords& words, unsigned long
   return __any_sync(kFull, bad);
 }
 
-// plan_pair (z80_plan.cuh) by a warp, lane g on field g: the names of the
-// fields are in the lanes, an instruction's dependency sets are met by ballots.
-__device__ __forceinline__ PairPlan plan_pair_warp(const PairWords& p, uint32_t reads, uint32_t keepF, uint32_t keepR) {
-  const unsigned lane = lane_id();
-  const uint32_t n = p.tl + p.cl;
-  unsigned long long row[kPlanMaxInsn];
-  uint32_t word[kPlanMaxInsn], in[kPlanMaxInsn], out[kPlanMaxInsn];
-#pragma unroll
-  for (int i = 0; i < kPlanMaxInsn; i++) {
-    word[i] = __shfl_sync(kFull, p.w, i);
-    row[i] = 0;
-    in[i] = out[i] = 0;
-    if (uint32_t(i) < n && lane < kFlowFields) row[i] = g_flow[word[i] & 0xFFFFu][lane];
-  }
-  const uint32_t varying = plan_varying(reads), cmp = plan_compared(keepF, keepR);
-  const uint32_t first = ((varying >> lane) & 1u) ? 256u + lane : 0u;
-  uint32_t cur = first, end_t = 0;
-#pragma unroll
-  for (int i = 0; i < kPlanMaxInsn; i++) {
-    if (uint32_t(i) >= n) break;
-    if (uint32_t(i) == p.tl) {
-      end_t = cur;
-      cur = first;
-    }
-    in[i] = cur;
-    const uint32_t dep = uint32_t(row[i]) & 0xFFFFFFu, src = uint32_t(row[i] >> 24) & 0xFFu;
-    const uint32_t cst = uint32_t(row[i] >> 32) & 0xFFFFu;
-    const uint32_t copy = __shfl_sync(kFull, cur, int(src & 31u));
-    uint32_t id;
-    if (!((row[i] >> 48) & 1u)) id = cur;
-    else if (src != 0xFFu) id = copy;
-    else if (cst < 256u) id = cst;
-    else if (cst == kFlowImmLo) id = (word[i] >> 16) & 0xFFu;
-    else if (cst == kFlowImmHi) id = word[i] >> 24;
-    else id = 280u + 24u * i + lane;
-    const bool computed = id == 280u + 24u * i + lane;
-    bool found = false;
-#pragma unroll
-    for (int j = 0; j < i; j++) {
-      if (word[j] != word[i]) continue;
-      const unsigned same = __ballot_sync(kFull, in[j] == in[i]);
-      if (computed && !found && (dep & ~same) == 0) {
-        id = out[j];
-        found = true;
-      }
-    }
-    out[i] = id;
-    cur = id;
-  }
-  if (p.cl == 0) end_t = cur;
-  const uint32_t open = __ballot_sync(kFull, end_t != cur) & cmp;
-  // what outputs can depend on, walked backwards over lanes [lo, hi)
-  auto relevant = [&](uint32_t lo, uint32_t hi, uint32_t o) {
-#pragma unroll
-    for (int i = kPlanMaxInsn - 1; i >= 0; i--) {
-      if (uint32_t(i) < lo || uint32_t(i) >= hi) continue;
-      const bool on = (o >> lane) & 1u, changed = (row[i] >> 48) & 1u;
-      o = __reduce_or_sync(kFull, !on ? 0u : (changed ? uint32_t(row[i]) & 0xFFFFFFu : 1u << lane));
-    }
-    return o;
-  };
-  bool keeps_t = true, keeps_c = true;
-#pragma unroll
-  for (int i = 0; i < kPlanMaxInsn; i++) {
-    const bool ch = __shfl_sync(kFull, uint32_t(row[i] >> 48) & 1u, 0) != 0u;
-    if (uint32_t(i) < p.tl) keeps_t = keeps_t && !ch;
-    else if (uint32_t(i) < n) keeps_c = keeps_c && !ch;
-  }
-  const uint32_t rest = open & ~uint32_t(kRegA), a = open & kRegA;
-  return plan_from(reads, open, relevant(0, p.tl, rest) | relevant(p.tl, n, rest), a ? relevant(0, p.tl, a) : 0u,
-                   a ? relevant(p.tl, n, a) : 0u, keeps_t, keeps_c);
-}
-
 // Plans the round's pairs (z80_plan.cuh), a warp each: compared outputs,
 // swept fields, class and chunks.  A pair that its programs prove equivalent
 // gets no chunk and keeps its zero flag; the pairs after it in its window
@@ -892,10 +813,10 @@ __global__ void __launch_bounds__(128, 8) k_pair_plan(const RoundArgs* __restric
     const PairWords words = pair_words(T, t, P, c);
     uint32_t reads;
     if (P.reads) reads = A->q.meta[t].reads | P.reads[c];
-    else reads = __reduce_or_sync(kFull, words.mine() ? uint32_t(g_ops[words.w & 0xFFFFu].reads) : 0u);
+    else reads = __reduce_or_sync(kFull, words.mine(lane) ? uint32_t(g_ops[words.w & 0xFFFFu].reads) : 0u);
     pr.keepF = masked ? uint8_t(~target_dead(T, t)) : uint8_t(0xFFu);
     pr.keepR = masked ? uint8_t((~target_dead_regs(T, t) & 0x3Fu) | 0x80u) : uint8_t(0x3Fu);
-    const PairPlan pl = plan_pair_warp(words, reads, pr.keepF, pr.keepR);
+    const PairPlan pl = plan_pair_warp(lane, g_flow, words, reads, pr.keepF, pr.keepR);
     pr.reads = pl.reads;
     pr.sweepf = pl.sweepf;
     pr.nblocks = pl.nblocks;
