@@ -129,6 +129,38 @@ static int search2(z80b_ctx* ctx) {
   uint64_t n = 0;
   return z80b_search(ctx, &job, rules, 8, &n, nullptr);
 }
+// One small search; lens: per-target lengths instead of one.
+static int search1(z80b_ctx* ctx, uint32_t n, uint32_t len, uint32_t stride, bool lens, bool masks) {
+  const std::vector<uint32_t> targets(size_t(n) * stride);
+  const std::vector<uint8_t> tl(n, uint8_t(len)), dead(n, 0x28);
+  z80b_job job{};
+  job.targets = targets.data();
+  job.n_targets = n;
+  job.target_len = lens ? 0 : len;
+  job.target_lens = lens ? tl.data() : nullptr;
+  job.target_stride = stride;
+  job.dead_flags = masks ? dead.data() : nullptr;
+  job.max_cand_len = 1;
+  job.mode = Z80B_MODE_FIRST;
+  job.path = Z80B_PATH_BATCHED;
+  std::vector<z80b_rule> rules(2 * n);
+  uint64_t got = 0;
+  return z80b_search(ctx, &job, rules.data(), rules.size(), &got, nullptr);
+}
+// The round loop of small searches is captured once, whatever the form of
+// their targets, and anew only when a search of twice the size comes.
+static int small_graphs(z80b_ctx* ctx) {
+  CHECK(search1(ctx, 8, 1, 1, false, false) == Z80B_OK);
+  CHECK(fake::graphs == 1);
+  for (uint32_t len = 1; len <= 4; len++)
+    for (uint32_t stride : {len, 4u, 7u})
+      for (int form = 0; form < 4; form++) CHECK(search1(ctx, 8, len, stride, form & 1, form & 2) == Z80B_OK);
+  CHECK(fake::graphs == 1);
+  for (uint32_t n = 1; n <= 1024; n += 3) CHECK(search1(ctx, n, 2, 2, false, false) == Z80B_OK);
+  CHECK(fake::graphs == 1 + 7);  // room for 16 .. 1,024 targets
+  z80b_destroy(ctx);
+  return 0;
+}
 // What goes up with the pair pool is ordered before the work that reads it.
 static int pair_pool_order(z80b_ctx* ctx) {
   CHECK(search2(ctx) == Z80B_OK);
@@ -304,7 +336,8 @@ int main(int argc, char** argv) {
                 {"pair_pool_order", pair_pool_order},
                 {"pair_pool_retry", pair_pool_retry}, {"chunks", chunks},
                 {"verify_events", verify_events}, {"verify_copies", verify_copies}, {"qc_index_memory", qc_index_memory},
-                {"query_counters", query_counters}, {"qc_index_debt", qc_index_debt}};
+                {"query_counters", query_counters}, {"qc_index_debt", qc_index_debt},
+                {"small_graphs", small_graphs}};
   for (const auto& c : checks)
     if (name == c.name) {
       z80b_ctx* ctx = nullptr;

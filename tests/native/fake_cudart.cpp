@@ -8,7 +8,7 @@
 #include <map>
 
 namespace fake {
-int unordered, copies_in, copies_out, events, launches, fail_malloc, fail_copy_in, fail_memset;
+int unordered, copies_in, copies_out, events, launches, graphs, fail_malloc, fail_copy_in, fail_memset;
 size_t bytes, peak, limit;
 static bool pending;                       // legacy-stream work that may still run
 static cudaError_t last;                   // what cudaGetLastError gives
@@ -224,6 +224,7 @@ cudaError_t cudaGraphDestroy(cudaGraph_t) { return cudaSuccess; }
 cudaError_t cudaGraphExecDestroy(cudaGraphExec_t) { return cudaSuccess; }
 cudaError_t cudaGraphInstantiate(cudaGraphExec_t* x, cudaGraph_t, unsigned long long) {
   *x = handle<cudaGraphExec_t>();
+  graphs++;
   return cudaSuccess;
 }
 cudaError_t cudaGraphLaunch(cudaGraphExec_t, cudaStream_t st) {

@@ -13,6 +13,7 @@ extern int unordered;
 extern int copies_in, copies_out;  // host-to-device and device-to-host copies
 extern int events;           // events alive
 extern int launches;         // kernels
+extern int graphs;           // graphs instantiated
 extern size_t bytes, peak;   // device memory alive, and the most there was
 // The n-th call from now on fails (0: none does); counted down to 0.
 extern int fail_malloc, fail_copy_in, fail_memset;

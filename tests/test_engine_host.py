@@ -24,7 +24,7 @@ def exe(tmp_path_factory):
 
 
 @pytest.mark.parametrize("check", ["error_reported_once", "mul_tables", "mul_no_room", "pair_pool_order", "pair_pool_retry", "chunks",
-                                   "verify_events", "verify_copies", "qc_index_memory", "query_counters", "qc_index_debt"])
+                                   "verify_events", "verify_copies", "qc_index_memory", "query_counters", "qc_index_debt", "small_graphs"])
 def test_engine_host(exe, check):
     r = subprocess.run([str(exe), check], capture_output=True, text=True, timeout=600)
     assert r.returncode == 0 and r.stdout.startswith("OK " + check), r.stdout + r.stderr

@@ -1224,6 +1224,11 @@ struct MulSearch {
 int run_pipeline(z80b_ctx* ctx, const DevTargets& T, const PipeOpts& opts, z80b_stats* st, uint64_t* nr) {
   const uint32_t mode = opts.mode;
   const uint32_t n = T.n;
+  // Room for the survivors and pairs of a job that is queued as a whole: by
+  // powers of two, as a round graph holds for the buffers it was captured with.
+  uint32_t room = n;
+  if (n <= kQueuedJob)
+    for (room = 1; room < n;) room *= 2;
   cudaStream_t s = ctx->stream;
   PoolBufs* pool = &ctx->pool8;
   QCConfig cfg{0xFFFFFFFFu, 0, 1, nullptr, 0};
@@ -1355,8 +1360,9 @@ int run_pipeline(z80b_ctx* ctx, const DevTargets& T, const PipeOpts& opts, z80b_
     trace("qc count done: %llu survivors", (unsigned long long)nsurv);
   }
   if (nsurv > 0xFFFFFFF0ull) return fail(ctx, Z80B_ECAPACITY, "too many QuickCheck survivors (%llu)", (unsigned long long)nsurv);
-  CK(ctx->surv.ensure(4ull * std::max<uint64_t>(nsurv, 1)));
-  CK(ctx->sdiff.ensure(2ull * std::max<uint64_t>(nsurv, 1)));
+  const uint64_t surv_room = queued ? uint64_t(room) * pool->qvalid : nsurv;
+  CK(ctx->surv.ensure(4ull * std::max<uint64_t>(surv_room, 1)));
+  CK(ctx->sdiff.ensure(2ull * std::max<uint64_t>(surv_room, 1)));
   q.surv = ctx->surv.as<uint32_t>();
   q.sdiff = ctx->sdiff.as<uint16_t>();
   if (nsurv && q.tmp) {
@@ -1393,7 +1399,7 @@ int run_pipeline(z80b_ctx* ctx, const DevTargets& T, const PipeOpts& opts, z80b_
     launch_lanes_init(L, n, s);
     CKR(check_launch(ctx, "lanes_init"));
     // pair slots per round: every lane once, and room for survivor windows
-    CKR(ensure_round(ctx, std::max<uint64_t>(2ull * n, std::min<uint64_t>(128ull * n, 1ull << 20)), true, &R));
+    CKR(ensure_round(ctx, std::max<uint64_t>(2ull * room, std::min<uint64_t>(128ull * room, 1ull << 20)), true, &R));
     RoundArgs* const args = ctx->roundargs.as<RoundArgs>();
     const bool small = n <= kSmallJob;
     RoundArgs ra{};
@@ -1732,27 +1738,33 @@ int upload_targets(z80b_ctx* ctx, Staged& S, const z80b_job* job, DevTargets* T,
   cudaStream_t s = ctx->stream;
   S.up_chunks = 0;
   if (!keep_host && n <= kSmallJob) {
-    // one copy from page-locked memory, to fixed places (a captured round
-    // graph holds the addresses)
-    const size_t head = 3 * size_t(kSmallJob), bytes = head + 4 * words;
-    CK(S.d_small.ensure(std::max<size_t>(bytes, head + 16 * size_t(kSmallJob))));
-    CK(ctx->h_up.ensure(std::max<size_t>(bytes, head + 16 * size_t(kSmallJob))));
+    // One copy from page-locked memory, to fixed places and in one form (a
+    // length for every target, kMaxSeq words each): a captured round graph
+    // holds the addresses, and a job of another length or stride would capture
+    // it anew (0.75 ms behind the 0.15 ms of a search of one target).
+    const size_t head = 3 * size_t(kSmallJob), per = 4 * size_t(kMaxSeq);
+    CK(S.d_small.ensure(head + per * kSmallJob));
+    CK(ctx->h_up.ensure(head + per * kSmallJob));
     uint8_t* const h = ctx->h_up.as<uint8_t>();
     uint8_t* const d = S.d_small.as<uint8_t>();
     if (n) {
+      // (lengths and opcodes out of range are found before anything reads them)
       if (job->target_lens) std::memcpy(h, job->target_lens, n);
+      else std::memset(h, int(job->target_len), n);
       if (job->dead_flags) std::memcpy(h + kSmallJob, job->dead_flags, n);
       if (job->dead_regs) std::memcpy(h + 2 * kSmallJob, job->dead_regs, n);
-      std::memcpy(h + head, job->targets, 4 * words);
-      CK(cudaMemcpyAsync(d, h, bytes, cudaMemcpyHostToDevice, s));
+      const size_t stride = job->target_stride, take = std::min<size_t>(4 * stride, per);
+      if (4 * stride == per) std::memcpy(h + head, job->targets, 4 * words);
+      else
+        for (uint32_t i = 0; i < n; i++) std::memcpy(h + head + per * i, job->targets + stride * i, take);
+      CK(cudaMemcpyAsync(d, h, head + per * n, cudaMemcpyHostToDevice, s));
     }
     *T = DevTargets{};
     T->insn = reinterpret_cast<const uint32_t*>(d + head);
     T->n = n;
-    T->stride = job->target_stride;
-    T->fixed_len = job->target_len;
+    T->stride = kMaxSeq;
     T->global_dead = job->global_dead_flags;
-    if (job->target_lens) T->len = d;
+    T->len = d;
     if (job->dead_flags) T->dead = d + kSmallJob;
     if (job->dead_regs) T->dead_regs = d + 2 * kSmallJob;
     S.T = *T;
