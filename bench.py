@@ -44,6 +44,9 @@ import numpy as np  # noqa: E402
 
 METRIC = "Z80 candidate checks/s on 1 B200, batched vs plain GPU; p50/p99 query latency"
 UNIT = "candidate checks/s"
+# What z80b_search brings back: the device's rule records, and two reports of
+# its counters (DevRule and Report of csrc/z80b_kernels.cuh).
+RULE_BYTES, REPORT_BYTES = 16, 320
 
 
 T0 = time.perf_counter()
@@ -512,7 +515,7 @@ def main():
         e2e_checks = float(c.item())
     e2e_value = e2e_checks / args.steps / e2e_step
     h2d = int(mine.nbytes)
-    d2h = int(nr.value) * 12 + 64
+    d2h = int(nr.value) * RULE_BYTES + 2 * REPORT_BYTES
 
     # ---- roofline of the dominant kernels (the ExhaustiveCheck sweep classes)
     # Integer issue-bound work (no contraction, nothing per state from

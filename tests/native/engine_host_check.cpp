@@ -327,6 +327,13 @@ static int query_counters(z80b_ctx* ctx) {
   return 0;
 }
 
+// The sizes of what a search brings back.
+static int sizes(z80b_ctx* ctx) {
+  std::printf("OK sizes %zu %zu\n", sizeof(z80b::DevRule), sizeof(z80b::Report));
+  z80b_destroy(ctx);
+  return 0;
+}
+
 int main(int argc, char** argv) {
   const std::string name = argc > 1 ? argv[1] : "";
   struct {
@@ -337,7 +344,7 @@ int main(int argc, char** argv) {
                 {"pair_pool_retry", pair_pool_retry}, {"chunks", chunks},
                 {"verify_events", verify_events}, {"verify_copies", verify_copies}, {"qc_index_memory", qc_index_memory},
                 {"query_counters", query_counters}, {"qc_index_debt", qc_index_debt},
-                {"small_graphs", small_graphs}};
+                {"small_graphs", small_graphs}, {"sizes", sizes}};
   for (const auto& c : checks)
     if (name == c.name) {
       z80b_ctx* ctx = nullptr;

@@ -28,3 +28,11 @@ def exe(tmp_path_factory):
 def test_engine_host(exe, check):
     r = subprocess.run([str(exe), check], capture_output=True, text=True, timeout=600)
     assert r.returncode == 0 and r.stdout.startswith("OK " + check), r.stdout + r.stderr
+
+
+def test_bench_counts_what_comes_back(exe):
+    import sys
+    sys.path.insert(0, ROOT)
+    import bench
+    r = subprocess.run([str(exe), "sizes"], capture_output=True, text=True, timeout=600)
+    assert r.stdout.split()[:4] == ["OK", "sizes", str(bench.RULE_BYTES), str(bench.REPORT_BYTES)], r.stdout
