@@ -14,10 +14,11 @@
 //  - none open: the pair is equivalent, nothing is swept;
 //  - else only the inputs that an open output depends on are swept, A at two
 //    values where that decides (see below), and the carry only if needed.
-// Measured (1 B200): the length-2 enumeration of 9.4M targets evaluates
+// Measured (1 B200): the length-2 enumeration of 9.4M targets evaluated
 // 1.3e9 states where leaving out only what nothing compared depends on took
 // 3.7e9 (ExhaustiveCheck 8.1 -> 3.1 ms); 100,003 targets with every flag dead
-// 2.3e7 where it took 1.3e8 to 6.8e8.
+// 2.3e7 where it took 1.3e8 to 6.8e8.  With the probe of long sweeps
+// (k_pair_plan) the enumeration evaluates 2.8e8.
 // What the sweep would find is unchanged: the outputs left out agree in
 // every state of it, and the inputs left out cannot change the others.
 #pragma once

@@ -38,6 +38,9 @@ uint32_t seq_aflow(const uint32_t* s, int n);
 // input fields they were computed from: a sound over-approximation (every
 // real dependency is in the set).
 constexpr int kDepF0 = 16, kDepFields = 24;
+// The plan of a pair takes op_flow below, which is the same run sharpened;
+// op_deps and what follows it up to pair_kept_out are the rule that the value
+// numbers replaced, kept as the statement that the host test checks.
 const uint32_t (*op_deps())[kDepFields];  // kNumOps rows
 // Input fields that the outputs in `out` (a mask of the layout above) of
 // the sequence s can depend on.

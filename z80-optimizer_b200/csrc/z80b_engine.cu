@@ -2376,7 +2376,7 @@ static int search_impl(z80b_ctx* ctx, const z80b_job* job, z80b_rule* out, uint6
   ctx->staged.valid = false;  // this job's targets are not kept for z80b_fetch_rules
   // The opcodes of a chunked batched job are checked by the QuickCheck count
   // that reads them anyway (the scan of 9.4M targets took 2.4 ms on 16 host
-  // threads, 1 ms longer than their upload).
+  // threads, as long as their upload, and no count is queued before it ends).
   const bool on_device = ctx->staged.up_chunks && job->path == Z80B_PATH_BATCHED;
   {
     // the host scan of the targets runs while their copy is in flight; on

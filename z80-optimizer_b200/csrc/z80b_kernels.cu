@@ -63,10 +63,11 @@ __device__ int16_t g_cren[kCompactSets][kNumOps];
 __device__ int8_t g_corig[kCompactSets][2];
 __device__ uint8_t g_cid[64];
 __device__ uint8_t g_opregs[kNumOps];
-// wide compact sweep: the same per register set of at most four registers
-// (wide_tables)
-// what each opcode's outputs are computed from (flow_word of z80_plan.cuh)
+// what each opcode's outputs are computed from (flow_word of z80_plan.cuh);
+// 87 KB, a row of 192 bytes per instruction read
 __device__ unsigned long long g_flow[kNumOps][kFlowFields];
+// wide compact sweep: as for the compact one, per register set of at most four
+// registers (wide_tables)
 __device__ int16_t g_wren[kWideSets][kNumOps];
 __device__ int8_t g_worig[kWideSets][4];
 __device__ uint8_t g_wid[64];
@@ -473,7 +474,6 @@ __global__ void __launch_bounds__(kBlock) k_qc_scan(DevTargets T, DevPool P, QCC
   if (!COLLECT && lane == 0 && my_checks) atomicAdd(o.checks, my_checks);
 }
 
-// Appends one pair per unresolved (target, kind) lane with an untried survivor.
 // Allocates w consecutive pair slots for this thread (one atomic per warp;
 // every lane of the warp takes part); returns the first slot.
 __device__ __forceinline__ uint32_t alloc_pairs(uint32_t* counter, uint32_t w) {
@@ -493,7 +493,7 @@ __device__ __forceinline__ uint32_t alloc_pairs(uint32_t* counter, uint32_t w) {
 
 // Puts the window of w survivors at sbase of lane (t, kind) into the pair
 // slots from p0: who the pairs are.  What their sweeps take is worked out by
-// k_pair_plan, a thread per pair (a window is up to 64 pairs and a plan some
+// k_pair_plan, a warp per pair (a window is up to 64 pairs and a plan some
 // microseconds: planned here, one thread would plan a window's pairs one
 // after the other).
 __device__ __forceinline__ void put_window(const RoundBuf& R, uint32_t p0, uint32_t w, uint32_t t, uint32_t kind,
@@ -790,8 +790,10 @@ __device__ __forceinline__ bool probe_pair(const PairWords& words, unsigned long
 // Bound by latency (some ten dependent loads and a few hundred instructions a
 // pair).  A lane per pair, each running plan_pair on arrays in local memory,
 // took 26 us a round however few its pairs (200 uneven targets: 1.75 ms a
-// search, 0.95 ms with this and k_qc_long; the 818,000 pairs of the 9.4M
-// length-2 targets' rounds pay for it with 0.4 ms of 5); in the round build, a
+// search, 0.95 ms with this and k_qc_long; the 851,000 pairs of the 9.8M
+// length-2 targets' rounds pay for it: 0.98 ms of a 5.1 ms step under ncu, and
+// at 64 registers a thread it spills, 370 bytes stored and 516 loaded, most of
+// them in the probe that few pairs run); in the round build, a
 // window's up to 64 pairs in one thread, 0.3 ms a round.  The probe and the polls between units:
 // 40,009 uneven targets evaluate 4.5e8 states where it was 1.6e10 (84 -> 43 ms
 // of sweeps), the 9.4M length-2 targets 2.7e8 where it was 1.3e9 (3.2 ->
@@ -1937,7 +1939,8 @@ __global__ void k_verify_small(const uint32_t* __restrict__ tgt, const uint8_t* 
 // lane; a lane whose slots are used up without a winner goes on from the
 // pair after the last one it took.
 
-// Bytes of the packed vector-0 word 0 / word 1 kept in the bucket key.
+// Bytes of an output's packed words 0 and 1 that count under a dead-register
+// mask whatever the dead flags are (A and the live registers; not F).
 __device__ __forceinline__ uint32_t key_keep0(uint32_t dregs) {
   return 0xFFu | ((dregs & 1u) ? 0u : 0xFF0000u) | ((dregs & 2u) ? 0u : 0xFF000000u);
 }
@@ -1947,7 +1950,8 @@ __device__ __forceinline__ uint32_t key_keep1(uint32_t dregs) {
 }
 // Hash of one vector's output (A, live registers, SP, M); the hash of a
 // sequence is the sum over the eight vectors, so that the lanes of a warp can
-// each hash one.
+// each hash one.  (The finalising multipliers are the published ones of
+// splitmix64, and in qc_mix below those of MurmurHash3.)
 __device__ __forceinline__ unsigned long long vector_hash(uint32_t w0, uint32_t w1, uint32_t w2, uint32_t v) {
   unsigned long long h = ((unsigned long long)w0 << 32) | w1;
   h ^= (unsigned long long)(w2 + (v << 24)) * 0x9E3779B97F4A7C15ull;
@@ -2315,7 +2319,8 @@ __device__ __forceinline__ void qc_bounds(const QCIndex& ix, const QCQuery& q, u
 // alone, gathering all eight outputs of every candidate that agreed on it and
 // broadcasting the target's eight outputs to every lane took 5.1 ms for 9.4M
 // length-2 targets and 1.0 ms for 100,003 targets with every flag dead, this
-// 1.9 and 0.13 ms (of the 1.9, the targets' upload 1.4).
+// 1.9 and 0.13 ms (the 1.9 are hardly more than the wait for the targets: 75 MB
+// take 2.3 ms to arrive, of which the last three chunks' 1.7 pass in here).
 // COLLECT: the collect pass; else the count pass, which with KEEP also keeps
 // the survivors of targets with at most kQCSlots (single pass).
 constexpr uint32_t kQCLong = 64;  // entries: eight steps of a group, two of a warp

@@ -341,8 +341,9 @@ __device__ __forceinline__ void run_digits(Pair& s, uint32_t idx, int len) {
     apply_at<P>(d, s.hi);
   }
 }
-// Hash of the state on all 256 inputs, the same in every lane.  salt: 0, or
-// the level where states of different levels are kept apart.
+// Hash of the state on all 256 inputs, the same in every lane (the multipliers
+// are splitmix64's).  salt: 0, or the level where states of different levels are
+// kept apart.
 __device__ __forceinline__ unsigned long long state_hash(const Pair& s, uint32_t salt) {
   const uint32_t w[14] = {s.lo.a, s.lo.b, s.lo.c, s.lo.as, s.lo.bs, s.lo.cs, s.lo.cf | (s.lo.cfs << 1),
                           s.hi.a, s.hi.b, s.hi.c, s.hi.as, s.hi.bs, s.hi.cs, s.hi.cf | (s.hi.cfs << 1)};
